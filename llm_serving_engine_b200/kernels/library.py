@@ -76,6 +76,7 @@ _SIGNATURES = {
                         c_longlong, c_longlong, c_int, c_longlong, c_void_p],
     "lse_gemm_f32_ranges": [c_int],
     "lse_gemm_f32_stack_ok": [c_void_p, c_void_p, c_int, c_int, c_longlong, c_longlong],
+    "lse_gemm_f32_stack_wanted": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong],
     "lse_paged_attention_generic": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                     c_int, c_int, c_int, c_void_p, c_int, c_void_p],

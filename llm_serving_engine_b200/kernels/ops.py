@@ -132,10 +132,18 @@ def gemm_f32_stack_ok(a: torch.Tensor, weight: torch.Tensor) -> bool:
                                                      a.stride(0), weight.stride(0)))
 
 
-def gemm_f32_stack(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+def gemm_f32_stack_wanted(a: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether a product of more rows than :func:`gemm_f32_stack_ok` takes is faster as a stack: its tiles alone would
+    leave much of the GPU idle."""
+    return bool(library.load().lse_gemm_f32_stack_wanted(a.data_ptr(), weight.data_ptr(), a.shape[0], weight.shape[0],
+                                                         a.shape[1], a.stride(0), weight.stride(0)))
+
+
+def gemm_f32_stack(a: torch.Tensor, weight: torch.Tensor, many_rows: bool = False) -> torch.Tensor:
     """a @ weight^T in true float32 as a stack [P, M, N] of the sums over the k ranges that the product is
     always cut into: a block per range, so that a product of few rows has enough blocks to stream the weights.
-    Added up in index order, starting from zero, the stack gives :func:`gemm_f32_nt`'s result bit for bit."""
+    Added up in index order, starting from zero, the stack gives :func:`gemm_f32_nt`'s result bit for bit.
+    ``many_rows``: more rows than :func:`gemm_f32_stack_ok` takes are accepted too."""
     _need_cuda(a, weight)
     m, k = a.shape
     n = weight.shape[0]
@@ -145,7 +153,8 @@ def gemm_f32_stack(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     ranges = int(lib.lse_gemm_f32_ranges(k))
     out = torch.empty((ranges, m, n), dtype=torch.float32, device=a.device)
     check(lib.lse_gemm_f32_nt(a.data_ptr(), weight.data_ptr(), None, out.data_ptr(), m, n, k,
-                              a.stride(0), weight.stride(0), out.stride(1), 1, out.stride(0), _stream()), "gemm_f32_stack")
+                              a.stride(0), weight.stride(0), out.stride(1), 2 if many_rows else 1, out.stride(0), _stream()),
+          "gemm_f32_stack")
     return out
 
 
@@ -190,16 +199,23 @@ GENERIC_SPLIT_MAX_ROWS = 64   # up to this many rows every chunk of keys of a ro
 def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                             out: torch.Tensor, block_tables: torch.Tensor,
                             segment_of_token: torch.Tensor, positions: torch.Tensor, scale: float,
-                            window: int = 0, split: bool | None = None) -> torch.Tensor:
+                            window: int = 0, split: bool | None = None, segment_start: torch.Tensor | None = None,
+                            segment_first_position: torch.Tensor | None = None, singles: bool = False,
+                            skip_single: bool = False) -> torch.Tensor:
     """Attention of every token of the step over its request's cached keys.
 
     q, out [T, n_q, D]; k_cache, v_cache [pages, n_kv, page_size, D];
     block_tables int32 [S, max_pages]; segment_of_token, positions int32 [T].
     A row's keys are summed in chunks of fixed size; ``split`` gives every chunk a block of its own
-    (default: with few rows, where one block per row would leave the GPU idle).  The result does not
-    depend on it, bit for bit.
+    (default: with few blocks, which would leave the GPU idle).  The result does not
+    depend on it, bit for bit, nor on what follows.
+
+    Without ``segment_start`` a block takes one row.  With ``segment_start`` (int32 [S + 1]) and ``segment_first_position``
+    (int32 [S]; the rows of a request neighbours in position order) a block takes a tile of rows that share their keys:
+    head sizes up to 128; ``skip_single`` leaves the requests of one row alone.  With ``segment_start`` and ``singles`` only
+    the requests of one row are worked on, a block a row.
     """
-    _need_cuda(q, k_cache, v_cache, out, block_tables, segment_of_token, positions)
+    _need_cuda(q, k_cache, v_cache, out, block_tables, segment_of_token, positions, segment_start, segment_first_position)
     tokens, n_q, head_dim = q.shape
     n_kv, page_size = k_cache.shape[1], k_cache.shape[2]
     if head_dim % 16 or head_dim > 256:
@@ -217,6 +233,12 @@ def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
         chunk = int(lib.lse_attention_generic_chunk())
         max_chunks = max(1, -(-(block_tables.stride(0) * page_size) // chunk))
         partials = torch.empty(tokens * n_q * max_chunks * (head_dim + 2), dtype=torch.float32, device=q.device)
+    segments = block_tables.shape[0]
+    tiles = segment_start is not None and not singles
+    if segment_start is not None:
+        assert segment_start.dtype == torch.int32 and segment_start.shape[0] == segments + 1
+    if tiles:
+        assert segment_first_position.dtype == torch.int32 and segment_first_position.shape[0] == segments
     check(lib.lse_paged_attention_generic(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                           out.data_ptr(), dtype_code(q.dtype), block_tables.data_ptr(),
                                           block_tables.stride(0), segment_of_token.data_ptr(),

@@ -113,7 +113,7 @@ class GroupedQueryAttention(Mixer):
         return next((bound for bound in self.PORTION_CLASSES if bound >= len(portions)), 0)
 
     def launch_signature(self, segment_counts):
-        if max(segment_counts) == 1 or not ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, self.ctx.dtype, self.window):
+        if max(segment_counts) == 1:
             return ()
         if sum(segment_counts) < ROWS_KERNEL_BELOW:
             return ("rows",)
@@ -123,7 +123,7 @@ class GroupedQueryAttention(Mixer):
     def forward(self, x, step, cache):
         tokens = x.shape[0]
         # bias is added with the rotation, in float32; at most 8 partial sums: the rotary kernel fetches them in one go
-        qkv = linear_partials(x, self.qkv_weight, max_splits=8)
+        qkv = linear_partials(x, self.qkv_weight, max_splits=8, stacks_of_many_rows=True)
         q = torch.empty((tokens, self.n_q, self.head_dim), dtype=x.dtype, device=x.device)
         self.position.encode_and_store(qkv, self.qkv_bias, step, cache, q, self.n_q, self.n_kv, self.head_dim)
         attended = torch.empty_like(q)

@@ -1,7 +1,7 @@
 """Matrix products of the layers: y = x W^T (+ b), W kept [out, in].
 
-float32: the engine's own FMA kernel (true 32-bit, fixed summation order: a few rows give the same bits as a
-stack of partial sums that the next kernel adds up as they do from the kernel that adds them up itself).
+float32: the engine's own FMA kernel (true 32-bit, fixed summation order: few rows, or few tiles, give the same bits
+as a stack of partial sums that the next kernel adds up as they do from the kernel that adds them up itself).
 bfloat16, few rows (decoding): the engine's tcgen05 kernel, which streams the
 weights with TMA and may cut the k range into splits; it returns a float32 stack
 of partial sums [P, rows, out] that the next kernel (norm, rotary, SiLU) adds up.
@@ -36,14 +36,18 @@ def reduce_partials(y: torch.Tensor) -> torch.Tensor:
     return y
 
 
-def linear_partials(x: torch.Tensor, weight: torch.Tensor, max_splits: int | None = None) -> torch.Tensor:
-    """x W^T as [rows, out] or, for few bfloat16 rows, as a float32 stack of partial sums
-    [P, rows, out].  For callers whose consumer kernel adds the partials itself."""
+def linear_partials(x: torch.Tensor, weight: torch.Tensor, max_splits: int | None = None,
+                    stacks_of_many_rows: bool = False) -> torch.Tensor:
+    """x W^T as [rows, out] or, for few rows, as a float32 stack of partial sums
+    [P, rows, out].  For callers whose consumer kernel adds the partials itself.  ``stacks_of_many_rows``: the consumer
+    reads every value once, so that a float32 product of more rows may come as a stack too where that is faster."""
     if (x.is_cuda and weight.dtype == torch.bfloat16 and x.shape[0] <= SKINNY_MAX_ROWS
             and ops.gemm_bf16_skinny_ok(x, weight)):
         return ops.gemm_bf16_skinny(x, weight, max_splits=max_splits)
-    if x.is_cuda and weight.dtype == torch.float32 and x.dtype == torch.float32 and ops.gemm_f32_stack_ok(x, weight):
-        return ops.gemm_f32_stack(x, weight)   # at most eight partial sums: what every consumer fetches in one go
+    if x.is_cuda and weight.dtype == torch.float32 and x.dtype == torch.float32:
+        # at most eight partial sums: what every consumer fetches in one go
+        if ops.gemm_f32_stack_ok(x, weight) or (stacks_of_many_rows and ops.gemm_f32_stack_wanted(x, weight)):
+            return ops.gemm_f32_stack(x, weight, many_rows=stacks_of_many_rows)
     return linear(x, weight)
 
 

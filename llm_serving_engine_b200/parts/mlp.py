@@ -51,10 +51,12 @@ class SwiGLU(FeedForward):
         }
 
     def forward(self, x):
-        gate_up = linear_partials(x, self.gate_up_weight)
+        gate_up = linear_partials(x, self.gate_up_weight, stacks_of_many_rows=True)
         act = torch.empty((x.shape[0], self.inter), dtype=x.dtype, device=x.device)
         ops.silu_mul(gate_up, act, self.activation, self.limit)
-        return linear_sums(act, self.down_weight) if self.float32_output else linear_partials(act, self.down_weight)
+        if self.float32_output:
+            return linear_sums(act, self.down_weight)
+        return linear_partials(act, self.down_weight, stacks_of_many_rows=True)
 
 
 register_feed_forward("gated_mlp", SwiGLU)   # the same part under the name that does not say which activation

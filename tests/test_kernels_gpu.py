@@ -108,6 +108,36 @@ def test_gemm_f32_is_true_float32_and_row_invariant(m, n, k):
     assert rel_err(no_bias, a.double() @ w.double().t()) < 1e-5
 
 
+@pytest.mark.parametrize("m, n, k", [(2, 31, 64), (4, 2100, 1100), (7, 20000, 132), (16, 20001, 68), (17, 65, 1028), (31, 127, 4100),
+                                     (33, 128, 260), (64, 129, 2052), (65, 9473, 512), (129, 255, 516), (257, 18945, 68)])
+def test_gemm_f32_sums_in_one_order_whatever_the_kernel(m, n, k):
+    """Edges of every kernel's tiles, as the kernel adds its ranges up and as a stack: each element is the sum over the k
+    ranges, in order from zero, of one fused multiply-add per k, worked out here in float64 a step at a time (a float32
+    product is exact in float64, and so is its sum with a float32 up to one rounding that float32 repeats: double
+    rounding can differ in the last place only at ties of the wider format, at most a few elements in a million)."""
+    torch.manual_seed(m + n + k)
+    a, w = torch.randn(m, k, device=DEV), torch.randn(n, k, device=DEV)
+    whole = torch.empty(m, n, device=DEV)
+    ops().gemm_f32_nt(a, w, None, whole)
+    stack = ops().gemm_f32_stack(a, w, many_rows=True)
+    length = -(-(-(-k // 8)) // 64) * 64
+    assert stack.shape == (-(-k // length), m, n)
+    total = torch.zeros(m, n, device=DEV)
+    for part in stack:
+        total += part
+    assert torch.equal(total, whole)
+    rows, cols = sorted({0, m // 2, m - 1}), sorted({0, 31, 32, 63, 64, 127, n // 2, n - 2, n - 1} & set(range(n)))
+    want = torch.zeros(len(rows), len(cols), device=DEV)
+    for lo in range(0, k, length):
+        acc = torch.zeros_like(want)
+        for kk in range(lo, min(k, lo + length)):
+            acc = (acc.double() + a[rows, kk].double()[:, None] * w[cols, kk].double()[None]).float()
+        want += acc
+    got = whole[rows][:, cols]
+    off = int((got != want).sum())
+    assert off <= 1 and float((got - want).abs().max()) <= 2.0 ** -20 * float(want.abs().max()), off
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 64, 64), (8, 1536, 8960), (3, 100, 1536), (16, 257, 520), (5, 96, 4100)])
 def test_gemm_f32_as_a_stack_of_range_sums(m, n, k):
     """Few rows as a stack of partial sums (a block per k range): added up in index order from zero, the stack gives
