@@ -194,6 +194,12 @@ def rope_kv_write(qkv: torch.Tensor, bias: torch.Tensor | None, positions: torch
 
 
 GENERIC_SPLIT_MAX_ROWS = 64   # up to this many rows every chunk of keys of a row gets a block of its own
+GENERIC_SCRATCH_FLOATS = 1 << 28    # most partial results that blocks of one chunk may leave (1 GiB)
+
+
+def attention_generic_tile_tokens(head_dim: int, n_q: int, n_kv: int) -> int:
+    """Tokens of a tile of the general attention's kernel for prompt portions (0: it does not take this shape)."""
+    return int(library.load().lse_attention_generic_tile_tokens(head_dim, n_q, n_kv))
 
 
 def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -227,25 +233,33 @@ def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     assert q.dtype == out.dtype == k_cache.dtype == v_cache.dtype
     assert block_tables.dtype == torch.int32 and block_tables.dim() == 2 and block_tables.stride(1) == 1
     assert segment_of_token.dtype == torch.int32 and positions.dtype == torch.int32
-    lib = library.load()
-    partials, max_chunks = None, 0
-    if split if split is not None else tokens <= GENERIC_SPLIT_MAX_ROWS:
-        chunk = int(lib.lse_attention_generic_chunk())
-        max_chunks = max(1, -(-(block_tables.stride(0) * page_size) // chunk))
-        partials = torch.empty(tokens * n_q * max_chunks * (head_dim + 2), dtype=torch.float32, device=q.device)
     segments = block_tables.shape[0]
     tiles = segment_start is not None and not singles
     if segment_start is not None:
         assert segment_start.dtype == torch.int32 and segment_start.shape[0] == segments + 1
     if tiles:
         assert segment_first_position.dtype == torch.int32 and segment_first_position.shape[0] == segments
-    check(lib.lse_paged_attention_generic(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                                          out.data_ptr(), dtype_code(q.dtype), block_tables.data_ptr(),
-                                          block_tables.stride(0), segment_of_token.data_ptr(),
-                                          positions.data_ptr(), tokens, n_q, n_kv, head_dim, page_size,
-                                          float(scale), int(window), k_cache.shape[0], block_tables.shape[0],
-                                          partials.data_ptr() if partials is not None else None, max_chunks,
-                                          _stream()), "paged_attention_generic")
+    lib = library.load()
+    chunk = int(lib.lse_attention_generic_chunk())
+    rows = segments if singles else tokens
+    max_chunks = max(1, -(-(block_tables.stride(0) * page_size) // chunk))
+    if split is None:
+        if tiles:
+            # a tile's blocks walk up to all its chunks one after the other, two blocks an SM at a time: with fewer than
+            # four blocks an SM the longest walk decides, and a block per chunk is faster
+            blocks = (-(-tokens // attention_generic_tile_tokens(head_dim, n_q, n_kv)) + segments) * n_kv
+            split = blocks < 4 * sm_count()
+        else:
+            split = rows <= GENERIC_SPLIT_MAX_ROWS
+        split = split and max_chunks > 1 and rows * n_q * max_chunks * (head_dim + 2) <= GENERIC_SCRATCH_FLOATS
+    partials = None
+    if split:
+        partials = torch.empty(rows * n_q * max_chunks * (head_dim + 2), dtype=torch.float32, device=q.device)
+    check(lib.lse_paged_attention_generic_portions(
+        q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), dtype_code(q.dtype), block_tables.data_ptr(),
+        block_tables.stride(0), segment_of_token.data_ptr(), positions.data_ptr(), tokens, n_q, n_kv, head_dim, page_size,
+        float(scale), int(window), k_cache.shape[0], segments, _ptr(partials), max_chunks if split else 0,
+        _ptr(segment_start), _ptr(segment_first_position), int(tiles), int(skip_single), _stream()), "paged_attention_generic")
     return out
 
 

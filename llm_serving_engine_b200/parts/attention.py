@@ -30,6 +30,10 @@ MIXED_DECODE_KERNEL = os.environ.get("LSE_MIXED_DECODE_KERNEL", "1") != "0"
 # step row by row, 1.85 / 2.15 / 2.07 on the tcgen05 kernel).  LSE_ROWS_KERNEL_BELOW=0 turns it off.
 ROWS_KERNEL_BELOW = int(os.environ.get("LSE_ROWS_KERNEL_BELOW", "64"))
 ROWS_KERNEL_BLOCKS = 256
+# The general kernels (float32, other head sizes, windows): a step's portions go to the kernel that takes tiles of rows with
+# a request's keys read once for them, its single tokens to the one that takes a row a block, as in a decode step.  Portions
+# of two rows do not fill a tile: they go row by row while the step is small.
+GENERIC_ROWS_UP_TO = 64
 
 
 @register_mixer("gqa_attention")
@@ -115,10 +119,33 @@ class GroupedQueryAttention(Mixer):
     def launch_signature(self, segment_counts):
         if max(segment_counts) == 1:
             return ()
+        if not ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, self.ctx.dtype, self.window):
+            return ("general", *self._general_kernels(segment_counts))
         if sum(segment_counts) < ROWS_KERNEL_BELOW:
             return ("rows",)
         portions, singles = self._portions(segment_counts)
         return (self.prompt_kernel(portions), singles, self._portion_class(portions, singles))
+
+    def _general_kernels(self, segment_counts: list[int]) -> tuple[bool, bool]:
+        """Whether the general attention's tiles kernel takes the portions of a step, and the rows kernel its single tokens."""
+        most = max(segment_counts)
+        if most == 1 or (most == 2 and sum(segment_counts) <= GENERIC_ROWS_UP_TO):
+            return False, False
+        if not ops.attention_generic_tile_tokens(self.head_dim, self.n_q, self.n_kv):
+            return False, False
+        return True, any(count == 1 for count in segment_counts)
+
+    def _general_attention(self, q, cache, attended, step):
+        arguments = (q, cache.keys, cache.values, attended, cache.block_tables, step.segment_of_token, step.positions,
+                     self.scale, self.window)
+        tiles, singles = (False, False) if step.decode_only else self._general_kernels([segment.count for segment in step.segments])
+        if not tiles:
+            ops.paged_attention_generic(*arguments)
+            return
+        if singles:
+            ops.paged_attention_generic(*arguments, segment_start=step.segment_start, singles=True)
+        ops.paged_attention_generic(*arguments, segment_start=step.segment_start,
+                                    segment_first_position=step.segment_first_position, skip_single=singles)
 
     def forward(self, x, step, cache):
         tokens = x.shape[0]
@@ -153,6 +180,5 @@ class GroupedQueryAttention(Mixer):
                        step.segment_first_position, self.scale, skip_single=singles,
                        max_portions=self._portion_class(portions, singles))
         else:   # float32, other head sizes, windows: the general kernel
-            ops.paged_attention_generic(q, cache.keys, cache.values, attended, cache.block_tables,
-                                        step.segment_of_token, step.positions, self.scale, self.window)
-        return linear_partials(attended.view(tokens, self.n_q * self.head_dim), self.o_weight)
+            self._general_attention(q, cache, attended, step)
+        return linear_partials(attended.view(tokens, self.n_q * self.head_dim), self.o_weight, stacks_of_many_rows=True)

@@ -382,6 +382,51 @@ def test_general_attention_gives_the_same_bits_with_a_block_per_chunk_of_keys(dt
     assert float((outs[0][-1, 5].double() - v[needle, 1].double()).abs().max()) < 0.05
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head_dim, n_q, n_kv, page, window", [(128, 12, 2, 16, 0), (64, 7, 1, 8, 0), (80, 5, 5, 32, 70), (48, 66, 1, 16, 0),
+                                                               (16, 4, 2, 1, 1), (128, 10, 2, 16, 200), (112, 28, 4, 64, 64)])
+def test_general_attention_gives_the_same_bits_tile_by_tile(dtype, head_dim, n_q, n_kv, page, window):
+    """Portions (and single tokens) of several requests, cut at the edges of tiles and chunks: row by row, as tiles with a
+    block per chunk, as tiles that walk all chunks, and split into single tokens and portions, all bit for bit the same
+    and right against dense attention; keys beyond a request's end hold NaN, a later row of a portion an infinite value."""
+    rng = random.Random(head_dim)
+    torch.manual_seed(head_dim)
+    portions = [(0, 1), (0, 9), (63, 2), (64, 1), (127, 66), (5, 11), (200, 33), (0, 130)]    # (first position, rows)
+    contexts = [first + count for first, count in portions]
+    k_cache, v_cache, tables, dense = paged_setup(rng, contexts, n_kv, head_dim, page, dtype)
+    poison_unowned(k_cache, v_cache, tables, contexts, page)
+    k, v = dense[-1]
+    v[-1] = float("inf")
+    v_cache[int(tables[len(portions) - 1, (contexts[-1] - 1) // page]), :, (contexts[-1] - 1) % page] = v[-1]
+    tokens = sum(count for _, count in portions)
+    q = torch.randn(tokens, n_q, head_dim, device=DEV).to(dtype)
+    segs = torch.cat([torch.full((count,), index) for index, (_, count) in enumerate(portions)]).to(torch.int32).to(DEV)
+    positions = torch.cat([torch.arange(first, first + count) for first, count in portions]).to(torch.int32).to(DEV)
+    start = torch.tensor([0] + [count for _, count in portions]).cumsum(0).to(torch.int32).to(DEV)
+    firsts = torch.tensor([first for first, _ in portions], dtype=torch.int32, device=DEV)
+    scale = 1.0 / math.sqrt(head_dim)
+    run = ops().paged_attention_generic
+    arguments = (k_cache, v_cache)
+    rows = torch.full_like(q, 9.0)
+    run(q, *arguments, rows, tables, segs, positions, scale, window, split=False)
+    for split in (True, False):
+        got = torch.full_like(q, 9.0)
+        run(q, *arguments, got, tables, segs, positions, scale, window, split=split, segment_start=start, segment_first_position=firsts)
+        assert torch.equal(got, rows) or torch.equal(got.nan_to_num(7.0), rows.nan_to_num(7.0)), split
+        apart = torch.full_like(q, 9.0)
+        run(q, *arguments, apart, tables, segs, positions, scale, window, split=split, segment_start=start, singles=True)
+        assert torch.equal(apart[start[2]:start[3]], torch.full_like(apart[start[2]:start[3]], 9.0))    # portions are left alone
+        run(q, *arguments, apart, tables, segs, positions, scale, window, split=split, segment_start=start,
+            segment_first_position=firsts, skip_single=True)
+        assert torch.equal(apart.nan_to_num(7.0), rows.nan_to_num(7.0)), split
+    bound = 1e-5 if dtype == torch.float32 else 2.0 ** -7
+    for r in rng.sample(range(tokens - 1), 40):
+        s, pos = int(segs[r]), int(positions[r])
+        want = dense_attention(q[r], dense[s][0][:pos + 1], dense[s][1][:pos + 1], scale, window=window)
+        assert float((rows[r].double() - want).abs().max()) < bound * max(1.0, float(want.abs().max())), (s, pos)
+    assert bool(torch.isinf(rows[-1]).all()) and bool(torch.isfinite(rows[:-1]).all())
+
+
 @pytest.mark.parametrize("window", [1, 5, 16, 33, 100])
 def test_window_edge(window):
     rng = random.Random(window)
