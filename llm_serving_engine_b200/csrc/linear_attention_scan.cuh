@@ -220,12 +220,12 @@ linear_attention_carry_kernel(const float* __restrict__ decay, float* __restrict
   float last_power = 1.f;
   for (int i = 0; i < b - a - (chunks - 1) * chunk_rows; ++i) last_power *= dk;
   float* own = chunk_state + (size_t)before * per_state + e;
-  for (int c0 = 0; c0 < chunks; c0 += 8) {      // eight chunks' states are fetched together, then carried in order
-    float mine[8];
+  for (int c0 = 0; c0 < chunks; c0 += 16) {      // sixteen chunks' states are fetched together, then carried in order
+    float mine[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) mine[i] = c0 + i < chunks ? own[(size_t)(c0 + i) * per_state] : 0.f;
+    for (int i = 0; i < 16; ++i) mine[i] = c0 + i < chunks ? own[(size_t)(c0 + i) * per_state] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 16; ++i) {
       if (c0 + i < chunks) {
         own[(size_t)(c0 + i) * per_state] = running;
         running = fmaf(c0 + i == chunks - 1 ? last_power : full, running, mine[i]);

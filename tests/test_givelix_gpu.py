@@ -363,6 +363,44 @@ def test_linear_attention_scan_against_the_recurrence():
             assert torch.equal(device_state[1].cpu(), state[1])                  # the empty request's slot is untouched
 
 
+@pytest.mark.parametrize("heads, dim, vdim, counts, dtype", [(2, 128, 128, [64, 65, 1, 130], "bfloat16"), (3, 68, 130, [127, 63], "float32"),
+                                                             (1, 127, 5, [200, 2], "bfloat16"), (2, 96, 256, [128], "float32")])
+def test_linear_attention_in_chunks_as_products(heads, dim, vdim, counts, dtype):
+    """The products over chunks of 64 rows at the edges of their tiles, against the recurrence in float64, from states that
+    are not zero; a decay that is gone within a chunk; and an infinite value in a request's last row, which must not reach
+    the rows before it."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(dim)
+    rows, width = sum(counts), heads * (2 * dim + 2 * vdim) + 3
+    proj = torch.randn(rows, width).to(getattr(torch, dtype))
+    v_last = 2 * heads * dim + heads * vdim - 1
+    proj[counts[0] - 1, v_last] = float("inf")
+    decay = torch.tensor([0.999, 0.02, 0.9][:heads])
+    state = torch.randn(len(counts), heads, dim, vdim) * 0.5
+    z = proj.double()
+    act = z * torch.sigmoid(z)
+    q, k = (act[:, i * heads * dim:(i + 1) * heads * dim].view(rows, heads, dim) for i in (0, 1))
+    v = act[:, 2 * heads * dim:2 * heads * dim + heads * vdim].view(rows, heads, vdim)
+    want, want_state, row = torch.zeros(rows, heads, vdim, dtype=torch.float64), state.double().clone(), 0
+    for request, count in enumerate(counts):
+        for t in range(row, row + count):
+            want_state[request] = decay.double()[:, None, None] * want_state[request] + k[t][:, :, None] * v[t][:, None, :]
+            want[t] = torch.einsum("hde,hd->he", want_state[request], q[t])
+        row += count
+    starts = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    got, device_state = torch.empty(rows, heads * vdim, device="cuda"), state.cuda()
+    ops.linear_attention_scan(proj.cuda(), 0, heads * dim, 2 * heads * dim, decay.cuda(), device_state, starts,
+                              torch.arange(len(counts), dtype=torch.int32).cuda(), got, heads, dim, vdim, "silu", chunked=True)
+    got = got.cpu().view(rows, heads, vdim).double()
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), finite) and int((~finite).sum()) == 1
+    # sums of up to 130 rows of 128 products, each a few units of 2^-24 of the largest terms
+    assert float((got - want)[finite].abs().max()) <= 2e-5 * float(want[finite].abs().max())
+    good = torch.isfinite(want_state)
+    assert float((device_state.cpu() - want_state)[good].abs().max()) <= 2e-5 * float(want_state[good].abs().max())
+
+
 def test_residual_copies_update_and_norm():
     from llm_serving_engine_b200.kernels import ops
 
