@@ -399,7 +399,9 @@ class StepRunner:
         if wanted > places:
             return None
         # which kernels the parts launch may depend on how the rows are cut into portions: such steps get graphs of their own
-        signature = self.model.launch_signature([len(entry.tokens) for entry in entries]) if hasattr(self.model, "launch_signature") else ()
+        counts = [len(entry.tokens) for entry in entries]
+        contexts = [self.cache.requests[entry.request_id].length + count for entry, count in zip(entries, counts)]
+        signature = self.model.launch_signature(counts, contexts) if hasattr(self.model, "launch_signature") else ()
         key = ("portions", tokens, segments, places, self._graph_width(self._pages_after(entries)), signature)
         slot = self._portion_graphs.get(key)
         if slot is None:

@@ -91,6 +91,15 @@ _SIGNATURES = {
     "lse_paged_attention_prefill": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                     c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p],
     "lse_attention_mma_supported": [c_int, c_int, c_int],
+    "lse_attention_expanded_supported": [c_int, c_int, c_int, c_int],
+    "lse_attention_expanded_tile": [],
+    "lse_attention_expanded_status": [],
+    "lse_attention_expanded_status_async": [c_void_p, c_void_p],
+    "lse_attention_expanded_status_reset": [],
+    "lse_latent_gather": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int,
+                          c_void_p],
+    "lse_attention_expanded": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                               c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p],
     "lse_paged_attention_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                        c_int, c_int, c_longlong, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                                        c_void_p, c_longlong, c_void_p],

@@ -507,16 +507,21 @@ def gemm_bf16_skinny_status() -> int:
     return int(library.load().lse_gemm_bf16_skinny_status())
 
 
+_STATUS_WORDS = (("gemm_tcgen05", "lse_gemm_bf16_skinny_status"), ("attention_tcgen05", "lse_attention_tc_status"),
+                 ("attention_expanded_tcgen05", "lse_attention_expanded_status"))
+
+
 def kernel_status_async(host_words: torch.Tensor) -> None:
     """Queue, on the current stream, copies of the status words of the kernels with bounded waits (the
-    few-rows product, the tcgen05 prompt attention) into ``host_words`` (pinned int32 [2]).  Once the
+    few-rows product, the tcgen05 prompt attention, the one over expanded latents) into ``host_words`` (pinned int32,
+    a word each; [2]: the first two).  Once the
     stream has got there, a non-zero word says that a wait gave up: that block wrote nothing, and
     what the step computed is not to be used."""
     assert host_words.dtype == torch.int32 and host_words.numel() >= 2 and host_words.is_pinned()
     lib = library.load()
     stream = _stream()
-    for index, (source, entry) in enumerate((("gemm_tcgen05", "lse_gemm_bf16_skinny_status_async"),
-                                             ("attention_tcgen05", "lse_attention_tc_status_async"))):
+    for index, (source, entry) in enumerate(_STATUS_WORDS[:host_words.numel()]):
+        entry += "_async"
         if not lib.source_loaded(source):       # a kernel that was never loaded has given up nothing
             host_words[index] = 0
         elif getattr(lib, entry)(host_words.data_ptr() + 4 * index, stream) != 0:
@@ -524,11 +529,11 @@ def kernel_status_async(host_words: torch.Tensor) -> None:
 
 
 def kernel_status_reset() -> None:
-    """Clear both status words (after a failure has been reported)."""
+    """Clear the status words (after a failure has been reported)."""
     lib = library.load()
-    for source, entry in (("gemm_tcgen05", "lse_gemm_bf16_skinny_status_reset"), ("attention_tcgen05", "lse_attention_tc_status_reset")):
+    for source, entry in _STATUS_WORDS:
         if lib.source_loaded(source):
-            getattr(lib, entry)()
+            getattr(lib, entry + "_reset")()
     for _, counters in _ATTENTION_TC_SCRATCH.values():   # a block that gave up may have left its arrival uncounted
         counters.zero_()
 
@@ -802,6 +807,63 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
                                    positions.data_ptr(), _ptr(sink), tokens, heads, dk, dv, page_size, float(scale),
                                    int(window), cache.shape[0], block_tables.shape[0], _ptr(partials), max_chunks,
                                    _stream()), "latent_attention")
+    return out
+
+
+def attention_expanded_supported(dim: int, rot: int, vdim: int, rank: int, dtype: torch.dtype) -> bool:
+    """Whether latent attention over expanded keys and values takes these sizes (:func:`attention_expanded`)."""
+    return dtype == torch.bfloat16 and bool(library.load().lse_attention_expanded_supported(int(dim), int(rot), int(vdim), int(rank)))
+
+
+def attention_expanded_tile() -> int:
+    """Keys of a tile of :func:`attention_expanded`: a request's gathered rows are a multiple of it."""
+    return int(library.load().lse_attention_expanded_tile())
+
+
+def latent_gather(cache: torch.Tensor, block_tables: torch.Tensor, segment_first_position: torch.Tensor,
+                  segment_context: torch.Tensor, capacity: int, window: int = 0) -> torch.Tensor:
+    """The cached rows (cache [pages, page_size, width] bfloat16) that each request of the step may read, positions
+    max(0, first + 1 - window) (window <= 0: 0) up to its context, request by request, each rounded up to whole key
+    tiles with zeros: [capacity, width], zeros behind the last.  ``capacity`` holds them all."""
+    _need_cuda(cache, block_tables, segment_first_position, segment_context)
+    segments, width = block_tables.shape[0], cache.shape[2]
+    assert cache.is_contiguous() and cache.dtype == torch.bfloat16 and block_tables.dtype == torch.int32 and block_tables.stride(1) == 1
+    assert segment_first_position.dtype == segment_context.dtype == torch.int32
+    assert segment_first_position.shape[0] == segment_context.shape[0] == segments
+    rows = torch.empty((int(capacity), width), dtype=cache.dtype, device=cache.device)
+    check(library.load().lse_latent_gather(cache.data_ptr(), block_tables.data_ptr(), block_tables.stride(0),
+                                           segment_first_position.data_ptr(), segment_context.data_ptr(), segments, width,
+                                           cache.shape[1], cache.shape[0], int(window), rows.data_ptr(), int(capacity),
+                                           _stream()), "latent_gather")
+    return rows
+
+
+def attention_expanded(q_plain: torch.Tensor, q_wide: torch.Tensor, rows: torch.Tensor, kv: torch.Tensor, out: torch.Tensor,
+                       segment_start: torch.Tensor, segment_first_position: torch.Tensor, segment_context: torch.Tensor,
+                       scale: float, window: int = 0, sink: torch.Tensor | None = None,
+                       gate: torch.Tensor | None = None) -> torch.Tensor:
+    """Causal attention of prompt portions over keys and values made from gathered latent rows.
+
+    q_plain [T, heads, 128]; q_wide [T, heads, rank + 64] (its last 64 columns are read: the rotated values); rows
+    [N, rank + 64] as :func:`latent_gather` leaves them; kv [N, 2 * heads, 128]: every head's key of a row, then every
+    head's value; out [T, heads, 128]; all bfloat16.  A score is (q_plain . key + q_rotated . row's last 64) * scale.
+    ``sink`` float32 [heads] joins the denominator as exp(sink); ``gate`` float32 [T, heads] multiplies a head's output."""
+    _need_cuda(q_plain, q_wide, rows, kv, out, segment_start, segment_first_position, segment_context, sink, gate)
+    tokens, heads, dim = q_plain.shape
+    segments, rank = segment_first_position.shape[0], rows.shape[1] - 64
+    assert q_wide.shape == (tokens, heads, rank + 64) and out.shape == q_plain.shape and kv.shape == (rows.shape[0], 2 * heads, dim)
+    for tensor in (q_plain, q_wide, rows, kv, out):
+        assert tensor.is_contiguous() and tensor.dtype == torch.bfloat16
+    for tensor, size in ((segment_start, segments + 1), (segment_first_position, segments), (segment_context, segments)):
+        assert tensor.dtype == torch.int32 and tensor.shape[0] == size
+    assert sink is None or (sink.dtype == torch.float32 and sink.shape == (heads,))
+    assert gate is None or (gate.dtype == torch.float32 and gate.is_contiguous() and gate.shape == (tokens, heads))
+    if not attention_expanded_supported(dim, 64, dim, rank, q_plain.dtype):
+        raise KernelError(f"attention over expanded latents: heads of {dim}, latents of {rank} are not supported")
+    check(library.load().lse_attention_expanded(q_plain.data_ptr(), q_wide.data_ptr(), rows.data_ptr(), kv.data_ptr(), out.data_ptr(),
+                                                segment_start.data_ptr(), segment_first_position.data_ptr(),
+                                                segment_context.data_ptr(), segments, tokens, heads, rank, rows.shape[0],
+                                                float(scale), int(window), _ptr(sink), _ptr(gate), _stream()), "attention_expanded")
     return out
 
 

@@ -172,9 +172,13 @@ class DecoderModel:
                 return False
         return bool(getattr(self.final_norm, "graph_safe", False))
 
-    def launch_signature(self, segment_counts: list[int]) -> tuple:
-        """The mixers' answers to ``Mixer.launch_signature`` for a step of this shape (each distinct answer once)."""
-        answers = {block.mixer.launch_signature(segment_counts) for block in self.blocks}
+    def launch_signature(self, segment_counts: list[int], contexts: list[int] | None = None) -> tuple:
+        """The mixers' answers to ``Mixer.launch_signature`` (``launch_signature_at``, given the requests' contexts) for a step
+        of this shape (each distinct answer once)."""
+        if contexts is None:
+            answers = {block.mixer.launch_signature(segment_counts) for block in self.blocks}
+        else:
+            answers = {block.mixer.launch_signature_at(segment_counts, contexts) for block in self.blocks}
         return tuple(sorted(answer for answer in answers if answer))
 
     @property

@@ -176,6 +176,11 @@ class Mixer(Part):
         are captured in CUDA graphs of their own; ``forward`` must choose by the same rule."""
         return ()
 
+    def launch_signature_at(self, segment_counts: list[int], contexts: list[int]) -> tuple:
+        """The same for mixers whose launches also depend on how many keys each request holds after the step
+        (``contexts``)."""
+        return self.launch_signature(segment_counts)
+
 
 def cache_needs(requirement) -> tuple:
     """A mixer's cache requirement as a tuple of single needs (empty for none)."""

@@ -12,6 +12,21 @@ from .linear import linear_partials
 
 PER_HEAD_LIBRARY_ROWS = 32    # above this many bfloat16 rows the per-head products are the library's batched product
 
+# Portions of prompts: keys and values of every head made from the gathered latent rows first, or attention over the latent
+# rows themselves.  The former costs one product over the rows that the requests hold (at EXPAND_FLOPS a microsecond) and
+# then 320 multiply-adds a (row, key, head) at EXPANDED_FLOPS; the latter none and 2 rank + 64 at LATENT_FLOPS (measured at
+# 16 heads, a latent of 512: 2,048 rows of a prompt 11 + 41 us, with 4 for the gathering, against 611; the two products
+# per head around the latter, 19 us, are saved too).  Both write into buffers of the step.
+EXPAND_FLOPS, EXPANDED_FLOPS, LATENT_FLOPS = 1.0e9, 4.0e8, 1.2e8
+EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an attention of few blocks
+EXPAND_MAX_ROWS = 65536       # keys and values of that many rows are held at once (8 KB a row at 16 heads)
+
+
+def _size_class(rows: int) -> int:
+    """``rows`` rounded up to a quarter of a power of two (captured steps are kept by it)."""
+    step = max(64, 1 << max(0, (rows - 1).bit_length() - 3))
+    return -(-rows // step) * step
+
 _DEFAULT_NAMES = {"q_down": "dq", "q_down_norm": "dq.norm", "q_up": "uq", "q": "q", "kv_down": "dkv",
                   "kv_down_norm": "dkv.norm", "k_up": "uk", "v_up": "uv", "sink": "sink", "gate": "g", "out": "o"}
 
@@ -58,7 +73,7 @@ class LatentAttention(Mixer):
     cached rows themselves (``csrc/attention_latent.cu``)."""
 
     graph_safe = True
-    kernel_sources = ("attention_latent", "attention_latent_mma", "gemm_heads",)
+    kernel_sources = ("attention_latent", "attention_latent_mma", "gemm_heads", "attention_expanded_tcgen05",)
 
     def __init__(self, params, weights, ctx) -> None:
         super().__init__(params, weights, ctx)
@@ -98,8 +113,9 @@ class LatentAttention(Mixer):
         if self.gates > self.heads and width % 16:       # whole tiles of the product, aligned rows of its result
             stacked.append(stacked[0].new_zeros((-width % 16, stacked[0].shape[1])))
         self.in_weight = torch.cat(stacked, dim=0).contiguous()
-        self.k_up = weights[names["k_up"]].contiguous().view(self.heads, self.dim, self.rank)
-        self.v_up = weights[names["v_up"]].contiguous().view(self.heads, self.vdim, self.rank).transpose(1, 2)
+        self.kv_up = torch.cat([weights[names["k_up"]], weights[names["v_up"]]], dim=0).contiguous()
+        self.k_up = self.kv_up[:self.heads * self.dim].view(self.heads, self.dim, self.rank)
+        self.v_up = self.kv_up[self.heads * self.dim:].view(self.heads, self.vdim, self.rank).transpose(1, 2)
         self.sink = weights[names["sink"]].to(torch.float32).contiguous() if p.get("sink", False) else None
         self.out_weight = weights[names["out"]].contiguous()
 
@@ -139,6 +155,34 @@ class LatentAttention(Mixer):
     @classmethod
     def cache_requirement(cls, params, hidden_size):
         return PagedLatent(int(params["kv_rank"]) + int(params["rot_dim"]), int(params.get("window", 0)))
+
+    def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
+        """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
+        the latent rows.  ``contexts``: keys of each request after the step."""
+        if min(segment_counts) == 1 or self.gates > self.heads or not ops.attention_expanded_supported(
+                self.dim, self.rot_dim, self.vdim, self.rank, self.ctx.dtype):
+            return 0
+        tile, rows, pairs = ops.attention_expanded_tile(), 0, 0
+        for count, context in zip(segment_counts, contexts):
+            first = max(0, context - count + 1 - self.window) if self.window > 0 else 0
+            rows += -(-(context - first) // tile) * tile
+            pairs += count * (min(context, self.window) if self.window > 0 else context - count // 2)
+        rows = _size_class(rows)
+        expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
+                    + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
+        latent = 2.0 * pairs * self.heads * (2 * self.rank + self.rot_dim) / LATENT_FLOPS
+        return rows if rows <= EXPAND_MAX_ROWS and expanded < latent else 0
+
+    def launch_signature_at(self, segment_counts, contexts):
+        rows = self._expanded_rows(segment_counts, contexts)
+        return ("expanded", rows) if rows else ()
+
+    def _expanded_attention(self, q_plain, q_wide, step, cache, gate, rows: int):
+        gathered = ops.latent_gather(cache.keys, cache.block_tables, step.segment_first_position, step.segment_context, rows, self.window)
+        kv = torch.mm(gathered[:, :self.rank], self.kv_up.t()).view(rows, 2 * self.heads, self.dim)
+        values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
+        return ops.attention_expanded(q_plain, q_wide, gathered, kv, values, step.segment_start, step.segment_first_position,
+                                      step.segment_context, self.scale, self.window, self.sink, gate)
 
     def _fold_queries(self, q_plain, q_wide) -> None:
         """q_wide[t, h, :rank] = W_uk,h^T q_plain[t, h]: many bfloat16 rows go to the library's batched product (the tensor
@@ -189,6 +233,12 @@ class LatentAttention(Mixer):
             queries = linear_partials(q_latent, self.q_up) if self.q_rank else proj
             ops.latent_query(queries, 0, heads, self.dim, self.rot_dim, self.rot_dims, self.freq, self.rot_factor,
                              step.positions, step.segment_of_token, q_plain, q_wide, self.rank)
+        expanded = (0 if step.decode_only else
+                    self._expanded_rows([segment.count for segment in step.segments],
+                                        [segment.first_position + segment.count for segment in step.segments]))
+        if expanded:
+            values = self._expanded_attention(q_plain, q_wide, step, cache, gate, expanded)
+            return linear_partials(values.view(tokens, heads * self.vdim), self.out_weight)
         self._fold_queries(q_plain, q_wide)
         attended = torch.empty((tokens, heads, self.rank), dtype=x.dtype, device=x.device)
         ops.latent_attention(q_wide, cache.keys, attended, cache.block_tables, step.segment_of_token, step.positions,

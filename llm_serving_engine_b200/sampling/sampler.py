@@ -54,7 +54,7 @@ class _Turn:
         self.dev_i = torch.empty((2, max_rows), dtype=torch.int64, device=device)
         self.out = torch.empty(max_rows, dtype=torch.int32, device=device)
         self.host_out = torch.empty(max_rows, dtype=torch.int32, pin_memory=pinned)
-        self.host_status = torch.zeros(2, dtype=torch.int32, pin_memory=pinned) if pinned else None
+        self.host_status = torch.zeros(3, dtype=torch.int32, pin_memory=pinned) if pinned else None
         self.done = torch.cuda.Event() if pinned else None
         self.rows = 0
 
@@ -118,8 +118,9 @@ class Sampler:
         turn = self._turns[self._last if ticket is None else ticket]
         if turn.done is not None:
             turn.done.synchronize()
-        if turn.host_status is not None and (turn.host_status[0] or turn.host_status[1]):
-            which = " and ".join(name for name, word in zip(("the few-rows product", "the tcgen05 prompt attention"),
+        if turn.host_status is not None and any(turn.host_status.tolist()):
+            which = " and ".join(name for name, word in zip(("the few-rows product", "the tcgen05 prompt attention",
+                                                             "the attention over expanded latents"),
                                                             turn.host_status.tolist()) if word)
             turn.host_status.zero_()
             ops.kernel_status_reset()

@@ -69,6 +69,11 @@ CONFIGS = {
                         # a reader of a cache that is not the first layer's, with other heads and sizes of its own
                         latent(heads=9, dim=8, rot_dim=6, vdim=10, kv_rank=36, q_rank=14, rot={"base": 777.0, "dims": 6}, kv_from=1)],
                        width=102, vocab=333, streams=2),
+    # heads of 128 and 64 rotated values: the attention over keys and values made from the latent
+    "expanded": model([latent(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, rot={"base": 500.0, "dims": 64}, mlp=DENSE),
+                       latent2(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=72, rot={"base": 900.0, "dims": 48}),
+                       latent(heads=1, dim=128, rot_dim=64, vdim=128, kv_rank=64, q_rank=24, rot={"base": 500.0, "dims": 64}, kv_from=0)],
+                      width=96),
 }
 NO_LAYER_SCALE = {"equal_sizes"}
 # bfloat16: the random models are made with large gains so that every mechanism matters; their rounding noise is
@@ -361,6 +366,104 @@ def test_linear_attention_scan_against_the_recurrence():
             assert float((got.cpu() - want).abs().max()) <= 2e-5 * scale, (heads, dim, vdim, chunked)
             assert float((device_state.cpu() - want_state).abs().max()) <= 2e-5 * float(want_state.abs().max())
             assert torch.equal(device_state[1].cpu(), state[1])                  # the empty request's slot is untouched
+
+
+def test_expanded_latent_attention_in_a_model(monkeypatch):
+    """Prompts in portions through the step function, layer by layer over expanded keys and values: launch by launch, from
+    a graph captured at a size class, and from that graph again with other contexts of the class; beside a decoding request the
+    layers go over the latent rows.  Every logit against the plain implementation."""
+    from llm_serving_engine_b200.kernels import ops
+    from llm_serving_engine_b200.parts import latent_attention
+
+    monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0)      # always worth it, whatever the sizes
+    sizes, real = [], ops.attention_expanded
+
+    def recorded(q_plain, q_wide, rows, *rest):
+        sizes.append((q_plain.shape[0], rows.shape[0]))
+        return real(q_plain, q_wide, rows, *rest)
+
+    monkeypatch.setattr(ops, "attention_expanded", recorded)
+    requests = some_requests("expanded", [230, 230, 215, 31])
+    steps, ids = [], list(requests)
+
+    def add(entries, end=()):
+        steps.append({"step": len(steps), "end": list(end),
+                      "entries": [{"id": rid, "tokens": requests[rid][lo:hi], "want": list(range(hi - lo))} for rid, lo, hi in entries]})
+
+    for rid in ids[:3]:                        # the same classes three times: launches, capture, replay
+        add([(rid, 0, 120)])
+        add([(rid, 120, len(requests[rid]))], end=[rid] if rid != ids[2] else ())
+    add([(ids[3], 0, 30)])
+    add([(ids[3], 30, 31)], end=[ids[2], ids[3]])
+    got = replay("expanded", "bfloat16", steps, 1024)
+    compare("expanded", "bfloat16", requests, got, "expanded")
+    assert sizes and len(sizes) % 3 == 0 and len(sizes) < 3 * 7      # some steps were replayed: nothing was launched from here
+    assert any(tokens > 120 for tokens, _ in sizes)                  # a captured class has padding rows
+
+
+@pytest.mark.parametrize("heads, rank, page, window, portions", [
+    (2, 64, 16, 0, [(0, 2), (0, 64), (63, 129), (700, 66)]), (3, 512, 8, 0, [(0, 300)]), (1, 24, 64, 37, [(0, 200), (500, 3), (36, 2)]),
+    (2, 512, 16, 512, [(1000, 130), (0, 640)]), (5, 72, 1, 1, [(5, 70)])])
+def test_latent_attention_over_expanded_keys_and_values(heads, rank, page, window, portions):
+    """Portions (first position, rows) behind prefixes, cut at the edges of row tiles (128) and key tiles (64), windows that
+    end inside a tile, a sink and a gate: the gathered rows exactly, the attention against float64 over the same bfloat16
+    keys and values.  Pages that no request owns hold NaN."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(rank + page)
+    rng = random.Random(rank)
+    width, tokens = rank + 64, sum(count for _, count in portions)
+    contexts = [first + count for first, count in portions]
+    pages = [-(-context // page) for context in contexts]
+    order = list(range(sum(pages) + 3))
+    rng.shuffle(order)
+    cache = torch.full((len(order), page, width), float("nan"), dtype=torch.bfloat16)
+    tables = torch.full((len(portions), max(pages)), -1, dtype=torch.int32)
+    dense = [torch.randn(context, width).bfloat16() for context in contexts]
+    for s, rows in enumerate(dense):
+        for logical in range(pages[s]):
+            tables[s, logical] = physical = order.pop()
+            part = rows[logical * page:(logical + 1) * page]
+            cache[physical, :len(part)] = part
+    starts = torch.tensor([0] + [count for _, count in portions] + [0]).cumsum(0).to(torch.int32).cuda()      # an empty request at the end
+    firsts = torch.tensor([first for first, _ in portions] + [0], dtype=torch.int32).cuda()
+    ends = torch.tensor(contexts + [0], dtype=torch.int32).cuda()
+    tables = torch.cat([tables, torch.full_like(tables[:1], -1)]).cuda()
+    low = [max(0, first + 1 - window) if window else 0 for first, _ in portions]
+    kept = [-(-(context - lo) // 64) * 64 for context, lo in zip(contexts, low)]
+    capacity = sum(kept) + 70
+    rows = ops.latent_gather(cache.cuda(), tables, firsts, ends, capacity, window)
+    want_rows = torch.zeros(capacity, width, dtype=torch.bfloat16)
+    at = 0
+    for part, lo, size in zip(dense, low, kept):
+        want_rows[at:at + len(part) - lo] = part[lo:]
+        at += size
+    assert torch.equal(rows.cpu(), want_rows)
+    kv = torch.randn(capacity, 2 * heads, 128).bfloat16()
+    q_plain, q_wide = torch.randn(tokens, heads, 128).bfloat16() * 0.4, torch.randn(tokens, heads, width).bfloat16()
+    sink, gate = torch.randn(heads), torch.rand(tokens, heads)
+    for with_extras in (False, True):
+        got = torch.empty(tokens, heads, 128, dtype=torch.bfloat16, device="cuda")
+        ops.attention_expanded(q_plain.cuda(), q_wide.cuda(), rows, kv.cuda(), got, starts, firsts, ends, 0.1, window,
+                               sink.cuda() if with_extras else None, gate.cuda() if with_extras else None)
+        assert int(ops.library.load().lse_attention_expanded_status()) == 0
+        row = at = 0
+        for (first, count), lo, size in zip(portions, low, kept):
+            keys = kv[at:at + size].double()
+            for t in sorted({0, 1, count // 2, min(127, count - 1), count - 1}):
+                pos = first + t
+                seen = slice(max(0, pos + 1 - window) - lo if window else 0, pos + 1 - lo)
+                scores = (torch.einsum("hd,khd->hk", q_plain[row + t].double(), keys[seen, :heads])
+                          + q_wide[row + t, :, rank:].double() @ want_rows[at:at + size][seen, rank:].double().t()) * 0.1
+                if with_extras:
+                    scores = torch.cat([scores, sink.double()[:, None]], dim=1)
+                weights = torch.softmax(scores, dim=1)[:, :keys[seen].shape[0]]
+                want = torch.einsum("hk,khd->hd", weights, keys[seen, heads:])
+                if with_extras:
+                    want = want * gate[row + t].double()[:, None]
+                # weights rounded to bfloat16, the result again: 2^-8 of the largest value each
+                assert float((got[row + t].cpu().double() - want).abs().max()) <= 2.0 ** -7 * max(1.0, float(want.abs().max())), (first, t)
+            row, at = row + count, at + size
 
 
 @pytest.mark.parametrize("heads, dim, vdim, counts, dtype", [(2, 128, 128, [64, 65, 1, 130], "bfloat16"), (3, 68, 130, [127, 63], "float32"),
