@@ -18,9 +18,9 @@
 //                 barrier.
 //   softmax       a thread owns one row of its group's tiles: it reads S (tcgen05.ld), masks, finds
 //                 the row maximum, takes exp2 in float32 and writes bfloat16 probabilities to shared memory in the swizzled K-major
-//                 layout the tensor cores read.  After a group's first tile the probabilities
-//                 are taken relative to the maximum in use, in one pass; O stays in tensor memory
-//                 and is only rescaled when a row maximum has grown by more than 2^8 (the sums
+//                 layout the tensor cores read.  The row is in registers before anything else, so that
+//                 the group's next scores are made meanwhile.  The probabilities are taken relative to
+//                 the maximum in use; O stays in tensor memory and is only rescaled when a row maximum has grown by more than 2^8 (the sums
 //                 carry the same factor, so the quotient is exact either way).  At the end the two groups' outputs
 //                 are weighted by 2^(their maximum - the common maximum), added, divided by the
 //                 sum and written out as bfloat16.
@@ -67,7 +67,7 @@ __device__ __forceinline__ unsigned sm_id() { unsigned v; asm volatile("mov.u32 
 #endif
 
 // per group g: index + g
-enum Bar { B_Q = 0, B_KF = 1, B_KE = 3, B_VF = 5, B_VE = 7, B_SF = 9, B_PF = 11, B_OD = 13, B_COUNT = 15 };
+enum Bar { B_Q = 0, B_KF = 1, B_KE = 3, B_VF = 5, B_VE = 7, B_SF = 9, B_PF = 11, B_SR = 13, B_OD = 15, B_COUNT = 17 };
 
 __device__ __forceinline__ float exp2_fast(float x) {   // 2^x, 2^-inf = 0
   float y;
@@ -166,7 +166,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
   if (tid == 0) {
     for (int i = 0; i < B_COUNT; ++i)
-      mbar_init(bar(i), (i >= B_PF && i < B_PF + 2) ? GROUP_THREADS : 1);
+      mbar_init(bar(i), (i >= B_PF && i < B_OD) ? GROUP_THREADS : 1);
     *abort_flag = 0;
     *reinterpret_cast<volatile int*>(tail + 8 * B_COUNT + 12) = 1;
     mbar_init_fence();
@@ -217,8 +217,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
-      // S_j = Q K_j^T as soon as the group of tile j has read the scores of its tile before (it has, when
-      // its probabilities are written).  The keys are waited for first: they have long arrived, and the
+      // S_j = Q K_j^T as soon as the group of tile j has read the scores of its tile before.  The keys are waited for first: they have long arrived, and the
       // wait that matters then comes last.
       const uint32_t idesc_s = instr_desc_bf16(BM, BN, false, false);
       bool ok = mbar_poll(bar(B_Q), 0, abort_flag, err);
@@ -228,7 +227,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         TC_STAMP2(j, 1)
         ok = mbar_poll(bar(B_KF + g), parity, abort_flag, err);
         TC_STAMP2(j, 2)
-        if (ok && j >= GROUPS) ok = mbar_poll(bar(B_PF + g), parity ^ 1u, abort_flag, err);
+        if (ok && j >= GROUPS) ok = mbar_poll(bar(B_SR + g), parity ^ 1u, abort_flag, err);
         if (!ok) break;
         fence_after_sync();
         TC_STAMP2(j, 6)
@@ -310,42 +309,54 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       fence_after_sync();
       const int kv0 = (j_lo + j) * BN;
       const bool diagonal = kv0 + BN - 1 > my_pos;   // some keys of this tile lie beyond this row's position
-      const bool first = j < GROUPS;                 // this group's first tile
+      // The whole row of scores into registers: the accumulator is free for the group's next tile at once, so that its
+      // product runs beside the exponentials of this one (with the scores read piece by piece while they were worked on,
+      // the group waited for its next ones after every tile: 4,500 cycles a pair of tiles, 2,600 of them exponentials).
+      uint32_t s[BN / 32][32];
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) tmem_ld32(s_addr + 32 * c, s[c]);
+      tmem_ld_wait();
+      fence_before_sync();
+      mbar_arrive(bar(B_SR + g));
       bool rescale = false;
       float alpha = 1.f;
+      float mx = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {
+        if (diagonal) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (kv0 + 32 * c + i > my_pos) s[c][i] = 0xff800000u;
+        }
+        if (PEN) {   // scaled and penalised first: the maximum is taken over what is exponentiated
+          const float ahead = (float)(my_pos - kv0 - 32 * c);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            s[c][i] = __float_as_uint(fmaf(__uint_as_float(s[c][i]), scale_log2e, -penalty(ahead - (float)i)));
+        }
+        if (!SIG) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])));
+        }
+      }
+      // a row of tile 0 always sees key 0; a row's last tile may be hidden entirely (-inf: nothing is added then)
+      const float m_tile = PEN ? mx : mx * scale_log2e;
       if (SIG) {
         m_used = m_seen = 0.f;      // the weights are taken as they are
-      } else if (first) {
-        // the row maximum of the first tile is found before anything is exponentiated
-        float mx = -INFINITY;
-#pragma unroll
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t s[32];
-          tmem_ld32(s_addr + c, s);
-          tmem_ld_wait();
-          if (diagonal) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (kv0 + c + i > my_pos) s[i] = 0xff800000u;
-          }
-          if (PEN) {
-            const float ahead = (float)(my_pos - kv0 - c);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fmaf(__uint_as_float(s[i]), scale_log2e, -penalty(ahead - (float)i)));
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) mx = fmaxf(mx, fmaxf(__uint_as_float(s[i]), __uint_as_float(s[i + 1])));
-          }
+      } else if (j < GROUPS) {
+        m_used = m_seen = m_tile;
+      } else {
+        // A maximum that grew by more than 2^8 in the tile before is taken over now: O and the sum follow.  One that grows by
+        // more than 2^64 in this tile is taken over at once (bfloat16 and float32 would run out of range a little further on).
+        m_seen = fmaxf(m_seen, m_tile);
+        if (pending || __any_sync(0xffffffffu, m_tile > m_used + REDO_STEP)) {
+          rescale = true;
+          alpha = m_used == -INFINITY ? 0.f : exp2_fast(m_used - m_seen);
+          m_used = m_seen;
+          l *= alpha;
         }
-        // a row of tile 0 always sees key 0; a row's last tile may be hidden entirely (-inf: nothing is added then)
-        m_used = m_seen = PEN ? mx : mx * scale_log2e;
-      } else if (pending) {   // the tile before raised the maximum by more than the step: O and the sum follow now
-        rescale = true;
-        alpha = m_used == -INFINITY ? 0.f : exp2_fast(m_used - m_seen);
-        m_used = m_seen;
-        l *= alpha;
-        pending = false;
       }
+      if (!SIG) pending = __any_sync(0xffffffffu, m_seen > m_used + RESCALE_STEP) != 0;
       TC_STAMP(j, 2)
       if (j >= GROUPS) {   // P V of this group's tile before has read the probabilities and added to O
         ok = wait_all(B_OD + g, parity ^ 1u);
@@ -353,101 +364,51 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         fence_after_sync();
       }
       TC_STAMP(j, 3)
-      // Later tiles take their probabilities relative to the maximum in use, in one pass, and find their
-      // own maximum on the way.  A maximum that grew by more than 2^8 is taken over before the next
-      // tile; one that grew by more than 2^64 (bfloat16 and float32 would run out of range a little
-      // further on) is taken over at once and the tile is done again.
+      if (rescale) {
 #pragma unroll 1
-      for (int attempt = 0; attempt < 2; ++attempt) {
-        if (rescale) {
-#pragma unroll
-          for (int c = 0; c < D; c += 32) {
-            uint32_t o[32];
-            tmem_ld32(o_addr + c, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st32(o_addr + c, o);
-          }
-          tmem_st_wait();
-          rescale = false;
-        }
-        const float neg = m_used == -INFINITY ? 0.f : -m_used;   // every score is -inf then as well: p = 0
-        float mx = -INFINITY, sum = 0.f;
-        // 32 keys = 4 chunks of 16 bytes at a time; the next 32 scores are on their way from tensor memory
-        // while these are worked on
-        auto take = [&](uint32_t (&s)[32], int c) {
-          if (diagonal) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (kv0 + c + i > my_pos) s[i] = 0xff800000u;
-          }
-          uint32_t pk[16];
-          const float ahead_of_chunk = (float)(my_pos - kv0 - c);
-#pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            float s0 = __uint_as_float(s[2 * i]), s1 = __uint_as_float(s[2 * i + 1]);
-            float s2 = __uint_as_float(s[2 * i + 2]), s3 = __uint_as_float(s[2 * i + 3]);
-            float p0, p1, p2, p3;
-            if (SIG) {   // capped, the head's number added, through the sigmoid; a hidden key (-inf) weighs nothing
-              auto weigh = [&](float raw) {
-                float x2 = raw * scale_log2e;
-                if (cap > 0.f) x2 = cap2 * (1.0f - __fdividef(2.0f, exp2_fast(raw * cap_step) + 1.0f));
-                const float w = __fdividef(1.0f, 1.0f + exp2_fast(-(x2 + bias2)));
-                return raw == -INFINITY ? 0.f : w;
-              };
-              p0 = weigh(s0); p1 = weigh(s1); p2 = weigh(s2); p3 = weigh(s3);
-              sum += (p0 + p1) + (p2 + p3);
-              pk[i] = pack_bf16(p0, p1);
-              pk[i + 1] = pack_bf16(p2, p3);
-              continue;
-            }
-            if (PEN) {   // scaled and penalised first: the maximum is taken over what is exponentiated
-              const float ahead = ahead_of_chunk - (float)(2 * i);
-              s0 = fmaf(s0, scale_log2e, -penalty(ahead)); s1 = fmaf(s1, scale_log2e, -penalty(ahead - 1.0f));
-              s2 = fmaf(s2, scale_log2e, -penalty(ahead - 2.0f)); s3 = fmaf(s3, scale_log2e, -penalty(ahead - 3.0f));
-              p0 = s0 + neg; p1 = s1 + neg; p2 = s2 + neg; p3 = s3 + neg;
-            } else {
-              p0 = fmaf(s0, scale_log2e, neg); p1 = fmaf(s1, scale_log2e, neg);
-              p2 = fmaf(s2, scale_log2e, neg); p3 = fmaf(s3, scale_log2e, neg);
-            }
-            mx = fmaxf(mx, fmaxf(fmaxf(s0, s1), fmaxf(s2, s3)));
-            p0 = exp2_fast(p0); p1 = exp2_fast(p1); p2 = exp2_fast(p2); p3 = exp2_fast(p3);
-            sum += (p0 + p1) + (p2 + p3);
-            pk[i] = pack_bf16(p0, p1);
-            pk[i + 1] = pack_bf16(p2, p3);
-          }
-          unsigned char* box = prow + (c / 64) * HALF_BYTES;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int chunk = (c % 64) / 8 + k;
-            *reinterpret_cast<uint4*>(box + ((chunk ^ (row & 7)) << 4)) = make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
-          }
-        };
-        uint32_t sa[32], sb[32];
-        tmem_ld32(s_addr, sa);
-#pragma unroll
-        for (int c = 0; c < BN; c += 64) {
+        for (int c = 0; c < D; c += 8) {
+          uint32_t o[8];
+          tmem_ld8(o_addr + c, o);
           tmem_ld_wait();
-          tmem_ld32(s_addr + c + 32, sb);
-          take(sa, c);
-          tmem_ld_wait();
-          if (c + 64 < BN) tmem_ld32(s_addr + c + 64, sa);
-          take(sb, c + 32);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st8(o_addr + c, o);
         }
-        const float m_tile = PEN ? mx : mx * scale_log2e;
-        if (first || !__any_sync(0xffffffffu, m_tile > m_used + REDO_STEP)) {
-          l += sum;
-          m_seen = fmaxf(m_seen, m_tile);
-          pending = __any_sync(0xffffffffu, m_seen > m_used + RESCALE_STEP) != 0;
-          break;
-        }
-        rescale = true;
-        alpha = m_used == -INFINITY ? 0.f : exp2_fast(m_used - fmaxf(m_used, m_tile));
-        m_used = fmaxf(m_used, m_tile);
-        m_seen = fmaxf(m_seen, m_used);
-        l *= alpha;
+        tmem_st_wait();
       }
+      const float neg = m_used == -INFINITY ? 0.f : -m_used;   // every score is -inf then as well: p = 0
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {      // 32 keys = 4 pieces of 16 bytes at a time
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float s0 = __uint_as_float(s[c][2 * i]), s1 = __uint_as_float(s[c][2 * i + 1]);
+          float p0, p1;
+          if (SIG) {   // capped, the head's number added, through the sigmoid; a hidden key (-inf) weighs nothing
+            auto weigh = [&](float raw) {
+              float x2 = raw * scale_log2e;
+              if (cap > 0.f) x2 = cap2 * (1.0f - __fdividef(2.0f, exp2_fast(raw * cap_step) + 1.0f));
+              const float w = __fdividef(1.0f, 1.0f + exp2_fast(-(x2 + bias2)));
+              return raw == -INFINITY ? 0.f : w;
+            };
+            p0 = weigh(s0); p1 = weigh(s1);
+          } else if (PEN) {
+            p0 = exp2_fast(s0 + neg); p1 = exp2_fast(s1 + neg);
+          } else {
+            p0 = exp2_fast(fmaf(s0, scale_log2e, neg)); p1 = exp2_fast(fmaf(s1, scale_log2e, neg));
+          }
+          sum += p0 + p1;
+          pk[i] = pack_bf16(p0, p1);
+        }
+        unsigned char* box = prow + (c / 2) * HALF_BYTES;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int chunk = (c % 2) * 4 + k;
+          *reinterpret_cast<uint4*>(box + ((chunk ^ (row & 7)) << 4)) = make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
+        }
+      }
+      l += sum;
       TC_STAMP(j, 4)
       if (j_lo + j == n_tiles - 1 && last_pos + 1 - kv0 < BN) {
         // rows of V beyond the last key: whatever lies there (stale keys, unwritten shared memory)
