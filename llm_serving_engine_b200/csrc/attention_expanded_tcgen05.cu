@@ -26,7 +26,7 @@ using namespace tc;
 
 constexpr int BM = 128, BN = 64;          // rows of a block, keys of a tile
 constexpr int GROUPS = 2, GROUP_THREADS = 128, STAGES = 3;
-constexpr int MMA_WARP = 8, LOADER_WARP = 9, PV_WARP = 10, THREADS = 352;
+constexpr int MMA_WARP = 8, LOADER_WARP = 9, PV_WARP = 10, V_LOADER_WARP = 11, THREADS = 384;
 constexpr int D = 128, ROT = 64;          // values of a head: unrotated (and of its value), rotated
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.0f, REDO_STEP = 64.0f;      // in powers of two
@@ -162,29 +162,26 @@ attn_expanded_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       tma_load_3d(q_s, &map_q, bar(B_Q), 0, head, row_base);
       tma_load_3d(q_s + Q_BOX, &map_q, bar(B_Q), 64, head, row_base);
       tma_load_3d(q_s + 2 * Q_BOX, &map_qr, bar(B_Q), rank, head, row_base);
-      auto load_k = [&](int j) {
+      for (int j = 0; j < n_local; ++j) {
         const int s = j % STAGES;
-        if (!mbar_wait(bar(B_KE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) return false;
+        if (!mbar_wait(bar(B_KE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) break;
         const uint32_t dst = k_s + s * K_BYTES;
         mbar_expect_tx(bar(B_KF + s), K_BYTES);
         tma_load_3d(dst, &map_kv, bar(B_KF + s), 0, head, key_row + j * BN);
         tma_load_3d(dst + KV_BOX, &map_kv, bar(B_KF + s), 64, head, key_row + j * BN);
         tma_load_2d(dst + 2 * KV_BOX, &map_kr, bar(B_KF + s), rank, key_row + j * BN);
-        return true;
-      };
-      auto load_v = [&](int j) {
+      }
+    }
+    __syncwarp();
+  } else if (warp == V_LOADER_WARP) {      // a thread of its own: keys are wanted long before the values of the same tile are
+    if (lane == 0) {
+      for (int j = 0; j < n_local; ++j) {
         const int s = j % STAGES;
-        if (!mbar_wait(bar(B_VE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) return false;
+        if (!mbar_wait(bar(B_VE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) break;
         const uint32_t dst = v_s + s * V_BYTES;
         mbar_expect_tx(bar(B_VF + s), V_BYTES);
         tma_load_3d(dst, &map_kv, bar(B_VF + s), 0, heads + head, key_row + j * BN);
         tma_load_3d(dst + KV_BOX, &map_kv, bar(B_VF + s), 64, heads + head, key_row + j * BN);
-        return true;
-      };
-      bool ok = load_k(0);
-      for (int j = 0; j < n_local && ok; ++j) {      // the keys of the next tile go before the values of this one
-        if (j + 1 < n_local) ok = load_k(j + 1);
-        if (ok) ok = load_v(j);
       }
     }
     __syncwarp();
