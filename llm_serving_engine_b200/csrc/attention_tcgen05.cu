@@ -18,7 +18,7 @@
 //                 barrier.
 //   softmax       a thread owns one row of its group's tiles: it reads S (tcgen05.ld), masks, finds
 //                 the row maximum, takes exp2 in float32 and writes bfloat16 probabilities to shared memory in the swizzled K-major
-//                 layout the tensor cores read.  The row is in registers before anything else, so that
+//                 layout the tensor cores read (scaled and summed up in pairs, two operations an instruction).  The row is in registers before anything else, so that
 //                 the group's next scores are made meanwhile.  The probabilities are taken relative to
 //                 the maximum in use; O stays in tensor memory and is only rescaled when a row maximum has grown by more than 2^8 (the sums
 //                 carry the same factor, so the quotient is exact either way).  At the end the two groups' outputs
@@ -377,7 +377,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tmem_st_wait();
       }
       const float neg = m_used == -INFINITY ? 0.f : -m_used;   // every score is -inf then as well: p = 0
-      float sum = 0.f;
+      const uint64_t scale_pair = f32_pair(scale_log2e, scale_log2e), neg_pair = f32_pair(neg, neg);
+      uint64_t sum_pair = 0;
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) {      // 32 keys = 4 pieces of 16 bytes at a time
         uint32_t pk[16];
@@ -396,9 +397,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           } else if (PEN) {
             p0 = exp2_fast(s0 + neg); p1 = exp2_fast(s1 + neg);
           } else {
-            p0 = exp2_fast(fmaf(s0, scale_log2e, neg)); p1 = exp2_fast(fmaf(s1, scale_log2e, neg));
+            f32_halves(f32_pair_fma(f32_pair(s0, s1), scale_pair, neg_pair), p0, p1);
+            p0 = exp2_fast(p0); p1 = exp2_fast(p1);
           }
-          sum += p0 + p1;
+          sum_pair = f32_pair_add(sum_pair, f32_pair(p0, p1));
           pk[i] = pack_bf16(p0, p1);
         }
         unsigned char* box = prow + (c / 2) * HALF_BYTES;
@@ -408,7 +410,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           *reinterpret_cast<uint4*>(box + ((chunk ^ (row & 7)) << 4)) = make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
         }
       }
-      l += sum;
+      float sum_even, sum_odd;
+      f32_halves(sum_pair, sum_even, sum_odd);
+      l += sum_even + sum_odd;
       TC_STAMP(j, 4)
       if (j_lo + j == n_tiles - 1 && last_pos + 1 - kv0 < BN) {
         // rows of V beyond the last key: whatever lies there (stale keys, unwritten shared memory)
