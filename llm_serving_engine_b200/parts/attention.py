@@ -156,7 +156,8 @@ class GroupedQueryAttention(Mixer):
         attended = torch.empty_like(q)
         if ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, x.dtype, self.window):
             if step.decode_only:
-                splits = ops.decode_splits(tokens, self.n_q, self.n_kv, step.max_context, getattr(step, "long_context", False))
+                splits = ops.decode_splits(tokens, self.n_q, self.n_kv, step.max_context, getattr(step, "long_context", False),
+                                           table_keys=cache.block_tables.shape[1] * cache.keys.shape[2])
                 ops.paged_attention_decode(q, cache.keys, cache.values, attended, cache.block_tables,
                                            step.segment_of_token, step.positions, self.scale, splits)
             elif sum(segment.count for segment in step.segments) < ROWS_KERNEL_BELOW:
@@ -170,7 +171,8 @@ class GroupedQueryAttention(Mixer):
                 portions, singles = self._portions([segment.count for segment in step.segments])
                 if singles:   # one block row per request of the step; requests with portions leave at once
                     requests = cache.block_tables.shape[0]
-                    splits = ops.decode_splits(requests, self.n_q, self.n_kv, None)
+                    splits = ops.decode_splits(requests, self.n_q, self.n_kv, None,
+                                               table_keys=cache.block_tables.shape[1] * cache.keys.shape[2])
                     ops.paged_attention_decode(q, cache.keys, cache.values, attended, cache.block_tables,
                                                step.segment_of_token, step.positions, self.scale, splits,
                                                segment_start=step.segment_start)
