@@ -152,6 +152,7 @@ class CacheManager:
         self._free_slots: deque[int] = deque(range(self.num_state_slots))
         self.requests: dict[str, RequestCache] = {}
         self._high_water = {"blocks": 0, "used_tokens": 0, "sequences": 0}
+        self._high_water_open = False       # the last reservation set the mark, its tokens and requests are not added up yet
 
         by_need: dict = {}
         self.layer_members: dict[int, int] = {}     # layers whose requirement is a tuple: how many members
@@ -199,6 +200,7 @@ class CacheManager:
     def create(self, request_id: str) -> RequestCache:
         if request_id in self.requests:
             raise ValueError(f"sequence {request_id!r} already exists")
+        self._settle_high_water()
         if not self._free_slots:
             raise CacheFullError("no free per-request state slot")
         slot = self._free_slots.popleft()
@@ -267,14 +269,25 @@ class CacheManager:
             if after - len(table) > group.pool.free_pages:
                 raise CacheFullError("paged KV cache has no free blocks")
         self._extend(request, after)
+        used = sum(group.pool.used_pages for group in self.groups)
+        highest = used >= self._high_water["blocks"]
+        if self._high_water_open and not highest:
+            self._settle_high_water()
         first = request.length
         request.length += count
-        used = sum(group.pool.used_pages for group in self.groups)
-        if used >= self._high_water["blocks"]:
-            self._high_water = {"blocks": used,
-                                "used_tokens": sum(item.length for item in self.requests.values()),
-                                "sequences": len(self.requests)}
+        if highest:
+            self._high_water["blocks"] = used
+            self._high_water_open = True
         return first
+
+    def _settle_high_water(self) -> None:
+        """Tokens and requests at the last reservation that held the most pages.  They are added up when something is about to
+        change them, or when they are asked for, and not at every reservation: a step of decoding requests reserves for
+        each, and adding up all of them every time took 250 of the 420 us that a step of 64 takes on the host."""
+        if self._high_water_open:
+            self._high_water["used_tokens"] = sum(item.length for item in self.requests.values())
+            self._high_water["sequences"] = len(self.requests)
+            self._high_water_open = False
 
     def release_passed(self, request_id: str) -> int:
         """Give back the pages of windowed groups that no later token can read:
@@ -299,6 +312,7 @@ class CacheManager:
         return given
 
     def free(self, request_id: str) -> None:
+        self._settle_high_water()
         request = self.requests.pop(request_id)
         for group, table in zip(self.groups, request.tables):
             for page in table:
@@ -364,6 +378,7 @@ class CacheManager:
         return sum(self.bytes_per_page(group) // self.page_size for group in self.groups)
 
     def stats(self, contiguous_max_length: int | None = None) -> dict[str, float]:
+        self._settle_high_water()
         used_tokens = sum(request.length for request in self.requests.values())
         used_pages = sum(group.pool.used_pages for group in self.groups)
         free_pages = sum(group.pool.free_pages for group in self.groups)
