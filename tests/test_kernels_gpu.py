@@ -84,6 +84,26 @@ def test_add_rmsnorm(hidden, delta_dtype, out_dtype):
     assert rel_err(picked, want[rows.long()]) < TOL[out_dtype] * 2
 
 
+@pytest.mark.parametrize("hidden", [2052, 3584, 5120, 8192, 512])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_add_rmsnorm_of_many_wide_rows(hidden, out_dtype):
+    """The kernel for many rows with one set of sums: the bits of the one that takes stacks of partial sums (given the same
+    sums and a second stack of zeros), and right against float64."""
+    torch.manual_seed(hidden)
+    rows = 257
+    residual, delta = torch.randn(rows, hidden, device=DEV), torch.randn(rows, hidden, device=DEV)
+    weight, eps = torch.rand(hidden, device=DEV) + 0.5, 1e-6
+    one, two = residual.clone(), residual.clone()
+    out, stacked = torch.empty(rows, hidden, device=DEV, dtype=out_dtype), torch.empty(rows, hidden, device=DEV, dtype=out_dtype)
+    ops().add_rmsnorm(one, delta, weight, eps, out)
+    ops().add_rmsnorm(two, torch.stack([delta, torch.zeros_like(delta)]), weight, eps, stacked)
+    assert torch.equal(one, two)
+    if hidden > 2048 or out_dtype == torch.float32:      # narrower bfloat16 rows go to a kernel of a warp a row
+        assert torch.equal(out, stacked)
+    want = qwen2_plain.rms_norm(residual.double() + delta.double(), weight.double(), eps)
+    assert rel_err(out, want) < TOL[out_dtype] * 2
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 33, 7), (5, 1000, 96), (17, 130, 1539), (70, 257, 300), (200, 64, 64)])
 def test_gemm_f32_is_true_float32_and_row_invariant(m, n, k):
     torch.manual_seed(m * n)
