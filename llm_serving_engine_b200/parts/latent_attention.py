@@ -19,7 +19,7 @@ PER_HEAD_LIBRARY_ROWS = 32    # above this many bfloat16 rows the per-head produ
 # per head around the latter, 19 us, are saved too).  Both write into buffers of the step.
 EXPAND_FLOPS, EXPANDED_FLOPS, LATENT_FLOPS = 1.0e9, 4.0e8, 1.2e8
 EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an attention of few blocks
-EXPAND_MAX_ROWS = 65536       # keys and values of that many rows are held at once (8 KB a row at 16 heads)
+EXPAND_MAX_BYTES = 1 << 30    # of keys and values that are held at once (8 KB a row at 16 heads)
 
 
 def _size_class(rows: int) -> int:
@@ -171,7 +171,7 @@ class LatentAttention(Mixer):
         expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
                     + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
         latent = 2.0 * pairs * self.heads * (2 * self.rank + self.rot_dim) / LATENT_FLOPS
-        return rows if rows <= EXPAND_MAX_ROWS and expanded < latent else 0
+        return rows if 2 * rows * self.kv_up.shape[0] <= EXPAND_MAX_BYTES and expanded < latent else 0
 
     def launch_signature_at(self, segment_counts, contexts):
         rows = self._expanded_rows(segment_counts, contexts)
