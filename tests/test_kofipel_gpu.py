@@ -626,6 +626,36 @@ def test_convolutions_unit_vectors_and_write_strengths(dtype, groups, heads, dim
             assert torch.equal(state[slots[i]].cpu(), proj[i][-(taps - 1):, :channels].float())
 
 
+@pytest.mark.parametrize("portions", [(127, 1, 2, 125), (127, 1, 2, 126), (255, 1, 1, 766), (255, 2, 1, 766), (255, 2, 1, 771)])
+@pytest.mark.parametrize("groups,heads,dim,vdim,taps", [(2, 4, 16, 24, 4), (1, 1, 150, 10, 2), (1, 2, 8, 8, 6)])
+def test_convolutions_of_many_rows(portions, groups, heads, dim, vdim, taps):
+    """255, 256, 1,023, 1,024 and 1,029 rows (one, four and eight rows a warp), with requests that begin and end inside a
+    warp's rows, from states that are not zero.  The limits are those of the test above."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(27)
+    slots, rank = [2, 0, 3, 1], 5
+    channels = 2 * groups * dim + heads * vdim
+    rows = torch.randn(sum(portions), -(-(channels + heads + rank) // 4) * 4)
+    conv, before = torch.randn(channels, taps) * 0.6, torch.randn(4, taps - 1, channels)
+    low, state, scale = torch.empty(sum(portions), 16, device="cuda"), before.cuda(), dim ** -0.5
+    result = ops.delta_prepare(rows.cuda(), conv.cuda(), state, _step(list(portions), slots=slots), low, groups, heads, dim, vdim,
+                               rank, scale)
+    at, qk = 0, groups * dim
+    for i, count in enumerate(portions):
+        mine = slice(at, at + count)
+        seen = torch.cat([before[slots[i]], rows[mine, :channels]])
+        y = torch.nn.functional.silu(plain.causal_conv(seen.double(), conv.double())[taps - 1:])
+        want = (plain.unit(y[:, :qk].view(count, groups, dim)).reshape(count, -1) * scale,
+                plain.unit(y[:, qk:2 * qk].view(count, groups, dim)).reshape(count, -1), y[:, 2 * qk:],
+                torch.sigmoid(rows[mine, channels:channels + heads].double()), rows[mine, channels + heads:channels + heads + rank].double())
+        for index, (tensor, expected) in enumerate(zip((*result, low[:, :rank]), want)):
+            error = (tensor[mine].cpu().double().reshape(count, -1) - expected).abs().max()
+            assert float(error) <= 3e-6 * max(1.0, float(expected.abs().max())), (i, index)
+        assert torch.equal(state[slots[i]].cpu(), seen[-(taps - 1):])
+        at += count
+
+
 @pytest.mark.parametrize("above", [0, 16, 10 ** 9])
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 48, 40), (2, 1, 128, 128), (3, 3, 20, 12), (1, 1, 200, 33), (2, 2, 64, 64), (1, 1, 1, 1)])
 @pytest.mark.parametrize("decay", ["mild", "strong"])
