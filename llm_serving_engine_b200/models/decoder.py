@@ -173,13 +173,15 @@ class DecoderModel:
         return bool(getattr(self.final_norm, "graph_safe", False))
 
     def launch_signature(self, segment_counts: list[int], contexts: list[int] | None = None) -> tuple:
-        """The mixers' answers to ``Mixer.launch_signature`` (``launch_signature_at``, given the requests' contexts) for a step
-        of this shape (each distinct answer once)."""
+        """What a captured step of this shape is kept by, besides its sizes: every layer's answer to
+        ``Mixer.launch_signature_at`` with the layer's index, layers without one left out.  Which layer gave which answer
+        matters: an answer may fix the size of a buffer, and two steps in which different layers give it launch different
+        things.  Without ``contexts``: the distinct answers to ``Mixer.launch_signature``, which only name kernels."""
         if contexts is None:
             answers = {block.mixer.launch_signature(segment_counts) for block in self.blocks}
-        else:
-            answers = {block.mixer.launch_signature_at(segment_counts, contexts) for block in self.blocks}
-        return tuple(sorted(answer for answer in answers if answer))
+            return tuple(sorted(answer for answer in answers if answer))
+        answers = [block.mixer.launch_signature_at(segment_counts, contexts) for block in self.blocks]
+        return tuple((index, answer) for index, answer in enumerate(answers) if answer)
 
     @property
     def vocab_size(self) -> int:

@@ -1,0 +1,49 @@
+"""What the captured steps with prompt portions are kept by (no GPU): steps that launch different things have different keys."""
+import torch
+
+from llm_serving_engine_b200.config.model_config import LayerSpec, ModelSpec, PartSpec
+from llm_serving_engine_b200.models import DecoderModel, expected_tensors
+
+
+def latent_model(windows, heads=16, rank=512, width=64, dtype=torch.bfloat16, device="cpu", scale=0.05, seed=0, positions=32768):
+    """Latent attention layers alone, one per window."""
+    norm = PartSpec("rmsnorm", {"eps": 1e-5})
+    layers = tuple(LayerSpec(prefix=f"l{index}.", block=PartSpec("residual_streams", {"feed_forward": False}),
+                             mixer=PartSpec("latent_attention", {"heads": heads, "dim": 128, "rot_dim": 64, "vdim": 128, "kv_rank": rank,
+                                                                 "scale": scale, "eps": 1e-5, "window": window,
+                                                                 "rot": {"base": 10000.0, "dims": 64}}),
+                             feed_forward=None, mixer_norm=norm, feed_forward_norm=None) for index, window in enumerate(windows))
+    spec = ModelSpec(architecture="latent layers", vocab_size=64, hidden_size=width, layers=layers, order=tuple(range(len(layers))),
+                     final_norm=norm, embedding_name="embed", final_norm_prefix="final.", lm_head_name="head",
+                     tie_word_embeddings=True, max_position_embeddings=positions)
+    generator = torch.Generator().manual_seed(seed)
+    weights = {}
+    for name, tensor in expected_tensors(spec).items():
+        values = torch.randn(tensor.shape, generator=generator)
+        if tensor.kind == "matrix":
+            weights[name] = (values * tensor.shape[-1] ** -0.5 * 1.5).to(dtype).to(device)
+        else:
+            weights[name] = (1.0 + 0.1 * values).to(device)
+    return DecoderModel(spec, weights, dtype, device)
+
+
+def test_a_layer_that_stops_expanding_its_latents_changes_the_key():
+    """A windowed and a full layer: at 20,000 keys a request the full one's keys and values would not fit, the windowed one's are
+    as many as before."""
+    model = latent_model([2048, 0])
+    counts = [256] * 8
+    short, long = (model.launch_signature(counts, [context] * 8) for context in (2304, 20000))
+    rows = [[block.mixer._expanded_rows(counts, [context] * 8) for block in model.blocks] for context in (2304, 20000)]
+    assert rows[0][0] == rows[0][1] == rows[1][0] > 0 and rows[1][1] == 0      # the layers' answers as a set are the same
+    assert short != long
+    assert model.launch_signature([256], [768]) != latent_model([0, 2048]).launch_signature([256], [20000])
+
+
+def test_the_order_of_the_answers_is_part_of_the_key():
+    a, b = latent_model([512, 0], heads=64), latent_model([0, 512], heads=64)
+    for contexts in ([20000], [9000]):
+        assert a.launch_signature([256], contexts) != b.launch_signature([256], contexts)
+
+
+def test_layers_without_an_answer_leave_the_key_empty():
+    assert latent_model([0, 512]).launch_signature([1, 1], [700, 20]) == ()

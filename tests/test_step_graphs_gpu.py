@@ -1,0 +1,48 @@
+"""Captured steps replayed at other contexts of their class, through the step function."""
+import pytest
+import torch
+
+from llm_serving_engine_b200.cache import CacheManager
+from llm_serving_engine_b200.config import CacheConfig
+from llm_serving_engine_b200.engine import StepEntry, StepRunner
+from llm_serving_engine_b200.models import cache_requirements
+from llm_serving_engine_b200.parts import latent_attention
+from test_launch_signature_cpu import latent_model
+
+pytestmark = pytest.mark.gpu
+
+
+def runner_for(model, use_graphs, positions=2048, page=16, pages=200, tokens=512, segments=8):
+    cache = CacheManager(cache_requirements(model.spec), CacheConfig(page, pages), model.dtype, "cuda", positions, num_state_slots=segments)
+    return StepRunner(model, cache, tokens, segments, use_graphs=use_graphs)
+
+
+def in_portions(runner, rid, tokens, size):
+    """The logits of every token of a request that is run alone in portions of ``size``."""
+    runner.cache.create(rid)
+    out = []
+    for lo in range(0, len(tokens), size):
+        part = tokens[lo:lo + size]
+        out.append(runner.run([StepEntry(rid, part, list(range(len(part))))]).clone())
+    runner.cache.free(rid)
+    return torch.cat(out)
+
+
+def test_a_captured_step_is_not_replayed_where_a_layer_launches_something_else(monkeypatch):
+    """A windowed and a full latent layer, keys and values bounded so that the full layer makes its own up to 128 keys only: the
+    second portions of two requests capture the step, the later portions of a third have the windowed layer's buffer of the same
+    size, but a full layer that goes over the latent rows.  Every logit against the latent rows' kernel launch by launch."""
+    model = latent_model([64, 0], heads=2, rank=64, device="cuda", scale=0.07)
+    generator = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, 64, (length,), generator=generator).tolist() for length in (128, 128, 448)]
+    plain = runner_for(model, use_graphs=False)
+    monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0e30)      # never worth it
+    want = [in_portions(plain, "r", tokens, 64) for tokens in prompts]
+    monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0)         # always worth it, where it fits
+    monkeypatch.setattr(latent_attention, "EXPAND_MAX_BYTES", 2 * 128 * model.blocks[0].mixer.kv_up.shape[0])
+    graphs = runner_for(model, use_graphs=True)
+    for index, tokens in enumerate(prompts):
+        got = in_portions(graphs, "r", tokens, 64)
+        # bfloat16 at other places of two layers: a few units in the last place of the largest logit
+        assert float((got - want[index]).abs().max()) <= 2.0 ** -4 * float(want[index].abs().max()), index
+    assert graphs.portion_graph_replays >= 4
