@@ -536,6 +536,10 @@ class ParallelMixers(Mixer):
     def launch_signature(self, segment_counts):
         return tuple(answer for branch in self.branches for answer in branch.launch_signature(segment_counts))
 
+    def launch_signature_at(self, segment_counts, contexts):
+        answers = [branch.launch_signature_at(segment_counts, contexts) for branch in self.branches]
+        return tuple((index, answer) for index, answer in enumerate(answers) if answer)
+
     def forward(self, x, step, cache):
         proj = input_projection(x, self.in_weight)
         mid = torch.empty((x.shape[0], self.mid_offsets[-1]), dtype=x.dtype, device=x.device)

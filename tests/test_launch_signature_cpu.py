@@ -3,6 +3,8 @@ import torch
 
 from llm_serving_engine_b200.config.model_config import LayerSpec, ModelSpec, PartSpec
 from llm_serving_engine_b200.models import DecoderModel, expected_tensors
+from llm_serving_engine_b200.parts.base import Mixer
+from llm_serving_engine_b200.parts.branches import ParallelMixers
 
 
 def latent_model(windows, heads=16, rank=512, width=64, dtype=torch.bfloat16, device="cpu", scale=0.05, seed=0, positions=32768):
@@ -47,3 +49,19 @@ def test_the_order_of_the_answers_is_part_of_the_key():
 
 def test_layers_without_an_answer_leave_the_key_empty():
     assert latent_model([0, 512]).launch_signature([1, 1], [700, 20]) == ()
+
+
+def test_parallel_mixers_hand_on_what_their_branches_answer_at_their_contexts():
+    class Branch(Mixer):
+        def __init__(self, from_keys):
+            self.from_keys = from_keys
+
+        def launch_signature_at(self, segment_counts, contexts):
+            return ("long",) if max(contexts) >= self.from_keys else ()
+
+    part = object.__new__(ParallelMixers)
+    part.branches = [Branch(100), Branch(1000)]
+    answers = [part.launch_signature_at([8], [context]) for context in (50, 500, 5000)]
+    assert answers[0] == () and len(set(answers)) == 3
+    part.branches.reverse()
+    assert part.launch_signature_at([8], [500]) != answers[1]      # another branch's answer
