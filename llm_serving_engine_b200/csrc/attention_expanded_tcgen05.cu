@@ -16,7 +16,8 @@
 // 2,048 rows, 16 heads: 41 us (524 TFLOP/s of the 320 multiply-adds a pair), bounded by the softmax threads' exponentials
 // and issue slots like the kernel it follows; over the latent rows themselves 611 us.
 //
-// Every wait is bounded (see tcgen05.cuh); lse_attention_expanded_status() reports one that gave up.
+// Every wait is bounded (see tcgen05.cuh); lse_attention_expanded_status() reports one that gave up, and contexts on the
+// device that ask for more rows than the host made room for (the rows beyond would be zeros, and count as keys).
 #include "tcgen05.cuh"
 
 LSE_CHECK_DEFINE(lse_check_attention_expanded)
@@ -34,6 +35,7 @@ constexpr uint32_t Q_BOX = BM * 128, KV_BOX = BN * 128;      // a box of 64 bflo
 constexpr uint32_t Q_BYTES = 3 * Q_BOX, K_BYTES = 3 * KV_BOX, V_BYTES = 2 * KV_BOX, P_BYTES = BM * 128;
 constexpr size_t SMEM = 1024 + Q_BYTES + STAGES * (K_BYTES + V_BYTES) + GROUPS * P_BYTES + GROUPS * 256 * 4 + 256;
 
+constexpr int TOO_MANY_ROWS = 2;      // in the error word: the requests hold more rows than were to be gathered (1: a wait gave up)
 __device__ int lse_attn_expanded_error;
 
 // barriers: stages of keys and values (full, empty), scores of a group (two accumulators: full, read), probabilities, outputs
@@ -93,6 +95,10 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
     before += __shfl_sync(0xffffffffu, upto, 31);
   }
   pdl_wait();      // the step's own rows come from the kernel before
+  if (blockIdx.x == 0 && threadIdx.x < 32) {      // capacity was fixed on the host (a captured step's when it was captured)
+    const int wanted = rows_before(first, context, window, num_segments);
+    if (threadIdx.x == 0 && wanted > capacity) atomicExch(&lse_attn_expanded_error, TOO_MANY_ROWS);
+  }
   const __nv_bfloat16* src = nullptr;
   if (seg >= 0) {
     const int pos = first_kept(first[seg], window) + local;
@@ -387,7 +393,8 @@ extern "C" int lse_attention_expanded_supported(int dim, int rot, int vdim, int 
 // Keys of a tile: a request's gathered rows are a multiple of it.
 extern "C" int lse_attention_expanded_tile(void) { return BN; }
 
-// 0: no bounded wait has given up since the word was last cleared (synchronises the device).
+// 0: no bounded wait has given up (1) and no request's rows were left out (2) since the word was last cleared (synchronises
+// the device).
 extern "C" int lse_attention_expanded_status(void) {
   int value = 0;
   if (cudaMemcpyFromSymbol(&value, lse_attn_expanded_error, sizeof(int)) != cudaSuccess) return -1;
@@ -403,7 +410,7 @@ extern "C" int lse_attention_expanded_status_reset(void) {
 
 // rows [capacity, width] bfloat16 receives the cached rows (cache [pages, page_size, width]) of every request, from its
 // first position - window + 1 on (window <= 0: from 0), up to context[s] (exclusive), rounded up to whole tiles; zeros beyond.
-// capacity holds the sum of them.  All 16-byte aligned.
+// capacity holds the sum of them (lse_attention_expanded_status: 2 if it does not).  All 16-byte aligned.
 extern "C" int lse_latent_gather(const void* cache, const int* block_tables, int bt_stride, const int* segment_first_pos,
                                  const int* segment_context, int num_segments, int width, int page_size, int num_pages,
                                  int window, void* rows, int capacity, cudaStream_t stream) {

@@ -831,11 +831,15 @@ def attention_expanded_tile() -> int:
     return int(library.load().lse_attention_expanded_tile())
 
 
+EXPANDED_ROWS_LEFT_OUT = 2      # in the status word of the attention over expanded latents (1: a wait gave up)
+
+
 def latent_gather(cache: torch.Tensor, block_tables: torch.Tensor, segment_first_position: torch.Tensor,
                   segment_context: torch.Tensor, capacity: int, window: int = 0) -> torch.Tensor:
     """The cached rows (cache [pages, page_size, width] bfloat16) that each request of the step may read, positions
     max(0, first + 1 - window) (window <= 0: 0) up to its context, request by request, each rounded up to whole key
-    tiles with zeros: [capacity, width], zeros behind the last.  ``capacity`` holds them all."""
+    tiles with zeros: [capacity, width], zeros behind the last.  ``capacity`` holds them all; if it does not, the kernels'
+    status word says so (``EXPANDED_ROWS_LEFT_OUT``)."""
     _need_cuda(cache, block_tables, segment_first_position, segment_context)
     segments, width = block_tables.shape[0], cache.shape[2]
     assert cache.is_contiguous() and cache.dtype == torch.bfloat16 and block_tables.dtype == torch.int32 and block_tables.stride(1) == 1

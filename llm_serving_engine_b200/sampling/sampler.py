@@ -122,7 +122,11 @@ class Sampler:
             which = " and ".join(name for name, word in zip(("the few-rows product", "the tcgen05 prompt attention",
                                                              "the attention over expanded latents"),
                                                             turn.host_status.tolist()) if word)
+            left_out = int(turn.host_status[2]) == ops.EXPANDED_ROWS_LEFT_OUT
             turn.host_status.zero_()
             ops.kernel_status_reset()
+            if left_out:
+                raise ops.KernelError("the attention over expanded latents was given room for fewer rows than the requests hold: "
+                                      "the step's results are not valid")
             raise ops.KernelError(f"a bounded wait inside {which} gave up: the step's results are not valid")
         return turn.host_out[:turn.rows].tolist()

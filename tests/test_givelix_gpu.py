@@ -466,6 +466,22 @@ def test_latent_attention_over_expanded_keys_and_values(heads, rank, page, windo
             row, at = row + count, at + size
 
 
+def test_a_gather_without_room_for_the_requests_rows_is_reported():
+    """Contexts of 100 and 130 keys are 128 and 192 rows: room for one row fewer is reported, and nothing behind it is written."""
+    from llm_serving_engine_b200.kernels import ops
+
+    cache = torch.randn(16, 16, 88).bfloat16().cuda()
+    tables = torch.arange(16, dtype=torch.int32).view(2, 8).cuda()
+    tables = torch.cat([tables, tables], dim=1)
+    firsts, contexts = torch.tensor([40, 0], dtype=torch.int32).cuda(), torch.tensor([100, 130], dtype=torch.int32).cuda()
+    library = ops.library.load()
+    for capacity, want in ((320, 0), (319, ops.EXPANDED_ROWS_LEFT_OUT), (400, 0)):
+        rows = ops.latent_gather(cache, tables, firsts, contexts, capacity)
+        assert library.lse_attention_expanded_status() == want and rows.shape[0] == capacity
+        ops.kernel_status_reset()
+    assert library.lse_attention_expanded_status() == 0
+
+
 @pytest.mark.parametrize("heads, dim, vdim, counts, dtype", [(2, 128, 128, [64, 65, 1, 130], "bfloat16"), (3, 68, 130, [127, 63], "float32"),
                                                              (1, 127, 5, [200, 2], "bfloat16"), (2, 96, 256, [128], "float32")])
 def test_linear_attention_in_chunks_as_products(heads, dim, vdim, counts, dtype):
