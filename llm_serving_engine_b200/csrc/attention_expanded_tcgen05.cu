@@ -6,7 +6,8 @@
 // one product over the rows, and to pay 192 and 128 a pair.  Two kernels, the product between them:
 //
 //   gather      copies the rows that the step's requests may read from their pages into one tensor, request by request, each
-//               request's rows rounded up to whole key tiles with zeros (a tile never meets another request's rows)
+//               request's rows rounded up to whole key tiles with zeros (a tile never meets another request's rows); a latent
+//               that is not finite becomes zeros with NaN in place of its rotated values
 //   attention   the kernel of attention_tcgen05.cu on these: a block takes 128 rows of one request and one head; key tiles of
 //               64 go alternately to two groups of four softmax warps.  A score product takes 128 columns of the head's key
 //               and the 64 rotated ones that all heads share (read from the gathered rows), so that a key tile is 24 KB;
@@ -67,6 +68,9 @@ __device__ __forceinline__ int rows_before(const int* __restrict__ first, const 
   return sum;
 }
 
+// Whether one of two bfloat16 numbers is infinite or NaN (an exponent of ones: it carries into the sign when it is raised by one).
+__device__ __forceinline__ bool not_finite(uint32_t two) { return (((two & 0x7f807f80u) + 0x00800080u) & 0x80008000u) != 0; }
+
 // rows[r] for r < capacity: a warp a row; rows of no request, and those that round a request up, are zeros.
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_tables, int bt_stride,
@@ -107,9 +111,20 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
       src = cache + ((size_t)page * page_size + pos % page_size) * width;
     }
   }
+  bool broken = false;
   for (int c = lane * 8; c < width; c += 256) {
     const uint4 v = src ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0u, 0u, 0u, 0u);
+    broken |= c < width - ROT && (not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w));
     *reinterpret_cast<uint4*>(rows + (size_t)r * width + c) = v;
+  }
+  // A latent that is not finite makes NaN of every row that attends to it, and must not reach those that do not: the values made
+  // of it would, as hidden keys of a tile have no weight but are multiplied by it.  So it has finite keys and values, and NaN
+  // where the scores are made, which hidden keys do not have.
+  if (__any_sync(0xffffffffu, broken)) {
+    for (int c = lane * 8; c < width; c += 256) {
+      const uint32_t x = c < width - ROT ? 0u : 0x7fc07fc0u;
+      *reinterpret_cast<uint4*>(rows + (size_t)r * width + c) = make_uint4(x, x, x, x);
+    }
   }
 }
 

@@ -839,7 +839,8 @@ def latent_gather(cache: torch.Tensor, block_tables: torch.Tensor, segment_first
     """The cached rows (cache [pages, page_size, width] bfloat16) that each request of the step may read, positions
     max(0, first + 1 - window) (window <= 0: 0) up to its context, request by request, each rounded up to whole key
     tiles with zeros: [capacity, width], zeros behind the last.  ``capacity`` holds them all; if it does not, the kernels'
-    status word says so (``EXPANDED_ROWS_LEFT_OUT``)."""
+    status word says so (``EXPANDED_ROWS_LEFT_OUT``).  A row whose latent is not finite comes as zeros with NaN in its last 64
+    values: who attends to it gets NaN, and nobody else does."""
     _need_cuda(cache, block_tables, segment_first_position, segment_context)
     segments, width = block_tables.shape[0], cache.shape[2]
     assert cache.is_contiguous() and cache.dtype == torch.bfloat16 and block_tables.dtype == torch.int32 and block_tables.stride(1) == 1

@@ -466,6 +466,48 @@ def test_latent_attention_over_expanded_keys_and_values(heads, rank, page, windo
             row, at = row + count, at + size
 
 
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_a_latent_that_is_not_finite_reaches_the_rows_that_read_it_only(value, window, monkeypatch):
+    """One cached row of 300 with a value that is not finite in its latent, through the layer: rows before it, and rows whose
+    window has passed it, are what they are without it, bit for bit; rows that read it are NaN, as over the latent rows.  Then an
+    infinite rotated value: the same rows are left alone."""
+    from llm_serving_engine_b200.kernels import ops
+    from llm_serving_engine_b200.parts import latent_attention
+    from test_launch_signature_cpu import latent_model
+    from test_step_graphs_gpu import runner_for
+    from llm_serving_engine_b200.engine import StepEntry
+
+    monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0)
+    mixer = latent_model([window], heads=2, rank=72, device="cuda", scale=0.07).blocks[0].mixer
+    torch.manual_seed(3)
+    x = torch.randn(300, 64, device="cuda").bfloat16()
+    real, at = ops.latent_gather, 193
+
+    def outputs(column):
+        runner = runner_for(latent_model([window], heads=2, rank=72, device="cuda"), use_graphs=False)
+        runner.cache.create("r")
+        step, caches = runner.prepare([StepEntry("r", [0] * 300, [])])
+
+        def gather(cache, tables, *rest):
+            if column is not None:
+                cache[tables[0, at // 16], at % 16, column] = value
+            return real(cache, tables, *rest)
+
+        monkeypatch.setattr(ops, "latent_gather", gather)
+        out = mixer.forward(x, step, caches[0])
+        return (out.sum(0) if out.dim() == 3 else out).float()
+
+    clean = outputs(None)
+    readers = torch.zeros(300, dtype=torch.bool, device="cuda")
+    readers[at:at + window if window else 300] = True
+    for column in (0, 71, 80):
+        got = outputs(column)
+        assert bool(clean.isfinite().all()) and torch.equal(got[~readers], clean[~readers]), column
+        if column < 72:
+            assert bool(got[readers].isnan().all()), column
+
+
 def test_a_gather_without_room_for_the_requests_rows_is_reported():
     """Contexts of 100 and 130 keys are 128 and 192 rows: room for one row fewer is reported, and nothing behind it is written."""
     from llm_serving_engine_b200.kernels import ops
