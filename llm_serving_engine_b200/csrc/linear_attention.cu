@@ -276,7 +276,10 @@ gated_group_rmsnorm_warp_kernel(const float* __restrict__ o, const TD* __restric
 // which is a third of the multiply-adds and lets a thread own 16 x 8 or 8 x 8 results: 116 us for the outputs and 56 for the
 // states (the multiply-adds alone take 32 and 15).  Everything is float32, products are
 // paired multiply-adds (two rounded operations an instruction).  For 64 < dim <= 128 (padded to 128 in shared memory); below, the
-// scan does as well.
+// scan does as well.  A chunk's products cost the same however few of its rows there are, so requests of up to LC_SHORT rows
+// go to the scan, row by row from and into their slots: 256 rows beside 64 single ones 914 to 248 us, 64 requests of four rows 872
+// to 192, eight of 17 115 to 58, 64 of 32 (where the two meet) 551 against 763 for 64 of 33 in chunks; 16 heads of 128 x 128.
+constexpr int LC_SHORT = 32;
 constexpr int LC_ROWS = 64, LC_DIM = 128, LC_THREADS = 128, LC_PITCH = LC_DIM + 4, LC_P_PITCH = LC_ROWS + 4;
 constexpr size_t LC_OWN_SMEM = sizeof(float) * 2 * LC_ROWS * LC_PITCH;
 constexpr size_t LC_OUT_SMEM = sizeof(float) * 3 * LC_ROWS * LC_PITCH;     // q | k, then P | v; at the end the state takes k's and v's place
@@ -359,7 +362,7 @@ __device__ __forceinline__ void lc_put(float* dst, const LcRaw<TD>& raw, const L
   }
 }
 // Which rows chunk `index` has (row0, n), the chunks being numbered request by request; n = 0: there is no such chunk.
-// Every thread of the block calls it; pow receives decay^0 .. decay^LC_ROWS.
+// Every thread of the block calls it; pow receives decay^0 .. decay^LC_ROWS.  Requests of up to LC_SHORT rows have none.
 __device__ __forceinline__ void lc_chunk(const int* __restrict__ segment_start, int num_segments, int index, float decay,
                                          float* pow, int* slot, int& row0, int& n) {
   if (threadIdx.x == 0) {
@@ -367,7 +370,7 @@ __device__ __forceinline__ void lc_chunk(const int* __restrict__ segment_start, 
     slot[0] = slot[1] = 0;
     for (int s = 0; s < num_segments; ++s) {
       const int a = segment_start[s], b = segment_start[s + 1];
-      const int chunks = (b - a + LC_ROWS - 1) / LC_ROWS;
+      const int chunks = la_chunks(b - a, LC_ROWS, LC_SHORT);
       if (index < before + chunks) {
         slot[0] = a + (index - before) * LC_ROWS;
         slot[1] = min(b - slot[0], LC_ROWS);
@@ -402,8 +405,8 @@ linear_attention_own_states_kernel(const LcInput<TD> in, int k_off, int v_off, c
   const int h = blockIdx.y, col0 = blockIdx.z * LC_DIM;
   int row0, n;
   lc_chunk(segment_start, num_segments, blockIdx.x, decay[h], pow_s, slot, row0, n);
+  pdl_wait();      // before any block leaves: a launch without chunks must not end ahead of the kernels before it
   if (n == 0) return;
-  pdl_wait();
   const int k_col = k_off + h * dim, v_col = v_off + h * vdim + col0;
   {
     LcRaw<TD> k_raw, v_raw;
@@ -513,8 +516,8 @@ linear_attention_outputs_kernel(const LcInput<TD> in, int q_off, int k_off, int 
   const int h = blockIdx.y, col0 = blockIdx.z * LC_DIM;
   int row0, n;
   lc_chunk(segment_start, num_segments, blockIdx.x, decay[h], pow_s, slot, row0, n);
+  pdl_wait();      // before any block leaves: a launch without chunks must not end ahead of the kernels before it
   if (n == 0) return;
-  pdl_wait();
   const int q_col = q_off + h * dim, k_col = k_off + h * dim, v_col = v_off + h * vdim + col0;
   {
     const auto one = [](int) { return 1.f; };
@@ -626,8 +629,8 @@ int linear_attention_chunks(const void* proj, int n_partials, long long partial_
   const size_t per_state = (size_t)heads * dim * vdim;
   lse_launch(linear_attention_own_states_kernel<TD>, grid, LC_THREADS, LC_OWN_SMEM, stream, in, k_off, v_off, decay, segment_start,
              chunk_state, heads, dim, vdim, max_segments);
-  lse_launch(linear_attention_carry_kernel, dim3((unsigned)((per_state + 255) / 256), max_segments), 256, 0, stream, decay, state,
-             segment_start, segment_slot, chunk_state, heads, dim, vdim, num_slots, LC_ROWS);
+  lse_launch(linear_attention_carry_kernel<16>, dim3((unsigned)((per_state + 255) / 256), max_segments), 256, 0, stream, decay, state,
+             segment_start, segment_slot, chunk_state, heads, dim, vdim, num_slots, LC_ROWS, LC_SHORT);
   lse_launch(linear_attention_outputs_kernel<TD>, grid, LC_THREADS, LC_OUT_SMEM, stream, in, q_off, k_off, v_off, decay,
              segment_start, (const float*)chunk_state, out, heads, dim, vdim, max_segments);
   LSE_LAUNCH_CHECK();
@@ -643,8 +646,14 @@ extern "C" int lse_linear_attention_scan(const void* proj, int proj_dtype, int n
       chunk_state != nullptr && max_chunks > 0 && n_partials >= 1 && (proj_dtype == LSE_DTYPE_F32 || proj_dtype == LSE_DTYPE_BF16)) {
 #define LSE_LC_ARGS proj, n_partials, partial_stride, ld, q_off, k_off, v_off, decay, state, segment_start, segment_slot, out, \
   max_segments, heads, dim, vdim, act, num_slots, chunk_state, max_chunks, stream
-    return proj_dtype == LSE_DTYPE_F32 ? linear_attention_chunks<float>(LSE_LC_ARGS) : linear_attention_chunks<__nv_bfloat16>(LSE_LC_ARGS);
+    const int err = proj_dtype == LSE_DTYPE_F32 ? linear_attention_chunks<float>(LSE_LC_ARGS)
+                                                : linear_attention_chunks<__nv_bfloat16>(LSE_LC_ARGS);
 #undef LSE_LC_ARGS
+    if (err != 0 || (max_segments == 1 && max_chunks > 1)) return err;      // one request of 64 rows or more: none is short
+    return linear_attention_scan_launch<MODE_PLAIN>(proj, proj_dtype, n_partials, partial_stride, ld, q_off, k_off, v_off,
+                                                    decay, state, segment_start, segment_slot, out, max_segments, heads,
+                                                    dim, vdim, act, num_slots, 0, nullptr, 0, nullptr, nullptr, 1.0f, 0, 1,
+                                                    nullptr, stream, LC_SHORT);
   }
   return linear_attention_scan_launch<MODE_PLAIN>(proj, proj_dtype, n_partials, partial_stride, ld, q_off, k_off, v_off,
                                                   decay, state, segment_start, segment_slot, out, max_segments, heads,

@@ -18,7 +18,8 @@ __device__ __forceinline__ float la_act(float z, int act) { return act == 1 ? z 
 // PARTS threads share a column (PARTS * 32 >= dim), CW = 32 / PARTS columns a warp, 4 * CW a block.
 //
 // A block's work item is a run of consecutive rows of one request:
-//   chunk_rows == 0: all rows of request blockIdx.x, from and into the request's state slot (few rows, decoding);
+//   chunk_rows == 0: all rows of request blockIdx.x, from and into the request's state slot (few rows, decoding;
+//     only_up_to > 0: requests of more rows than that are left alone);
 //   chunk_rows  > 0: the rows of every request are cut into chunks of chunk_rows rows, numbered request by request,
 //     and blockIdx.x is a chunk.  phase 1: from a zero state, no outputs, the chunk's own state goes to
 //     chunk_state[chunk].  phase 2: from chunk_state[chunk] (which linear_attention_carry_kernel has turned into the
@@ -47,7 +48,7 @@ linear_attention_scan_kernel(const TD* __restrict__ proj, int n_partials, long l
                              const int* __restrict__ segment_slot, float* __restrict__ out, int heads, int dim,
                              int vdim, int act, int num_slots, int num_segments, int chunk_rows, int phase,
                              float* __restrict__ chunk_state, const float* __restrict__ token_keep,
-                             const float* __restrict__ token_take, float q_scale, int norm_col, int qk_share) {
+                             const float* __restrict__ token_take, float q_scale, int norm_col, int qk_share, int only_up_to) {
   constexpr bool GATED = MODE == MODE_GATED;
   constexpr bool VECTOR = MODE == MODE_VECTOR;
   constexpr int CW = 32 / PARTS;
@@ -90,7 +91,7 @@ linear_attention_scan_kernel(const TD* __restrict__ proj, int n_partials, long l
     seg = item[0]; row0 = item[1]; row1 = item[2];
     if (seg < 0) return;
   }
-  if (row1 <= row0) return;
+  if (row1 <= row0 || (only_up_to > 0 && row1 - row0 > only_up_to)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int part = lane / CW, cb = warp * CW + lane % CW, col = col0 + cb;
   const float decay_h = MODE == MODE_PLAIN ? decay[h] : 1.f;
@@ -194,38 +195,46 @@ linear_attention_scan_kernel(const TD* __restrict__ proj, int n_partials, long l
 
 // Between the two phases: chunk_state[c] holds chunk c's own state (from zero); it becomes the state at the chunk's
 // start, S_start(c + 1) = decay^rows(c) * S_start(c) + own(c), beginning with the request's slot, which receives the
-// state after the request's last chunk.  One thread per element of (request, head, dim, vdim).
+// state after the request's last chunk.  One thread per element of (request, head, dim, vdim).  Requests of up to
+// short_rows rows have no chunks.  BATCH chunks' states are fetched together, then carried in order: sixteen over long
+// prompts (40 to 22 us at 32 chunks), eight for the scan's forms (64 requests of four rows, 32 heads of 64 x 64: a tenth less).
+__device__ __forceinline__ int la_chunks(int rows, int chunk_rows, int short_rows) {
+  return rows <= short_rows ? 0 : (rows + chunk_rows - 1) / chunk_rows;
+}
+template <int BATCH>
 __global__ void __launch_bounds__(256)
 linear_attention_carry_kernel(const float* __restrict__ decay, float* __restrict__ state,
                               const int* __restrict__ segment_start, const int* __restrict__ segment_slot,
                               float* __restrict__ chunk_state, int heads, int dim, int vdim, int num_slots,
-                              int chunk_rows) {
+                              int chunk_rows, int short_rows) {
   pdl_launch_dependents();
   pdl_wait();
   const int seg = blockIdx.y;
   const int a = segment_start[seg], b = segment_start[seg + 1];
-  if (b <= a) return;
+  const int chunks = la_chunks(b - a, chunk_rows, short_rows);
+  if (chunks <= 0) return;
   const size_t per_state = (size_t)heads * dim * vdim;
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int before = 0;      // chunks of the requests before: a warp adds them up (a thread alone took most of a step of many requests)
+  for (int s = threadIdx.x & 31; s < seg; s += 32) before += la_chunks(segment_start[s + 1] - segment_start[s], chunk_rows, short_rows);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
   if (e >= per_state) return;
-  int before = 0;
-  for (int s = 0; s < seg; ++s) before += (segment_start[s + 1] - segment_start[s] + chunk_rows - 1) / chunk_rows;
   const int h = (int)(e / ((size_t)dim * vdim));
   const float dk = decay[h];
   float full = 1.f;
   for (int i = 0; i < chunk_rows; ++i) full *= dk;
   float* slot = state + (size_t)LSE_CHECKED(segment_slot[seg], 0, num_slots, 0, LSE_CHECK_ROW) * per_state + e;
   float running = *slot;
-  const int chunks = (b - a + chunk_rows - 1) / chunk_rows;
   float last_power = 1.f;
   for (int i = 0; i < b - a - (chunks - 1) * chunk_rows; ++i) last_power *= dk;
   float* own = chunk_state + (size_t)before * per_state + e;
-  for (int c0 = 0; c0 < chunks; c0 += 16) {      // sixteen chunks' states are fetched together, then carried in order
-    float mine[16];
+  for (int c0 = 0; c0 < chunks; c0 += BATCH) {
+    float mine[BATCH];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) mine[i] = c0 + i < chunks ? own[(size_t)(c0 + i) * per_state] : 0.f;
+    for (int i = 0; i < BATCH; ++i) mine[i] = c0 + i < chunks ? own[(size_t)(c0 + i) * per_state] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < BATCH; ++i) {
       if (c0 + i < chunks) {
         own[(size_t)(c0 + i) * per_state] = running;
         running = fmaf(c0 + i == chunks - 1 ? last_power : full, running, mine[i]);
@@ -358,10 +367,11 @@ static int linear_attention_scan_launch(const void* proj, int proj_dtype, int n_
                                         int max_segments, int heads, int dim, int vdim, int act, int num_slots,
                                         int chunk_rows, float* chunk_state, int max_chunks, const float* token_keep,
                                         const float* token_take, float q_scale, int norm_col, int qk_share,
-                                        float* chunk_keep, cudaStream_t stream) {
+                                        float* chunk_keep, cudaStream_t stream, int only_up_to = 0) {
   if (max_segments <= 0) return 0;
   if (heads <= 0 || dim <= 0 || vdim <= 0 || dim > 8 * LA_DPT || heads > 65535) return LSE_ERR_BAD_ARGUMENT;
   if (qk_share <= 0 || heads % qk_share) return LSE_ERR_BAD_ARGUMENT;
+  if (only_up_to > 0 && chunk_rows) return LSE_ERR_BAD_ARGUMENT;
   if (chunk_rows < 0 || (chunk_rows > 0 && (chunk_state == nullptr || max_chunks <= 0))) return LSE_ERR_BAD_ARGUMENT;
   if (MODE == MODE_VECTOR && chunk_rows > 0 && chunk_keep == nullptr) return LSE_ERR_BAD_ARGUMENT;
   const int vs = vdim + (MODE == MODE_GATED && norm_col ? 1 : 0);
@@ -376,12 +386,12 @@ static int linear_attention_scan_launch(const void* proj, int proj_dtype, int n_
         lse_launch(linear_attention_scan_kernel<TD, P, false, MODE>, grid, LA_THREADS, 0, stream,                \
                    (const TD*)proj, n_partials, partial_stride, ld, q_off, k_off, v_off, decay, state,           \
                    segment_start, segment_slot, out, heads, dim, vdim, act, num_slots, max_segments, chunk_rows, \
-                   phase, chunk_state, token_keep, token_take, q_scale, norm_col, qk_share);                     \
+                   phase, chunk_state, token_keep, token_take, q_scale, norm_col, qk_share, only_up_to);         \
       else                                                                                                       \
         lse_launch(linear_attention_scan_kernel<TD, P, true, MODE>, grid, LA_THREADS, 0, stream,                 \
                    (const TD*)proj, n_partials, partial_stride, ld, q_off, k_off, v_off, decay, state,           \
                    segment_start, segment_slot, out, heads, dim, vdim, act, num_slots, max_segments, chunk_rows, \
-                   phase, chunk_state, token_keep, token_take, q_scale, norm_col, qk_share);                     \
+                   phase, chunk_state, token_keep, token_take, q_scale, norm_col, qk_share, only_up_to);         \
       if (chunk_rows && phase == 1) {                                                                            \
         const size_t per_state = (size_t)heads * dim * vs;                                                       \
         if (MODE == MODE_GATED)                                                                                  \
@@ -397,9 +407,9 @@ static int linear_attention_scan_launch(const void* proj, int proj_dtype, int n_
                      256, 0, stream, (const float*)chunk_keep, state, segment_start, segment_slot, chunk_state,  \
                      heads, dim, vs, num_slots, chunk_rows);                                                     \
         } else                                                                                                   \
-          lse_launch(linear_attention_carry_kernel, dim3((unsigned)((per_state + 255) / 256), max_segments),     \
+          lse_launch(linear_attention_carry_kernel<8>, dim3((unsigned)((per_state + 255) / 256), max_segments),  \
                      256, 0, stream, decay, state, segment_start, segment_slot, chunk_state, heads, dim, vdim,   \
-                     num_slots, chunk_rows);                                                                     \
+                     num_slots, chunk_rows, 0);                                                                  \
       }                                                                                                          \
     }                                                                                                            \
   }

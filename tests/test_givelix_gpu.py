@@ -562,6 +562,34 @@ def test_linear_attention_in_chunks_as_products(heads, dim, vdim, counts, dtype)
     assert float((device_state.cpu() - want_state)[good].abs().max()) <= 2e-5 * float(want_state[good].abs().max())
 
 
+@pytest.mark.parametrize("counts", [[32, 33, 1, 80, 3], [1] * 40, [5], [300] + [1] * 9, [32], [33]])
+def test_short_requests_beside_chunks_are_scanned_row_by_row(counts):
+    """Requests of up to 32 rows do not pay for a chunk of 64: beside longer ones and alone they give the row-by-row scan's bits,
+    outputs and states; the longer ones' agree with it up to rounding."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(len(counts))
+    heads, dim, vdim, rows = 2, 96, 130, sum(counts)
+    proj = torch.randn(rows, heads * (2 * dim + 2 * vdim)).bfloat16().cuda()
+    decay, first = torch.tensor([0.97, 0.5]).cuda(), torch.randn(len(counts), heads, dim, vdim).cuda()
+    starts = torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda()
+    slots = torch.arange(len(counts), dtype=torch.int32).flip(0).cuda()
+    results = []
+    for chunked in (False, True):
+        out, state = torch.full((rows, heads * vdim), float("nan"), device="cuda"), first.clone()
+        ops.linear_attention_scan(proj, 0, heads * dim, 2 * heads * dim, decay, state, starts, slots, out, heads, dim, vdim, "silu",
+                                  chunked=chunked)
+        results.append((out, state))
+    (want, want_state), (got, got_state) = results
+    for index, count in enumerate(counts):
+        mine, slot = slice(int(starts[index]), int(starts[index + 1])), int(slots[index])
+        if count <= 32:
+            assert torch.equal(got[mine], want[mine]) and torch.equal(got_state[slot], want_state[slot]), index
+        # sums of up to 300 rows of 96 products, each a few units of 2^-24 of the largest terms
+        assert float((got[mine] - want[mine]).abs().max()) <= 2e-5 * float(want[mine].abs().max()), index
+        assert float((got_state[slot] - want_state[slot]).abs().max()) <= 2e-5 * float(want_state[slot].abs().max()), index
+
+
 def test_residual_copies_update_and_norm():
     from llm_serving_engine_b200.kernels import ops
 
