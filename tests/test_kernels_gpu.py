@@ -158,6 +158,24 @@ def test_gemm_f32_sums_in_one_order_whatever_the_kernel(m, n, k):
     assert off <= 1 and float((got - want).abs().max()) <= 2.0 ** -20 * float(want.abs().max()), off
 
 
+@pytest.mark.parametrize("m, n, k", [(9, 31, 64), (16, 33, 100), (12, 129, 1540), (16, 2048, 1536), (13, 20000, 132), (16, 19000, 8)])
+def test_gemm_f32_of_nine_to_sixteen_rows_with_few_and_with_many_columns(m, n, k):
+    """One column a lane where blocks of 128 columns would be few, four where they are many: the bits of the many-rows kernel
+    either way, whole, with a bias and as a stack."""
+    torch.manual_seed(m + n + k)
+    many, w, bias = torch.randn(40, k, device=DEV), torch.randn(n, k, device=DEV), torch.randn(n, device=DEV)
+    a = many[3:3 + m].contiguous()
+    large, whole, biased = torch.empty(40, n, device=DEV), torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops().gemm_f32_nt(many, w, None, large)
+    ops().gemm_f32_nt(a, w, None, whole)
+    ops().gemm_f32_nt(a, w, bias, biased)
+    assert torch.equal(whole, large[3:3 + m]) and torch.equal(biased, whole + bias)
+    total = torch.zeros(m, n, device=DEV)
+    for part in ops().gemm_f32_stack(a, w):
+        total += part
+    assert torch.equal(total, whole)
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 64, 64), (8, 1536, 8960), (3, 100, 1536), (16, 257, 520), (5, 96, 4100)])
 def test_gemm_f32_as_a_stack_of_range_sums(m, n, k):
     """Few rows as a stack of partial sums (a block per k range): added up in index order from zero, the stack gives
