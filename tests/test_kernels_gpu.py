@@ -176,6 +176,15 @@ def test_gemm_f32_of_nine_to_sixteen_rows_with_few_and_with_many_columns(m, n, k
     assert torch.equal(total, whole)
 
 
+def test_gemm_f32_of_more_columns_than_a_grid_has_rows():
+    """65,537 tiles of columns and more, whichever tile is taken: a row of unaligned length, and eighteen rows."""
+    for m, n, k in ((1, 65536 * 128 + 5, 5), (18, 65536 * 64 + 1, 4)):
+        a, w, out = torch.randn(m, k, device=DEV), torch.randn(n, k, device=DEV), torch.empty(m, n, device=DEV)
+        ops().gemm_f32_nt(a, w, None, out)
+        for cols in (slice(0, 300), slice(n - 300, n)):
+            assert float((out[:, cols].double() - a.double() @ w[cols].double().t()).abs().max()) <= 1e-5
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 64, 64), (8, 1536, 8960), (3, 100, 1536), (16, 257, 520), (5, 96, 4100)])
 def test_gemm_f32_as_a_stack_of_range_sums(m, n, k):
     """Few rows as a stack of partial sums (a block per k range): added up in index order from zero, the stack gives
