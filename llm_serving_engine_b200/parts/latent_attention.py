@@ -19,7 +19,9 @@ PER_HEAD_LIBRARY_ROWS = 32    # above this many bfloat16 rows the per-head produ
 # per head around the latter, 19 us, are saved too).  Both write into buffers of the step.
 EXPAND_FLOPS, EXPANDED_FLOPS, LATENT_FLOPS = 1.0e9, 4.0e8, 1.2e8
 EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an attention of few blocks
-EXPAND_MAX_BYTES = 1 << 30    # of keys and values that are held at once (8 KB a row at 16 heads)
+# Keys and values that are held at once (8 KB a row at 16 heads).  They are taken in the middle of a step, beside a cache that
+# was sized before: no more than the buffers of a step of a few thousand rows over the latent rows take.
+EXPAND_MAX_BYTES = 1 << 28
 
 
 def _size_class(rows: int) -> int:

@@ -36,6 +36,7 @@ def test_a_layer_that_stops_expanding_its_latents_changes_the_key():
     counts = [256] * 8
     short, long = (model.launch_signature(counts, [context] * 8) for context in (2304, 20000))
     rows = [[block.mixer._expanded_rows(counts, [context] * 8) for block in model.blocks] for context in (2304, 20000)]
+    assert 2 * rows[0][0] * model.blocks[0].mixer.kv_up.shape[0] <= 1 << 28      # bytes of keys and values
     assert rows[0][0] == rows[0][1] == rows[1][0] > 0 and rows[1][1] == 0      # the layers' answers as a set are the same
     assert short != long
     assert model.launch_signature([256], [768]) != latent_model([0, 2048]).launch_signature([256], [20000])
