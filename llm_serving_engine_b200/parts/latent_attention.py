@@ -161,7 +161,7 @@ class LatentAttention(Mixer):
     def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
         the latent rows.  ``contexts``: keys of each request after the step."""
-        if min(segment_counts) == 1 or self.gates > self.heads or not ops.attention_expanded_supported(
+        if min(segment_counts) == 1 or self.gates > self.heads or not self.scale > 0.0 or not ops.attention_expanded_supported(
                 self.dim, self.rot_dim, self.vdim, self.rank, self.ctx.dtype):
             return 0
         tile, rows, pairs = ops.attention_expanded_tile(), 0, 0

@@ -48,6 +48,13 @@ def test_the_order_of_the_answers_is_part_of_the_key():
         assert a.launch_signature([256], contexts) != b.launch_signature([256], contexts)
 
 
+def test_scales_that_the_expanded_attention_refuses_go_over_the_latent_rows():
+    """Its maximum is taken before the scale; over the latent rows any scale is taken, zero and negative ones too."""
+    counts, contexts = [512], [512]
+    for scale, expanded in ((0.05, True), (0.0, False), (-0.05, False)):
+        assert (latent_model([0], scale=scale).blocks[0].mixer._expanded_rows(counts, contexts) > 0) == expanded, scale
+
+
 def test_layers_without_an_answer_leave_the_key_empty():
     assert latent_model([0, 512]).launch_signature([1, 1], [700, 20]) == ()
 
