@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import gc
 import os
+from collections import OrderedDict
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -130,6 +131,9 @@ class StepRunner:
     PORTION_BUCKETS = (16, 32, 48, 64, 96, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024, 1280, 1536, 2048,
                        2560, 3072, 4096, 5120, 6144, 8192)
     PORTION_REQUEST_BUCKETS = (1, 8, 32, 128, 256)
+    # Captured steps with prompt portions that are kept: what mixers launch by the requests' contexts multiplies the classes, and
+    # every graph holds its nodes and buffers.  The one that was not used for longest goes first.
+    MAX_PORTION_GRAPHS = 256
 
     def __init__(self, model, cache: CacheManager, max_tokens_per_step: int, max_segments: int,
                  use_graphs: bool = True) -> None:
@@ -155,8 +159,8 @@ class StepRunner:
         self._capture_stream = None
         self._arange = np.arange(max(self.GRAPH_BUCKETS), dtype=np.int32)
         self.graph_portions = os.environ.get("LSE_PORTION_GRAPHS", "1") != "0"
-        self._portion_classes_seen: dict = {}
-        self._portion_graphs: dict = {}
+        self._portion_classes_seen: dict = {}     # classes that were met once and are not captured yet
+        self._portion_graphs: OrderedDict = OrderedDict()      # the one used last is the last one
         self.portion_graph_replays = 0
         self.steps_run = 0
         self.graph_replays = 0
@@ -405,12 +409,18 @@ class StepRunner:
         key = ("portions", tokens, segments, places, self._graph_width(self._pages_after(entries)), signature)
         slot = self._portion_graphs.get(key)
         if slot is None:
-            seen = self._portion_classes_seen.get(key, 0) + 1
-            self._portion_classes_seen[key] = seen
-            if seen < 2:
+            if self._portion_classes_seen.pop(key, None) is None:
+                self._portion_classes_seen[key] = True
+                if len(self._portion_classes_seen) > 16 * self.MAX_PORTION_GRAPHS:
+                    self._portion_classes_seen.pop(next(iter(self._portion_classes_seen)))
                 return None
+            if len(self._portion_graphs) >= self.MAX_PORTION_GRAPHS:
+                torch.cuda.current_stream().synchronize()      # it may still run, or its buffers be on their way
+                self._portion_graphs.popitem(last=False)
             slot = _Graph(_Layout(tokens, segments, places, key[4], self._groups), self.device, True)
             self._portion_graphs[key] = slot
+        else:
+            self._portion_graphs.move_to_end(key)
         if self._copy_pending:
             self._copied.synchronize()
             self._copy_pending = False

@@ -25,8 +25,10 @@ EXPAND_MAX_BYTES = 1 << 28
 
 
 def _size_class(rows: int) -> int:
-    """``rows`` rounded up to a quarter of a power of two (captured steps are kept by it)."""
-    step = max(64, 1 << max(0, (rows - 1).bit_length() - 3))
+    """``rows`` rounded up to half a power of two: captured steps are kept by it, so a prompt in portions meets two classes for
+    every doubling of its context (four had nearly every portion captured anew), and the product makes at most half as many
+    rows again as there are.  Steps launched one by one make the rows that there are."""
+    step = max(64, 1 << max(0, (rows - 1).bit_length() - 2))
     return -(-rows // step) * step
 
 _DEFAULT_NAMES = {"q_down": "dq", "q_down_norm": "dq.norm", "q_up": "uq", "q": "q", "kv_down": "dkv",
@@ -158,18 +160,21 @@ class LatentAttention(Mixer):
     def cache_requirement(cls, params, hidden_size):
         return PagedLatent(int(params["kv_rank"]) + int(params["rot_dim"]), int(params.get("window", 0)))
 
+    def _gathered_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
+        """Latent rows that a step of this shape may read, each request's rounded up to whole key tiles."""
+        tile = ops.attention_expanded_tile()
+        return sum(-(-(context - (max(0, context - count + 1 - self.window) if self.window > 0 else 0)) // tile) * tile
+                   for count, context in zip(segment_counts, contexts))
+
     def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
         the latent rows.  ``contexts``: keys of each request after the step."""
         if min(segment_counts) == 1 or self.gates > self.heads or not self.scale > 0.0 or not ops.attention_expanded_supported(
                 self.dim, self.rot_dim, self.vdim, self.rank, self.ctx.dtype):
             return 0
-        tile, rows, pairs = ops.attention_expanded_tile(), 0, 0
-        for count, context in zip(segment_counts, contexts):
-            first = max(0, context - count + 1 - self.window) if self.window > 0 else 0
-            rows += -(-(context - first) // tile) * tile
-            pairs += count * (min(context, self.window) if self.window > 0 else context - count // 2)
-        rows = _size_class(rows)
+        pairs = sum(count * (min(context, self.window) if self.window > 0 else context - count // 2)
+                    for count, context in zip(segment_counts, contexts))
+        rows = _size_class(self._gathered_rows(segment_counts, contexts))
         expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
                     + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
         latent = 2.0 * pairs * self.heads * (2 * self.rank + self.rot_dim) / LATENT_FLOPS
@@ -235,9 +240,10 @@ class LatentAttention(Mixer):
             queries = linear_partials(q_latent, self.q_up) if self.q_rank else proj
             ops.latent_query(queries, 0, heads, self.dim, self.rot_dim, self.rot_dims, self.freq, self.rot_factor,
                              step.positions, step.segment_of_token, q_plain, q_wide, self.rank)
-        expanded = (0 if step.decode_only else
-                    self._expanded_rows([segment.count for segment in step.segments],
-                                        [segment.first_position + segment.count for segment in step.segments]))
+        shape = ([segment.count for segment in step.segments], [segment.first_position + segment.count for segment in step.segments])
+        expanded = 0 if step.decode_only else self._expanded_rows(*shape)
+        if expanded and not torch.cuda.is_current_stream_capturing():
+            expanded = self._gathered_rows(*shape)
         if expanded:
             values = self._expanded_attention(q_plain, q_wide, step, cache, gate, expanded)
             return linear_partials(values.view(tokens, heads * self.vdim), self.out_weight)

@@ -48,6 +48,19 @@ def test_the_order_of_the_answers_is_part_of_the_key():
         assert a.launch_signature([256], contexts) != b.launch_signature([256], contexts)
 
 
+def test_a_long_prompt_in_portions_meets_few_classes():
+    """Contexts of a prompt of 16,384 keys in portions of 512: at most two keys for every doubling, and room for all rows."""
+    model = latent_model([0])
+    mixer = model.blocks[0].mixer
+    keys = set()
+    for context in range(512, 16385, 512):
+        key = model.launch_signature([512], [context])
+        keys.add(key)
+        rows, exact = mixer._expanded_rows([512], [context]), mixer._gathered_rows([512], [context])
+        assert key == ((0, ("expanded", rows)),) and exact == context <= rows <= 1.5 * exact
+    assert len(keys) <= 2 * 5 + 1
+
+
 def test_scales_that_the_expanded_attention_refuses_go_over_the_latent_rows():
     """Its maximum is taken before the scale; over the latent rows any scale is taken, zero and negative ones too."""
     counts, contexts = [512], [512]

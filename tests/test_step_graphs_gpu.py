@@ -46,3 +46,20 @@ def test_a_captured_step_is_not_replayed_where_a_layer_launches_something_else(m
         # bfloat16 at other places of two layers: a few units in the last place of the largest logit
         assert float((got - want[index]).abs().max()) <= 2.0 ** -4 * float(want[index].abs().max()), index
     assert graphs.portion_graph_replays >= 4
+
+
+def test_captured_steps_beyond_the_bound_make_room_for_each_other():
+    """Three classes of steps in turn where two graphs are kept: captured, dropped, captured again, and always the same logits;
+    the class used last stays."""
+    model = latent_model([0], heads=1, rank=64, device="cuda", scale=0.07)
+    generator = torch.Generator().manual_seed(7)
+    prompts = [torch.randint(0, 64, (length,), generator=generator).tolist() for length in (16, 30, 45)]
+    plain, graphs = runner_for(model, use_graphs=False), runner_for(model, use_graphs=True)
+    graphs.MAX_PORTION_GRAPHS = 2
+    want = [in_portions(plain, "r", tokens, 64) for tokens in prompts]
+    for index in (0, 0, 1, 1, 0, 2, 2, 0, 1, 1, 1, 2, 2, 2, 0):
+        got = in_portions(graphs, "r", prompts[index], 64)
+        assert float((got - want[index]).abs().max()) <= 2.0 ** -5 * float(want[index].abs().max()), index
+        assert len(graphs._portion_graphs) <= 2
+    assert [key[1] for key in graphs._portion_graphs] == [32, 48] or [key[1] for key in graphs._portion_graphs] == [48, 32]
+    assert graphs.portion_graph_replays >= 6
