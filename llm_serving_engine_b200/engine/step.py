@@ -614,8 +614,8 @@ class StepRunner:
     def warmup(self, batch_sizes=None) -> None:
         """Capture the decode graphs of the given batch sizes (default: every bucket up to
         ``max_segments``) with temporary one-token requests, then give their pages back.  Before that, one
-        step with a prompt portion as long as a step may be, beside a single token of another request: the
-        library's products and the prompt kernels load and configure themselves at their first use, which
+        step with a prompt portion as long as a step may be, beside a single token of another request (and one without it, where
+        a portion alone goes to other kernels): the library's products and the prompt kernels load and configure themselves at their first use, which
         would otherwise cost the first request a tenth of a second."""
         self._warm_prompt_path()
         if not self.use_graphs:
@@ -641,16 +641,25 @@ class StepRunner:
         tokens = min(self.max_tokens - 1, self.model.spec.max_position_embeddings - 1, room - cache.page_size)
         if tokens < 2 or self.max_segments < 2:
             return
-        names = ["__warmup_portion", "__warmup_token"]
-        try:
-            for name in names:
-                cache.create(name)
-            self.run([StepEntry(names[0], [0] * tokens, [tokens - 1]), StepEntry(names[1], [0], [0])])
-            torch.cuda.current_stream().synchronize()
-        finally:
-            for name in names:
-                if name in cache.requests:
-                    cache.free(name)
+        portion, token = (StepEntry("__warmup_portion", [0] * tokens, [tokens - 1]), StepEntry("__warmup_token", [0], [0]))
+        steps = [[portion, token]]
+        if hasattr(self.model, "launch_signature"):
+            def kinds(entries):
+                counts = [len(entry.tokens) for entry in entries]
+                return {(index, answer[:1]) for index, answer in self.model.launch_signature(counts, counts)}
+
+            if not kinds([portion]) <= kinds(steps[0]):      # a portion alone goes to kernels of its own
+                steps.append([portion])
+        for entries in steps:
+            try:
+                for entry in entries:
+                    cache.create(entry.request_id)
+                self.run(entries)
+                torch.cuda.current_stream().synchronize()
+            finally:
+                for entry in entries:
+                    if entry.request_id in cache.requests:
+                        cache.free(entry.request_id)
 
     def finish(self, entries: list[StepEntry]) -> None:
         """After the step: give back pages that a window has passed."""

@@ -48,6 +48,25 @@ def test_a_captured_step_is_not_replayed_where_a_layer_launches_something_else(m
     assert graphs.portion_graph_replays >= 4
 
 
+def test_warmup_runs_the_kernels_of_a_portion_alone(monkeypatch):
+    """A latent layer's portion alone goes over expanded keys and values, beside a single token over the latent rows: both are run
+    once before the first request, and the cache is left empty."""
+    from llm_serving_engine_b200.kernels import ops
+
+    calls = []
+    for name in ("attention_expanded", "latent_attention"):
+        def recorded(*args, _real=getattr(ops, name), _name=name, **more):
+            calls.append(_name)
+            return _real(*args, **more)
+
+        monkeypatch.setattr(ops, name, recorded)
+    monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0)
+    runner = runner_for(latent_model([0], heads=1, rank=64, device="cuda", scale=0.07), use_graphs=True, segments=2)
+    runner.warmup()
+    assert calls[:2] == ["latent_attention", "attention_expanded"] and not runner.cache.requests
+    assert runner.cache.groups[0].pool.used_pages == 0
+
+
 def test_captured_steps_beyond_the_bound_make_room_for_each_other():
     """Three classes of steps in turn where two graphs are kept: captured, dropped, captured again, and always the same logits;
     the class used last stays."""
