@@ -19,6 +19,7 @@
 //
 // Every wait is bounded (see tcgen05.cuh); lse_attention_expanded_status() reports one that gave up, and contexts on the
 // device that ask for more rows than the host made room for (the rows beyond would be zeros, and count as keys).
+#include "smem_allowance.cuh"
 #include "tcgen05.cuh"
 
 LSE_CHECK_DEFINE(lse_check_attention_expanded)
@@ -448,19 +449,16 @@ extern "C" int lse_attention_expanded(const void* q_plain, const void* q_wide, c
   if (heads <= 0 || capacity <= 0 || !(scale > 0.f) || !lse_attention_expanded_supported(D, ROT, D, rank) ||
       (((uintptr_t)q_plain | (uintptr_t)q_wide | (uintptr_t)rows | (uintptr_t)kv | (uintptr_t)out) & 15))
     return LSE_ERR_BAD_ARGUMENT;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(attn_expanded_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  static SmemAllowance allowed;
+  cudaError_t err = allow_smem(attn_expanded_tc_kernel, SMEM, allowed);
+  if (err != cudaSuccess) return (int)err;
   CUtensorMap map_q, map_qr, map_kv, map_kr;
   if (!make_map_3d(&map_q, q_plain, tokens, heads, D, BM) || !make_map_3d(&map_qr, q_wide, tokens, heads, rank + ROT, BM) ||
       !make_map_3d(&map_kv, kv, capacity, 2 * heads, D, BN) || !make_map_2d(&map_kr, rows, capacity, rank + ROT, BN))
     return LSE_ERR_BAD_ARGUMENT;
   const long long blocks = ((long long)(tokens + BM - 1) / BM + num_segments) * heads;      // every request may end with a partial tile
   if (blocks > 0x7fffffffLL) return LSE_ERR_TOO_LARGE;
-  cudaError_t err = lse_launch(attn_expanded_tc_kernel, (unsigned)blocks, THREADS, SMEM, stream, map_q, map_qr, map_kv, map_kr,
+  err = lse_launch(attn_expanded_tc_kernel, (unsigned)blocks, THREADS, SMEM, stream, map_q, map_qr, map_kv, map_kr,
                                (__nv_bfloat16*)out, segment_start, segment_first_pos, segment_context, num_segments, heads, rank,
                                scale * LOG2E, window, sink, out_gate);
   if (err != cudaSuccess) return (int)err;

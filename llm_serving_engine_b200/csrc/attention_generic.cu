@@ -23,6 +23,7 @@
 //
 // Cache layout: [page][kv head][offset in page][D].
 #include "common.cuh"
+#include "smem_allowance.cuh"
 
 LSE_CHECK_DEFINE(lse_check_attention_generic)
 
@@ -568,20 +569,12 @@ paged_attention_generic_merge_kernel(const float* __restrict__ partials, T* __re
 size_t rows_smem(int D) { return sizeof(float) * ((size_t)GC * D + 2 * (size_t)CHUNK * (D + 4) + CHUNK * GC + 2 * GC); }
 size_t tiles_smem(int DT) { return sizeof(float) * ((size_t)(ROWS + 2 * CHUNK) * (DT + 4) + 4 * ROWS); }
 
-template <typename Kernel>
-cudaError_t allow_smem(Kernel kernel, size_t bytes, bool& done) {      // once per process (not repeated while a stream is captured)
-  if (done) return cudaSuccess;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  done = err == cudaSuccess;
-  return err;
-}
-
 template <typename T, bool SPLIT, bool VEC>
 cudaError_t launch_rows(const void* q, const void* k, const void* v, void* out, const Step& p, int rows, float* partials,
                         int max_chunks, cudaStream_t stream) {
   auto kernel = paged_attention_generic_kernel<T, SPLIT, VEC>;
-  static bool done = false;
-  cudaError_t err = allow_smem(kernel, rows_smem(MAX_D), done);
+  static SmemAllowance allowed;
+  cudaError_t err = allow_smem(kernel, rows_smem(MAX_D), allowed);
   if (err != cudaSuccess) return err;
   const int gchunks = (p.n_q / p.n_kv + GC - 1) / GC;
   const dim3 grid((unsigned)((long long)rows * gchunks * (SPLIT ? max_chunks : 1)), p.n_kv);
@@ -593,8 +586,8 @@ template <typename T, int DT, bool SPLIT, bool VEC>
 cudaError_t launch_tiles(const void* q, const void* k, const void* v, void* out, const Step& p, const int* segment_first,
                          int tiles, float* partials, int max_chunks, cudaStream_t stream) {
   auto kernel = paged_attention_tiles_kernel<T, DT, SPLIT, VEC>;
-  static bool done = false;
-  cudaError_t err = allow_smem(kernel, tiles_smem(DT), done);
+  static SmemAllowance allowed;
+  cudaError_t err = allow_smem(kernel, tiles_smem(DT), allowed);
   if (err != cudaSuccess) return err;
   const int group = p.n_q / p.n_kv, heads = group < ROWS ? group : ROWS, gchunks = (group + heads - 1) / heads;
   const dim3 grid((unsigned)((long long)tiles * gchunks * (SPLIT ? max_chunks : 1)), p.n_kv);

@@ -12,6 +12,7 @@
 // partial sums.
 //
 // Both kernels bring their tiles through a ring of shared-memory stages with cp.async.
+#include "smem_allowance.cuh"
 #include "tcgen05.cuh"
 
 // Length of a k range: an eighth of K rounded up to a multiple of 64.
@@ -354,19 +355,11 @@ struct Product {
   int ranges;      // 1: the kernel adds the ranges up
 };
 
-template <typename Kernel>
-cudaError_t allow_smem(Kernel kernel, size_t bytes, size_t& allowed) {
-  if (bytes <= allowed) return cudaSuccess;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err == cudaSuccess) allowed = bytes;
-  return err;
-}
-
 template <int BM, int BN, int WM, int WN, int TM, int TN, bool IN_TMEM>
 cudaError_t launch_tiles(const Product& p, cudaStream_t stream) {
   auto kernel = gemm_f32_tiles_kernel<BM, BN, WM, WN, TM, TN, IN_TMEM>;
   const size_t smem = sizeof(float) * STAGES * BK * (BM + BN + 8);
-  static size_t allowed = 48 * 1024;
+  static SmemAllowance allowed;
   cudaError_t err = allow_smem(kernel, smem, allowed);
   if (err != cudaSuccess) return err;
   const long long blocks = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
@@ -383,7 +376,7 @@ cudaError_t launch_few(const Product& p, cudaStream_t stream) {
   const int length = p.ranges > 1 ? f32_range(p.K) : p.K;
   const int tiles = (length + FEW_BK - 1) / FEW_BK, stages = tiles < FEW_STAGES ? tiles : FEW_STAGES;
   const size_t smem = sizeof(float) * stages * (COLS * (FEW_BK + 4) + ROWS * FEW_BK);
-  static size_t allowed = 48 * 1024;
+  static SmemAllowance allowed;
   cudaError_t err = allow_smem(kernel, smem, allowed);
   if (err != cudaSuccess) return err;
   const dim3 grid((p.N + COLS - 1) / COLS, p.ranges);

@@ -12,6 +12,7 @@
 // memory a few at a time.  Everything is float32: the projections arrive in float32, in bfloat16 or as a
 // stack of float32 partial sums, and are activated in float32.
 #include "common.cuh"
+#include "smem_allowance.cuh"
 
 LSE_CHECK_DEFINE(lse_check_linear_attention)
 
@@ -614,14 +615,10 @@ int linear_attention_chunks(const void* proj, int n_partials, long long partial_
                             int v_off, const float* decay, float* state, const int* segment_start, const int* segment_slot,
                             float* out, int max_segments, int heads, int dim, int vdim, int act, int num_slots,
                             float* chunk_state, int max_chunks, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(linear_attention_own_states_kernel<TD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LC_OWN_SMEM);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(linear_attention_outputs_kernel<TD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LC_OUT_SMEM);
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  static SmemAllowance own_allowed, out_allowed;
+  cudaError_t err = allow_smem(linear_attention_own_states_kernel<TD>, LC_OWN_SMEM, own_allowed);
+  if (err == cudaSuccess) err = allow_smem(linear_attention_outputs_kernel<TD>, LC_OUT_SMEM, out_allowed);
+  if (err != cudaSuccess) return (int)err;
   const bool wide = n_partials == 1 && (((uintptr_t)proj) & (4 * sizeof(TD) - 1)) == 0 && ld % 4 == 0 && q_off % 4 == 0 &&
                     k_off % 4 == 0 && v_off % 4 == 0 && dim % 4 == 0 && vdim % 4 == 0;
   const LcInput<TD> in = {(const TD*)proj, n_partials, partial_stride, ld, act, wide ? 1 : 0};

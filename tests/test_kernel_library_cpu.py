@@ -2,6 +2,7 @@
 includes, and a model names the sources of its parts and no others."""
 import ctypes
 import re
+import subprocess
 
 import pytest
 import torch
@@ -80,3 +81,33 @@ def test_libraries_share_the_switch_of_dependent_launches():
     paths = build.library_paths(["elementwise", "tanh_norm"], verbose=False)
     places = {ctypes.addressof(ctypes.c_int.in_dll(ctypes.CDLL(str(path)), "lse_pdl_enabled")) for path in paths.values()}
     assert len(places) == 1
+
+
+def test_shared_memory_is_allowed_on_every_device_and_never_lowered(tmp_path):
+    """The table that kernels of more than 48 KB of shared memory are kept in, compiled here with calls that are counted in
+    place of the runtime's: once per device, again for more, not for less, again after an error, and from eight threads at once
+    never down."""
+    (tmp_path / "trial.cpp").write_text('''
+#include <cstddef>
+#include <thread>
+#include <vector>
+#include "smem_allowance.cuh"
+static SmemAllowance one, many;
+static int calls = 0;
+extern "C" int raise_(int device, int bytes, int err) { int before = calls; one.raise(device, bytes, [&](int) { ++calls; return err; }); return calls - before; }
+extern "C" int together() {
+  int limit = 0, lowered = 0;      // both under the table's lock
+  std::vector<std::thread> threads;
+  for (int t = 0; t < 8; ++t)
+    threads.emplace_back([&, t] { for (int i = 0; i < 1000; ++i) many.raise(0, 50000 + (i * 37 + t * 101) % 5000, [&](int most) { lowered += most < limit; limit = most; return 0; }); });
+  for (auto& thread : threads) thread.join();
+  return lowered;
+}
+''')
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-pthread", f"-I{build.CSRC}", str(tmp_path / "trial.cpp"), "-o",
+                    str(tmp_path / "trial.so")], check=True)
+    trial = ctypes.CDLL(str(tmp_path / "trial.so"))
+    for device, bytes_, err, calls in ((0, 49152, 0, 0), (0, 70000, 0, 1), (0, 70000, 0, 0), (1, 70000, 0, 1), (0, 60000, 0, 0),
+                                       (0, 90000, 7, 1), (0, 90000, 0, 1), (1, 90000, 0, 1), (1, 90000, 0, 0), (70, 90000, 0, 1)):
+        assert trial.raise_(device, bytes_, err) == calls, (device, bytes_, err)
+    assert trial.together() == 0
