@@ -15,11 +15,11 @@
 // result is the same bit for bit whatever else is in the batch, however the prompt was cut and whichever kernel ran.
 //
 // Three kernels:
-//   rows    a block takes one row and up to GC query heads that share a key/value head (decoding): one chunk, whose
-//           partial result it leaves in global memory, or (many rows) all chunks of its row;
+//   rows    a block takes one row and up to GC query heads that share a key/value head (decoding): some of its chunks, whose
+//           partial results it leaves in global memory, or (many rows) all chunks of its row;
 //   tiles   a block takes ROWS (token, query head) pairs of one key/value head, the tokens neighbouring rows of one
-//           request (prompts): all chunks, or one chunk, as above;
-//   merge   adds up the chunks that blocks of one chunk left.
+//           request (prompts): all chunks, or some, as above;
+//   merge   adds up the chunks that several blocks left.
 //
 // Cache layout: [page][kv head][offset in page][D].
 #include "common.cuh"
@@ -34,6 +34,10 @@ constexpr int THREADS = 128;  // 4 warps
 constexpr int MAX_D = 256;
 constexpr int ROWS = 64;      // (token, head) pairs per block of the tiles kernel
 constexpr int TILES_MAX_D = 128;
+// About so many blocks share the chunks of a launch, sixteen an SM.  float32, 64 requests, 12 / 2 heads of 128, a block a
+// chunk against 1,184, 2,368 and 9,472 blocks: 2,000 keys 106 against 90, 88 and 93 us; 100 keys in tables of 16,384 50
+// against 15, 17 and 24 us; 8 heads of 64: 155 against 143, 126 and 130 us, 140 against 16, 17 and 23 us.
+constexpr long long SPLIT_BLOCKS = 2368;
 
 // Merge a chunk's (m, l) into the running (M, L); wa and wb are the factors for the outputs.
 __device__ __forceinline__ void merge_chunk(float& M, float& L, float m, float l, float& wa, float& wb) {
@@ -104,6 +108,7 @@ struct Step {      // what the kernels take from the step
   float scale;
   int window;
   int skip;                       // rows kernel and merge: see which_row
+  int max_chunks, parts;          // SPLIT: chunks that a row's partial results have room for; blocks that share them
 };
 enum { ALL_ROWS = 0, SINGLE_ROWS = 1, ROWS_OF_PORTIONS = 2 };
 
@@ -121,6 +126,14 @@ __device__ __forceinline__ int which_row(const Step& p, int index, int& seg) {
   return index;
 }
 
+// SPLIT: the block of number `part` takes every parts-th of the chunks lo .. hi of its rows: lo becomes its first one.
+// (The chunks of a row are known on the device only: with a block for every chunk that the block tables have room for, 64
+// rows of 100 keys in tables of 16,384 made 16,384 blocks at two key/value heads, nearly all of them without work.)
+__device__ __forceinline__ void my_chunks(const Step& p, int part, int& lo, int& hi) {
+  hi = min(hi, p.max_chunks - 1);
+  lo += (part - lo % p.parts + p.parts) % p.parts;
+}
+
 // ---------------------------------------------------------------- rows
 // Element offset of key j of the request in the cache.
 __device__ __forceinline__ long long key_offset(const Step& p, const int* bt, int kv_head, int j) {
@@ -128,7 +141,7 @@ __device__ __forceinline__ long long key_offset(const Step& p, const int* bt, in
   return (((long long)page * p.n_kv + kv_head) * p.page_size + (j % p.page_size)) * p.head_dim;
 }
 
-// grid (rows * head chunks * chunks, kv heads).  SPLIT: the block takes one chunk and writes acc [D], m, l of it and its
+// grid (rows * head chunks * parts, kv heads).  SPLIT: the block takes some chunks and writes acc [D], m, l of each and its
 // heads to `partials` [row][head][chunk][D + 2].  Else it merges all chunks of its row and writes `out`.
 // The chunk's keys and values (2 x 33 KB at 128 values of float32) are asked for at once; scores: a lane owns two keys and
 // two heads, sums: two columns and four heads, which keeps the register writes from shared memory, 128 bytes a clock,
@@ -136,7 +149,7 @@ __device__ __forceinline__ long long key_offset(const Step& p, const int* bt, in
 template <typename T, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__(THREADS)
 paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                               T* __restrict__ out, const Step p, float* __restrict__ partials, int max_chunks, int rows) {
+                               T* __restrict__ out, const Step p, float* __restrict__ partials, int rows) {
   extern __shared__ __align__(16) float smem[];
   pdl_launch_dependents();
   pdl_wait();
@@ -153,9 +166,8 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
   const int kv_begin = p.window > 0 ? max(0, pos + 1 - p.window) : 0;
   int chunk_lo = kv_begin / CHUNK, chunk_hi = pos / CHUNK;
   if (SPLIT) {
-    const int mine = rest / gchunks;
-    if (mine < chunk_lo || mine > chunk_hi) return;
-    chunk_lo = chunk_hi = mine;
+    my_chunks(p, rest / gchunks, chunk_lo, chunk_hi);
+    if (chunk_lo > chunk_hi) return;
   }
   const int* bt = p.block_tables + (size_t)seg * p.bt_stride;
   const int D = p.head_dim, pitch = D + 4;
@@ -180,7 +192,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 #pragma unroll
     for (int i = 0; i < 4; ++i) total[g][i] = 0.f;
   }
-  for (int chunk = chunk_lo; chunk <= chunk_hi; ++chunk) {
+  for (int chunk = chunk_lo; chunk <= chunk_hi; chunk += SPLIT ? p.parts : 1) {
     const int first_key = chunk * CHUNK;
     if (tid < CHUNK) {      // (read by the fills of the chunk before, which all threads have left)
       const int j = first_key + tid;
@@ -253,7 +265,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
       if (h0 + g >= gcount) continue;
       const float m = stat_s[h0 + g], l = stat_s[GC + h0 + g];
       if (SPLIT) {
-        float* dst = partials + (((size_t)index * p.n_q + first_head + h0 + g) * max_chunks + chunk) * (D + 2);
+        float* dst = partials + (((size_t)index * p.n_q + first_head + h0 + g) * p.max_chunks + chunk) * (D + 2);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int col = 2 * (tid % 64) + 128 * (i / 2) + i % 2;
@@ -282,15 +294,15 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ k_
 // ---------------------------------------------------------------- tiles
 // A block's rows are pairs (token, head): pair r is token r / heads and head r % heads of the tile, heads = min(group, ROWS)
 // query heads that share the key/value head, so that its keys are read once for all of them and a short portion still
-// fills a tile.  grid (tiles of tokens * head chunks * (SPLIT ? chunks : 1), kv heads).
+// fills a tile.  grid (tiles of tokens * head chunks * (SPLIT ? parts : 1), kv heads).
 // Scores: a thread owns 8 rows x 4 keys, sums: 8 rows x TN columns; a chunk's two products are bounded by the register
 // writes from shared memory about as much as by the multiply-adds.  Keys and weights share a buffer, which leaves room
 // for two blocks an SM (102 KB each at 128 values): one loads while the other multiplies.
 template <typename T, int DT, bool SPLIT, bool VEC>
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(THREADS, SPLIT && DT <= 64 ? 4 : 2)
 paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                              T* __restrict__ out, const Step p, const int* __restrict__ segment_first,
-                             float* __restrict__ partials, int max_chunks, int tiles) {
+                             float* __restrict__ partials, int tiles) {
   constexpr int TN = DT / 16;                 // columns of a thread: 4 (up to 64 values) or 8, in groups of four
   constexpr int PITCH = DT + 4, P_PITCH = CHUNK + 4;
   extern __shared__ __align__(16) float smem[];
@@ -309,9 +321,8 @@ paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_ca
   const int first_key_read = p.window > 0 ? max(0, pos0 + 1 - p.window) : 0;
   int chunk_lo = first_key_read / CHUNK, chunk_hi = last_pos / CHUNK;
   if (SPLIT) {
-    const int mine = rest / gchunks;
-    if (mine < chunk_lo || mine > chunk_hi) return;
-    chunk_lo = chunk_hi = mine;
+    my_chunks(p, rest / gchunks, chunk_lo, chunk_hi);
+    if (chunk_lo > chunk_hi) return;
   }
   const int first_head = kv_head * group + (rest % gchunks) * heads;
   const int head_count = min(heads, group - (rest % gchunks) * heads);
@@ -353,7 +364,7 @@ paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_ca
 #pragma unroll
     for (int j = 0; j < TN; ++j) total[i][j] = 0.f;
 
-  for (int chunk = chunk_lo; chunk <= chunk_hi; ++chunk) {
+  for (int chunk = chunk_lo; chunk <= chunk_hi; chunk += SPLIT ? p.parts : 1) {
     const int first_key = chunk * CHUNK;
     float m_chunk = -INFINITY, l_chunk = 0.f;
     if (tid < CHUNK) {
@@ -481,7 +492,7 @@ paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_ca
         if (!row_of(r, token, head)) continue;
         const int pos = pos_s[r];          // the merge asks for the chunks with a visible key only
         if (first_key > pos || (p.window > 0 && first_key + CHUNK - 1 <= pos - p.window)) continue;
-        float* dst = partials + (((size_t)(row_base + token) * p.n_q + first_head + head) * max_chunks + chunk) * (D + 2);
+        float* dst = partials + (((size_t)(row_base + token) * p.n_q + first_head + head) * p.max_chunks + chunk) * (D + 2);
 #pragma unroll
         for (int c = 0; c < TN; ++c) {
           const int col = oc + 32 * (c / 4) + c % 4;
@@ -517,7 +528,7 @@ paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_ca
 constexpr int MERGE_BATCH = 32;
 template <typename T>
 __global__ void __launch_bounds__(MAX_D)
-paged_attention_generic_merge_kernel(const float* __restrict__ partials, T* __restrict__ out, const Step p, int max_chunks) {
+paged_attention_generic_merge_kernel(const float* __restrict__ partials, T* __restrict__ out, const Step p) {
   __shared__ float wa_s[MERGE_BATCH], wb_s[MERGE_BATCH], sum_s[MERGE_BATCH];
   pdl_launch_dependents();
   const int index = blockIdx.x, head = blockIdx.y, d = threadIdx.x;
@@ -526,8 +537,8 @@ paged_attention_generic_merge_kernel(const float* __restrict__ partials, T* __re
   if (seg < 0) return;
   const int pos = p.positions[t];
   const int kv_begin = p.window > 0 ? max(0, pos + 1 - p.window) : 0;
-  const float* src = partials + ((size_t)index * p.n_q + head) * max_chunks * (D + 2);
-  const int hi = pos / CHUNK;
+  const float* src = partials + ((size_t)index * p.n_q + head) * p.max_chunks * (D + 2);
+  const int hi = min(pos / CHUNK, p.max_chunks - 1);
   float total = 0.f, M = -INFINITY, L = 0.f;      // M: the first warp's
   pdl_wait();
   for (int c0 = kv_begin / CHUNK; c0 <= hi; c0 += MERGE_BATCH) {
@@ -571,53 +582,53 @@ size_t tiles_smem(int DT) { return sizeof(float) * ((size_t)(ROWS + 2 * CHUNK) *
 
 template <typename T, bool SPLIT, bool VEC>
 cudaError_t launch_rows(const void* q, const void* k, const void* v, void* out, const Step& p, int rows, float* partials,
-                        int max_chunks, cudaStream_t stream) {
+                        cudaStream_t stream) {
   auto kernel = paged_attention_generic_kernel<T, SPLIT, VEC>;
   static SmemAllowance allowed;
   cudaError_t err = allow_smem(kernel, rows_smem(MAX_D), allowed);
   if (err != cudaSuccess) return err;
   const int gchunks = (p.n_q / p.n_kv + GC - 1) / GC;
-  const dim3 grid((unsigned)((long long)rows * gchunks * (SPLIT ? max_chunks : 1)), p.n_kv);
+  const dim3 grid((unsigned)((long long)rows * gchunks * (SPLIT ? p.parts : 1)), p.n_kv);
   return lse_launch(kernel, grid, THREADS, rows_smem(p.head_dim), stream, (const T*)q, (const T*)k, (const T*)v, (T*)out, p,
-                    partials, max_chunks, rows);
+                    partials, rows);
 }
 
 template <typename T, int DT, bool SPLIT, bool VEC>
 cudaError_t launch_tiles(const void* q, const void* k, const void* v, void* out, const Step& p, const int* segment_first,
-                         int tiles, float* partials, int max_chunks, cudaStream_t stream) {
+                         int tiles, float* partials, cudaStream_t stream) {
   auto kernel = paged_attention_tiles_kernel<T, DT, SPLIT, VEC>;
   static SmemAllowance allowed;
   cudaError_t err = allow_smem(kernel, tiles_smem(DT), allowed);
   if (err != cudaSuccess) return err;
   const int group = p.n_q / p.n_kv, heads = group < ROWS ? group : ROWS, gchunks = (group + heads - 1) / heads;
-  const dim3 grid((unsigned)((long long)tiles * gchunks * (SPLIT ? max_chunks : 1)), p.n_kv);
+  const dim3 grid((unsigned)((long long)tiles * gchunks * (SPLIT ? p.parts : 1)), p.n_kv);
   return lse_launch(kernel, grid, THREADS, tiles_smem(DT), stream, (const T*)q, (const T*)k, (const T*)v, (T*)out, p,
-                    segment_first, partials, max_chunks, tiles);
+                    segment_first, partials, tiles);
 }
 
 template <typename T>
-cudaError_t launch_merge(void* out, const Step& p, int rows, const float* partials, int max_chunks, cudaStream_t stream) {
+cudaError_t launch_merge(void* out, const Step& p, int rows, const float* partials, cudaStream_t stream) {
   return lse_launch(paged_attention_generic_merge_kernel<T>, dim3(rows, p.n_q), ((p.head_dim + 31) / 32) * 32, 0, stream,
-                    partials, (T*)out, p, max_chunks);
+                    partials, (T*)out, p);
 }
 
 template <typename T, bool VEC>
 cudaError_t run(const void* q, const void* k, const void* v, void* out, const Step& p, const int* segment_first, int rows,
-                int tiles, float* partials, int max_chunks, cudaStream_t stream) {
+                int tiles, float* partials, cudaStream_t stream) {
   cudaError_t err;
   if (tiles > 0) {
     const bool small = p.head_dim <= 64;
     if (partials)
-      err = small ? launch_tiles<T, 64, true, VEC>(q, k, v, out, p, segment_first, tiles, partials, max_chunks, stream)
-                  : launch_tiles<T, 128, true, VEC>(q, k, v, out, p, segment_first, tiles, partials, max_chunks, stream);
+      err = small ? launch_tiles<T, 64, true, VEC>(q, k, v, out, p, segment_first, tiles, partials, stream)
+                  : launch_tiles<T, 128, true, VEC>(q, k, v, out, p, segment_first, tiles, partials, stream);
     else
-      err = small ? launch_tiles<T, 64, false, VEC>(q, k, v, out, p, segment_first, tiles, nullptr, 0, stream)
-                  : launch_tiles<T, 128, false, VEC>(q, k, v, out, p, segment_first, tiles, nullptr, 0, stream);
+      err = small ? launch_tiles<T, 64, false, VEC>(q, k, v, out, p, segment_first, tiles, nullptr, stream)
+                  : launch_tiles<T, 128, false, VEC>(q, k, v, out, p, segment_first, tiles, nullptr, stream);
   } else {
-    err = partials ? launch_rows<T, true, VEC>(q, k, v, out, p, rows, partials, max_chunks, stream)
-                   : launch_rows<T, false, VEC>(q, k, v, out, p, rows, nullptr, 0, stream);
+    err = partials ? launch_rows<T, true, VEC>(q, k, v, out, p, rows, partials, stream)
+                   : launch_rows<T, false, VEC>(q, k, v, out, p, rows, nullptr, stream);
   }
-  if (err == cudaSuccess && partials) err = launch_merge<T>(out, p, rows, partials, max_chunks, stream);
+  if (err == cudaSuccess && partials) err = launch_merge<T>(out, p, rows, partials, stream);
   return err;
 }
 }  // namespace
@@ -634,24 +645,26 @@ extern "C" int lse_attention_generic_tile_tokens(int head_dim, int n_q, int n_kv
 // segment_start null: the rows kernel over all `tokens` rows.  Else (with segment_first, [segments]) portions != 0: the tiles
 // kernel over the rows of the requests that bring several (skip_single) or all requests; portions == 0: the rows kernel
 // over the requests that bring one.
-// partials != null: every chunk gets a block of its own and a second kernel merges them; partials holds rows * n_q *
+// partials != null: a row's chunks are shared by several blocks and a second kernel merges them; partials holds rows * n_q *
 // max_chunks * (head_dim + 2) floats (rows: tokens, or segments for single rows), and max_chunks chunks cover the longest
-// context that the block tables can describe.  The result is the same bit for bit either way.
+// context of the step (max_context; 0: what the block tables can describe).  The result is the same bit for bit either way.
 extern "C" int lse_paged_attention_generic_portions(const void* q, const void* k_cache, const void* v_cache, void* out, int dtype,
                                                     const int* block_tables, int bt_stride, const int* segment_of_token,
                                                     const int* positions, int tokens, int n_q, int n_kv, int head_dim,
                                                     int page_size, float scale, int window, int num_pages, int num_segments,
-                                                    float* partials, int max_chunks, const int* segment_start,
-                                                    const int* segment_first, int portions, int skip_single,
-                                                    cudaStream_t stream) {
+                                                    float* partials, int max_chunks, int max_context,
+                                                    const int* segment_start, const int* segment_first, int portions,
+                                                    int skip_single, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (head_dim <= 0 || head_dim > MAX_D || head_dim % 16 || n_kv <= 0 || n_q % n_kv || page_size <= 0)
     return LSE_ERR_BAD_ARGUMENT;
   if (segment_start && (num_segments <= 0 || (portions && (!segment_first || !lse_attention_generic_tile_tokens(head_dim, n_q, n_kv)))))
     return LSE_ERR_BAD_ARGUMENT;
-  if (partials && (max_chunks <= 0 || (long long)max_chunks * CHUNK < (long long)bt_stride * page_size)) return LSE_ERR_BAD_ARGUMENT;
+  long long keys = (long long)bt_stride * page_size;
+  if (max_context > 0 && max_context < keys) keys = max_context;
+  if (partials && (max_chunks <= 0 || (long long)max_chunks * CHUNK < keys)) return LSE_ERR_BAD_ARGUMENT;
   Step p = {block_tables, bt_stride, segment_of_token, positions, segment_start, num_pages, num_segments,
-            n_q, n_kv, head_dim, page_size, scale, window, ALL_ROWS};
+            n_q, n_kv, head_dim, page_size, scale, window, ALL_ROWS, max_chunks, 1};
   int rows = tokens, tiles = 0;
   if (segment_start && portions) {
     const int per_tile = lse_attention_generic_tile_tokens(head_dim, n_q, n_kv);
@@ -661,27 +674,21 @@ extern "C" int lse_paged_attention_generic_portions(const void* q, const void* k
     rows = num_segments;
     p.skip = SINGLE_ROWS;
   }
-  const long long blocks = (long long)(tiles > 0 ? tiles : rows) * ((n_q / n_kv + GC - 1) / GC) * (partials ? max_chunks : 1);
+  const int group = n_q / n_kv, heads = tiles > 0 ? (group < ROWS ? group : ROWS) : GC;
+  const long long whole = (long long)(tiles > 0 ? tiles : rows) * ((group + heads - 1) / heads);
+  if (partials) {
+    const long long wanted = SPLIT_BLOCKS / (whole * n_kv) + 1;
+    p.parts = (int)(wanted < max_chunks ? wanted : max_chunks);
+  }
+  const long long blocks = whole * p.parts;
   if (blocks > 0x7fffffffLL) return LSE_ERR_TOO_LARGE;
   const bool vec = (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
   cudaError_t err;
-#define LSE_GENERIC_ARGS q, k_cache, v_cache, out, p, segment_first, rows, tiles, partials, max_chunks, stream
+#define LSE_GENERIC_ARGS q, k_cache, v_cache, out, p, segment_first, rows, tiles, partials, stream
   if (dtype == LSE_DTYPE_F32) err = vec ? run<float, true>(LSE_GENERIC_ARGS) : run<float, false>(LSE_GENERIC_ARGS);
   else if (dtype == LSE_DTYPE_BF16) err = vec ? run<__nv_bfloat16, true>(LSE_GENERIC_ARGS) : run<__nv_bfloat16, false>(LSE_GENERIC_ARGS);
   else return LSE_ERR_BAD_ARGUMENT;
 #undef LSE_GENERIC_ARGS
   if (err != cudaSuccess) return (int)err;
   LSE_LAUNCH_CHECK();
-}
-
-extern "C" int lse_paged_attention_generic(const void* q, const void* k_cache, const void* v_cache,
-                                           void* out, int dtype, const int* block_tables,
-                                           int bt_stride, const int* segment_of_token,
-                                           const int* positions, int tokens, int n_q, int n_kv,
-                                           int head_dim, int page_size, float scale, int window,
-                                           int num_pages, int num_segments, float* partials, int max_chunks,
-                                           cudaStream_t stream) {
-  return lse_paged_attention_generic_portions(q, k_cache, v_cache, out, dtype, block_tables, bt_stride, segment_of_token,
-                                              positions, tokens, n_q, n_kv, head_dim, page_size, scale, window, num_pages,
-                                              num_segments, partials, max_chunks, nullptr, nullptr, 0, 0, stream);
 }

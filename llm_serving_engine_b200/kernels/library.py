@@ -77,12 +77,9 @@ _SIGNATURES = {
     "lse_gemm_f32_ranges": [c_int],
     "lse_gemm_f32_stack_ok": [c_void_p, c_void_p, c_int, c_int, c_longlong, c_longlong],
     "lse_gemm_f32_stack_wanted": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong],
-    "lse_paged_attention_generic": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
-                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
-                                    c_int, c_int, c_int, c_void_p, c_int, c_void_p],
     "lse_paged_attention_generic_portions": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
-                                             c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
+                                             c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "lse_attention_generic_chunk": [],
     "lse_attention_generic_tile_tokens": [c_int, c_int, c_int],
     "lse_paged_attention_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,

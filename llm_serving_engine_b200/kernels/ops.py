@@ -193,8 +193,8 @@ def rope_kv_write(qkv: torch.Tensor, bias: torch.Tensor | None, positions: torch
           "rope_kv_write")
 
 
-GENERIC_SPLIT_MAX_ROWS = 64   # up to this many rows every chunk of keys of a row gets a block of its own
-GENERIC_SCRATCH_FLOATS = 1 << 28    # most partial results that blocks of one chunk may leave (1 GiB)
+GENERIC_SPLIT_MAX_ROWS = 64   # up to this many rows the chunks of keys of a row are shared by several blocks
+GENERIC_SCRATCH_FLOATS = 1 << 26    # most partial results that a launch may leave (256 MiB): beyond, some rows at a time
 
 
 def attention_generic_tile_tokens(head_dim: int, n_q: int, n_kv: int) -> int:
@@ -207,19 +207,20 @@ def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
                             segment_of_token: torch.Tensor, positions: torch.Tensor, scale: float,
                             window: int = 0, split: bool | None = None, segment_start: torch.Tensor | None = None,
                             segment_first_position: torch.Tensor | None = None, singles: bool = False,
-                            skip_single: bool = False) -> torch.Tensor:
+                            skip_single: bool = False, max_context: int = 0) -> torch.Tensor:
     """Attention of every token of the step over its request's cached keys.
 
     q, out [T, n_q, D]; k_cache, v_cache [pages, n_kv, page_size, D];
     block_tables int32 [S, max_pages]; segment_of_token, positions int32 [T].
-    A row's keys are summed in chunks of fixed size; ``split`` gives every chunk a block of its own
+    A row's keys are summed in chunks of fixed size; ``split`` has several blocks share a row's chunks
     (default: with few blocks, which would leave the GPU idle).  The result does not
     depend on it, bit for bit, nor on what follows.
 
     Without ``segment_start`` a block takes one row.  With ``segment_start`` (int32 [S + 1]) and ``segment_first_position``
     (int32 [S]; the rows of a request neighbours in position order) a block takes a tile of rows that share their keys:
     head sizes up to 128; ``skip_single`` leaves the requests of one row alone.  With ``segment_start`` and ``singles`` only
-    the requests of one row are worked on, a block a row.
+    the requests of one row are worked on, a block a row.  ``max_context``: keys that any request of the step holds at most
+    (0: what the block tables have room for); it sizes the partial results.
     """
     _need_cuda(q, k_cache, v_cache, out, block_tables, segment_of_token, positions, segment_start, segment_first_position)
     tokens, n_q, head_dim = q.shape
@@ -242,24 +243,35 @@ def paged_attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     lib = library.load()
     chunk = int(lib.lse_attention_generic_chunk())
     rows = segments if singles else tokens
-    max_chunks = max(1, -(-(block_tables.stride(0) * page_size) // chunk))
+    keys = block_tables.stride(0) * page_size
+    max_chunks = max(1, -(-(min(keys, max_context) if max_context > 0 else keys) // chunk))
+    per_row = n_q * max_chunks * (head_dim + 2)      # partial results of a row
+    at_once = rows
     if split is None:
         if tiles:
             # a tile's blocks walk up to all its chunks one after the other, two blocks an SM at a time: with fewer than
-            # four blocks an SM the longest walk decides, and a block per chunk is faster
+            # four blocks an SM the longest walk decides, and sharing the chunks is faster
             blocks = (-(-tokens // attention_generic_tile_tokens(head_dim, n_q, n_kv)) + segments) * n_kv
-            split = blocks < 4 * sm_count()
+            split = blocks < 4 * sm_count() and rows * per_row <= GENERIC_SCRATCH_FLOATS
         else:
             split = rows <= GENERIC_SPLIT_MAX_ROWS
-        split = split and max_chunks > 1 and rows * n_q * max_chunks * (head_dim + 2) <= GENERIC_SCRATCH_FLOATS
-    partials = None
-    if split:
-        partials = torch.empty(rows * n_q * max_chunks * (head_dim + 2), dtype=torch.float32, device=q.device)
-    check(lib.lse_paged_attention_generic_portions(
-        q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), dtype_code(q.dtype), block_tables.data_ptr(),
-        block_tables.stride(0), segment_of_token.data_ptr(), positions.data_ptr(), tokens, n_q, n_kv, head_dim, page_size,
-        float(scale), int(window), k_cache.shape[0], segments, _ptr(partials), max_chunks if split else 0,
-        _ptr(segment_start), _ptr(segment_first_position), int(tiles), int(skip_single), _stream()), "paged_attention_generic")
+        split = split and max_chunks > 1
+        if split and not tiles:
+            at_once = max(1, min(rows, GENERIC_SCRATCH_FLOATS // per_row))
+    partials = torch.empty(at_once * per_row, dtype=torch.float32, device=q.device) if split else None
+    for row in range(0, rows, at_once):
+        count = min(at_once, rows - row)
+        # single rows are numbered by their requests, the others by themselves
+        first, requests = (row, count) if singles else (0, segments)
+        own = 0 if singles else row
+        at = own * n_q * head_dim * q.element_size()
+        check(lib.lse_paged_attention_generic_portions(
+            q.data_ptr() + at, k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr() + at, dtype_code(q.dtype),
+            block_tables.data_ptr() + 4 * first * block_tables.stride(0), block_tables.stride(0),
+            segment_of_token.data_ptr() + 4 * own, positions.data_ptr() + 4 * own, tokens if singles else count, n_q, n_kv, head_dim,
+            page_size, float(scale), int(window), k_cache.shape[0], requests, _ptr(partials), max_chunks if split else 0,
+            int(max_context), None if segment_start is None else segment_start.data_ptr() + 4 * first,
+            _ptr(segment_first_position), int(tiles), int(skip_single), _stream()), "paged_attention_generic")
     return out
 
 

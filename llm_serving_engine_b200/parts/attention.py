@@ -126,6 +126,16 @@ class GroupedQueryAttention(Mixer):
         portions, singles = self._portions(segment_counts)
         return (self.prompt_kernel(portions), singles, self._portion_class(portions, singles))
 
+    def launch_signature_at(self, segment_counts, contexts):
+        answer = self.launch_signature(segment_counts)
+        return (*answer, self._context_class(contexts)) if answer[:1] == ("general",) else answer
+
+    @staticmethod
+    def _context_class(contexts: list[int]) -> int:
+        """An upper bound on the requests' contexts (a power of two): the general kernels' partial results have room for so many
+        keys a row, not for all that the block tables could hold."""
+        return 1 << max(7, (max(contexts) - 1).bit_length())
+
     def _general_kernels(self, segment_counts: list[int]) -> tuple[bool, bool]:
         """Whether the general attention's tiles kernel takes the portions of a step, and the rows kernel its single tokens."""
         most = max(segment_counts)
@@ -138,14 +148,18 @@ class GroupedQueryAttention(Mixer):
     def _general_attention(self, q, cache, attended, step):
         arguments = (q, cache.keys, cache.values, attended, cache.block_tables, step.segment_of_token, step.positions,
                      self.scale, self.window)
-        tiles, singles = (False, False) if step.decode_only else self._general_kernels([segment.count for segment in step.segments])
-        if not tiles:
+        if step.decode_only:      # a captured step's contexts grow until its tables are full
             ops.paged_attention_generic(*arguments)
             return
+        tiles, singles = self._general_kernels([segment.count for segment in step.segments])
+        longest = self._context_class([segment.first_position + segment.count for segment in step.segments])
+        if not tiles:
+            ops.paged_attention_generic(*arguments, max_context=longest)
+            return
         if singles:
-            ops.paged_attention_generic(*arguments, segment_start=step.segment_start, singles=True)
-        ops.paged_attention_generic(*arguments, segment_start=step.segment_start,
-                                    segment_first_position=step.segment_first_position, skip_single=singles)
+            ops.paged_attention_generic(*arguments, segment_start=step.segment_start, singles=True, max_context=longest)
+        ops.paged_attention_generic(*arguments, segment_start=step.segment_start, segment_first_position=step.segment_first_position,
+                                    skip_single=singles, max_context=longest)
 
     def forward(self, x, step, cache):
         tokens = x.shape[0]

@@ -474,6 +474,65 @@ def test_general_attention_gives_the_same_bits_tile_by_tile(dtype, head_dim, n_q
     assert bool(torch.isinf(rows[-1]).all()) and bool(torch.isfinite(rows[:-1]).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head_dim, n_q, n_kv, window", [(32, 16, 16, 0), (48, 24, 8, 0), (32, 16, 16, 150), (128, 20, 20, 0)])
+def test_general_attention_whose_blocks_share_a_rows_chunks(dtype, head_dim, n_q, n_kv, window):
+    """Tables far wider than the contexts, and so many rows and heads that a block takes several of a row's chunks: single rows,
+    single rows beside portions and tiles, with the tables' room, with a bound on the contexts, and with so little room for
+    partial results that a launch takes a few rows at a time, all bit for bit what a block per row gives."""
+    rng = random.Random(head_dim + window)
+    torch.manual_seed(head_dim + window)
+    portions = [(rng.choice([0, 63, 64, 200, 700, 1000]), 1) for _ in range(50)] + [(100, 2), (960, 9), (0, 65), (640, 3)]
+    contexts = [first + count for first, count in portions]
+    k_cache, v_cache, tables, _ = paged_setup(rng, contexts, n_kv, head_dim, 16, dtype)
+    poison_unowned(k_cache, v_cache, tables, contexts, 16)
+    tables = torch.cat([tables, torch.full((len(portions), 700), -1, dtype=torch.int32, device=DEV)], dim=1)
+    tokens = sum(count for _, count in portions)
+    q = torch.randn(tokens, n_q, head_dim, device=DEV).to(dtype)
+    segs = torch.cat([torch.full((count,), index) for index, (_, count) in enumerate(portions)]).to(torch.int32).to(DEV)
+    positions = torch.cat([torch.arange(first, first + count) for first, count in portions]).to(torch.int32).to(DEV)
+    start = torch.tensor([0] + [count for _, count in portions]).cumsum(0).to(torch.int32).to(DEV)
+    firsts = torch.tensor([first for first, _ in portions], dtype=torch.int32, device=DEV)
+    run, scale = ops().paged_attention_generic, 1.0 / math.sqrt(head_dim)
+    want = torch.full_like(q, 9.0)
+    run(q, k_cache, v_cache, want, tables, segs, positions, scale, window, split=False)
+    kept, singles = ops().GENERIC_SCRATCH_FLOATS, slice(0, 50)
+    try:
+        for room in (kept, 7 * n_q * 189 * (head_dim + 2)):
+            ops().GENERIC_SCRATCH_FLOATS = room
+            for bound in (0, 1024, max(contexts)):
+                got = torch.full_like(q, 9.0)
+                run(q[singles], k_cache, v_cache, got[singles], tables, segs[singles], positions[singles], scale, window, max_context=bound)
+                assert torch.equal(got[singles], want[singles]), (room, bound)
+                got = torch.full_like(q, 9.0)
+                run(q, k_cache, v_cache, got, tables, segs, positions, scale, window, segment_start=start, singles=True, max_context=bound)
+                assert bool((got[50:] == 9.0).all())
+                for split in (None, True):
+                    run(q, k_cache, v_cache, got, tables, segs, positions, scale, window, split=split, segment_start=start,
+                        segment_first_position=firsts, skip_single=True, max_context=bound)
+                    assert torch.equal(got, want), (room, bound, split)
+    finally:
+        ops().GENERIC_SCRATCH_FLOATS = kept
+
+
+def test_general_attention_keeps_its_partial_results_within_bounds():
+    """64 single rows of 40 heads behind tables of 32,768 keys: 680 MB of partial results if all rows left theirs at once."""
+    tokens, n_q, n_kv, head_dim, page = 64, 40, 8, 128, 16
+    cache = torch.randn(8, n_kv, page, head_dim, device=DEV)
+    tables = torch.zeros(tokens, 32768 // page, dtype=torch.int32, device=DEV)
+    q = torch.randn(tokens, n_q, head_dim, device=DEV)
+    out = torch.empty_like(q)
+    segs = torch.arange(tokens, dtype=torch.int32, device=DEV)
+    positions = torch.full((tokens,), 99, dtype=torch.int32, device=DEV)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    ops().paged_attention_generic(q, cache, cache, out, tables, segs, positions, 0.1)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before <= (1 << 28) + (1 << 21)
+
+
 @pytest.mark.parametrize("window", [1, 5, 16, 33, 100])
 def test_window_edge(window):
     rng = random.Random(window)
