@@ -126,6 +126,13 @@ __device__ __forceinline__ int which_row(const Step& p, int index, int& seg) {
   return index;
 }
 
+// What a block without work does that has not waited for the kernels before yet.  A launch over some of the rows may have none
+// at all (every request brings one row): it must not end ahead of the kernel before it, for the kernel after it waits for
+// this launch only.
+__device__ __forceinline__ void leave_unneeded(const Step& p) {
+  if (p.skip != ALL_ROWS) pdl_wait();
+}
+
 // SPLIT: the block of number `part` takes every parts-th of the chunks lo .. hi of its rows: lo becomes its first one.
 // (The chunks of a row are known on the device only: with a block for every chunk that the block tables have room for, 64
 // rows of 100 keys in tables of 16,384 made 16,384 blocks at two key/value heads, nearly all of them without work.)
@@ -314,7 +321,7 @@ paged_attention_tiles_kernel(const T* __restrict__ q, const T* __restrict__ k_ca
   const int kv_head = blockIdx.y;
   int seg, r0, cnt;
   lse_find_tile(p.segment_start, p.num_segments, tokens_per_tile, p.skip == ROWS_OF_PORTIONS, rank, tile_slot, seg, r0, cnt);
-  if (seg < 0) return;
+  if (seg < 0) { leave_unneeded(p); return; }
   const int tokens = min(tokens_per_tile, cnt - r0);
   const int row_base = p.segment_start[seg] + r0;
   const int pos0 = segment_first[seg] + r0, last_pos = pos0 + tokens - 1;
@@ -534,7 +541,7 @@ paged_attention_generic_merge_kernel(const float* __restrict__ partials, T* __re
   const int index = blockIdx.x, head = blockIdx.y, d = threadIdx.x;
   int seg;
   const int t = which_row(p, index, seg), D = p.head_dim;
-  if (seg < 0) return;
+  if (seg < 0) { leave_unneeded(p); return; }
   const int pos = p.positions[t];
   const int kv_begin = p.window > 0 ? max(0, pos + 1 - p.window) : 0;
   const float* src = partials + ((size_t)index * p.n_q + head) * p.max_chunks * (D + 2);

@@ -515,6 +515,36 @@ def test_general_attention_whose_blocks_share_a_rows_chunks(dtype, head_dim, n_q
         ops().GENERIC_SCRATCH_FLOATS = kept
 
 
+def test_a_launch_over_portions_of_a_step_without_portions_does_not_end_ahead_of_the_one_before():
+    """Single rows, then a launch over the portions, of which there are none, then a norm of what the first left, queued behind
+    one another: the norm reads the finished rows every time."""
+    torch.manual_seed(3)
+    tokens, n_q, n_kv, head_dim, page, context = 64, 8, 8, 128, 16, 1500
+    pages = -(-context // page)
+    k_cache, v_cache = (torch.randn(pages * 4, n_kv, page, head_dim, device=DEV) for _ in range(2))
+    tables = (torch.arange(pages, dtype=torch.int32)[None] + pages * (torch.arange(tokens, dtype=torch.int32) % 4)[:, None]).to(DEV)
+    q = torch.randn(tokens, n_q, head_dim, device=DEV)
+    segs = torch.arange(tokens, dtype=torch.int32, device=DEV)
+    positions = torch.full((tokens,), context - 1, dtype=torch.int32, device=DEV)
+    start = torch.arange(tokens + 1, dtype=torch.int32, device=DEV)
+    weight = torch.ones(n_q * head_dim, device=DEV)
+    run, arguments = ops().paged_attention_generic, (tables, segs, positions, 0.2)
+    want = torch.empty_like(q)
+    run(q, k_cache, v_cache, want, *arguments, split=False)
+    torch.cuda.synchronize()
+    wanted = torch.empty(tokens, n_q * head_dim, device=DEV)
+    ops().add_rmsnorm(torch.zeros_like(wanted), want.view(tokens, -1), weight, 1e-6, wanted)
+    outs = [(torch.full_like(q, 9.0), torch.empty_like(wanted), torch.zeros_like(wanted)) for _ in range(24)]
+    torch.cuda.synchronize()
+    for index, (out, normed, residual) in enumerate(outs):
+        split = index % 2 == 0
+        run(q, k_cache, v_cache, out, *arguments, split=split, segment_start=start, singles=True)
+        run(q, k_cache, v_cache, out, *arguments, split=split, segment_start=start, segment_first_position=positions, skip_single=True)
+        ops().add_rmsnorm(residual, out.view(tokens, -1), weight, 1e-6, normed)
+    for out, normed, _ in outs:
+        assert torch.equal(out, want) and torch.equal(normed, wanted)
+
+
 def test_general_attention_keeps_its_partial_results_within_bounds():
     """64 single rows of 40 heads behind tables of 32,768 keys: 680 MB of partial results if all rows left theirs at once."""
     tokens, n_q, n_kv, head_dim, page = 64, 40, 8, 128, 16
