@@ -14,7 +14,7 @@ device with one transfer; ``StepContext`` holds views into the device copy.
 
 Steps in which every request brings exactly one token (decoding) are replayed
 from CUDA graphs: the model's launches are captured once per (batch bucket,
-block-table width) with the metadata at fixed addresses, rows beyond the batch
+block-table width, class of the longest context) with the metadata at fixed addresses, rows beyond the batch
 being padding (segment -1, cache slot -1) that every kernel skips.  Only models
 whose mixers all say ``graph_safe`` are captured; others run launch by launch.
 """
@@ -29,6 +29,7 @@ import numpy as np
 import torch
 
 from ..cache.manager import CacheFullError, CacheManager, LayerCache
+from ..kernels import ops
 
 
 @dataclass
@@ -72,6 +73,7 @@ class StepContext:
         self.decode_only = False                     # every segment brings exactly one token
         self.long_context = False                    # some request holds more than LONG_CONTEXT keys (known on the host always:
                                                      # graphs of decode steps are captured for either case)
+        self.many_keys = False                       # some request holds ops.DECODE_MANY_KEYS keys or more (likewise)
 
 
 def _round4(n: int) -> int:
@@ -79,6 +81,9 @@ def _round4(n: int) -> int:
 
 
 LONG_CONTEXT = 8192   # keys of a request beyond which a decode step counts as one over long contexts
+# what a decode graph was captured for: contexts below ops.DECODE_MANY_KEYS keys (or a model that launches the same there),
+# contexts from there on, contexts beyond LONG_CONTEXT
+SHORT, MANY_KEYS, LONG = 0, 1, 2
 
 
 class _Layout:
@@ -154,7 +159,8 @@ class StepRunner:
         self._copied = torch.cuda.Event() if pinned else None
         self._copy_pending = False
         self.use_graphs = bool(use_graphs) and pinned and getattr(model, "graph_safe", False)
-        self._graphs: dict[tuple[int, int, bool], _Graph] = {}   # (batch bucket, block-table width, long contexts)
+        self._graphs: dict[tuple[int, int, int], _Graph] = {}   # (batch bucket, block-table width, SHORT / MANY_KEYS / LONG)
+        self._depends_on_keys: dict[int, bool] = {}              # by batch bucket (DecoderModel.decode_depends_on_keys)
         self._graph_pool = None          # one memory pool for all graphs: only one of them runs at a time
         self._capture_stream = None
         self._arange = np.arange(max(self.GRAPH_BUCKETS), dtype=np.int32)
@@ -259,6 +265,7 @@ class StepRunner:
             row += count
         host[lay.start[0] + len(entries): lay.start[1]] = row      # padding segments are empty
         step.long_context = step.max_context > LONG_CONTEXT
+        step.many_keys = step.max_context >= ops.DECODE_MANY_KEYS
         if wanted_all_rows:
             host[lay.want[0]:lay.want[1]] = np.arange(lay.wanted, dtype=np.int32)
         step.decode_only = step.max_segment_tokens == 1
@@ -303,6 +310,7 @@ class StepRunner:
         step.max_segment_tokens = 1
         step.max_context = max(firsts) + 1
         step.long_context = step.max_context > LONG_CONTEXT
+        step.many_keys = step.max_context >= ops.DECODE_MANY_KEYS
         step.decode_only = True
         return step
 
@@ -350,14 +358,25 @@ class StepRunner:
         return self._views(step, self._device, lay)
 
     # -- decode steps from CUDA graphs ---------------------------------------------
-    def _run_graph(self, entries: list[StepEntry]) -> torch.Tensor:
+    def _decode_key(self, bucket: int, pages: int, at_least: int = SHORT) -> tuple[int, int, int]:
+        """Which graph a decode step belongs to whose longest request has ``pages`` pages after it."""
+        keys = pages * self.cache.page_size
+        kind = max(at_least, LONG if keys > LONG_CONTEXT else MANY_KEYS if keys >= ops.DECODE_MANY_KEYS else SHORT)
+        if kind == MANY_KEYS:
+            if bucket not in self._depends_on_keys:
+                asked = getattr(self.model, "decode_depends_on_keys", None)
+                self._depends_on_keys[bucket] = bool(asked(bucket)) if asked else False
+            kind = MANY_KEYS if self._depends_on_keys[bucket] else SHORT
+        return bucket, self._graph_width(pages), kind
+
+    def _run_graph(self, entries: list[StepEntry], at_least: int = SHORT) -> torch.Tensor:
         count = len(entries)
         bucket = next((b for b in self.GRAPH_BUCKETS if b >= count), None)
         if bucket is None:
             step, caches = self.prepare(entries, validated=True)
             return self.model.forward(step, caches)
         pages = self._pages_after(entries)
-        key = (bucket, self._graph_width(pages), pages * self.cache.page_size > LONG_CONTEXT)
+        key = self._decode_key(bucket, pages, at_least)
         slot = self._graphs.get(key)
         if slot is None:
             slot = _Graph(_Layout(bucket, bucket, bucket, key[1], self._groups), self.device, True)
@@ -367,7 +386,7 @@ class StepRunner:
             self._copy_pending = False
         step = self._pack_decode(entries, slot.host_np, slot.layout)
         step.max_context = None
-        step.long_context = key[2]   # what the graph was, or is now, captured for
+        step.long_context, step.many_keys = key[2] == LONG, key[2] >= MANY_KEYS   # what the graph was, or is now, captured for
         slot.device.copy_(slot.host, non_blocking=True)
         self.last_h2d_bytes = slot.layout.size * 4
         self._copied.record()
@@ -464,7 +483,7 @@ class StepRunner:
                 return None          # the token opens a page and none is free: the ordinary path decides
             firsts.append(first)
         pages = max(1, max(first // page_size + 1 for first in firsts))
-        key = (bucket, self._graph_width(pages), pages * page_size > LONG_CONTEXT)
+        key = self._decode_key(bucket, pages)
         slot = self._graphs.get(key)
         if slot is None or slot.graph is None:
             return None
@@ -628,7 +647,13 @@ class StepRunner:
             try:
                 for name in names:
                     self.cache.create(name)
-                self.run([StepEntry(name, [0], [0]) for name in names])
+                entries = [StepEntry(name, [0], [0]) for name in names]
+                self.run(entries)
+                bucket = next((b for b in self.GRAPH_BUCKETS if b >= size), None)
+                if (bucket is not None and self._decode_key(bucket, 1, MANY_KEYS)[2] == MANY_KEYS
+                        and self.cache.fits([(name, 1) for name in names])):
+                    self._run_graph(entries, MANY_KEYS)      # the same for longer contexts
+                    self.finish(entries)
                 torch.cuda.current_stream().synchronize()
             finally:
                 for name in names:

@@ -289,15 +289,15 @@ _DECODE_MAX_SPLITS = int(__import__("os").environ.get("LSE_DECODE_MAX_SPLITS", "
 _DECODE_MAX_SPLITS_LONG = 32    # the kernel's own limit
 
 
-_DECODE_TABLE_FOR_TWO = 1024    # keys that the block tables describe, from which many rows get two blocks an SM
+DECODE_MANY_KEYS = 1024         # keys of a step's longest context from which many rows get two blocks an SM
 
 
 def decode_splits(tokens: int, n_q: int, n_kv: int, max_context: int | None, long_context: bool = False,
-                  table_keys: int = 0) -> int:
+                  many_keys: bool = False) -> int:
     """How many splits of the keys a decode launch uses: enough blocks to fill the GPU and a little
     more (a block that ends early makes room for the next kernel's blocks), at least one 16-key
-    tile per warp and split.  (A block takes up to 8 query heads of a group.)  ``table_keys``: keys that the step's block
-    tables have room for (known where the contexts are not)."""
+    tile per warp and split.  (A block takes up to 8 query heads of a group.)  ``many_keys``: some request of the step holds
+    DECODE_MANY_KEYS keys or more (steps are captured for either case)."""
     base = tokens * n_kv * ((n_q // n_kv + 7) // 8)
     # about 1.4 blocks per SM (measured best from 12 to 64 rows on 148 SMs: 192 blocks beat 128 and 256); at most
     # 8 splits: one cluster adds them up.  Over long contexts (more than 8,192 keys) with so few rows that 8 splits
@@ -307,10 +307,13 @@ def decode_splits(tokens: int, n_q: int, n_kv: int, max_context: int | None, lon
     if long_context and 10 * base * cap < 7 * sm_count():
         cap = max(cap, _DECODE_MAX_SPLITS_LONG)
     blocks = (sm_count() * 7 + 4) // 5
-    if 2 * base >= sm_count() and table_keys >= _DECODE_TABLE_FOR_TWO:
+    if 2 * base >= sm_count() and many_keys:
         # rows enough for half the SMs or more: up to 1.75 blocks an SM, so that a launch does not last as long as one block
-        # on the longest context (64 requests of 950 to 2,850 keys: 24.1 against 30.9 us a layer; all of 1,900: 23.2 against
-        # 23.4; 32 of 2,048: 14.3 against 15.0).  Not over short contexts: 64 of 500 keys take 10.2 us split, 8.9 whole.
+        # on the longest context.  On 148 SMs two splits in place of one at 105 to 129 blocks, three of two at 74 to 86.  12 / 2
+        # heads, 64 requests of 950 to 2,850 keys: 23.5 against 30.4 us, all of 2,000: 23.9 against 24.3, all of 1,100: 12.3
+        # against 14.2; 28 / 4 heads, 32 requests: 24.2 against 31.1, 24.4 against 24.3, 12.8 against 14.7; 40 / 8 heads, 16:
+        # 23.3 against 30.7, 23.5 against 23.8, 12.0 against 14.0.  Not over short contexts: 64 requests of 800 keys 11.0
+        # against 10.5, of 500 9.1 against 7.9, of 60 6.8 against 3.7.
         blocks = sm_count() * 7 // 4
     splits = max(1, min(cap, blocks // base))
     if max_context is not None:

@@ -183,6 +183,11 @@ class DecoderModel:
         answers = [block.mixer.launch_signature_at(segment_counts, contexts) for block in self.blocks]
         return tuple((index, answer) for index, answer in enumerate(answers) if answer)
 
+    def decode_depends_on_keys(self, rows: int) -> bool:
+        """Whether a decode step of ``rows`` requests launches something else where the longest context holds
+        ``ops.DECODE_MANY_KEYS`` keys or more."""
+        return any(block.mixer.decode_signature(rows, False) != block.mixer.decode_signature(rows, True) for block in self.blocks)
+
     @property
     def vocab_size(self) -> int:
         return self.spec.vocab_size

@@ -130,6 +130,11 @@ class GroupedQueryAttention(Mixer):
         answer = self.launch_signature(segment_counts)
         return (*answer, self._context_class(contexts)) if answer[:1] == ("general",) else answer
 
+    def decode_signature(self, rows, many_keys):
+        if not ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, self.ctx.dtype, self.window):
+            return ()
+        return (ops.decode_splits(rows, self.n_q, self.n_kv, None, False, many_keys),)
+
     @staticmethod
     def _context_class(contexts: list[int]) -> int:
         """An upper bound on the requests' contexts (a power of two): the general kernels' partial results have room for so many
@@ -171,7 +176,7 @@ class GroupedQueryAttention(Mixer):
         if ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, x.dtype, self.window):
             if step.decode_only:
                 splits = ops.decode_splits(tokens, self.n_q, self.n_kv, step.max_context, getattr(step, "long_context", False),
-                                           table_keys=cache.block_tables.shape[1] * cache.keys.shape[2])
+                                           getattr(step, "many_keys", False))
                 ops.paged_attention_decode(q, cache.keys, cache.values, attended, cache.block_tables,
                                            step.segment_of_token, step.positions, self.scale, splits)
             elif sum(segment.count for segment in step.segments) < ROWS_KERNEL_BELOW:
@@ -185,8 +190,7 @@ class GroupedQueryAttention(Mixer):
                 portions, singles = self._portions([segment.count for segment in step.segments])
                 if singles:   # one block row per request of the step; requests with portions leave at once
                     requests = cache.block_tables.shape[0]
-                    splits = ops.decode_splits(requests, self.n_q, self.n_kv, None,
-                                               table_keys=cache.block_tables.shape[1] * cache.keys.shape[2])
+                    splits = ops.decode_splits(requests, self.n_q, self.n_kv, None)
                     ops.paged_attention_decode(q, cache.keys, cache.values, attended, cache.block_tables,
                                                step.segment_of_token, step.positions, self.scale, splits,
                                                segment_start=step.segment_start)

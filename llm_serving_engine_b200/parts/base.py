@@ -181,6 +181,11 @@ class Mixer(Part):
         (``contexts``)."""
         return self.launch_signature(segment_counts)
 
+    def decode_signature(self, rows: int, many_keys: bool) -> tuple:
+        """What this mixer's launches in a decode step of ``rows`` requests depend on besides the number of rows, where the
+        longest context holds ``ops.DECODE_MANY_KEYS`` keys or more, or fewer (empty: on nothing)."""
+        return ()
+
 
 def cache_needs(requirement) -> tuple:
     """A mixer's cache requirement as a tuple of single needs (empty for none)."""

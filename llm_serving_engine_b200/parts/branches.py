@@ -540,6 +540,9 @@ class ParallelMixers(Mixer):
         answers = [branch.launch_signature_at(segment_counts, contexts) for branch in self.branches]
         return tuple((index, answer) for index, answer in enumerate(answers) if answer)
 
+    def decode_signature(self, rows, many_keys):
+        return tuple(branch.decode_signature(rows, many_keys) for branch in self.branches)
+
     def forward(self, x, step, cache):
         proj = input_projection(x, self.in_weight)
         mid = torch.empty((x.shape[0], self.mid_offsets[-1]), dtype=x.dtype, device=x.device)

@@ -82,3 +82,55 @@ def test_captured_steps_beyond_the_bound_make_room_for_each_other():
         assert len(graphs._portion_graphs) <= 2
     assert [key[1] for key in graphs._portion_graphs] == [32, 48] or [key[1] for key in graphs._portion_graphs] == [48, 32]
     assert graphs.portion_graph_replays >= 6
+
+
+def attention_model(heads=(12, 2), layers=1):
+    """Grouped-query attention layers of 128 values a head in bfloat16, as the large models have them, with a narrow feed-forward."""
+    config = {"architectures": ["Qwen2ForCausalLM"], "model_type": "qwen2", "num_hidden_layers": layers, "hidden_size": 128 * heads[0],
+              "intermediate_size": 64, "num_attention_heads": heads[0], "num_key_value_heads": heads[1],
+              "vocab_size": 64, "max_position_embeddings": 4096, "rope_theta": 10000.0, "rms_norm_eps": 1e-6,
+              "tie_word_embeddings": True, "attention_bias": True}
+    from llm_serving_engine_b200.config import load_config
+    from llm_serving_engine_b200.models import DecoderModel, expected_tensors
+
+    _, _, spec = load_config(config)
+    generator = torch.Generator().manual_seed(2)
+    weights = {}
+    for name, tensor in expected_tensors(spec).items():
+        values = torch.randn(tensor.shape, generator=generator)
+        weights[name] = ((values * tensor.shape[-1] ** -0.5).bfloat16() if tensor.kind == "matrix" else 1.0 + 0.1 * values).cuda()
+    return DecoderModel(spec, weights, torch.bfloat16, "cuda")
+
+
+def test_decode_steps_split_their_keys_by_the_contexts_and_not_by_the_tables(monkeypatch):
+    """64 requests in tables of 4,096 keys, captured: whole while the longest context is below 1,024 keys, in two splits from
+    there on, each from a graph of its own that the warm-up has made, with the logits of the step launched one by one."""
+    from llm_serving_engine_b200.kernels import ops
+
+    model, splits, real = attention_model(), [], ops.paged_attention_decode
+    assert model.decode_depends_on_keys(64) and not model.decode_depends_on_keys(1)
+
+    def recorded(*args, **more):
+        splits.append(args[8])
+        return real(*args, **more)
+
+    monkeypatch.setattr(ops, "paged_attention_decode", recorded)
+    sizes = dict(positions=4096, pages=6000, tokens=2100, segments=64)
+    graphs, plain = runner_for(model, use_graphs=True, **sizes), runner_for(model, use_graphs=False, **sizes)
+    graphs.warmup([64])
+    assert {1, 2} <= set(splits) and len(graphs._graphs) == 2
+    generator = torch.Generator().manual_seed(9)
+    lengths = [1006 if index == 5 else 20 + index for index in range(64)]      # + 1: 63 pages of 16 keys; then 1,008 and 1,009
+    tokens = [torch.randint(0, 64, (length + 3,), generator=generator).tolist() for length in lengths]
+    for runner in (graphs, plain):
+        for index, length in enumerate(lengths):
+            runner.cache.create(str(index))
+            runner.run([StepEntry(str(index), tokens[index][:length], [])])
+    for turn, (eager, kind) in enumerate(((1, 0), (1, 0), (1, 1))):
+        entries = [StepEntry(str(index), tokens[index][length + turn:length + turn + 1], [0]) for index, length in enumerate(lengths)]
+        splits.clear()
+        replays = graphs.graph_replays
+        got, want = graphs.run(entries).clone(), plain.run(entries)
+        assert splits == [eager] and graphs.graph_replays == replays + 1 and len(graphs._graphs) == 2
+        assert graphs._decode_key(64, graphs._pages_after([StepEntry(e.request_id, [], []) for e in entries]))[2] == kind, turn
+        assert float((got - want).abs().max()) <= 2.0 ** -5 * float(want.abs().max())      # bfloat16, another order of sums

@@ -74,3 +74,23 @@ def test_decode_fast_path_packs_what_the_general_path_packs(lengths):
     assert step_a.decode_only and step_b.decode_only and step_a.max_context == step_b.max_context
     assert [(s.request_id, s.first_position, s.row_start) for s in step_a.segments] == \
            [(s.request_id, s.first_position, s.row_start) for s in step_b.segments]
+
+
+def test_decode_graphs_are_kept_by_the_longest_context_where_the_launches_depend_on_it():
+    """Tables of 16,384 keys for every captured step: what a step launches follows from its longest context, with a graph for
+    either side only where the model launches something else there, and the eager path says the same of its context."""
+    from llm_serving_engine_b200.engine.step import LONG, LONG_CONTEXT, MANY_KEYS, SHORT
+    from llm_serving_engine_b200.kernels.ops import DECODE_MANY_KEYS
+
+    runner, cache = make_runner(groups=(PagedKV(2, 16),), pages=8, page=16)
+    asked = []
+    runner.model.decode_depends_on_keys = lambda rows: asked.append(rows) or rows >= 64
+    edge, far = DECODE_MANY_KEYS // 16, LONG_CONTEXT // 16
+    for bucket, depends in ((64, True), (8, False)):
+        kinds = [runner._decode_key(bucket, pages)[2] for pages in (1, edge - 1, edge, far, far + 1)]
+        assert kinds == [SHORT, SHORT, MANY_KEYS if depends else SHORT, MANY_KEYS if depends else SHORT, LONG]
+        assert runner._decode_key(bucket, 1, MANY_KEYS)[2] == (MANY_KEYS if depends else SHORT)
+    assert asked == [64, 8]                      # once each
+    cache.create("a")
+    step, _ = runner.prepare([StepEntry("a", [1] * 60, [])])
+    assert not step.many_keys and not step.long_context and step.max_context == 60
