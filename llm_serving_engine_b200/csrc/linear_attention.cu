@@ -664,9 +664,10 @@ extern "C" int lse_gated_rmsnorm(const float* o, const void* proj, int proj_dtyp
                                  cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (n <= 0) return LSE_ERR_BAD_ARGUMENT;
-  // one set of sums, groups of four values aligned wherever they are read or written
+  // one set of sums, groups of four values aligned wherever they are read or written; from 512 values on (2,048 rows of 512: 6.4
+  // us either way, of 100: 6.4 against 4.2 with a value a thread)
   const size_t proj_group = proj_dtype == LSE_DTYPE_F32 ? 16 : 8, out_group = out_dtype == LSE_DTYPE_F32 ? 16 : 8;
-  const bool vec = n_partials == 1 && n % 4 == 0 && n <= 4 * 256 * GN_GROUPS && ld % 4 == 0 && g_off % 4 == 0 &&
+  const bool vec = n_partials == 1 && n % 4 == 0 && n >= 512 && n <= 4 * 256 * GN_GROUPS && ld % 4 == 0 && g_off % 4 == 0 &&
                    (((uintptr_t)o | (uintptr_t)weight) & 15) == 0 && ((uintptr_t)proj & (proj_group - 1)) == 0 &&
                    ((uintptr_t)out & (out_group - 1)) == 0;
 #define LSE_GN_CASE(TD, TO)                                                                                   \

@@ -590,6 +590,31 @@ def test_short_requests_beside_chunks_are_scanned_row_by_row(counts):
         assert float((got_state[slot] - want_state[slot]).abs().max()) <= 2e-5 * float(want_state[slot].abs().max()), index
 
 
+@pytest.mark.parametrize("rows, n, off, partials", [(3, 100, 4, 1), (5, 508, 0, 1), (5, 512, 8, 1), (300, 512, 3, 1), (2, 2052, 4, 1),
+                                                    (7, 4096, 0, 1), (4, 4100, 0, 1), (9, 1024, 4, 3)])
+@pytest.mark.parametrize("proj_type, out_type", [("float32", "float32"), ("bfloat16", "bfloat16"), ("float32", "bfloat16")])
+def test_gated_norm_on_either_side_of_its_rules(rows, n, off, partials, proj_type, out_type):
+    """Widths below and above the one-pass kernel's, gates at columns that are not aligned, stacks of partial sums; rows of no
+    request are left alone."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(n + rows)
+    kind = getattr(torch, proj_type if partials == 1 else "float32")
+    values, weight = torch.randn(rows, n).cuda(), (torch.rand(n) + 0.5).cuda()
+    proj = torch.randn(*((partials,) if partials > 1 else ()), rows, n + off + 1).to(kind).cuda()
+    segments = torch.zeros(rows, dtype=torch.int32)
+    segments[rows // 2] = -1
+    got = torch.full((rows, n), 9.0, dtype=getattr(torch, out_type)).cuda()
+    ops.gated_rmsnorm(values, proj, off, weight, 1e-5, got, segments.cuda())
+    z = proj.double().sum(0) if partials > 1 else proj.double()
+    x = values.double()
+    want = x / torch.sqrt(x.pow(2).mean(-1, keepdim=True) + 1e-5) * weight.double() * torch.sigmoid(z[:, off:off + n])
+    kept = segments >= 0
+    assert bool((got[~kept] == 9.0).all())
+    bound = 2.0 ** -8 if out_type == "bfloat16" else 2e-6
+    assert float((got.double() - want)[kept].abs().max()) <= bound * float(want.abs().max())
+
+
 def test_residual_copies_update_and_norm():
     from llm_serving_engine_b200.kernels import ops
 
