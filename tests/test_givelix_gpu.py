@@ -466,6 +466,56 @@ def test_latent_attention_over_expanded_keys_and_values(heads, rank, page, windo
             row, at = row + count, at + size
 
 
+@pytest.mark.parametrize("window", [0, 330])
+@pytest.mark.parametrize("per_tile", [5.0, 9.5, 40.0, 90.0])
+def test_expanded_latent_attention_while_the_maximum_grows(per_tile, window):
+    """Scores that grow along the keys, by 2^5 a tile of 64 (a tile's probabilities stay relative to an older maximum), 2^9.5 and
+    2^40 (the sums are taken over to the new maximum a tile later) and 2^90 (at once), in the unrotated and the rotated part, over
+    enough tiles for both groups and all their accumulators; the values shrink as the weights grow (up to 2^9.5 a tile), so that
+    every tile counts and a factor that is lost or applied twice shows.  Against float64 over the same bfloat16 keys and values."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(int(per_tile) + window)
+    heads, rank, portions = 2, 64, [(0, 600), (500, 130)]
+    contexts = [first + count for first, count in portions]
+    low = [max(0, first + 1 - window) if window else 0 for first, _ in portions]
+    kept = [-(-(context - lo) // 64) * 64 for context, lo in zip(contexts, low)]
+    tokens, capacity, scale = sum(count for _, count in portions), sum(kept), 0.1
+    sign, rot_sign = torch.randint(0, 2, (heads, 128)) * 2.0 - 1, torch.randint(0, 2, (64,)) * 2.0 - 1
+    q_plain = (sign * 0.5).expand(tokens, heads, 128).contiguous().bfloat16()
+    q_wide = torch.cat([torch.randn(tokens, heads, rank), (rot_sign * 0.5).expand(tokens, heads, 64)], dim=2).bfloat16()
+    rows, kv = torch.zeros(capacity, rank + 64), torch.zeros(capacity, 2 * heads, 128)
+    at = 0
+    for lo, context, size in zip(low, contexts, kept):
+        n = context - lo
+        growth = torch.arange(n) * per_tile / 64                       # of the score, in powers of two
+        natural = growth * 0.6931471805599453 / scale
+        kv[at:at + n, :heads] = (natural * 0.6 / 64)[:, None, None] * sign + torch.randn(n, heads, 128) * 0.02
+        rows[at:at + n, rank:] = (natural * 0.4 / 32)[:, None] * rot_sign + torch.randn(n, 64) * 0.02
+        shrink = torch.exp2(-growth if per_tile < 10 else torch.zeros(n))
+        kv[at:at + n, heads:] = (1.0 + torch.rand(n, heads, 128)) * shrink[:, None, None]
+        at += size
+    rows, kv = rows.bfloat16(), kv.bfloat16()
+    starts = torch.tensor([0, 600, 730], dtype=torch.int32).cuda()
+    firsts, ends = (torch.tensor(values, dtype=torch.int32).cuda() for values in ([0, 500], contexts))
+    got = torch.empty(tokens, heads, 128, dtype=torch.bfloat16, device="cuda")
+    ops.attention_expanded(q_plain.cuda(), q_wide.cuda(), rows.cuda(), kv.cuda(), got, starts, firsts, ends, scale, window)
+    assert int(ops.library.load().lse_attention_expanded_status()) == 0
+    row = at = 0
+    for (first, count), lo, size in zip(portions, low, kept):
+        keys, rotated = kv[at:at + size].double(), rows[at:at + size, rank:].double()
+        for t in sorted({0, 63, 64, 127, min(128, count - 1), min(200, count - 1), min(400, count - 1), count - 1}):
+            pos = first + t
+            seen = slice(max(0, pos + 1 - window) - lo if window else 0, pos + 1 - lo)
+            scores = (torch.einsum("hd,khd->hk", q_plain[row + t].double(), keys[seen, :heads])
+                      + q_wide[row + t, :, rank:].double() @ rotated[seen].t()) * scale
+            want = torch.einsum("hk,khd->hd", torch.softmax(scores, dim=1), keys[seen, heads:])
+            # weights rounded to bfloat16 and the result again, all values positive: 2^-8 each of the value
+            error = ((got[row + t].cpu().double() - want).abs() / want).max()
+            assert float(error) <= 2.0 ** -6, (first, t, float(error))
+        row, at = row + count, at + size
+
+
 @pytest.mark.parametrize("window", [0, 70])
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
 def test_a_latent_that_is_not_finite_reaches_the_rows_that_read_it_only(value, window, monkeypatch):
