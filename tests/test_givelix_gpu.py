@@ -651,7 +651,7 @@ def test_gated_norm_on_either_side_of_its_rules(rows, n, off, partials, proj_typ
     torch.manual_seed(n + rows)
     kind = getattr(torch, proj_type if partials == 1 else "float32")
     values, weight = torch.randn(rows, n).cuda(), (torch.rand(n) + 0.5).cuda()
-    proj = torch.randn(*((partials,) if partials > 1 else ()), rows, n + off + 1).to(kind).cuda()
+    proj = torch.randn(*((partials,) if partials > 1 else ()), rows, n + off + -(n + off) % 4).to(kind).cuda()
     segments = torch.zeros(rows, dtype=torch.int32)
     segments[rows // 2] = -1
     got = torch.full((rows, n), 9.0, dtype=getattr(torch, out_type)).cuda()
