@@ -14,7 +14,7 @@
 //               three key and value stages are shared by the groups, and a group has two score accumulators, so that its
 //               next scores are made while it works on the last.
 //
-// 2,048 rows, 16 heads: 41 us (524 TFLOP/s of the 320 multiply-adds a pair), bounded by the softmax threads' exponentials
+// 2,048 rows, 16 heads: 39.5 us (544 TFLOP/s of the 320 multiply-adds a pair), bounded by the softmax threads' exponentials
 // and issue slots like the kernel it follows; over the latent rows themselves 611 us.
 //
 // Every wait is bounded (see tcgen05.cuh); lse_attention_expanded_status() reports one that gave up, and contexts on the

@@ -15,7 +15,7 @@ PER_HEAD_LIBRARY_ROWS = 32    # above this many bfloat16 rows the per-head produ
 # Portions of prompts: keys and values of every head made from the gathered latent rows first, or attention over the latent
 # rows themselves.  The former costs one product over the rows that the requests hold (at EXPAND_FLOPS a microsecond) and
 # then 320 multiply-adds a (row, key, head) at EXPANDED_FLOPS; the latter none and 2 rank + 64 at LATENT_FLOPS (measured at
-# 16 heads, a latent of 512: 2,048 rows of a prompt 11 + 41 us, with 4 for the gathering, against 611; the two products
+# 16 heads, a latent of 512: 2,048 rows of a prompt 11 + 39.5 us, with 4 for the gathering, against 611; the two products
 # per head around the latter, 19 us, are saved too).  Both write into buffers of the step.
 EXPAND_FLOPS, EXPANDED_FLOPS, LATENT_FLOPS = 1.0e9, 4.0e8, 1.2e8
 EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an attention of few blocks
