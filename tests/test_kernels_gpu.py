@@ -399,7 +399,7 @@ def test_one_far_key_among_hundreds_is_found(dtype, needle):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("window", [0, 300])
 def test_general_attention_gives_the_same_bits_with_a_block_per_chunk_of_keys(dtype, window):
-    """The general kernel sums a row's keys chunk by chunk (256 keys): one block walks all chunks of its row, or every
+    """The general kernel sums a row's keys chunk by chunk (64 keys): one block walks all chunks of its row, or every
     chunk has a block of its own and a second kernel merges them.  Rows at the edges of chunks (255, 256, 257 keys, ...),
     a far key that carries a row's weight: both ways against dense attention, and bit for bit against each other."""
     rng = random.Random(21)
