@@ -240,10 +240,12 @@ class LatentAttention(Mixer):
             queries = linear_partials(q_latent, self.q_up) if self.q_rank else proj
             ops.latent_query(queries, 0, heads, self.dim, self.rot_dim, self.rot_dims, self.freq, self.rot_factor,
                              step.positions, step.segment_of_token, q_plain, q_wide, self.rank)
-        shape = ([segment.count for segment in step.segments], [segment.first_position + segment.count for segment in step.segments])
-        expanded = 0 if step.decode_only else self._expanded_rows(*shape)
-        if expanded and not torch.cuda.is_current_stream_capturing():
-            expanded = self._gathered_rows(*shape)
+        expanded = 0
+        if not step.decode_only:
+            shape = ([segment.count for segment in step.segments], [segment.first_position + segment.count for segment in step.segments])
+            expanded = self._expanded_rows(*shape)
+            if expanded and not torch.cuda.is_current_stream_capturing():
+                expanded = self._gathered_rows(*shape)
         if expanded:
             values = self._expanded_attention(q_plain, q_wide, step, cache, gate, expanded)
             return linear_partials(values.view(tokens, heads * self.vdim), self.out_weight)
