@@ -130,12 +130,14 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
 }
 
 // map_q: [rows][heads][128]; map_qr: [rows][heads][rank + 64], the rotated values behind column `rank`; map_kv: [gathered
-// rows][2 heads][128], keys of the heads and then values; map_kr: the gathered rows, [rows][rank + 64].
+// rows][2 own_heads][128], keys and then values of the heads first_head .. first_head + own_heads - 1, those that this launch
+// works on; map_kr: the gathered rows, [rows][rank + 64].
 __global__ void __launch_bounds__(THREADS, 1)
 attn_expanded_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_qr,
                         const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_kr,
                         __nv_bfloat16* __restrict__ out, const int* __restrict__ segment_start, const int* __restrict__ first,
-                        const int* __restrict__ context, int num_segments, int heads, int rank, float scale_log2e, int window,
+                        const int* __restrict__ context, int num_segments, int heads, int first_head, int own_heads, int rank,
+                        float scale_log2e, int window,
                         const float* __restrict__ sink, const float* __restrict__ out_gate) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -149,11 +151,11 @@ attn_expanded_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // blocks are numbered tile by tile, all heads of a tile side by side, late tiles (the longest walks) first
-  const int head = blockIdx.x % heads;
+  const int own_head = blockIdx.x % own_heads, head = first_head + own_head;
   pdl_launch_dependents();
   int seg, r0, cnt;
   __shared__ int tile_slot[3];
-  lse_find_tile(segment_start, num_segments, BM, 0, (int)(blockIdx.x / heads), tile_slot, seg, r0, cnt);
+  lse_find_tile(segment_start, num_segments, BM, 0, (int)(blockIdx.x / own_heads), tile_slot, seg, r0, cnt);
   if (seg < 0) return;
   const int nrows = min(BM, cnt - r0);
   const int row_base = segment_start[seg] + r0;
@@ -189,8 +191,8 @@ attn_expanded_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (!mbar_wait(bar(B_KE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) break;
         const uint32_t dst = k_s + s * K_BYTES;
         mbar_expect_tx(bar(B_KF + s), K_BYTES);
-        tma_load_3d(dst, &map_kv, bar(B_KF + s), 0, head, key_row + j * BN);
-        tma_load_3d(dst + KV_BOX, &map_kv, bar(B_KF + s), 64, head, key_row + j * BN);
+        tma_load_3d(dst, &map_kv, bar(B_KF + s), 0, own_head, key_row + j * BN);
+        tma_load_3d(dst + KV_BOX, &map_kv, bar(B_KF + s), 64, own_head, key_row + j * BN);
         tma_load_2d(dst + 2 * KV_BOX, &map_kr, bar(B_KF + s), rank, key_row + j * BN);
       }
     }
@@ -202,8 +204,8 @@ attn_expanded_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (!mbar_wait(bar(B_VE + s), ((uint32_t)(j / STAGES) & 1u) ^ 1u, abort_flag, err)) break;
         const uint32_t dst = v_s + s * V_BYTES;
         mbar_expect_tx(bar(B_VF + s), V_BYTES);
-        tma_load_3d(dst, &map_kv, bar(B_VF + s), 0, heads + head, key_row + j * BN);
-        tma_load_3d(dst + KV_BOX, &map_kv, bar(B_VF + s), 64, heads + head, key_row + j * BN);
+        tma_load_3d(dst, &map_kv, bar(B_VF + s), 0, own_heads + own_head, key_row + j * BN);
+        tma_load_3d(dst + KV_BOX, &map_kv, bar(B_VF + s), 64, own_heads + own_head, key_row + j * BN);
       }
     }
     __syncwarp();
@@ -439,14 +441,15 @@ extern "C" int lse_latent_gather(const void* cache, const int* block_tables, int
 }
 
 // q_plain [tokens, heads, 128], q_wide [tokens, heads, rank + 64] (the rotated values behind column rank), rows [capacity,
-// rank + 64] as gathered, kv [capacity, 2 heads, 128] (every head's key, then every head's value), out [tokens, heads, 128],
-// all bfloat16, contiguous, 16-byte aligned.  sink float32 [heads] or null; out_gate float32 [tokens, heads] or null.
+// rank + 64] as gathered, kv [capacity, 2 own_heads, 128] (the keys of heads first_head .. first_head + own_heads - 1, then
+// their values; the other heads' outputs are left alone), out [tokens, heads, 128], all bfloat16, contiguous, 16-byte aligned.  sink float32 [heads] or null; out_gate float32 [tokens, heads] or null.
 extern "C" int lse_attention_expanded(const void* q_plain, const void* q_wide, const void* rows, const void* kv, void* out,
                                       const int* segment_start, const int* segment_first_pos, const int* segment_context,
-                                      int num_segments, int tokens, int heads, int rank, int capacity, float scale, int window,
+                                      int num_segments, int tokens, int heads, int first_head, int own_heads, int rank,
+                                      int capacity, float scale, int window,
                                       const float* sink, const float* out_gate, cudaStream_t stream) {
   if (tokens <= 0 || num_segments <= 0) return 0;
-  if (heads <= 0 || capacity <= 0 || !(scale > 0.f) || !lse_attention_expanded_supported(D, ROT, D, rank) ||
+  if (heads <= 0 || first_head < 0 || own_heads <= 0 || first_head + own_heads > heads || capacity <= 0 || !(scale > 0.f) || !lse_attention_expanded_supported(D, ROT, D, rank) ||
       (((uintptr_t)q_plain | (uintptr_t)q_wide | (uintptr_t)rows | (uintptr_t)kv | (uintptr_t)out) & 15))
     return LSE_ERR_BAD_ARGUMENT;
   static SmemAllowance allowed;
@@ -454,13 +457,13 @@ extern "C" int lse_attention_expanded(const void* q_plain, const void* q_wide, c
   if (err != cudaSuccess) return (int)err;
   CUtensorMap map_q, map_qr, map_kv, map_kr;
   if (!make_map_3d(&map_q, q_plain, tokens, heads, D, BM) || !make_map_3d(&map_qr, q_wide, tokens, heads, rank + ROT, BM) ||
-      !make_map_3d(&map_kv, kv, capacity, 2 * heads, D, BN) || !make_map_2d(&map_kr, rows, capacity, rank + ROT, BN))
+      !make_map_3d(&map_kv, kv, capacity, 2 * own_heads, D, BN) || !make_map_2d(&map_kr, rows, capacity, rank + ROT, BN))
     return LSE_ERR_BAD_ARGUMENT;
-  const long long blocks = ((long long)(tokens + BM - 1) / BM + num_segments) * heads;      // every request may end with a partial tile
+  const long long blocks = ((long long)(tokens + BM - 1) / BM + num_segments) * own_heads;      // every request may end with a partial tile
   if (blocks > 0x7fffffffLL) return LSE_ERR_TOO_LARGE;
   err = lse_launch(attn_expanded_tc_kernel, (unsigned)blocks, THREADS, SMEM, stream, map_q, map_qr, map_kv, map_kr,
-                               (__nv_bfloat16*)out, segment_start, segment_first_pos, segment_context, num_segments, heads, rank,
-                               scale * LOG2E, window, sink, out_gate);
+                               (__nv_bfloat16*)out, segment_start, segment_first_pos, segment_context, num_segments, heads, first_head,
+                               own_heads, rank, scale * LOG2E, window, sink, out_gate);
   if (err != cudaSuccess) return (int)err;
   return (int)cudaGetLastError();
 }

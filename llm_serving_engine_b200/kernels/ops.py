@@ -872,17 +872,19 @@ def latent_gather(cache: torch.Tensor, block_tables: torch.Tensor, segment_first
 def attention_expanded(q_plain: torch.Tensor, q_wide: torch.Tensor, rows: torch.Tensor, kv: torch.Tensor, out: torch.Tensor,
                        segment_start: torch.Tensor, segment_first_position: torch.Tensor, segment_context: torch.Tensor,
                        scale: float, window: int = 0, sink: torch.Tensor | None = None,
-                       gate: torch.Tensor | None = None) -> torch.Tensor:
+                       gate: torch.Tensor | None = None, first_head: int = 0) -> torch.Tensor:
     """Causal attention of prompt portions over keys and values made from gathered latent rows.
 
     q_plain [T, heads, 128]; q_wide [T, heads, rank + 64] (its last 64 columns are read: the rotated values); rows
-    [N, rank + 64] as :func:`latent_gather` leaves them; kv [N, 2 * heads, 128]: every head's key of a row, then every
-    head's value; out [T, heads, 128]; all bfloat16.  A score is (q_plain . key + q_rotated . row's last 64) * scale.
+    [N, rank + 64] as :func:`latent_gather` leaves them; kv [N, 2 * n, 128]: the keys of heads first_head .. first_head + n - 1
+    of a row, then their values (the other heads' outputs are left alone); out [T, heads, 128]; all bfloat16.  A score is (q_plain . key + q_rotated . row's last 64) * scale.
     ``sink`` float32 [heads] joins the denominator as exp(sink); ``gate`` float32 [T, heads] multiplies a head's output."""
     _need_cuda(q_plain, q_wide, rows, kv, out, segment_start, segment_first_position, segment_context, sink, gate)
     tokens, heads, dim = q_plain.shape
     segments, rank = segment_first_position.shape[0], rows.shape[1] - 64
-    assert q_wide.shape == (tokens, heads, rank + 64) and out.shape == q_plain.shape and kv.shape == (rows.shape[0], 2 * heads, dim)
+    own_heads = kv.shape[1] // 2
+    assert q_wide.shape == (tokens, heads, rank + 64) and out.shape == q_plain.shape
+    assert kv.shape == (rows.shape[0], 2 * own_heads, dim) and 0 <= first_head <= heads - own_heads
     for tensor in (q_plain, q_wide, rows, kv, out):
         assert tensor.is_contiguous() and tensor.dtype == torch.bfloat16
     for tensor, size in ((segment_start, segments + 1), (segment_first_position, segments), (segment_context, segments)):
@@ -893,7 +895,8 @@ def attention_expanded(q_plain: torch.Tensor, q_wide: torch.Tensor, rows: torch.
         raise KernelError(f"attention over expanded latents: heads of {dim}, latents of {rank} are not supported")
     check(library.load().lse_attention_expanded(q_plain.data_ptr(), q_wide.data_ptr(), rows.data_ptr(), kv.data_ptr(), out.data_ptr(),
                                                 segment_start.data_ptr(), segment_first_position.data_ptr(),
-                                                segment_context.data_ptr(), segments, tokens, heads, rank, rows.shape[0],
+                                                segment_context.data_ptr(), segments, tokens, heads, int(first_head), own_heads, rank,
+                                                rows.shape[0],
                                                 float(scale), int(window), _ptr(sink), _ptr(gate), _stream()), "attention_expanded")
     return out
 

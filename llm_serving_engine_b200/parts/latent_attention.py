@@ -19,8 +19,10 @@ PER_HEAD_LIBRARY_ROWS = 32    # above this many bfloat16 rows the per-head produ
 # per head around the latter, 19 us, are saved too).  Both write into buffers of the step.
 EXPAND_FLOPS, EXPANDED_FLOPS, LATENT_FLOPS = 1.0e9, 4.0e8, 1.2e8
 EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an attention of few blocks
-# Keys and values that are held at once (8 KB a row at 16 heads).  They are taken in the middle of a step, beside a cache that
-# was sized before: no more than the buffers of a step of a few thousand rows over the latent rows take.
+# Keys and values that are held at once (512 bytes a row and head), and gathered rows.  They are taken in the middle of a step,
+# beside a cache that was sized before: no more than the buffers of a step of a few thousand rows over the latent rows take.
+# Where the heads' keys and values take more, some heads at a time are made and attended to: 128 heads, 256 rows behind 8,000
+# keys, GROUPED us with all of them at once, against 4,540 over the latent rows.
 EXPAND_MAX_BYTES = 1 << 28
 
 
@@ -178,7 +180,8 @@ class LatentAttention(Mixer):
         expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
                     + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
         latent = 2.0 * pairs * self.heads * (2 * self.rank + self.rot_dim) / LATENT_FLOPS
-        return rows if 2 * rows * self.kv_up.shape[0] <= EXPAND_MAX_BYTES and expanded < latent else 0
+        fits = 2 * rows * max(self.dim + self.vdim, self.rank + self.rot_dim) <= EXPAND_MAX_BYTES      # a head, the gathered rows
+        return rows if fits and expanded < latent else 0
 
     def launch_signature_at(self, segment_counts, contexts):
         rows = self._expanded_rows(segment_counts, contexts)
@@ -186,10 +189,22 @@ class LatentAttention(Mixer):
 
     def _expanded_attention(self, q_plain, q_wide, step, cache, gate, rows: int):
         gathered = ops.latent_gather(cache.keys, cache.block_tables, step.segment_first_position, step.segment_context, rows, self.window)
-        kv = torch.mm(gathered[:, :self.rank], self.kv_up.t()).view(rows, 2 * self.heads, self.dim)
         values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
-        return ops.attention_expanded(q_plain, q_wide, gathered, kv, values, step.segment_start, step.segment_first_position,
-                                      step.segment_context, self.scale, self.window, self.sink, gate)
+        latent, dim = gathered[:, :self.rank], self.dim
+        at_once = min(self.heads, EXPAND_MAX_BYTES // (4 * rows * dim))      # heads whose keys and values are made together
+        buffer = torch.empty(rows * 2 * at_once * dim, dtype=q_plain.dtype, device=q_plain.device)
+        for first in range(0, self.heads, at_once):
+            count = min(at_once, self.heads - first)
+            kv = buffer[:rows * 2 * count * dim].view(rows, 2 * count * dim)
+            if count == self.heads:
+                torch.mm(latent, self.kv_up.t(), out=kv)
+            else:
+                keys, vals = (self.kv_up[at:at + count * dim] for at in (first * dim, (self.heads + first) * dim))
+                torch.mm(latent, keys.t(), out=kv[:, :count * dim])
+                torch.mm(latent, vals.t(), out=kv[:, count * dim:])
+            ops.attention_expanded(q_plain, q_wide, gathered, kv.view(rows, 2 * count, dim), values, step.segment_start,
+                                   step.segment_first_position, step.segment_context, self.scale, self.window, self.sink, gate, first)
+        return values
 
     def _fold_queries(self, q_plain, q_wide) -> None:
         """q_wide[t, h, :rank] = W_uk,h^T q_plain[t, h]: many bfloat16 rows go to the library's batched product (the tensor

@@ -558,6 +558,32 @@ def test_a_latent_that_is_not_finite_reaches_the_rows_that_read_it_only(value, w
             assert bool(got[readers].isnan().all()), column
 
 
+def test_expanded_latent_attention_some_heads_at_a_time():
+    """Five heads, two, two and one at a time, with a sink and gates, bit for bit as all of them at once; a launch leaves the other
+    heads' outputs alone."""
+    from llm_serving_engine_b200.kernels import ops
+
+    torch.manual_seed(8)
+    heads, rank, counts, first = 5, 72, [130, 65], [0, 63]
+    contexts = [a + b for a, b in zip(first, counts)]
+    tokens, capacity = sum(counts), sum(-(-context // 64) * 64 for context in contexts)
+    rows, kv = torch.randn(capacity, rank + 64).bfloat16().cuda(), torch.randn(capacity, 2, heads, 128).bfloat16().cuda()
+    q_plain, q_wide = torch.randn(tokens, heads, 128).bfloat16().cuda(), torch.randn(tokens, heads, rank + 64).bfloat16().cuda()
+    starts, firsts, ends = (torch.tensor(values, dtype=torch.int32).cuda() for values in ([0, 130, 195], first, contexts))
+    sink, gate = torch.randn(heads).cuda(), torch.rand(tokens, heads).cuda()
+    want, got = torch.empty_like(q_plain), torch.full_like(q_plain, 9.0)
+    rest = (starts, firsts, ends, 0.1, 0, sink, gate)
+    ops.attention_expanded(q_plain, q_wide, rows, kv.view(capacity, 2 * heads, 128), want, *rest)
+    for at, count in ((3, 2), (0, 2), (2, 1)):
+        part = kv[:, :, at:at + count].reshape(capacity, 2 * count, 128)
+        before = got.clone()
+        ops.attention_expanded(q_plain, q_wide, rows, part, got, *rest, first_head=at)
+        assert torch.equal(got[:, at:at + count], want[:, at:at + count])
+        others = [head for head in range(heads) if not at <= head < at + count]
+        assert torch.equal(got[:, others], before[:, others])
+    assert int(ops.library.load().lse_attention_expanded_status()) == 0
+
+
 def test_a_gather_without_room_for_the_requests_rows_is_reported():
     """Contexts of 100 and 130 keys are 128 and 192 rows: room for one row fewer is reported, and nothing behind it is written."""
     from llm_serving_engine_b200.kernels import ops

@@ -30,13 +30,13 @@ def latent_model(windows, heads=16, rank=512, width=64, dtype=torch.bfloat16, de
 
 
 def test_a_layer_that_stops_expanding_its_latents_changes_the_key():
-    """A windowed and a full layer: at 20,000 keys a request the full one's keys and values would not fit, the windowed one's are
-    as many as before."""
+    """A windowed and a full layer: at 40,000 keys a request the full one's gathered rows would not fit, the windowed one's are as
+    many as before."""
     model = latent_model([2048, 0])
     counts = [256] * 8
-    short, long = (model.launch_signature(counts, [context] * 8) for context in (2304, 20000))
-    rows = [[block.mixer._expanded_rows(counts, [context] * 8) for block in model.blocks] for context in (2304, 20000)]
-    assert 2 * rows[0][0] * model.blocks[0].mixer.kv_up.shape[0] <= 1 << 28      # bytes of keys and values
+    short, long = (model.launch_signature(counts, [context] * 8) for context in (2304, 40000))
+    rows = [[block.mixer._expanded_rows(counts, [context] * 8) for block in model.blocks] for context in (2304, 40000)]
+    assert 2 * rows[0][0] * 576 <= 1 << 28      # bytes of gathered rows
     assert rows[0][0] == rows[0][1] == rows[1][0] > 0 and rows[1][1] == 0      # the layers' answers as a set are the same
     assert short != long
     assert model.launch_signature([256], [768]) != latent_model([0, 2048]).launch_signature([256], [20000])

@@ -29,8 +29,8 @@ def in_portions(runner, rid, tokens, size):
 
 
 def test_a_captured_step_is_not_replayed_where_a_layer_launches_something_else(monkeypatch):
-    """A windowed and a full latent layer, keys and values bounded so that the full layer makes its own up to 128 keys only: the
-    second portions of two requests capture the step, the later portions of a third have the windowed layer's buffer of the same
+    """A windowed and a full latent layer, room bounded so that the full layer makes keys and values up to 128 keys only, a head at
+    a time: the second portions of two requests capture the step, the later portions of a third have the windowed layer's buffer of the same
     size, but a full layer that goes over the latent rows.  Every logit against the latent rows' kernel launch by launch."""
     model = latent_model([64, 0], heads=2, rank=64, device="cuda", scale=0.07)
     generator = torch.Generator().manual_seed(5)
@@ -39,7 +39,7 @@ def test_a_captured_step_is_not_replayed_where_a_layer_launches_something_else(m
     monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0e30)      # never worth it
     want = [in_portions(plain, "r", tokens, 64) for tokens in prompts]
     monkeypatch.setattr(latent_attention, "LATENT_FLOPS", 1.0)         # always worth it, where it fits
-    monkeypatch.setattr(latent_attention, "EXPAND_MAX_BYTES", 2 * 128 * model.blocks[0].mixer.kv_up.shape[0])
+    monkeypatch.setattr(latent_attention, "EXPAND_MAX_BYTES", 128 * 512)
     graphs = runner_for(model, use_graphs=True)
     for index, tokens in enumerate(prompts):
         got = in_portions(graphs, "r", tokens, 64)
