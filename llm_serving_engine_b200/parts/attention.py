@@ -32,8 +32,12 @@ ROWS_KERNEL_BELOW = int(os.environ.get("LSE_ROWS_KERNEL_BELOW", "64"))
 ROWS_KERNEL_BLOCKS = 256
 # The general kernels (float32, other head sizes, windows): a step's portions go to the kernel that takes tiles of rows with
 # a request's keys read once for them, its single tokens to the one that takes a row a block, as in a decode step.  Portions
-# of two rows do not fill a tile: they go row by row while the step is small.
-GENERIC_ROWS_UP_TO = 64
+# of two rows do not fill a tile, and a step of few rows over short contexts has not enough tiles: up to GENERIC_ROWS_UP_TO rows
+# such steps go row by row, all rows in one launch.  Few are GENERIC_ROWS_CHUNKS chunks of 64 keys, over all rows and groups of
+# up to eight heads (float32; row by row against tiles: 40 rows of a prompt, 12 / 2 heads of 128, 80 chunks, 8.8 against 20.0 us;
+# 8 heads of 64, 320 chunks, 7.4 against 14.0; eight rows behind 2,000 keys, 512 chunks, 21.4 against 27.6; 20 rows of 32 heads
+# of 128, 640 chunks, 16.6 against 19.7; at 1,024 chunks the two are alike, 64 rows behind 2,000 keys are slower).
+GENERIC_ROWS_UP_TO, GENERIC_ROWS_CHUNKS = 64, 640
 
 
 @register_mixer("gqa_attention")
@@ -120,7 +124,7 @@ class GroupedQueryAttention(Mixer):
         if max(segment_counts) == 1:
             return ()
         if not ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, self.ctx.dtype, self.window):
-            return ("general", *self._general_kernels(segment_counts))
+            return ("general",)
         if sum(segment_counts) < ROWS_KERNEL_BELOW:
             return ("rows",)
         portions, singles = self._portions(segment_counts)
@@ -128,7 +132,10 @@ class GroupedQueryAttention(Mixer):
 
     def launch_signature_at(self, segment_counts, contexts):
         answer = self.launch_signature(segment_counts)
-        return (*answer, self._context_class(contexts)) if answer[:1] == ("general",) else answer
+        if answer[:1] != ("general",):
+            return answer
+        longest = self._context_class(contexts)
+        return ("general", *self._general_kernels(segment_counts, longest), longest)
 
     def decode_signature(self, rows, many_keys):
         if not ops.attention_mma_supported(self.head_dim, self.n_q, self.n_kv, self.ctx.dtype, self.window):
@@ -141,10 +148,12 @@ class GroupedQueryAttention(Mixer):
         keys a row, not for all that the block tables could hold."""
         return 1 << max(7, (max(contexts) - 1).bit_length())
 
-    def _general_kernels(self, segment_counts: list[int]) -> tuple[bool, bool]:
-        """Whether the general attention's tiles kernel takes the portions of a step, and the rows kernel its single tokens."""
-        most = max(segment_counts)
-        if most == 1 or (most == 2 and sum(segment_counts) <= GENERIC_ROWS_UP_TO):
+    def _general_kernels(self, segment_counts: list[int], longest: int) -> tuple[bool, bool]:
+        """Whether the general attention's tiles kernel takes the portions of a step whose contexts are within the class ``longest``,
+        and the rows kernel its single tokens."""
+        most, rows = max(segment_counts), sum(segment_counts)
+        chunks = rows * self.n_kv * -(-(self.n_q // self.n_kv) // 8) * -(-longest // 64)
+        if most == 1 or (rows <= GENERIC_ROWS_UP_TO and (most == 2 or chunks <= GENERIC_ROWS_CHUNKS)):
             return False, False
         if not ops.attention_generic_tile_tokens(self.head_dim, self.n_q, self.n_kv):
             return False, False
@@ -156,8 +165,8 @@ class GroupedQueryAttention(Mixer):
         if step.decode_only:      # a captured step's contexts grow until its tables are full
             ops.paged_attention_generic(*arguments)
             return
-        tiles, singles = self._general_kernels([segment.count for segment in step.segments])
         longest = self._context_class([segment.first_position + segment.count for segment in step.segments])
+        tiles, singles = self._general_kernels([segment.count for segment in step.segments], longest)
         if not tiles:
             ops.paged_attention_generic(*arguments, max_context=longest)
             return

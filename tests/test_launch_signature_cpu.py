@@ -1,8 +1,11 @@
 """What the captured steps with prompt portions are kept by (no GPU): steps that launch different things have different keys."""
+from types import SimpleNamespace
+
 import torch
 
 from llm_serving_engine_b200.config.model_config import LayerSpec, ModelSpec, PartSpec
 from llm_serving_engine_b200.models import DecoderModel, expected_tensors
+from llm_serving_engine_b200.parts.attention import GroupedQueryAttention
 from llm_serving_engine_b200.parts.base import Mixer
 from llm_serving_engine_b200.parts.branches import ParallelMixers
 
@@ -86,3 +89,24 @@ def test_parallel_mixers_hand_on_what_their_branches_answer_at_their_contexts():
     assert answers[0] == () and len(set(answers)) == 3
     part.branches.reverse()
     assert part.launch_signature_at([8], [500]) != answers[1]      # another branch's answer
+
+
+def test_general_attention_takes_few_rows_over_short_contexts_row_by_row():
+    """The rule by rows and chunks at its edges, and that everything it follows from is in the key."""
+    mixer = object.__new__(GroupedQueryAttention)
+    mixer.head_dim, mixer.n_q, mixer.n_kv, mixer.window = 128, 12, 2, 0
+    mixer.ctx = SimpleNamespace(dtype=torch.float32)
+
+    def route(counts, contexts):
+        signature = mixer.launch_signature_at(counts, contexts)
+        longest = mixer._context_class(contexts)
+        assert signature == ("general", *mixer._general_kernels(counts, longest), longest)
+        return signature[1:3]
+
+    assert route([64], [64]) == (False, False) and route([65], [65]) == (True, False)
+    assert route([64], [256]) == (False, False) and route([64], [512]) == (True, False)      # 512 and 1,024 chunks
+    assert route([8], [2048]) == (False, False) and route([10, 1], [2048, 5]) == (True, True)
+    assert route([2] * 32, [4096] * 32) == (False, False) and route([2] * 33, [200] * 33) == (True, False)
+    assert mixer.launch_signature_at([1, 1], [9, 9]) == ()
+    mixer.head_dim = 192                                                                     # tiles take heads of up to 128
+    assert route([500], [500]) == (False, False)
