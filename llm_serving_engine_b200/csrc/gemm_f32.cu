@@ -429,9 +429,10 @@ cudaError_t few_rows(const Product& p, cudaStream_t stream) {
   if (p.M == 2) return launch_few<2, 2, 1, 1, 64, 4>(p, stream);
   if (p.M <= 4) return launch_few<4, 2, 1, 1, 64, 4>(p, stream);
   if (p.M <= 8) return wide ? launch_few<8, 4, 2, 1, 32, 4>(p, stream) : launch_few<8, 4, 1, 1, 64, 4>(p, stream);
-  // four columns a lane leave blocks of 128 columns: too few of them, each walking the whole of k, and one column is better
-  // (2,048 x 1,536 whole: 43.6 us with 16 blocks, FEW_16 with 64)
-  if ((long long)((p.N + 127) / 128) * p.ranges < gpu_sms()) return launch_few<16, 4, 1, 1, 64, 4>(p, stream);
+  // four columns a lane leave blocks of 128 columns: where those are few, one column a lane is better (2,048 x 1,536 whole 21.6
+  // against 43.6 us with 16 blocks of 128 columns, 1,536 x 8,960 whole 120 against 251 with 12; as stacks 8.0 against 6.5 with
+  // 128, 33 either way with 84)
+  if ((long long)((p.N + 127) / 128) * p.ranges < 64) return launch_few<16, 4, 1, 1, 64, 4>(p, stream);
   return wide ? launch_few<16, 4, 4, 1, 32, 3>(p, stream) : launch_few<16, 4, 4, 1, 64, 3>(p, stream);
 }
 }  // namespace
