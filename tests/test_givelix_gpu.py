@@ -575,7 +575,7 @@ def test_expanded_latent_attention_some_heads_at_a_time():
     rest = (starts, firsts, ends, 0.1, 0, sink, gate)
     ops.attention_expanded(q_plain, q_wide, rows, kv.view(capacity, 2 * heads, 128), want, *rest)
     for at, count in ((3, 2), (0, 2), (2, 1)):
-        part = kv[:, :, at:at + count].reshape(capacity, 2 * count, 128)
+        part = kv[:, :, at:at + count].reshape(capacity, 2 * count, 128).contiguous()
         before = got.clone()
         ops.attention_expanded(q_plain, q_wide, rows, part, got, *rest, first_head=at)
         assert torch.equal(got[:, at:at + count], want[:, at:at + count])
