@@ -39,8 +39,8 @@ template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile
 // Tiles lie transposed in shared memory (cp.async of four bytes, which needs no alignment either), so that neighbouring
 // rows of A come as register pairs for the paired multiply-add, two rounded operations an instruction: it leaves issue
 // slots for the reads, which single ones do not.
-// gridDim.y == 1: the block adds the ranges up itself.  Else block row y takes range y and writes its sum to
-// C + y * part_stride (no bias).
+// gridDim.z == 1: the block adds the ranges up itself.  Else block z takes range z and writes its sum to
+// C + z * part_stride (no bias).
 __device__ __forceinline__ void fma_pair(uint64_t& c, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(c) : "l"(a), "l"(b));
 }
@@ -68,13 +68,12 @@ gemm_f32_tiles_kernel(const float* __restrict__ A, const float* __restrict__ B, 
   float* const As = tiles;                              // [STAGES][BK][A_PITCH]
   float* const Bs = tiles + STAGES * BK * A_PITCH;      // [STAGES][BK][B_PITCH]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row_tiles = (M + BM - 1) / BM;      // tiles that share columns of B side by side; all in x, which has no small limit
-  const int m0 = (int)(blockIdx.x % row_tiles) * BM, n0 = (int)(blockIdx.x / row_tiles) * BN;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int am = (warp % (BM / WM)) * WM + (lane % LM) * 4;        // this thread's first four rows; the others 4 LM apart
   const int bn = (warp / (BM / WM)) * WN + (lane / LM) * 4;        // its first four columns; the others 4 LN apart
   const int range = f32_range(K);
-  const bool split = gridDim.y > 1;
-  const int k_lo = split ? blockIdx.y * range : 0;
+  const bool split = gridDim.z > 1;
+  const int k_lo = split ? blockIdx.z * range : 0;
   const int k_hi = split ? min(K, k_lo + range) : K;
   const int n_tiles = (k_hi - k_lo + BK - 1) / BK;
   pdl_launch_dependents();
@@ -191,7 +190,7 @@ gemm_f32_tiles_kernel(const float* __restrict__ A, const float* __restrict__ B, 
       }
     }
   }
-  float* const dst = C + (split ? (size_t)blockIdx.y * part_stride : 0);
+  float* const dst = C + (split ? (size_t)blockIdx.z * part_stride : 0);
   const bool wide = (((uintptr_t)dst) & 15) == 0 && ldc % 4 == 0;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -362,11 +361,15 @@ cudaError_t launch_tiles(const Product& p, cudaStream_t stream) {
   static SmemAllowance allowed;
   cudaError_t err = allow_smem(kernel, smem, allowed);
   if (err != cudaSuccess) return err;
-  const long long blocks = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const dim3 grid((unsigned)blocks, p.ranges);
-  return lse_launch(kernel, grid, (BM / WM) * (BN / WN) * 32, smem, stream, p.A, p.B, p.bias, p.C, p.M, p.N, p.K,
-                    p.lda, p.ldb, p.ldc, p.part_stride);
+  // tiles of columns lie in the grid's second dimension, which ends at 65,535 (numbered in the first they cost a hundredth of
+  // the product: the compiler schedules the loop worse)
+  for (long long n = 0; n < p.N && err == cudaSuccess; n += 65535LL * BN) {
+    const int cols = (int)(p.N - n < 65535LL * BN ? p.N - n : 65535LL * BN);
+    const dim3 grid((p.M + BM - 1) / BM, (cols + BN - 1) / BN, p.ranges);
+    err = lse_launch(kernel, grid, (BM / WM) * (BN / WN) * 32, smem, stream, p.A, p.B + n * p.ldb,
+                     p.bias ? p.bias + n : nullptr, p.C + n, p.M, cols, p.K, p.lda, p.ldb, p.ldc, p.part_stride);
+  }
+  return err;
 }
 
 template <int ROWS, int TM, int TN, int GROUPS, int FEW_BK, int FEW_STAGES>
