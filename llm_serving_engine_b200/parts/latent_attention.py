@@ -22,7 +22,7 @@ EXPAND_OVERHEAD_US = 15.0     # two more launches, and the first tiles of an att
 # Keys and values that are held at once (512 bytes a row and head), and gathered rows.  They are taken in the middle of a step,
 # beside a cache that was sized before: no more than the buffers of a step of a few thousand rows over the latent rows take.
 # Where the heads' keys and values take more, some heads at a time are made and attended to: 128 heads, 256 rows behind 8,000
-# keys, GROUPED us with all of them at once, against 4,540 over the latent rows.
+# keys, captured: 891 us (572 with all of them at once, in 805 MB) against 4,540 over the latent rows.
 EXPAND_MAX_BYTES = 1 << 28
 
 
@@ -124,6 +124,7 @@ class LatentAttention(Mixer):
         self.v_up = self.kv_up[self.heads * self.dim:].view(self.heads, self.vdim, self.rank).transpose(1, 2)
         self.sink = weights[names["sink"]].to(torch.float32).contiguous() if p.get("sink", False) else None
         self.out_weight = weights[names["out"]].contiguous()
+        self._tile: int | None = None      # keys of a tile of the expanded attention, 0: not for this layer (see _key_tile)
 
     @staticmethod
     def _gates(params) -> int:
@@ -162,17 +163,24 @@ class LatentAttention(Mixer):
     def cache_requirement(cls, params, hidden_size):
         return PagedLatent(int(params["kv_rank"]) + int(params["rot_dim"]), int(params.get("window", 0)))
 
+    def _key_tile(self) -> int:
+        """Keys of a tile of the attention over expanded keys and values, 0 if it does not take this layer."""
+        if self._tile is None:
+            taken = self.gates <= self.heads and self.scale > 0.0 and ops.attention_expanded_supported(
+                self.dim, self.rot_dim, self.vdim, self.rank, self.ctx.dtype)
+            self._tile = ops.attention_expanded_tile() if taken else 0
+        return self._tile
+
     def _gathered_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """Latent rows that a step of this shape may read, each request's rounded up to whole key tiles."""
-        tile = ops.attention_expanded_tile()
+        tile = self._key_tile()
         return sum(-(-(context - (max(0, context - count + 1 - self.window) if self.window > 0 else 0)) // tile) * tile
                    for count, context in zip(segment_counts, contexts))
 
     def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
         the latent rows.  ``contexts``: keys of each request after the step."""
-        if min(segment_counts) == 1 or self.gates > self.heads or not self.scale > 0.0 or not ops.attention_expanded_supported(
-                self.dim, self.rot_dim, self.vdim, self.rank, self.ctx.dtype):
+        if min(segment_counts) == 1 or not self._key_tile():
             return 0
         pairs = sum(count * (min(context, self.window) if self.window > 0 else context - count // 2)
                     for count, context in zip(segment_counts, contexts))
@@ -191,17 +199,18 @@ class LatentAttention(Mixer):
         gathered = ops.latent_gather(cache.keys, cache.block_tables, step.segment_first_position, step.segment_context, rows, self.window)
         values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
         latent, dim = gathered[:, :self.rank], self.dim
-        at_once = min(self.heads, EXPAND_MAX_BYTES // (4 * rows * dim))      # heads whose keys and values are made together
+        at_once = EXPAND_MAX_BYTES // (4 * rows * dim)      # heads whose keys and values are made together
+        if at_once >= self.heads:
+            kv = torch.mm(latent, self.kv_up.t()).view(rows, 2 * self.heads, dim)
+            return ops.attention_expanded(q_plain, q_wide, gathered, kv, values, step.segment_start, step.segment_first_position,
+                                          step.segment_context, self.scale, self.window, self.sink, gate)
         buffer = torch.empty(rows * 2 * at_once * dim, dtype=q_plain.dtype, device=q_plain.device)
         for first in range(0, self.heads, at_once):
             count = min(at_once, self.heads - first)
             kv = buffer[:rows * 2 * count * dim].view(rows, 2 * count * dim)
-            if count == self.heads:
-                torch.mm(latent, self.kv_up.t(), out=kv)
-            else:
-                keys, vals = (self.kv_up[at:at + count * dim] for at in (first * dim, (self.heads + first) * dim))
-                torch.mm(latent, keys.t(), out=kv[:, :count * dim])
-                torch.mm(latent, vals.t(), out=kv[:, count * dim:])
+            keys, vals = (self.kv_up[at:at + count * dim] for at in (first * dim, (self.heads + first) * dim))
+            torch.mm(latent, keys.t(), out=kv[:, :count * dim])
+            torch.mm(latent, vals.t(), out=kv[:, count * dim:])
             ops.attention_expanded(q_plain, q_wide, gathered, kv.view(rows, 2 * count, dim), values, step.segment_start,
                                    step.segment_first_position, step.segment_context, self.scale, self.window, self.sink, gate, first)
         return values
