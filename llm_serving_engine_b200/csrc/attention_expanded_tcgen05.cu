@@ -69,8 +69,8 @@ __device__ __forceinline__ int rows_before(const int* __restrict__ first, const 
   return sum;
 }
 
-// Whether one of two bfloat16 numbers is infinite or NaN (an exponent of ones: it carries into the sign when it is raised by one).
-__device__ __forceinline__ bool not_finite(uint32_t two) { return (((two & 0x7f807f80u) + 0x00800080u) & 0x80008000u) != 0; }
+// Not zero if one of two bfloat16 numbers is infinite or NaN (an exponent of ones: it carries into the sign when it is raised by one).
+__device__ __forceinline__ uint32_t not_finite(uint32_t two) { return ((two & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
 
 // rows[r] for r < capacity: a warp a row; rows of no request, and those that round a request up, are zeros.
 __global__ void __launch_bounds__(256)
@@ -112,16 +112,24 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
       src = cache + ((size_t)page * page_size + pos % page_size) * width;
     }
   }
-  bool broken = false;
-  for (int c = lane * 8; c < width; c += 256) {
-    const uint4 v = src ? *reinterpret_cast<const uint4*>(src + c) : make_uint4(0u, 0u, 0u, 0u);
-    broken |= c < width - ROT && (not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w));
-    *reinterpret_cast<uint4*>(rows + (size_t)r * width + c) = v;
+  uint32_t broken = 0;
+  for (int base = lane * 8; base < width; base += 4 * 256) {      // all pieces of a row of up to 1,024 values on their way together
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[i] = src && base + 256 * i < width ? *reinterpret_cast<const uint4*>(src + base + 256 * i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = base + 256 * i;
+      if (c >= width) continue;
+      *reinterpret_cast<uint4*>(rows + (size_t)r * width + c) = v[i];
+      broken |= c < width - ROT ? not_finite(v[i].x) | not_finite(v[i].y) | not_finite(v[i].z) | not_finite(v[i].w) : 0u;
+    }
   }
   // A latent that is not finite makes NaN of every row that attends to it, and must not reach those that do not: the values made
   // of it would, as hidden keys of a tile have no weight but are multiplied by it.  So it has finite keys and values, and NaN
   // where the scores are made, which hidden keys do not have.
-  if (__any_sync(0xffffffffu, broken)) {
+  if (__any_sync(0xffffffffu, broken != 0)) {
     for (int c = lane * 8; c < width; c += 256) {
       const uint32_t x = c < width - ROT ? 0u : 0x7fc07fc0u;
       *reinterpret_cast<uint4*>(rows + (size_t)r * width + c) = make_uint4(x, x, x, x);

@@ -180,16 +180,21 @@ class LatentAttention(Mixer):
     def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
         the latent rows.  ``contexts``: keys of each request after the step."""
+        return _size_class(rows) if (rows := self._worth_expanding(segment_counts, contexts)) else 0
+
+    def _worth_expanding(self, segment_counts: list[int], contexts: list[int]) -> int:
+        """The same without the size class: the rows that there are.  Whether it is worth it goes by the class."""
         if min(segment_counts) == 1 or not self._key_tile():
             return 0
         pairs = sum(count * (min(context, self.window) if self.window > 0 else context - count // 2)
                     for count, context in zip(segment_counts, contexts))
-        rows = _size_class(self._gathered_rows(segment_counts, contexts))
+        exact = self._gathered_rows(segment_counts, contexts)
+        rows = _size_class(exact)
         expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
                     + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
         latent = 2.0 * pairs * self.heads * (2 * self.rank + self.rot_dim) / LATENT_FLOPS
         fits = 2 * rows * max(self.dim + self.vdim, self.rank + self.rot_dim) <= EXPAND_MAX_BYTES      # a head, the gathered rows
-        return rows if fits and expanded < latent else 0
+        return exact if fits and expanded < latent else 0
 
     def launch_signature_at(self, segment_counts, contexts):
         rows = self._expanded_rows(segment_counts, contexts)
@@ -197,13 +202,14 @@ class LatentAttention(Mixer):
 
     def _expanded_attention(self, q_plain, q_wide, step, cache, gate, rows: int):
         gathered = ops.latent_gather(cache.keys, cache.block_tables, step.segment_first_position, step.segment_context, rows, self.window)
-        values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
         latent, dim = gathered[:, :self.rank], self.dim
         at_once = EXPAND_MAX_BYTES // (4 * rows * dim)      # heads whose keys and values are made together
         if at_once >= self.heads:
             kv = torch.mm(latent, self.kv_up.t()).view(rows, 2 * self.heads, dim)
+            values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
             return ops.attention_expanded(q_plain, q_wide, gathered, kv, values, step.segment_start, step.segment_first_position,
                                           step.segment_context, self.scale, self.window, self.sink, gate)
+        values = torch.empty((q_plain.shape[0], self.heads, self.vdim), dtype=q_plain.dtype, device=q_plain.device)
         buffer = torch.empty(rows * 2 * at_once * dim, dtype=q_plain.dtype, device=q_plain.device)
         for first in range(0, self.heads, at_once):
             count = min(at_once, self.heads - first)
@@ -267,9 +273,9 @@ class LatentAttention(Mixer):
         expanded = 0
         if not step.decode_only:
             shape = ([segment.count for segment in step.segments], [segment.first_position + segment.count for segment in step.segments])
-            expanded = self._expanded_rows(*shape)
-            if expanded and not torch.cuda.is_current_stream_capturing():
-                expanded = self._gathered_rows(*shape)
+            expanded = self._worth_expanding(*shape)
+            if expanded and torch.cuda.is_current_stream_capturing():
+                expanded = _size_class(expanded)
         if expanded:
             values = self._expanded_attention(q_plain, q_wide, step, cache, gate, expanded)
             return linear_partials(values.view(tokens, heads * self.vdim), self.out_weight)
