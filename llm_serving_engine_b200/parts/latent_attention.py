@@ -171,24 +171,22 @@ class LatentAttention(Mixer):
             self._tile = ops.attention_expanded_tile() if taken else 0
         return self._tile
 
-    def _gathered_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
-        """Latent rows that a step of this shape may read, each request's rounded up to whole key tiles."""
-        tile = self._key_tile()
-        return sum(-(-(context - (max(0, context - count + 1 - self.window) if self.window > 0 else 0)) // tile) * tile
-                   for count, context in zip(segment_counts, contexts))
-
     def _expanded_rows(self, segment_counts: list[int], contexts: list[int]) -> int:
         """How many rows of keys and values are made for a step of this shape (a size class), or 0: the attention runs over
         the latent rows.  ``contexts``: keys of each request after the step."""
         return _size_class(rows) if (rows := self._worth_expanding(segment_counts, contexts)) else 0
 
     def _worth_expanding(self, segment_counts: list[int], contexts: list[int]) -> int:
-        """The same without the size class: the rows that there are.  Whether it is worth it goes by the class."""
-        if min(segment_counts) == 1 or not self._key_tile():
+        """The same without the size class: the rows that there are, each request's rounded up to whole key tiles.  Whether it is
+        worth it goes by the class."""
+        tile = self._key_tile() if self._tile is None else self._tile
+        if min(segment_counts) == 1 or not tile:
             return 0
-        pairs = sum(count * (min(context, self.window) if self.window > 0 else context - count // 2)
-                    for count, context in zip(segment_counts, contexts))
-        exact = self._gathered_rows(segment_counts, contexts)
+        window, exact, pairs = self.window, 0, 0
+        for count, context in zip(segment_counts, contexts):
+            first = max(0, context - count + 1 - window) if window > 0 else 0
+            exact += -(-(context - first) // tile) * tile
+            pairs += count * (min(context, window) if window > 0 else context - count // 2)
         rows = _size_class(exact)
         expanded = (2.0 * rows * self.kv_up.numel() / EXPAND_FLOPS
                     + 2.0 * pairs * self.heads * (self.dim + self.rot_dim + self.vdim) / EXPANDED_FLOPS + EXPAND_OVERHEAD_US)
@@ -274,7 +272,7 @@ class LatentAttention(Mixer):
         if not step.decode_only:
             shape = ([segment.count for segment in step.segments], [segment.first_position + segment.count for segment in step.segments])
             expanded = self._worth_expanding(*shape)
-            if expanded and torch.cuda.is_current_stream_capturing():
+            if expanded and step.max_context is None:      # a step that is captured for its class
                 expanded = _size_class(expanded)
         if expanded:
             values = self._expanded_attention(q_plain, q_wide, step, cache, gate, expanded)

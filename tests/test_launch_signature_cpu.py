@@ -59,7 +59,7 @@ def test_a_long_prompt_in_portions_meets_few_classes():
     for context in range(512, 16385, 512):
         key = model.launch_signature([512], [context])
         keys.add(key)
-        rows, exact = mixer._expanded_rows([512], [context]), mixer._gathered_rows([512], [context])
+        rows, exact = mixer._expanded_rows([512], [context]), mixer._worth_expanding([512], [context])
         assert key == ((0, ("expanded", rows)),) and exact == context <= rows <= 1.5 * exact
     assert len(keys) <= 2 * 5 + 1
 
