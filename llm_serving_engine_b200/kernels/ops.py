@@ -2,6 +2,8 @@
 current CUDA stream.  Every function needs CUDA tensors; there is no CPU path."""
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import library
@@ -838,7 +840,12 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
 
 def attention_expanded_supported(dim: int, rot: int, vdim: int, rank: int, dtype: torch.dtype) -> bool:
     """Whether latent attention over expanded keys and values takes these sizes (:func:`attention_expanded`)."""
-    return dtype == torch.bfloat16 and bool(library.load().lse_attention_expanded_supported(int(dim), int(rot), int(vdim), int(rank)))
+    return dtype == torch.bfloat16 and _expanded_sizes(int(dim), int(rot), int(vdim), int(rank))
+
+
+@functools.lru_cache(maxsize=256)
+def _expanded_sizes(dim: int, rot: int, vdim: int, rank: int) -> bool:
+    return bool(library.load().lse_attention_expanded_supported(dim, rot, vdim, rank))      # follows from the sizes alone
 
 
 def attention_expanded_tile() -> int:
