@@ -1443,6 +1443,7 @@ def timeline(args) -> int:
     import torch
 
     os.environ["LSE_TRACE"] = "1"   # before the library is loaded
+    os.environ["LSE_DECODE_LAYERS"] = "0"   # the kernels one by one: the step in one launch has no hand-overs to show
     from llm_serving_engine_b200.cache.manager import CacheManager
     from llm_serving_engine_b200.config.runtime_config import CacheConfig
     from llm_serving_engine_b200.engine.step import StepEntry, StepRunner

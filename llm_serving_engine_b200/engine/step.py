@@ -71,6 +71,7 @@ class StepContext:
         self.max_segment_tokens = 0
         self.max_context = 0                         # None: not known on the host (a replayed graph)
         self.decode_only = False                     # every segment brings exactly one token
+        self.every_row_wanted = False                # want_rows is 0, 1, ... (known on the host)
         self.long_context = False                    # some request holds more than LONG_CONTEXT keys (known on the host always:
                                                      # graphs of decode steps are captured for either case)
         self.many_keys = False                       # some request holds ops.DECODE_MANY_KEYS keys or more (likewise)
@@ -269,6 +270,7 @@ class StepRunner:
         if wanted_all_rows:
             host[lay.want[0]:lay.want[1]] = np.arange(lay.wanted, dtype=np.int32)
         step.decode_only = step.max_segment_tokens == 1
+        step.every_row_wanted = wanted_all_rows or (step.decode_only and all(entry.want == [0] for entry in entries))
         return step
 
     def _pack_decode(self, entries: list[StepEntry], host: np.ndarray, lay: _Layout) -> StepContext:
@@ -311,7 +313,7 @@ class StepRunner:
         step.max_context = max(firsts) + 1
         step.long_context = step.max_context > LONG_CONTEXT
         step.many_keys = step.max_context >= ops.DECODE_MANY_KEYS
-        step.decode_only = True
+        step.decode_only = step.every_row_wanted = True
         return step
 
     def _views(self, step: StepContext, dev: torch.Tensor, lay: _Layout):

@@ -3,6 +3,7 @@ current CUDA stream.  Every function needs CUDA tensors; there is no CPU path.""
 from __future__ import annotations
 
 import functools
+from ctypes import c_float, c_longlong
 
 import torch
 
@@ -536,13 +537,13 @@ def gemm_bf16_skinny_status() -> int:
 
 
 _STATUS_WORDS = (("gemm_tcgen05", "lse_gemm_bf16_skinny_status"), ("attention_tcgen05", "lse_attention_tc_status"),
-                 ("attention_expanded_tcgen05", "lse_attention_expanded_status"))
+                 ("attention_expanded_tcgen05", "lse_attention_expanded_status"), ("decode_layers", "lse_decode_layers_status"))
 
 
 def kernel_status_async(host_words: torch.Tensor) -> None:
     """Queue, on the current stream, copies of the status words of the kernels with bounded waits (the
-    few-rows product, the tcgen05 prompt attention, the one over expanded latents) into ``host_words`` (pinned int32,
-    a word each; [2]: the first two).  Once the
+    few-rows product, the tcgen05 prompt attention, the one over expanded latents, the decode step in one launch) into
+    ``host_words`` (pinned int32, a word each; [2]: the first two).  Once the
     stream has got there, a non-zero word says that a wait gave up: that block wrote nothing, and
     what the step computed is not to be used."""
     assert host_words.dtype == torch.int32 and host_words.numel() >= 2 and host_words.is_pinned()
@@ -564,6 +565,39 @@ def kernel_status_reset() -> None:
             getattr(lib, entry + "_reset")()
     for _, counters in _ATTENTION_TC_SCRATCH.values():   # a block that gave up may have left its arrival uncounted
         counters.zero_()
+
+
+def decode_layers_supported(layers: int, rows: int, hidden: int, inter: int, n_q: int, n_kv: int, vocab: int) -> bool:
+    """Whether :func:`decode_layers` takes a step of these sizes on this GPU."""
+    return bool(library.load().lse_decode_layers_supported(sm_count(), layers, rows, hidden, inter, n_q, n_kv, vocab))
+
+
+def decode_layers(layer_pointers: list, eps: list, embedding: torch.Tensor, embedding_scale: float, head: torch.Tensor,
+                  final_norm: torch.Tensor, final_eps: float, inv_freq: torch.Tensor, pairing: int, token_ids: torch.Tensor,
+                  positions: torch.Tensor, segment_of_token: torch.Tensor, slot_mapping: torch.Tensor, block_tables: torch.Tensor,
+                  keys: torch.Tensor, inter: int, n_q: int, scale: float) -> torch.Tensor:
+    """A step of single tokens through all layers and the head: float32 logits [rows, vocab].
+
+    ``layer_pointers``: per layer the addresses of qkv, o, gate_up and down weights, the qkv bias (or None), both norms'
+    weights, the cached keys and values; ``eps``: both norms' of every layer; ``keys``: one layer's cache, for its shape."""
+    _need_cuda(embedding, head, token_ids, keys)
+    rows, hidden, vocab = token_ids.shape[0], embedding.shape[1], head.shape[0]
+    pages, n_kv, page_size, _ = keys.shape
+    lib = library.load()
+    blocks, layers = sm_count(), len(layer_pointers)
+    flat = (c_longlong * (9 * layers))(*[pointer or 0 for layer in layer_pointers for pointer in layer])
+    places = (c_longlong * 14)()
+    if lib.lse_decode_layers_scratch(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, places) != 0:
+        raise KernelError("decode_layers: a step of these sizes does not fit")
+    scratch = torch.empty(places[13], dtype=torch.uint8, device=embedding.device)
+    logits = torch.empty((rows, vocab), dtype=torch.float32, device=embedding.device)
+    check(lib.lse_decode_layers(flat, (c_float * (2 * layers))(*eps), layers, embedding.data_ptr(), embedding.shape[0],
+                                float(embedding_scale), head.data_ptr(), final_norm.data_ptr(), float(final_eps), inv_freq.data_ptr(),
+                                int(pairing), token_ids.data_ptr(), positions.data_ptr(), segment_of_token.data_ptr(),
+                                slot_mapping.data_ptr(), block_tables.data_ptr(), block_tables.stride(0), block_tables.shape[0], rows,
+                                hidden, inter, n_q, n_kv, vocab, page_size, pages, float(scale), scratch.data_ptr(),
+                                logits.data_ptr(), blocks, _stream()), "decode_layers")
+    return logits
 
 
 def argmax(logits: torch.Tensor, out: torch.Tensor) -> torch.Tensor:

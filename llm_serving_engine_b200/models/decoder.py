@@ -11,6 +11,7 @@ from ..parts.base import (BLOCKS, FEED_FORWARDS, MIXERS, NORMS, POSITION_ENCODIN
                           ResidualStream, cache_needs)
 from ..parts.linear import linear
 from ..weights.tensor_spec import TensorSpec
+from .decode_layers import DecodeLayers
 
 _PART_ROLES = ("mixer_norm", "mixer", "feed_forward_norm", "feed_forward")
 
@@ -160,6 +161,7 @@ class DecoderModel:
         local = {name[len(prefix):]: tensor for name, tensor in weights.items() if name.startswith(prefix)}
         self.final_norm = NORMS.get(spec.final_norm.kind)(spec.final_norm.params, local, ctx)
         self.layer_hook = None   # for inspection: called as hook(position in the order, stream) after every layer run
+        self._decode_layers = DecodeLayers.of(self)    # decode steps in one launch, where the layers are of that kind
 
     @property
     def graph_safe(self) -> bool:
@@ -214,6 +216,12 @@ class DecoderModel:
     def forward(self, step, caches) -> torch.Tensor:
         """Run the step's rows through the layers and return float32 logits
         [number of wanted rows, vocab] (an empty tensor when nothing is wanted)."""
+        if self._decode_layers is not None and step.decode_only and self.layer_hook is None:
+            logits = self._decode_layers.forward(step, caches)
+            if logits is not None:
+                if not step.every_row_wanted:
+                    logits = logits.index_select(0, step.want_rows)
+                return self._finish_logits(logits)
         tokens = step.num_tokens
         step.carried = {}      # what a layer leaves for later layers of the same step
         copies = self.spec.residual_streams
@@ -247,7 +255,9 @@ class DecoderModel:
             return torch.empty((0, self.spec.vocab_size), dtype=torch.float32, device=self.device)
         stream.read = None     # the head reads the sum of the copies
         x = self.final_norm.forward(stream, rows=step.want_rows)
-        logits = linear(x, self.lm_head, out_dtype=torch.float32)
+        return self._finish_logits(linear(x, self.lm_head, out_dtype=torch.float32))
+
+    def _finish_logits(self, logits: torch.Tensor) -> torch.Tensor:
         if self.spec.logit_scale != 1.0:
             logits.mul_(self.spec.logit_scale)
         if self.spec.logit_softcap > 0.0:
