@@ -8,6 +8,7 @@
 // the kernels add them in index order before anything else, so the sum is the
 // same whatever else runs.
 #include "common.cuh"
+#include "gate_act.cuh"
 
 LSE_TL_DEFINE(lse_timeline_elementwise)
 LSE_CHECK_DEFINE(lse_check_elementwise)
@@ -678,29 +679,6 @@ extern "C" int lse_rope_kv_write(const void* qkv, int in_dtype, int n_partials, 
 }
 
 // ------------------------------------------------------------------ gated activation (SiLU or tanh-form GELU)
-// ACT 0: silu(g) = g / (1 + exp(-g)).  ACT 1: gelu(g) = 0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))).
-// FAST: the result is rounded to bfloat16, far more coarsely than the fast exponential and division err.
-template <int ACT, bool FAST>
-__device__ __forceinline__ float gate_act(float g) {
-  if (ACT == 2) return fmaxf(g, 0.f);
-  if (ACT == 3) return FAST ? __fdividef(g, 1.0f + __expf(-1.702f * g)) : g / (1.0f + expf(-1.702f * g));
-  if (ACT == 0) return FAST ? __fdividef(g, 1.0f + __expf(-g)) : g / (1.0f + expf(-g));
-  const float inner = 0.7978845608028654f * fmaf(0.044715f * g * g, g, g);
-  if (FAST) return g - __fdividef(g, 1.0f + __expf(2.0f * inner));   // 0.5 g (1 + tanh x) = g - g / (1 + exp(2x))
-  return 0.5f * g * (1.0f + tanhf(inner));
-}
-
-// The product of the activated gate and the up value.  ACT 3 (clamped swish): g' = min(g, limit), u' = clamp(u, -limit,
-// limit), g' sigmoid(1.702 g') (u' + 1); the others: act(g) u, `limit` not read.
-template <int ACT, bool FAST>
-__device__ __forceinline__ float gate_mul(float g, float u, float limit) {
-  if (ACT == 3) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit) + 1.0f;
-  }
-  return gate_act<ACT, FAST>(g) * u;
-}
-
 // gate_up[t] = [gate (I values) | up (I values)];  out[t, i] = silu(gate_i) * up_i
 // grid: (chunks of the row, tokens); a thread handles 4 consecutive i when I % 4 == 0.
 template <typename TI, typename TO, int VEC, int ACT>

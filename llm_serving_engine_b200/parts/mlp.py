@@ -51,9 +51,15 @@ class SwiGLU(FeedForward):
         }
 
     def forward(self, x):
-        gate_up = linear_partials(x, self.gate_up_weight, stacks_of_many_rows=True)
         act = torch.empty((x.shape[0], self.inter), dtype=x.dtype, device=x.device)
+        if ops.gated_product_wanted(x, self.gate_up_weight):
+            ops.gated_product(x, self.gate_up_weight, act, self.activation, self.limit)
+            return self._down(act)
+        gate_up = linear_partials(x, self.gate_up_weight, stacks_of_many_rows=True)
         ops.silu_mul(gate_up, act, self.activation, self.limit)
+        return self._down(act)
+
+    def _down(self, act):
         if self.float32_output:
             return linear_sums(act, self.down_weight)
         return linear_partials(act, self.down_weight, stacks_of_many_rows=True)

@@ -47,11 +47,13 @@ class ClampedMoE(FeedForward):
       expert's columns by the token's weight for it (zero where it was not chosen), so that the second product is the
       weighted sum over the experts.  With a handful of tokens nearly every expert's weights are read anyway.
     * many bfloat16 rows: every (token, chosen expert) pair gets a row in a buffer grouped by expert (two small
-      kernels), the library's grouped product runs over views of the same stacked matrices, and a kernel adds each
-      token's rows times their weights in float32, with the identity experts' share, onto the shared expert's output."""
+      kernels), two products run over the groups and the shared expert at once, the activation inside the first, and a
+      kernel adds each token's rows times their weights in float32, with the identity experts' share, onto the shared
+      expert's output.  (Experts without a gate, or of a width that is no multiple of 64: the library's grouped product
+      over views of the same stacked matrices, and the activation kernel.)"""
 
     graph_safe = True
-    kernel_sources = ("moe",)
+    kernel_sources = ("moe", "gemm_pairs")
 
     def __init__(self, params, weights, ctx) -> None:
         super().__init__(params, weights, ctx)
@@ -110,6 +112,9 @@ class ClampedMoE(FeedForward):
             self._grouped_gate_up = (self.gate_up_weight[:self.columns * routed]
                                      .view(self.experts, self.columns * self.ff, width).transpose(1, 2))
             self._grouped_down = self.down_weight.as_strided((self.experts, self.ff, width), (self.ff, 1, self.inter))
+        # the engine's own products over groups of rows: gated experts whose columns are whole pieces of 64
+        self._in_pairs = (self._grouped_gate_up is not None and self.activation in ("clamped_swish", "silu") and self.ff % 64 == 0
+                          and self.shared_ff % 8 == 0 and self.experts <= ops.PAIRS_MAX_GROUPS)
 
     @classmethod
     def expected_tensors(cls, params, hidden_size):
@@ -146,6 +151,8 @@ class ClampedMoE(FeedForward):
         tokens, width = x.shape
         chosen = torch.empty((tokens, self.top), dtype=torch.int32, device=x.device)
         expert_weights, identity_weight, shared_gate = self._route(x, chosen)
+        if self._in_pairs:
+            return self._grouped_in_pairs(x, chosen, expert_weights, identity_weight, shared_gate)
         y = None
         if self.shared_ff:   # the shared expert: two plain products, its gate folded into the activation
             routed = self.experts * self.ff
@@ -166,6 +173,26 @@ class ClampedMoE(FeedForward):
         out = y if y is not None else torch.empty((tokens, width), dtype=torch.float32, device=x.device)
         return ops.moe_combine(down, row_of, chosen, expert_weights, identity_weight if self.identity else None, x, out,
                                accumulate=y is not None)
+
+    def _grouped_in_pairs(self, x, chosen, expert_weights, identity_weight, shared_gate):
+        """The experts and the shared expert together in two products of the engine's own, the activation inside the first."""
+        tokens, width = x.shape
+        row_of, offsets = ops.moe_group_rows(chosen, self.experts)
+        rows = tokens * self.top
+        grouped = torch.empty((rows, width), dtype=x.dtype, device=x.device)
+        ops.moe_gather_rows(x, row_of, grouped)
+        act = torch.empty((rows, self.ff), dtype=x.dtype, device=x.device)
+        down = torch.empty((rows, width), dtype=x.dtype, device=x.device)
+        out = torch.empty((tokens, width), dtype=torch.float32, device=x.device)
+        shared = shared_act = shared_out = None
+        if self.shared_ff:
+            shared, shared_out = x, out
+            shared_act = torch.empty((tokens, self.shared_ff), dtype=x.dtype, device=x.device)
+        ops.gated_product_groups(grouped, offsets, act, self.limit, shared, shared_act, shared_gate if self.shared_gated else None,
+                                 self.shared_limit, self.gate_up_weight, self.activation)
+        ops.product_groups(act, offsets, down, shared_act, shared_out, self.down_weight)
+        return ops.moe_combine(down, row_of, chosen, expert_weights, identity_weight if self.identity else None, x, out,
+                               accumulate=shared is not None)
 
     def _route(self, x, chosen=None):
         """The router's logits as a product with float32 sums (partial sums for few rows), then the routing kernel."""

@@ -54,7 +54,7 @@ class _Turn:
         self.dev_i = torch.empty((2, max_rows), dtype=torch.int64, device=device)
         self.out = torch.empty(max_rows, dtype=torch.int32, device=device)
         self.host_out = torch.empty(max_rows, dtype=torch.int32, pin_memory=pinned)
-        self.host_status = torch.zeros(4, dtype=torch.int32, pin_memory=pinned) if pinned else None
+        self.host_status = torch.zeros(5, dtype=torch.int32, pin_memory=pinned) if pinned else None
         self.done = torch.cuda.Event() if pinned else None
         self.rows = 0
 
@@ -120,7 +120,8 @@ class Sampler:
             turn.done.synchronize()
         if turn.host_status is not None and any(turn.host_status.tolist()):
             which = " and ".join(name for name, word in zip(("the few-rows product", "the tcgen05 prompt attention",
-                                                             "the attention over expanded latents", "the decode step"),
+                                                             "the attention over expanded latents", "the decode step",
+                                                             "the product on pairs of SMs"),
                                                             turn.host_status.tolist()) if word)
             left_out = int(turn.host_status[2]) == ops.EXPANDED_ROWS_LEFT_OUT
             turn.host_status.zero_()

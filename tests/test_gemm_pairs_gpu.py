@@ -1,0 +1,116 @@
+"""The product on pairs of SMs (``csrc/gemm_pairs.cu``): gated, and over groups of rows, at the edges of its tiles, against
+float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def ops():
+    from llm_serving_engine_b200.kernels import ops
+    return ops
+
+
+def _act(kind, g, u, limit):
+    if kind == "silu":
+        return g * torch.sigmoid(g) * u
+    if kind == "relu":
+        return g.clamp(min=0) * u
+    if kind == "gelu_tanh":
+        return 0.5 * g * (1 + torch.tanh(0.7978845608028654 * (g + 0.044715 * g ** 3))) * u
+    g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+    return g * torch.sigmoid(1.702 * g) * (u + 1)
+
+
+def _check(got, want, x, w):
+    """Rounded once to bfloat16 (2^-9 of the value; 2^-8 allows for a neighbour), and float32 sums of k terms: k 2^-24 of the
+    magnitudes, times what the activation and the other factor make of it (all factors here are below 16)."""
+    sums = x.shape[1] * 2.0 ** -24 * float((x.abs().double() @ w.abs().double().t()).max())
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * sums + 1e-6).all())
+
+
+def _random(rows, k, scale=1.0):
+    return (torch.randn(rows, k, device=DEV) * scale).bfloat16()
+
+
+@pytest.mark.parametrize("rows,k,inter,kind", [(1, 64, 128, "silu"), (31, 72, 8, "silu"), (33, 64, 136, "relu"), (96, 200, 320, "gelu_tanh"),
+                                               (256, 128, 1000, "silu"), (257, 448, 64, "clamped_swish"), (300, 512, 264, "silu"),
+                                               (522, 64, 9480, "clamped_swish"), (1349, 96, 2000, "silu")])
+def test_gated_product(rows, k, inter, kind):
+    torch.manual_seed(rows + k)
+    x, w = _random(rows, k), _random(2 * inter, k, k ** -0.5)
+    out = torch.full((rows, inter + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    ops().gated_product(x, w, out[:, :inter], kind, 1.5)
+    sums = x.double() @ w.double().t()
+    _check(out[:, :inter], _act(kind, sums[:, :inter], sums[:, inter:], 1.5), x, w)
+    assert bool((out[:, inter:] == 7.0).all())             # nothing beside the results is written
+    from llm_serving_engine_b200.kernels import library
+    assert library.load().lse_gemm_pairs_status() == 0
+
+
+@pytest.mark.parametrize("counts,k,columns,whole,whole_columns,kind", [
+    ([64], 64, 64, 0, 0, "silu"), ([0, 1, 33, 0, 300], 128, 192, 40, 72, "clamped_swish"), ([256, 522, 5], 192, 128, 257, 200, "silu"),
+    ([2, 0, 3] + [1] * 60, 72, 64, 1, 8, "silu"), ([0, 0], 64, 64, 70, 136, "clamped_swish")])
+def test_groups_of_rows_with_weights_of_their_own(counts, k, columns, whole, whole_columns, kind):
+    """Both products of a mixture of experts: rows behind the last group stay as they are, a group may have none."""
+    torch.manual_seed(sum(counts) + k)
+    used, groups = sum(counts), len(counts)
+    x, everyone = _random(used + 3, k), _random(whole, k) if whole else None
+    offsets = torch.tensor(counts, device=DEV).cumsum(0).int()
+    w = _random(2 * (groups * columns + whole_columns), k, k ** -0.5)
+    act = torch.full((used + 3, columns), 7.0, device=DEV, dtype=torch.bfloat16)
+    scale = torch.rand(whole, device=DEV) if whole else None
+    if whole:
+        scale[0] = 0.0
+        w[2 * groups * columns] = float("nan")             # a row whose factor is zero takes nothing from anywhere
+    shared = torch.empty(whole, whole_columns, device=DEV, dtype=torch.bfloat16) if whole else None
+    ops().gated_product_groups(x, offsets, act, 1.5, everyone, shared, scale, 2.0, w, kind)
+    assert bool((act[used:] == 7.0).all())
+    start = 0
+    for group, count in enumerate(counts):
+        if count:
+            piece = w[2 * group * columns:2 * (group + 1) * columns]
+            sums = x[start:start + count].double() @ piece.double().t()
+            _check(act[start:start + count], _act(kind, sums[:, :columns], sums[:, columns:], 1.5), x[start:start + count], piece)
+        start += count
+    if whole:
+        assert bool((shared[0] == 0).all())
+        piece = w[2 * groups * columns:].clone()
+        piece[0] = 0
+        sums = everyone.double() @ piece.double().t()
+        want = _act(kind, sums[:, :whole_columns], sums[:, whole_columns:], 2.0) * scale.double()[:, None]
+        _check(shared[1:, 1:], want[1:, 1:], everyone, piece)
+        assert kind == "clamped_swish" or bool(torch.isnan(shared[1:, 0]).all())      # a clamp takes the number beside a NaN
+
+    width = 328
+    down_w = _random(width, groups * columns + whole_columns, columns ** -0.5)
+    act[used:] = 0
+    if whole:
+        shared = _random(whole, whole_columns)
+    down = torch.full((used + 3, width), 7.0, device=DEV, dtype=torch.bfloat16)
+    total = torch.empty(whole, width, device=DEV) if whole else None
+    ops().product_groups(act, offsets, down, shared, total, down_w)
+    assert bool((down[used:] == 7.0).all())
+    start = 0
+    for group, count in enumerate(counts):
+        if count:
+            piece = down_w[:, group * columns:(group + 1) * columns]
+            _check(down[start:start + count], act[start:start + count].double() @ piece.double().t(), act[start:start + count], piece)
+        start += count
+    if whole:
+        piece = down_w[:, groups * columns:]
+        want = shared.double() @ piece.double().t()
+        bound = whole_columns * 2.0 ** -24 * (shared.abs().double() @ piece.abs().double().t()) + 1e-6
+        assert bool(((total.double() - want).abs() <= bound).all())
+
+
+def test_what_the_product_does_not_take():
+    o = ops()
+    x, w = _random(40, 64), _random(128, 64)
+    assert o.gemm_pairs_ok(x, w)
+    assert not o.gemm_pairs_ok(x.float(), w) and not o.gemm_pairs_ok(_random(40, 60), _random(128, 60))
+    assert not o.gemm_pairs_ok(torch.empty(0, 64, device=DEV, dtype=torch.bfloat16), w)
+    assert not o.gemm_pairs_ok(_random(41, 64).flatten()[4:4 + 40 * 64].view(40, 64), w)
+    with pytest.raises(o.KernelError):
+        o.gated_product(x.float(), w, torch.empty(40, 64, device=DEV, dtype=torch.bfloat16))
