@@ -34,12 +34,28 @@ template <> __device__ __forceinline__ void dm_load4<__nv_bfloat16>(const __nv_b
 template <bool VEC> __device__ __forceinline__ int dm_column(int lane, int slot) {
   return VEC ? (lane + 32 * (slot / 4)) * 4 + slot % 4 : lane + 32 * slot;
 }
-template <typename TD, bool VEC, int NS>
+// ONE: the row is whole (a single partial sum).
+template <typename TD, bool VEC, int NS, bool ONE>
 __device__ __forceinline__ void dm_fetch(const TD* p, int n_partials, long long partial_stride, int lane, int width,
                                          float (&v)[NS]) {
 #pragma unroll
   for (int s = 0; s < NS; ++s) v[s] = 0.f;
-  if (VEC) {
+  if (ONE) {
+#pragma unroll
+    for (int k = 0; k < (VEC ? NS / 4 : NS); ++k) {
+      const int c = VEC ? (lane + 32 * k) * 4 : lane + 32 * k;
+      if (c < width) {
+        float a[4];
+        if (VEC) {
+          dm_load4<TD>(p + c, a);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[4 * k + e] = a[e];
+        } else {
+          v[k] = to_f32<TD>(p[c]);
+        }
+      }
+    }
+  } else if (VEC) {
 #pragma unroll
     for (int k = 0; k < NS / 4; ++k) {
       const int c = (lane + 32 * k) * 4;
@@ -91,8 +107,13 @@ __device__ __forceinline__ void dm_put(float* p, int lane, int width, const floa
 // head of q, a head of k, a piece of v, a piece of the columns behind it) of rows_per_warp rows and walks them with the
 // channels' last taps - 1 inputs in registers, DM_AHEAD rows fetched at a time (TAPS known; TAPS = 0: any number, fetched
 // again for every row).  NS: values a lane holds (4 for items of up to 128 columns, 8 up to 256).
+//
+// A warp meets the kernel's code once or a few times, so what bounds it is how much code there is: a third to half of the
+// warps' waits were for instructions.  Rows that come whole (ONE: no partial sums) have loads without loops, and the rows
+// fetched together share one copy of the work on a row, the fetched values moving up a place after each.  501 rows of 16 heads
+// of 128: 29.0 to 17.0 us.
 constexpr int DM_AHEAD = 4;
-template <typename TD, typename TO, int TAPS, bool VEC, int NS>
+template <typename TD, typename TO, int TAPS, bool VEC, int NS, bool ONE>
 __global__ void __launch_bounds__(128)
 delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long partial_stride, long long ld,
                      const float* __restrict__ conv_weight, float* __restrict__ state,
@@ -163,14 +184,21 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
       segs[g] = -1;
       if (base + g < end) {
         segs[g] = segment_of_token[base + g];
-        dm_fetch<TD, VEC, NS>(proj + (size_t)(base + g) * ld + column, n_partials, partial_stride, lane, width, ahead[g]);
+        dm_fetch<TD, VEC, NS, ONE>(proj + (size_t)(base + g) * ld + column, n_partials, partial_stride, lane, width, ahead[g]);
       }
     }
+#pragma unroll 1
+    for (int r = base; r < min(base + DM_AHEAD, end); ++r) {
+      int seg = segs[0];
+      float now[NS];
 #pragma unroll
-    for (int g = 0; g < DM_AHEAD; ++g) {
-      const int r = base + g;
-      if (r >= end) break;
-      int seg = segs[g];
+      for (int s = 0; s < NS; ++s) now[s] = ahead[0][s];
+#pragma unroll
+      for (int g = 0; g + 1 < DM_AHEAD; ++g) {
+        segs[g] = segs[g + 1];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) ahead[g][s] = ahead[g + 1][s];
+      }
       if (seg < 0) { held = -1; continue; }
       seg = LSE_CHECKED(seg, 0, num_segments, 0, LSE_CHECK_SEGMENT);
       float* window = back_rt > 0 ? state + (size_t)LSE_CHECKED(segment_slot[seg], 0, num_slots, 0, LSE_CHECK_ROW) * back_rt * channels + column : nullptr;
@@ -181,8 +209,8 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
 #pragma unroll
           for (int i = 0; i < BACK; ++i) {
             const int back = BACK - i;
-            if (l - back >= 0) dm_fetch<TD, VEC, NS>(proj + (size_t)(r - back) * ld + column, n_partials, partial_stride, lane, width, before[i]);
-            else dm_fetch<float, VEC, NS>(window + (size_t)(BACK + l - back) * channels, 1, 0, lane, width, before[i]);
+            if (l - back >= 0) dm_fetch<TD, VEC, NS, ONE>(proj + (size_t)(r - back) * ld + column, n_partials, partial_stride, lane, width, before[i]);
+            else dm_fetch<float, VEC, NS, true>(window + (size_t)(BACK + l - back) * channels, 1, 0, lane, width, before[i]);
           }
           held = seg;
         }
@@ -191,7 +219,7 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
           float sum = 0.f;
 #pragma unroll
           for (int j = 0; j < BACK; ++j) sum = fmaf(w[j][s], before[j][s], sum);
-          y[s] = fmaf(w[TAPS > 0 ? TAPS - 1 : 0][s], ahead[g][s], sum);
+          y[s] = fmaf(w[TAPS > 0 ? TAPS - 1 : 0][s], now[s], sum);
         }
         if (BACK > 0) {
 #pragma unroll
@@ -199,7 +227,7 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
 #pragma unroll
             for (int s = 0; s < NS; ++s) before[i][s] = before[i + 1][s];
 #pragma unroll
-          for (int s = 0; s < NS; ++s) before[HELD - 1][s] = ahead[g][s];
+          for (int s = 0; s < NS; ++s) before[HELD - 1][s] = now[s];
           if (move_windows)
 #pragma unroll
             for (int i = 0; i < BACK; ++i) dm_put<VEC, NS>(window + (size_t)i * channels, lane, width, before[i]);
@@ -213,7 +241,7 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
           if (c < width)
             for (int j = 0; j < taps_rt; ++j) {
               const int back = taps_rt - 1 - j;
-              const float u = back == 0 ? ahead[g][s]
+              const float u = back == 0 ? now[s]
                   : l - back >= 0 ? sum_partials<TD>(proj + (size_t)(r - back) * ld + column + c, n_partials, partial_stride)
                                   : window[(size_t)(taps_rt - 1 + l - back) * channels + c];
               sum = fmaf(conv_weight[(size_t)(column + c) * taps_rt + j], u, sum);
@@ -221,7 +249,7 @@ delta_prepare_kernel(const TD* __restrict__ proj, int n_partials, long long part
           y[s] = sum;
           if (move_windows && c < width) {
             for (int i = 0; i + 1 < back_rt; ++i) window[(size_t)i * channels + c] = window[(size_t)(i + 1) * channels + c];
-            if (back_rt > 0) window[(size_t)(back_rt - 1) * channels + c] = ahead[g][s];
+            if (back_rt > 0) window[(size_t)(back_rt - 1) * channels + c] = now[s];
           }
         }
       }
@@ -389,11 +417,16 @@ extern "C" int lse_delta_prepare(const void* proj, int proj_dtype, int n_partial
   const long long blocks = (warps + 3) / 4;
   if (blocks > 0x7fffffffLL) return LSE_ERR_TOO_LARGE;
   const bool vec = dim % 4 == 0 && value % 4 == 0 && ld % 4 == 0 && partial_stride % 4 == 0 && (((uintptr_t)proj) & 15) == 0;
-#define LSE_DM_NS(TD, TO, TAPS, VEC, NS)                                                                               \
-  lse_launch(delta_prepare_kernel<TD, TO, TAPS, VEC, NS>, (unsigned)blocks, 128, 0, stream, (const TD*)proj, n_partials,    \
+#define LSE_DM_ONE(TD, TO, TAPS, VEC, NS, ONE)                                                                         \
+  lse_launch(delta_prepare_kernel<TD, TO, TAPS, VEC, NS, ONE>, (unsigned)blocks, 128, 0, stream, (const TD*)proj, n_partials,    \
              partial_stride, ld, conv_weight, state, segment_of_token, segment_start, segment_slot, q_out, k_out, v_out, \
              beta_out, (TO*)low_out, low_ld, tokens, rows_per_warp, groups, heads, dim, vdim, rank, taps, q_scale,      \
              move_windows, num_slots, num_segments, items)
+#define LSE_DM_NS(TD, TO, TAPS, VEC, NS)                               \
+  do {                                                                 \
+    if (n_partials == 1) LSE_DM_ONE(TD, TO, TAPS, VEC, NS, true);      \
+    else LSE_DM_ONE(TD, TO, TAPS, VEC, NS, false);                     \
+  } while (0)
 #define LSE_DM_GO(TD, TO, TAPS, VEC)                          \
   do {                                                        \
     if (dim <= 128) LSE_DM_NS(TD, TO, TAPS, VEC, 4);          \
@@ -418,6 +451,7 @@ extern "C" int lse_delta_prepare(const void* proj, int proj_dtype, int n_partial
 #undef LSE_DM_TAPS
 #undef LSE_DM_GO
 #undef LSE_DM_NS
+#undef LSE_DM_ONE
   LSE_LAUNCH_CHECK();
 }
 
