@@ -33,6 +33,7 @@
 // once or none is.
 #include <type_traits>
 
+#include "key_ring.cuh"
 #include "mma_common.cuh"
 #include "smem_allowance.cuh"
 #include "tcgen05.cuh"
@@ -192,15 +193,6 @@ struct Shared {
   int row_segment[MAX_ROWS], row_position[MAX_ROWS];
   __nv_bfloat16 new_k[HEAD], new_v[HEAD];
   int pages[KEY_TILES];      // rows of the cache, in groups of 8, at which the item's tiles begin
-};
-
-// A place in the ring and the parity of its barriers' phase.
-struct Slot {
-  int at = 0;
-  uint32_t parity = 0;
-  __device__ __forceinline__ void step(int stages) {
-    if (++at == stages) { at = 0; parity ^= 1u; }
-  }
 };
 
 __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* abort) {
@@ -616,79 +608,76 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
         if (!block_sync_ok(ok)) break;
         STAMP(5)
         // A warp's tiles of 16 keys: S = Q K^T (heads x keys), probabilities relative to the running maximum, O += P V.
-        // Stage st holds tiles 3 st .. 3 st + 2; the warps take the tiles in turn.
+        // A stage holds three tiles; the warps take the tiles in turn.
         const int r = lane >> 2, q = lane & 3;
         float o[HEAD / 8][2] = {};
         float m_run = -INFINITY, l_run = 0.f;
         uint4 qf[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) qf[j] = lds128(smem_u32(q_s) + r * Q_STRIDE + j * 64 + q * 16);
-        const int kv_stages = (it.tiles + STAGE_KEYS - 1) / STAGE_KEYS;
-#pragma unroll 1
-        for (int st = 0; st < kv_stages; ++st) {
-          const int i = (warp - st * STAGE_KEYS) & (WARPS - 1), t = st * STAGE_KEYS + i;
-          if (i < STAGE_KEYS && t < it.tiles) {
-            ok = ok && wait_for(smem_u32(&s.full[slot.at]), slot.parity, &s.abort);
-            const uint32_t kt = ring + slot.at * STAGE + i * 8192, vt = kt + 4096;
-            const int left = it.limit - (it.tile + t) * 16;   // keys of the tile that are the request's
-            if (left < 16) {   // whatever else lies there (NaN included) counts as zero
-              const int row16 = lane >> 1;
-              if (row16 >= left) {
-                const uint32_t dst = vt + (row16 >> 3) * 2048 + (row16 & 7) * 128 + (lane & 1) * 1024;
-                const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                for (int c = 0; c < 8; ++c) sts128(dst + c * 16, zero);
-              }
-              __syncwarp();
-            }
-            float c[2][2] = {};
-#pragma unroll
-            for (int k8 = 0; k8 < 2; ++k8)
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 b = lds128(kt + k8 * 2048 + (j >> 1) * 1024 + r * 128 + ((((j & 1) * 4 + q) ^ r) << 4));
-                mma_heads(c[k8][0], c[k8][1], qf[j].x, qf[j].y, b.x, b.y);
-                mma_heads(c[k8][0], c[k8][1], qf[j].z, qf[j].w, b.z, b.w);
-              }
-            float m_tile = -INFINITY;
-#pragma unroll
-            for (int k8 = 0; k8 < 2; ++k8)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                c[k8][e] = k8 * 8 + 2 * q + e < left ? c[k8][e] * a.scale_log2e : -INFINITY;
-                m_tile = fmaxf(m_tile, c[k8][e]);
-              }
-            m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
-            m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
-            const float m_new = fmaxf(m_run, m_tile);
-            const float base = m_new == -INFINITY ? 0.f : m_new;
-            const float keep = fast_exp2(m_run - base);
-            m_run = m_new;
-            l_run *= keep;
-#pragma unroll
-            for (int k8 = 0; k8 < 2; ++k8)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                c[k8][e] = fast_exp2(c[k8][e] - base);
-                l_run += c[k8][e];
-              }
-#pragma unroll
-            for (int d = 0; d < HEAD / 8; ++d) { o[d][0] *= keep; o[d][1] *= keep; }
-            const uint32_t p0 = pack_bf16(c[0][0], c[0][1]), p1 = pack_bf16(c[1][0], c[1][1]);
-            const uint32_t v_row = vt + ((lane >> 3) & 1) * 2048 + (lane & 7) * 128;
-#pragma unroll
-            for (int d = 0; d < HEAD / 16; ++d) {
-              uint32_t b[4];
-              ldmatrix_x4_trans(b, v_row + (d >> 2) * 1024 + ((((d & 3) * 2 + (lane >> 4)) ^ (lane & 7)) << 4));
-              mma_heads(o[2 * d][0], o[2 * d][1], p0, p1, b[0], b[1]);
-              mma_heads(o[2 * d + 1][0], o[2 * d + 1][1], p0, p1, b[2], b[3]);
-            }
-            if (left < 16) tc::fence_async_smem();
-          }
+        auto wait_stage = [&](const Slot& at) { ok = ok && wait_for(smem_u32(&s.full[at.at]), at.parity, &s.abort); };
+        auto stage_read = [&](const Slot& at) {
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(smem_u32(&s.empty[slot.at]));
-          slot.step(a.stages);
-        }
+          if (lane == 0) tc::mbar_arrive(smem_u32(&s.empty[at.at]));
+        };
+        auto tile = [&](const Slot& at, int i, int t) {
+          const uint32_t kt = ring + at.at * STAGE + i * 8192, vt = kt + 4096;
+          const int left = it.limit - (it.tile + t) * 16;   // keys of the tile that are the request's
+          if (left < 16) {   // whatever else lies there (NaN included) counts as zero
+            const int row16 = lane >> 1;
+            if (row16 >= left) {
+              const uint32_t dst = vt + (row16 >> 3) * 2048 + (row16 & 7) * 128 + (lane & 1) * 1024;
+              const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+              for (int c = 0; c < 8; ++c) sts128(dst + c * 16, zero);
+            }
+            __syncwarp();
+          }
+          float c[2][2] = {};
+#pragma unroll
+          for (int k8 = 0; k8 < 2; ++k8)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 b = lds128(kt + k8 * 2048 + (j >> 1) * 1024 + r * 128 + ((((j & 1) * 4 + q) ^ r) << 4));
+              mma_heads(c[k8][0], c[k8][1], qf[j].x, qf[j].y, b.x, b.y);
+              mma_heads(c[k8][0], c[k8][1], qf[j].z, qf[j].w, b.z, b.w);
+            }
+          float m_tile = -INFINITY;
+#pragma unroll
+          for (int k8 = 0; k8 < 2; ++k8)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              c[k8][e] = k8 * 8 + 2 * q + e < left ? c[k8][e] * a.scale_log2e : -INFINITY;
+              m_tile = fmaxf(m_tile, c[k8][e]);
+            }
+          m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 1));
+          m_tile = fmaxf(m_tile, __shfl_xor_sync(0xffffffffu, m_tile, 2));
+          const float m_new = fmaxf(m_run, m_tile);
+          const float base = m_new == -INFINITY ? 0.f : m_new;
+          const float keep = fast_exp2(m_run - base);
+          m_run = m_new;
+          l_run *= keep;
+#pragma unroll
+          for (int k8 = 0; k8 < 2; ++k8)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              c[k8][e] = fast_exp2(c[k8][e] - base);
+              l_run += c[k8][e];
+            }
+#pragma unroll
+          for (int d = 0; d < HEAD / 8; ++d) { o[d][0] *= keep; o[d][1] *= keep; }
+          const uint32_t p0 = pack_bf16(c[0][0], c[0][1]), p1 = pack_bf16(c[1][0], c[1][1]);
+          const uint32_t v_row = vt + ((lane >> 3) & 1) * 2048 + (lane & 7) * 128;
+#pragma unroll
+          for (int d = 0; d < HEAD / 16; ++d) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, v_row + (d >> 2) * 1024 + ((((d & 3) * 2 + (lane >> 4)) ^ (lane & 7)) << 4));
+            mma_heads(o[2 * d][0], o[2 * d][1], p0, p1, b[0], b[1]);
+            mma_heads(o[2 * d + 1][0], o[2 * d + 1][1], p0, p1, b[2], b[3]);
+          }
+          if (left < 16) tc::fence_async_smem();
+        };
+        walk_key_stages(warp, WARPS, it.tiles, STAGE_KEYS, a.stages, slot, wait_stage, tile, stage_read);
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
         STAMP(6)

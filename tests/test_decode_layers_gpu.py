@@ -16,17 +16,20 @@ SIZES = {
     "small": (192, 320, 2, 1, 528),
     "odd": (1600, 4672, 16, 2, 1040),
     "wide": (576, 3136, 4, 4, 4112),
+    "two_heads": (192, 320, 4, 2, 528),
+    "eight_heads": (256, 320, 16, 8, 528),
+    "many_heads": (256, 320, 36, 36, 528),
 }
 CONTEXTS = [0, 1, 15, 16, 17, 31, 127, 128, 129, 300, 64, 5, 48, 200, 33, 3]
 
 
-def _build(name, pairing="interleaved"):
+def _build(name, pairing="interleaved", layers=3):
     from llm_serving_engine_b200.config import load_config
     from llm_serving_engine_b200.models import DecoderModel, expected_tensors
 
     hidden, inter, n_q, n_kv, vocab = SIZES[name]
     config = {"architectures": ["Qwen2ForCausalLM"], "model_type": "qwen2", "vocab_size": vocab, "hidden_size": hidden, "head_dim": 128,
-              "intermediate_size": inter, "num_hidden_layers": 3, "num_attention_heads": n_q, "num_key_value_heads": n_kv,
+              "intermediate_size": inter, "num_hidden_layers": layers, "num_attention_heads": n_q, "num_key_value_heads": n_kv,
               "max_position_embeddings": 1024, "rope_theta": 10000.0, "rms_norm_eps": 1e-6, "tie_word_embeddings": False}
     _, _, spec = load_config(config)
     for layer in spec.layers:
@@ -96,6 +99,81 @@ def test_halves_turned_as_launch_by_launch(name, rows):
     sequences = [helpers.random_tokens(rng, config["vocab_size"], context + 1) for context in CONTEXTS[2:2 + rows]]
     got, want = (_decode(model, sequences, 1, one_launch) for one_launch in (True, False))
     assert float((got - want).abs().max()) <= helpers.tolerance("bfloat16", want)
+
+
+def _plain_step(config, weights, kept, context, token):
+    """Logits of ``token`` behind ``context`` cached keys and values (``kept``: [layers, 2, context, heads, 128], turned)."""
+    n_q, n_kv, eps, positions = config["num_attention_heads"], config["num_key_value_heads"], config["rms_norm_eps"], torch.tensor([context])
+    h = qwen2_plain.embedding(weights["model.embed_tokens.weight"], torch.tensor([token]))
+    for index in range(config["num_hidden_layers"]):
+        base = f"model.layers.{index}."
+        x = qwen2_plain.rms_norm(h, weights[base + "input_layernorm.weight"], eps)
+        q, k, v = (qwen2_plain.linear(x, weights[base + f"self_attn.{part}_proj.weight"], weights[base + f"self_attn.{part}_proj.bias"])
+                   .view(1, -1, 128) for part in "qkv")
+        q, k = (qwen2_plain.rope(part, positions, config["rope_theta"]) for part in (q, k))
+        keys, values = torch.cat([kept[index, 0], k]), torch.cat([kept[index, 1], v])
+        scores = torch.einsum("hgd,khd->hgk", q.view(n_kv, n_q // n_kv, 128), keys) / 128 ** 0.5
+        out = torch.einsum("hgk,khd->hgd", scores.softmax(-1), values).reshape(1, n_q * 128)
+        h = h + qwen2_plain.linear(out, weights[base + "self_attn.o_proj.weight"])
+        h = h + qwen2_plain.swiglu(qwen2_plain.rms_norm(h, weights[base + "post_attention_layernorm.weight"], eps), weights, base + "mlp.")
+    return qwen2_plain.linear(qwen2_plain.rms_norm(h, weights["model.norm.weight"], eps), weights["lm_head.weight"])[0]
+
+
+# the ring (18 tiles) just filled and refilled, shares of many stages, one request's keys in more than ten shares and in as many as
+# there may be, eight key/value heads, requests of very different lengths, a share of more tiles than are looked up ahead
+@pytest.mark.parametrize("name,layers,contexts", [
+    ("small", 3, [1280]), ("small", 3, [1281, 3072]), ("small", 3, [6912, 6913, 31, 7200]), ("two_heads", 3, [8192]),
+    ("two_heads", 3, [30000]), ("two_heads", 2, [30000, 16]), ("eight_heads", 2, [4000, 3985]),
+    ("eight_heads", 2, [6000, 129, 5999, 2650]), ("many_heads", 1, [17000, 20, 15, 33])])
+def test_long_contexts(name, layers, contexts, monkeypatch):
+    """Against the plain implementation and launch by launch.  The cached keys are large enough (scores of a spread of two) that some
+    hundreds of them carry the result: a share that is lost or read twice moves it by a tenth and more.  Such scores carry the
+    queries' rounding to bfloat16 (2^-9) into the probabilities a few times over, whichever way the step runs: hence the wider of
+    the two bounds."""
+    from llm_serving_engine_b200.cache import CacheManager
+    from llm_serving_engine_b200.config import CacheConfig
+    from llm_serving_engine_b200.engine import StepEntry, StepRunner
+    from llm_serving_engine_b200.kernels import library, ops
+    from llm_serving_engine_b200.models import cache_requirements
+
+    config, model, weights = _build(name, layers=layers)
+    n_kv, rows = config["num_key_value_heads"], len(contexts)
+    assert model._decode_layers is not None and model._decode_layers.wanted(rows)
+    generator = torch.Generator().manual_seed(sum(contexts))
+    spread = torch.tensor([4.0, 1.0]).view(1, 2, 1, 1, 1)
+    kept = [(torch.randn((layers, 2, context, n_kv, 128), generator=generator) * spread).bfloat16() for context in contexts]
+    tokens = [7 + index for index in range(rows)]
+    pages = sum(-(-(context + 1) // 16) for context in contexts)
+    calls = []
+    launch = ops.decode_layers
+    monkeypatch.setattr(ops, "decode_layers", lambda *given: calls.append(1) or launch(*given))
+
+    def run():
+        cache = CacheManager(cache_requirements(model.spec), CacheConfig(16, pages), model.dtype, "cuda", 40000, num_state_slots=rows)
+        cache.groups[0].storage.fill_(float("nan"))
+        runner = StepRunner(model, cache, max_tokens_per_step=rows, max_segments=rows, use_graphs=False)
+        for index, context in enumerate(contexts):
+            cache.create(str(index))
+            cache.reserve(str(index), context)
+            slots = torch.from_numpy(cache.slot_mapping(0, str(index), 0, context)).cuda().long()
+            for position in range(layers):
+                view = cache.layer_view(position)
+                view.keys[slots // 16, :, slots % 16] = kept[index][position, 0].cuda()
+                view.values[slots // 16, :, slots % 16] = kept[index][position, 1].cuda()
+        return runner.run([StepEntry(str(index), [token], [0]) for index, token in enumerate(tokens)]).cpu()
+
+    got, again = run(), run()
+    assert len(calls) == 2 and library.load().lse_decode_layers_status() == 0
+    assert torch.equal(got, again)
+    model._decode_layers = None
+    chain = run()
+    assert len(calls) == 2
+    for index, (context, token) in enumerate(zip(contexts, tokens)):
+        want = _plain_step(config, weights, kept[index].float(), context, token)
+        limit = helpers.tolerance("bfloat16", want)
+        for answer in (got[index], chain[index]):
+            assert float((answer - want).abs().max()) <= limit, (context, "one launch" if answer is got[index] else "launch by launch")
+            assert helpers.rms_ratio(answer[None], want[None]) <= helpers.RMS_RATIO_LARGE_LAYERS
 
 
 def test_some_rows_wanted():
