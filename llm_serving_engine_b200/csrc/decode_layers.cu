@@ -29,8 +29,8 @@
 // gate/up 8, down 6, each 1.2 to 2 of it waiting for the others); more sizes beside the rule in models/decode_layers.py.
 //
 // Every wait is bounded: a block whose wait gives up sets the kernel's error word and the launch's abort word, the others see
-// it while they wait, and all leave (copies in flight land first).  The launch is cooperative: all blocks are on the GPU at
-// once or none is.
+// it while they wait, and all leave.  Whichever way a block leaves, the warps that bring its data wait until all that they have
+// started has landed.  The launch is cooperative: all blocks are on the GPU at once or none is.
 #include <type_traits>
 
 #include "key_ring.cuh"
@@ -64,6 +64,8 @@ static_assert(STAGE % 1024 == 0 && STAGE >= STAGE_KEYS * 8192 && STAGE >= 8 * RO
 constexpr int MAX_DOWN_GROUPS = 2048;
 
 __device__ int lse_decode_layers_error;
+__device__ unsigned lse_decode_layers_spin_limit = SPIN_LIMIT;
+__device__ int lse_decode_layers_withhold;    // test hook: the first sum of squares never comes
 
 // Tuning builds: when the blocks passed the marks of the last layer (nanoseconds of the global timer).
 #ifdef LSE_TRACE
@@ -187,6 +189,8 @@ struct Shared {
   int down_first_chunk;      // of this block's part of the down product's k range
   int down_split;
   int abort;
+  unsigned spin_limit;
+  int started[MAX_STAGES];   // parity of the phase in which a slot was filled last, -1: never
   float inverse[MAX_ROWS];   // 1 / rms of the rows
   float cs[HEAD / 2], sn[HEAD / 2];
   float ml[WARPS + 1][MAX_HEADS][2];
@@ -195,8 +199,9 @@ struct Shared {
   int pages[KEY_TILES];      // rows of the cache, in groups of 8, at which the item's tiles begin
 };
 
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, volatile int* abort) {
-  for (unsigned i = 0; i < SPIN_LIMIT; ++i) {
+__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, Shared& s) {
+  volatile int* abort = &s.abort;
+  for (unsigned i = 0; i < s.spin_limit; ++i) {
     if (tc::mbar_test_suspend(bar, parity)) return true;
     if (*abort) return false;
   }
@@ -211,6 +216,7 @@ __device__ __noinline__ void deal(const Common& a, Shared& s, int block, int blo
   for (int i = 0; i < a.stages; ++i) {
     tc::mbar_init(smem_u32(&s.full[i]), 1);
     tc::mbar_init(smem_u32(&s.empty[i]), WARPS);
+    s.started[i] = -1;
   }
   tc::mbar_init_fence();
   int at = 0;
@@ -298,8 +304,11 @@ __device__ __forceinline__ void bring(const Args& args, const Layer* layers, Sha
         for (int h = 0; h < 2; ++h) {
           if (mine && ok) {
             const uint32_t bar = smem_u32(&s.full[slot.at]);
-            ok = wait_for(smem_u32(&s.empty[slot.at]), slot.parity ^ 1u, &s.abort);
-            if (ok && lane == 0) tc::mbar_expect_tx(bar, 8u * bytes);
+            ok = __all_sync(0xffffffffu, wait_for(smem_u32(&s.empty[slot.at]), slot.parity ^ 1u, s));   // one answer for the warp
+            if (ok && lane == 0) {
+              tc::mbar_expect_tx(bar, 8u * bytes);
+              s.started[slot.at] = (int)slot.parity;
+            }
             __syncwarp();
             if (ok && lane < 8) bulk_copy(ring + slot.at * STAGE + lane * ROW_BYTES, from + (h ? half : 0), bytes, bar, once);
           }
@@ -307,7 +316,6 @@ __device__ __forceinline__ void bring(const Args& args, const Layer* layers, Sha
           slot.step(stages);
         }
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
   };
   auto small_weights = [&](int layer) {   // (the second warp) into the L2, so that who needs them does not wait behind the stream
@@ -332,8 +340,11 @@ __device__ __forceinline__ void bring(const Args& args, const Layer* layers, Sha
       const int tiles = min(STAGE_KEYS, s.item.tiles - t0);
       if (mine) {
         const uint32_t bar = smem_u32(&s.full[slot.at]), dst = ring + slot.at * STAGE;
-        ok = __all_sync(0xffffffffu, wait_for(smem_u32(&s.empty[slot.at]), slot.parity ^ 1u, &s.abort));
-        if (ok && lane == 0) tc::mbar_expect_tx(bar, tiles * 8192u);
+        ok = __all_sync(0xffffffffu, wait_for(smem_u32(&s.empty[slot.at]), slot.parity ^ 1u, s));
+        if (ok && lane == 0) {
+          tc::mbar_expect_tx(bar, tiles * 8192u);
+          s.started[slot.at] = (int)slot.parity;
+        }
         __syncwarp();
         if (ok && lane < 2 * tiles) {
           const int t = t0 + (lane >> 1);
@@ -357,8 +368,13 @@ __device__ __forceinline__ void bring(const Args& args, const Layer* layers, Sha
     product(DOWN, L.down, a.inter, s.down_first_chunk * 32, 16, 8);
   }
   product(HEADS, a.head, a.hidden, 0, 16, 8);
-  if (!ok) {   // a wait gave up: copies in flight land before the block leaves
-    for (int i = 0; i < 2000; ++i) __nanosleep(100);
+  // Neither warp starts anything any more: all that is in flight lands before the block leaves, also where the computing warps
+  // have left already.
+  asm volatile("bar.sync 2, 64;\n" ::: "memory");
+  if (which == 0 && lane < stages) {
+    const int parity = s.started[lane];
+    for (unsigned i = 0; parity >= 0 && i < SPIN_LIMIT; ++i)
+      if (tc::mbar_test_suspend(smem_u32(&s.full[lane]), (uint32_t)parity)) break;
   }
 }
 
@@ -389,6 +405,7 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
     s.row_segment[tid] = LSE_CHECKED(a.segment_of_token[tid], -1, a.num_segments, -1, LSE_CHECK_SEGMENT);
     s.row_position[tid] = a.positions[tid];
   }
+  if (tid == THREADS) s.spin_limit = lse_decode_layers_spin_limit;
   __syncthreads();
   if (tid == 0) deal(a, s, block, blocks);
   __syncthreads();
@@ -422,8 +439,8 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
     if (++turns & 255u) return true;
     unsigned stop;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(stop) : "l"(a.abort) : "memory");
-    if (turns >= SPIN_LIMIT) atomicExch(&lse_decode_layers_error, 1);
-    if (turns >= SPIN_LIMIT || stop || *(volatile int*)&s.abort) {
+    if (turns >= s.spin_limit) atomicExch(&lse_decode_layers_error, 1);
+    if (turns >= s.spin_limit || stop || *(volatile int*)&s.abort) {
       *(volatile int*)&s.abort = 1;
       atomicExch(a.abort, 1u);
       ok = false;
@@ -615,7 +632,7 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
         uint4 qf[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) qf[j] = lds128(smem_u32(q_s) + r * Q_STRIDE + j * 64 + q * 16);
-        auto wait_stage = [&](const Slot& at) { ok = ok && wait_for(smem_u32(&s.full[at.at]), at.parity, &s.abort); };
+        auto wait_stage = [&](const Slot& at) { ok = ok && wait_for(smem_u32(&s.full[at.at]), at.parity, s); };
         auto stage_read = [&](const Slot& at) {
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(smem_u32(&s.empty[at.at]));
@@ -843,8 +860,8 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
               slot.step(a.stages);
               const Slot high = slot;
               slot.step(a.stages);
-              ok = ok && wait_for(smem_u32(&s.full[low.at]), low.parity, &s.abort) &&
-                   wait_for(smem_u32(&s.full[high.at]), high.parity, &s.abort);
+              ok = ok && wait_for(smem_u32(&s.full[low.at]), low.parity, s) &&
+                   wait_for(smem_u32(&s.full[high.at]), high.parity, s);
               const int c0 = p * sh.per_piece, chunks = min(sh.per_piece, sh.chunks - c0);
               const uint32_t w_low = w0 + low.at * STAGE, w_high = w0 + high.at * STAGE;
 #pragma unroll 3
@@ -944,7 +961,7 @@ decode_layers_start_kernel(const __nv_bfloat16* __restrict__ table, const int* _
     float sq = v.x * v.x + v.y * v.y;
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffu << (threadIdx.x & 24), sq, o);
-    if ((p & 7) == 0) input_sq[p / 8] = make_uint2(__float_as_uint(sq), 1u << 16);
+    if ((p & 7) == 0 && !(p == 0 && lse_decode_layers_withhold)) input_sq[p / 8] = make_uint2(__float_as_uint(sq), 1u << 16);
   }
 }
 
@@ -1052,6 +1069,14 @@ extern "C" int lse_decode_layers_status_async(int* host_dst, cudaStream_t stream
 extern "C" int lse_decode_layers_status_reset(void) {
   const int zero = 0;
   return (int)cudaMemcpyToSymbol(lse_decode_layers_error, &zero, sizeof(int));
+}
+// Test hooks.  spin_limit: attempts of a bounded wait before it gives up (0: the default); withhold != 0: a value that every block
+// with a unit of the first product waits for never comes.
+extern "C" int lse_decode_layers_test_hooks(unsigned int spin_limit, int withhold) {
+  const unsigned int limit = spin_limit ? spin_limit : SPIN_LIMIT;
+  cudaError_t err = cudaMemcpyToSymbol(lse_decode_layers_spin_limit, &limit, sizeof(limit));
+  if (err != cudaSuccess) return (int)err;
+  return (int)cudaMemcpyToSymbol(lse_decode_layers_withhold, &withhold, sizeof(withhold));
 }
 
 // One decode step.  layer_pointers [layers][9]: qkv, o, gate_up, down, qkv_bias (may be 0), norm1, norm2, keys, values;

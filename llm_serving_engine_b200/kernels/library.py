@@ -229,6 +229,7 @@ _SIGNATURES = {
     "lse_decode_layers_status": [],
     "lse_decode_layers_status_async": [c_void_p, c_void_p],
     "lse_decode_layers_status_reset": [],
+    "lse_decode_layers_test_hooks": [c_uint, c_int],
     "lse_argmax": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p],
     "lse_sample": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                    c_void_p, c_void_p, c_void_p],

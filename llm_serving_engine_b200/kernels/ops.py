@@ -649,6 +649,13 @@ def decode_layers_supported(layers: int, rows: int, hidden: int, inter: int, n_q
     return bool(library.load().lse_decode_layers_supported(sm_count(), layers, rows, hidden, inter, n_q, n_kv, vocab))
 
 
+def decode_layers_test_hooks(spin_limit: int = 0, withhold: bool = False) -> None:
+    """For tests of the bounded waits: ``spin_limit`` attempts before a wait gives up (0: the default), ``withhold``: a value
+    that the first product waits for never comes."""
+    torch.cuda.synchronize()
+    check(library.load().lse_decode_layers_test_hooks(int(spin_limit), int(bool(withhold))), "decode_layers test hooks")
+
+
 def decode_layers(layer_pointers: list, eps: list, embedding: torch.Tensor, embedding_scale: float, head: torch.Tensor,
                   final_norm: torch.Tensor, final_eps: float, inv_freq: torch.Tensor, pairing: int, token_ids: torch.Tensor,
                   positions: torch.Tensor, segment_of_token: torch.Tensor, slot_mapping: torch.Tensor, block_tables: torch.Tensor,

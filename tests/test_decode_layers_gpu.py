@@ -196,3 +196,30 @@ def test_some_rows_wanted():
     assert torch.equal(run([[0], [], [0]]), whole[[0, 2]])
     assert torch.equal(run([[], [0, 0], [0]]), whole[[1, 1, 2]])
     assert run([[], [], []]).shape == (0, whole.shape[1])
+
+
+@pytest.mark.parametrize("name,rows,layers", [("small", 1, 3), ("odd", 4, 2)])
+def test_a_wait_that_runs_out_is_reported_and_the_kernel_returns(name, rows, layers):
+    """A value that the first product waits for does not come, and the waits give up after a few thousand attempts: the blocks that
+    wait for it, those that wait for what these would have made, and the warps whose ring nobody empties.  The launch ends, its
+    status word reaches the host as the sampler reads it, and after a reset the next step is right.  Nothing faults: a value is
+    simply not written."""
+    from llm_serving_engine_b200.kernels import library, ops
+    from llm_serving_engine_b200.sampling.sampler import GenerationConfig, Sampler
+
+    config, model, _ = _build(name, layers=layers)
+    sequences = [[5 + index, 9] for index in range(rows)]
+    want = _decode(model, sequences, 1, True)
+    sampler = Sampler(config["vocab_size"], rows, torch.device("cuda"))
+    ops.decode_layers_test_hooks(spin_limit=2000, withhold=True)
+    try:
+        broken = _decode(model, sequences, 1, True)[:, 0].cuda()
+        assert library.load().lse_decode_layers_status() == 1
+        ticket = sampler.launch(broken, [GenerationConfig() for _ in range(rows)], [0] * rows)
+        with pytest.raises(ops.KernelError, match="the decode step"):
+            sampler.collect(ticket)
+    finally:
+        ops.decode_layers_test_hooks()
+        ops.kernel_status_reset()
+    assert torch.equal(_decode(model, sequences, 1, True), want)
+    assert library.load().lse_decode_layers_status() == 0
