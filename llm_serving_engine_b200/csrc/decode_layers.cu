@@ -19,9 +19,11 @@
 //     it took 3.4.  A packet's place is written again only by blocks whose own input depends, over the phases between, on every
 //     reader having read.
 //   * Norms are not phases: who adds to the residual multiplies by the next norm's weight and leaves the sums of squares of its
-//     16 columns; who reads it adds these up and scales.  Rotation, bias and the cache write belong to the attention, the SiLU
-//     gate to the gate/up product (a unit is eight gate rows and the eight up rows beside them).  The down product's k range may
-//     be cut into parts, and a request's keys into shares: the blocks add up one another's parts, in their order.
+//     16 columns; who reads it adds these up and scales.  These values are float32 in places of their own for every norm, cleared
+//     to a pattern that no value has: four values a read, where packets would hold two.  Rotation, bias and the cache write belong
+//     to the attention, the SiLU gate to the gate/up product (a unit is eight gate rows and the eight up rows beside them).  The
+//     down product's k range may be cut into parts, and a request's keys into shares: the blocks add up one another's parts, in
+//     their order.
 // Sums do not depend on timing: every order is fixed.
 //
 // Measured against nine launches a layer, one B200: 28 layers of the 1.5B sizes and the head, one request of 100 keys, 879 us a
@@ -87,18 +89,19 @@ struct Common {
   const __nv_bfloat16* head;
   const float *final_norm, *inv_freq;
   const int *positions, *segment_of_token, *slot_mapping, *block_tables;
-  // Packets of 8 bytes: a value (float32, or two bfloat16) or two values of 24 bits, and in the upper 16 bits the epoch that they
-  // belong to.
-  uint2 *input, *middle;       // the residual that a layer begins with, and behind its attention [rows][hidden],
-  uint2 *input_x, *middle_x;   // times the weight of the norm that reads it, 24 bits a value [rows][hidden / 2],
-  uint2 *input_sq, *middle_sq; // and the sums of squares of 16 columns at a time [rows][hidden / 16]
+  // Packets of 8 bytes: a value (float32, or two bfloat16), and in the upper 16 bits the epoch that it belongs to.
+  uint2 *input, *middle;       // the residual that a layer begins with, and behind its attention [rows][hidden]
   uint2 *qkv, *attended, *act; // [rows][n], [rows][n_q * 64], [rows][inter / 2]
   uint2 *part_o, *part_ml;     // an attention share's sums [blocks][heads][128], maximum and sum [blocks][heads][2]
   uint2* down_part;            // [splits][rows][hidden]
+  // What the norms read, float32 without epochs: the residual times the norm's weight [rows][hidden], and its sums of squares of
+  // 16 columns at a time [rows][hidden / 16].  Every norm of the step has a place of its own (2 l and 2 l + 1 in layer l, 2 layers
+  // at the end), which holds UNSET until its values come: four values a read, where packets would hold two.
+  uint32_t* normed;
   unsigned* abort;             // set: a wait gave up somewhere
   float* logits;
   int layers, rows, hidden, inter, n_q, n_kv, vocab, page_size, bt_stride, num_pages, num_slots, num_segments, pairing;
-  int down_splits, batch_units, x_bytes, stages;
+  int down_splits, batch_units, x_bytes, stages, norm_stride;   // values from a norm's place to the next one's
   float final_eps, scale_log2e;
 };
 
@@ -132,17 +135,20 @@ __device__ __forceinline__ uint2 load_packet(const uint2* p) {
 __device__ __forceinline__ void store_packet(uint2* p, uint32_t value, uint32_t epoch) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"((unsigned long long)epoch << 48 | value) : "memory");
 }
-// The upper 24 bits of a float32, rounded to nearest: what is rounded to bfloat16 after one more product keeps nine bits more
-// than that needs, in the room of four bytes a value.
-__device__ __forceinline__ uint32_t upper24(float v) {
+// A float32 in a place that held UNSET: a NaN of these bits is stored as another.
+constexpr uint32_t UNSET = 0xffffffffu;
+__device__ __forceinline__ uint32_t set_bits(float v) {
   const uint32_t u = __float_as_uint(v);
-  return ((u & 0x7f800000u) == 0x7f800000u ? u : u + 0x7fu + (u >> 8 & 1u)) >> 8;    // infinities and NaN as they are
+  return u == UNSET ? 0x7fffffffu : u;
 }
-__device__ __forceinline__ unsigned long long packet24(float lo, float hi, uint32_t epoch) {
-  return (unsigned long long)epoch << 48 | (unsigned long long)upper24(hi) << 24 | upper24(lo);
+__device__ __forceinline__ void store_value(uint32_t* p, float v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(set_bits(v)) : "memory");
 }
-__device__ __forceinline__ float low24(uint32_t x) { return __uint_as_float(x << 8); }
-__device__ __forceinline__ float high24(uint32_t x, uint32_t y) { return __uint_as_float((x >> 24 | (y & 0xffffu) << 8) << 8); }
+__device__ __forceinline__ uint4 load_values(const uint32_t* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, unsigned long long policy) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy) : "memory");
@@ -447,19 +453,22 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
     }
     return ok;
   };
-  // Waits for the pairs of packets at(k), k in `todo` (a bit each): every round asks for all that have not come together, so
-  // that what came late costs one round trip, not one each.
-  auto fetch = [&](auto& v, uint32_t todo, uint32_t epoch, auto at) {
+  // Waits for the 16 bytes load(k), k in `todo` (a bit each), until came(v[k]): every round asks for all that have not come together,
+  // so that what came late costs one round trip, not one each.
+  auto fetch_until = [&](auto& v, uint32_t todo, auto came, auto load) {
     constexpr int COUNT = sizeof(v) / sizeof(uint4);
     for (unsigned turns = 0; todo;) {
 #pragma unroll
       for (int k = 0; k < COUNT; ++k)
-        if (todo >> k & 1u) v[k] = load_packets(at(k));
+        if (todo >> k & 1u) v[k] = load(k);
 #pragma unroll
       for (int k = 0; k < COUNT; ++k)
-        if ((todo >> k & 1u) && v[k].y >> 16 == epoch && v[k].w >> 16 == epoch) todo &= ~(1u << k);
+        if ((todo >> k & 1u) && came(v[k])) todo &= ~(1u << k);
       if (todo && !patience(turns)) break;
     }
+  };
+  auto fetch = [&](auto& v, uint32_t todo, uint32_t epoch, auto at) {   // pairs of packets
+    fetch_until(v, todo, [&](const uint4& got) { return got.y >> 16 == epoch && got.w >> 16 == epoch; }, [&](int k) { return load_packets(at(k)); });
   };
   auto fetch_single = [&](auto& v, uint32_t todo, auto epoch, auto at) {
     constexpr int COUNT = sizeof(v) / sizeof(uint2);
@@ -473,60 +482,61 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
       if (todo && !patience(turns)) break;
     }
   };
-  // Rows of x (bfloat16) into shared memory, COUNT pairs of packets a thread in flight, and the rows' sums of squares.
-  auto load_x = [&](auto count, int tid, const uint2* src, int row_packets, int pairs, uint32_t epoch, const uint2* squares,
+  // Rows of x (bfloat16) into shared memory, COUNT times 16 bytes a thread in flight: pairs of packets of two bfloat16 each, or
+  // (normed) four values of a norm's place, whose sums of squares say what they are multiplied by.
+  auto load_x = [&](auto count, auto normed, int tid, const void* src, int row_quads, int quads, uint32_t epoch, const uint32_t* squares,
                     int x_row_bytes, uint32_t rows_mask, float eps) {
-    constexpr int COUNT = decltype(count)::value, SQUARES = 2;
+    constexpr int COUNT = decltype(count)::value;
+    constexpr bool NORMED = decltype(normed)::value;
+    constexpr int SQUARES = NORMED ? 1 : 0;
     const int lane = tid & 31, warp = tid >> 5, groups = a.hidden / 16;
-    float sq = 0.f;
-    const int all = pairs * a.rows;
+    auto came = [&](const uint4& v) {
+      if (NORMED) return v.x != UNSET && v.y != UNSET && v.z != UNSET && v.w != UNSET;
+      return v.y >> 16 == epoch && v.w >> 16 == epoch;
+    };
+    auto sum_of = [](const uint4& v) { return (__uint_as_float(v.x) + __uint_as_float(v.y)) + (__uint_as_float(v.z) + __uint_as_float(v.w)); };
+    const int all = quads * a.rows;
     int row = 0, column = tid;
     auto settle = [&]() {
-      while (column >= pairs) {
-        column -= pairs;
+      while (column >= quads) {
+        column -= quads;
         if (++row == a.rows) row = 0;
       }
     };
     settle();
     for (int e = tid, round = 0; round == 0 || e < all; ++round) {
       uint4 v[COUNT + SQUARES] = {};    // set on every path: a register that is not stays occupied through all phases
-      uint32_t pair_of[COUNT];          // row and column of the pair
+      uint32_t quad_of[COUNT];          // row and column of the 16 bytes
       uint32_t todo = 0u;
 #pragma unroll
       for (int k = 0; k < COUNT; ++k) {
-        pair_of[k] = (uint32_t)row << 24 | (uint32_t)column;
+        quad_of[k] = (uint32_t)row << 24 | (uint32_t)column;
         if (e < all && (rows_mask >> row & 1u)) todo |= 1u << k;     // padding rows: nobody writes them
         e += THREADS;
         column += THREADS;
         settle();
       }
       const uint32_t mine = todo;
-      if (squares != nullptr && round == 0 && warp < a.rows) {     // a warp adds up a row's: lanes, then the butterfly
-#pragma unroll
-        for (int k = 0; k < SQUARES; ++k)
-          if (2 * lane + k * 64 < groups) todo |= 1u << (COUNT + k);
-      }
-      auto at = [&](int k) { return k < COUNT ? src + (size_t)(pair_of[k] >> 24) * row_packets + 2 * (pair_of[k] & 0xffffffu) : squares + warp * groups + 2 * lane + (k - COUNT) * 64; };
+      if (NORMED && round == 0 && warp < a.rows && 4 * lane < groups) todo |= 1u << COUNT;   // a warp adds up a row's: lanes, then the butterfly
+      auto load = [&](int k) -> uint4 {
+        if (NORMED && k >= COUNT) return load_values(squares + warp * groups + 4 * lane);
+        const size_t at = (size_t)(quad_of[k] >> 24) * row_quads + (quad_of[k] & 0xffffffu);
+        return NORMED ? load_values(reinterpret_cast<const uint32_t*>(src) + 4 * at) : load_packets(reinterpret_cast<const uint2*>(src) + 2 * at);
+      };
       if (COUNT > 4) {                                        // many: one of them is waited for, then the others asked for
-        fetch(v, todo & 1u, epoch, at);
+        fetch_until(v, todo & 1u, came, load);
         todo &= ~1u;
       }
-      fetch(v, todo, epoch, at);
-      if (squares != nullptr && round == 0) {
-#pragma unroll
-        for (int k = COUNT; k < COUNT + SQUARES; ++k) {
-          sq += __uint_as_float(v[k].x);
-          sq += __uint_as_float(v[k].z);
-        }
+      fetch_until(v, todo, came, load);
+      if (NORMED && round == 0) {
 #pragma unroll 1
         for (int r = warp; r < a.rows; r += WARPS) {
-          if (r != warp) sq = 0.f;
+          float sq = r == warp ? sum_of(v[COUNT + SQUARES - 1]) : 0.f;
 #pragma unroll 1
-          for (int i = 2 * lane + (r == warp ? SQUARES * 64 : 0); i < groups; i += 64) {
+          for (int i = 4 * lane + (r == warp ? 128 : 0); i < groups; i += 128) {
             uint4 more[1] = {};
-            fetch(more, 1u, epoch, [&](int) { return squares + r * groups + i; });
-            sq += __uint_as_float(more[0].x);
-            sq += __uint_as_float(more[0].z);
+            fetch_until(more, 1u, came, [&](int) { return load_values(squares + r * groups + i); });
+            sq += sum_of(more[0]);
           }
           sq = warp_sum(sq);
           if (lane == 0) s.inverse[r] = 1.0f / sqrtf(sq / (float)a.hidden + eps);
@@ -537,12 +547,12 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
       for (int k = 0; k < COUNT; ++k) {
         if (mine >> k & 1u) {
           uint2 out = make_uint2(v[k].x, v[k].z);
-          if (squares != nullptr) {
-            const float inverse = s.inverse[pair_of[k] >> 24];
-            out.x = pack_bf16(low24(v[k].x) * inverse, high24(v[k].x, v[k].y) * inverse);
-            out.y = pack_bf16(low24(v[k].z) * inverse, high24(v[k].z, v[k].w) * inverse);
+          if (NORMED) {
+            const float inverse = s.inverse[quad_of[k] >> 24];
+            out.x = pack_bf16(__uint_as_float(v[k].x) * inverse, __uint_as_float(v[k].y) * inverse);
+            out.y = pack_bf16(__uint_as_float(v[k].z) * inverse, __uint_as_float(v[k].w) * inverse);
           }
-          *reinterpret_cast<uint2*>(work + (pair_of[k] >> 24) * x_row_bytes + (pair_of[k] & 0xffffffu) * 8) = out;
+          *reinterpret_cast<uint2*>(work + (quad_of[k] >> 24) * x_row_bytes + (quad_of[k] & 0xffffffu) * 8) = out;
         }
       }
     }
@@ -820,29 +830,33 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
           }
         };
         look_up(j0);
-        const uint2* src = phase == O ? a.attended : phase == DOWN ? a.act + s.down_first_chunk * 16 : phase == GATE_UP ? a.middle_x : a.input_x;
-        const uint2* squares = phase == GATE_UP ? a.middle_sq : normed ? a.input_sq : nullptr;
-        const int row_packets = (phase == O ? a.n_q * HEAD : phase == DOWN ? a.inter : a.hidden) / 2;
-        const int x_pairs = sh.chunks * 8, mine = (x_pairs * a.rows + THREADS - 1) / THREADS;
-        const uint32_t rows_mask = phase == O ? valid_rows : 0xffffu;
-        const float eps = phase == QKV ? L.eps1 : phase == GATE_UP ? L.eps2 : a.final_eps;
-        if (mine > 4) load_x(std::integral_constant<int, 12>(), tid, src, row_packets, x_pairs, epoch, squares, x_row_bytes, rows_mask, eps);
-        else load_x(std::integral_constant<int, 4>(), tid, src, row_packets, x_pairs, epoch, squares, x_row_bytes, rows_mask, eps);
+        const int quads = sh.chunks * 8, mine = (quads * a.rows + THREADS - 1) / THREADS;
+        auto take = [&](auto count) {
+          if (normed) {
+            const uint32_t* src = a.normed + (size_t)(2 * layer + (phase == GATE_UP ? 1 : 0)) * a.norm_stride;
+            const float eps = phase == QKV ? L.eps1 : phase == GATE_UP ? L.eps2 : a.final_eps;
+            load_x(count, std::true_type(), tid, src, a.hidden / 4, quads, epoch, src + a.rows * a.hidden, x_row_bytes, 0xffffu, eps);
+          } else {
+            const uint2* src = phase == O ? a.attended : a.act + s.down_first_chunk * 16;
+            load_x(count, std::false_type(), tid, src, (phase == O ? a.n_q * HEAD : a.inter) / 4, quads, epoch, nullptr, x_row_bytes,
+                   phase == O ? valid_rows : 0xffffu, 0.f);
+          }
+        };
+        if (mine > 4) take(std::integral_constant<int, 12>());
+        else take(std::integral_constant<int, 4>());
         if (!block_sync_ok(ok)) break;
         STAMP(phase * 4 + 1)
         // A new value of the residual, and what the norm that reads it needs of it (the 16 threads of a unit's row together).
         auto publish = [&](int row, int at, float v, float weight) {
           const size_t there = (size_t)row * a.hidden + at;
           const unsigned mask = 0xffffu << (lane & 16);
+          uint32_t* normed_there = a.normed + (size_t)(2 * layer + (phase == DOWN ? 2 : 1)) * a.norm_stride;
           store_packet(fresh + there, __float_as_uint(v), fresh_epoch);
-          const float x = v * weight, next = __shfl_down_sync(mask, x, 1);
-          if ((i & 1) == 0)
-            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"((phase == DOWN ? a.input_x : a.middle_x) + there / 2),
-                         "l"(packet24(x, next, fresh_epoch)) : "memory");
+          store_value(normed_there + there, v * weight);
           float sq = v * v;
 #pragma unroll
           for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(mask, sq, o);
-          if (i == 0) store_packet((phase == DOWN ? a.input_sq : a.middle_sq) + there / 16, __float_as_uint(sq), fresh_epoch);
+          if (i == 0) store_value(normed_there + a.rows * a.hidden + there / 16, sq);
         };
         const uint32_t x0 = x_s + min(lane >> 2, a.rows - 1) * x_row_bytes + (lane & 3) * 16;
         const uint32_t w0 = ring + (lane >> 2) * ROW_BYTES + (lane & 3) * 16;
@@ -936,15 +950,17 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
   LSE_TL_MARK(3)
 }
 
-// The rows' embeddings as the first layer's residual (packets of epoch 1), and no epoch in every other packet.
+// The rows' embeddings as the first layer's residual (packets of epoch 1) and what its norm reads; no epoch in every other packet,
+// UNSET in the other norms' places.
 __global__ void __launch_bounds__(256)
 decode_layers_start_kernel(const __nv_bfloat16* __restrict__ table, const int* __restrict__ ids, const float* __restrict__ norm,
-                           uint2* __restrict__ input, uint2* __restrict__ input_x, uint2* __restrict__ input_sq, uint4* __restrict__ rest,
-                           long long rest_count, int rows, int hidden, int vocab, float scale) {
+                           uint2* __restrict__ input, uint32_t* __restrict__ normed, uint4* __restrict__ rest, long long rest_count,
+                           uint4* __restrict__ unset, long long unset_count, int rows, int hidden, int vocab, float scale) {
   pdl_launch_dependents();
   pdl_wait();
   const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = first; i < rest_count; i += stride) rest[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = first; i < unset_count; i += stride) unset[i] = make_uint4(UNSET, UNSET, UNSET, UNSET);
   for (int p = first; p < rows * hidden / 2; p += stride) {    // pairs of columns: eight threads hold a group of 16 (hidden % 64 == 0)
     const int row = p / (hidden / 2), column = 2 * (p % (hidden / 2));
     const int id = LSE_CHECKED(ids[row], 0, vocab, -1, LSE_CHECK_TOKEN_ID);
@@ -956,12 +972,11 @@ decode_layers_start_kernel(const __nv_bfloat16* __restrict__ table, const int* _
     }
     input[2 * p] = make_uint2(__float_as_uint(v.x), 1u << 16);
     input[2 * p + 1] = make_uint2(__float_as_uint(v.y), 1u << 16);
-    const unsigned long long both = packet24(v.x * norm[column], v.y * norm[column + 1], 1u);
-    input_x[p] = make_uint2((uint32_t)both, (uint32_t)(both >> 32));
+    reinterpret_cast<uint2*>(normed)[p] = make_uint2(set_bits(v.x * norm[column]), set_bits(v.y * norm[column + 1]));
     float sq = v.x * v.x + v.y * v.y;
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffu << (threadIdx.x & 24), sq, o);
-    if ((p & 7) == 0 && !(p == 0 && lse_decode_layers_withhold)) input_sq[p / 8] = make_uint2(__float_as_uint(sq), 1u << 16);
+    if ((p & 7) == 0) normed[rows * hidden + p / 8] = p == 0 && lse_decode_layers_withhold ? UNSET : set_bits(sq);
   }
 }
 
@@ -1040,21 +1055,22 @@ extern "C" int lse_decode_layers_supported(int blocks, int layers, int rows, int
   return layers >= 1 && layers <= MAX_LAYERS && make_plan(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, &plan) ? 1 : 0;
 }
 
-// Bytes of scratch memory of a launch: the packets that blocks exchange, and the abort word.
-// offsets (14 values): where each begins, every one 256-byte aligned, and the whole.
+// Bytes of scratch memory of a launch: the packets that blocks exchange, the abort word, and the norms' places.
+// offsets (11 values): where each begins, every one 256-byte aligned, and the whole.
 extern "C" int lse_decode_layers_scratch(int blocks, int layers, int rows, int hidden, int inter, int n_q, int n_kv, int vocab, long long* offsets) {
   Plan plan;
   if (!make_plan(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, &plan)) return LSE_ERR_TOO_LARGE;
   const long long residual = (long long)rows * hidden;
-  const long long packets[13] = {residual, residual / 2, residual / 16, residual, residual / 2, residual / 16,
-                                 (long long)rows * (n_q + 2 * n_kv) * HEAD, (long long)rows * n_q * HEAD / 2, (long long)rows * inter / 2,
-                                 (long long)blocks * MAX_HEADS * HEAD, (long long)blocks * MAX_HEADS * 2, plan.down_splits * residual, 1};
+  const long long packets[9] = {residual, residual, (long long)rows * (n_q + 2 * n_kv) * HEAD, (long long)rows * n_q * HEAD / 2,
+                                (long long)rows * inter / 2, (long long)blocks * MAX_HEADS * HEAD, (long long)blocks * MAX_HEADS * 2,
+                                plan.down_splits * residual, 1};
   long long at = 0;
-  for (int i = 0; i < 13; ++i) {
+  for (int i = 0; i < 9; ++i) {
     offsets[i] = at;
     at += (packets[i] * 8 + 255) / 256 * 256;
   }
-  offsets[13] = at;
+  offsets[9] = at;
+  offsets[10] = at + ((2LL * layers + 1) * (residual + residual / 16) * 4 + 255) / 256 * 256;
   return 0;
 }
 
@@ -1109,17 +1125,18 @@ extern "C" int lse_decode_layers(const long long* layer_pointers, const float* l
         !tc::make_map_row_groups(&args.maps[i][1], L.values, cache_rows, HEAD, 16))
       return LSE_ERR_BAD_ARGUMENT;
   }
-  long long at[14];
+  long long at[11];
   lse_decode_layers_scratch(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, at);
   unsigned char* base = (unsigned char*)scratch;
   Common& c = args.common;
   c.head = (const __nv_bfloat16*)head; c.final_norm = final_norm; c.inv_freq = inv_freq;
   c.positions = positions; c.segment_of_token = segment_of_token; c.slot_mapping = slot_mapping;
   c.block_tables = block_tables;
-  uint2** parts[12] = {&c.input, &c.input_x, &c.input_sq, &c.middle, &c.middle_x, &c.middle_sq,
-                       &c.qkv, &c.attended, &c.act, &c.part_o, &c.part_ml, &c.down_part};
-  for (int i = 0; i < 12; ++i) *parts[i] = (uint2*)(base + at[i]);
-  c.abort = (unsigned*)(base + at[12]);
+  uint2** parts[8] = {&c.input, &c.middle, &c.qkv, &c.attended, &c.act, &c.part_o, &c.part_ml, &c.down_part};
+  for (int i = 0; i < 8; ++i) *parts[i] = (uint2*)(base + at[i]);
+  c.abort = (unsigned*)(base + at[8]);
+  c.normed = (uint32_t*)(base + at[9]);
+  c.norm_stride = rows * hidden + rows * hidden / 16;
   c.logits = logits;
   c.layers = layers; c.rows = rows; c.hidden = hidden; c.inter = inter; c.n_q = n_q; c.n_kv = n_kv;
   c.vocab = vocab; c.page_size = page_size; c.bt_stride = bt_stride; c.num_pages = num_pages;
@@ -1128,8 +1145,8 @@ extern "C" int lse_decode_layers(const long long* layer_pointers, const float* l
   c.stages = plan.stages;
   c.final_eps = final_eps; c.scale_log2e = scale * LOG2E;
   cudaError_t err = lse_launch(decode_layers_start_kernel, 2 * blocks, 256, 0, stream, (const __nv_bfloat16*)embedding, token_ids,
-                               args.layer[0].norm1, c.input, c.input_x, c.input_sq, (uint4*)c.middle, (at[13] - at[3]) / 16, rows, hidden,
-                               embedding_rows, embedding_scale);
+                               args.layer[0].norm1, c.input, c.normed, (uint4*)c.middle, (at[9] - at[1]) / 16,
+                               (uint4*)(c.normed + c.norm_stride), 2LL * layers * c.norm_stride / 4, rows, hidden, embedding_rows, embedding_scale);
   if (err != cudaSuccess) return (int)err;
   return launch(args, blocks, plan.smem, stream);
 }

@@ -670,10 +670,10 @@ def decode_layers(layer_pointers: list, eps: list, embedding: torch.Tensor, embe
     lib = library.load()
     blocks, layers = sm_count(), len(layer_pointers)
     flat = (c_longlong * (9 * layers))(*[pointer or 0 for layer in layer_pointers for pointer in layer])
-    places = (c_longlong * 14)()
+    places = (c_longlong * 11)()
     if lib.lse_decode_layers_scratch(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, places) != 0:
         raise KernelError("decode_layers: a step of these sizes does not fit")
-    scratch = torch.empty(places[13], dtype=torch.uint8, device=embedding.device)
+    scratch = torch.empty(places[10], dtype=torch.uint8, device=embedding.device)
     logits = torch.empty((rows, vocab), dtype=torch.float32, device=embedding.device)
     check(lib.lse_decode_layers(flat, (c_float * (2 * layers))(*eps), layers, embedding.data_ptr(), embedding.shape[0],
                                 float(embedding_scale), head.data_ptr(), final_norm.data_ptr(), float(final_eps), inv_freq.data_ptr(),

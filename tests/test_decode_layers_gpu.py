@@ -19,6 +19,7 @@ SIZES = {
     "two_heads": (192, 320, 4, 2, 528),
     "eight_heads": (256, 320, 16, 8, 528),
     "many_heads": (256, 320, 36, 36, 528),
+    "square": (2560, 320, 2, 1, 2560),
 }
 CONTEXTS = [0, 1, 15, 16, 17, 31, 127, 128, 129, 300, 64, 5, 48, 200, 33, 3]
 
@@ -174,6 +175,25 @@ def test_long_contexts(name, layers, contexts, monkeypatch):
         for answer in (got[index], chain[index]):
             assert float((answer - want).abs().max()) <= limit, (context, "one launch" if answer is got[index] else "launch by launch")
             assert helpers.rms_ratio(answer[None], want[None]) <= helpers.RMS_RATIO_LARGE_LAYERS
+
+
+@pytest.mark.parametrize("one_launch", [True, False])
+def test_the_head_reads_rows_that_were_rounded_once(one_launch):
+    """Branches that add nothing and a head that is the identity: the logits are the normed embeddings as the product reads them,
+    float32 up to one rounding to bfloat16.  Float32's own rounding (a few 2^-24) puts a value on the other side of a bfloat16
+    boundary once in 2^13: 5 of the 40,960 values here.  Sixteen bits on the way (2^-18 on average) would do so once in 2^9.5."""
+    config, model, weights = _build("square", layers=1)
+    block = model.blocks[0]
+    block.mixer.o_weight.zero_()
+    block.feed_forward.down_weight.zero_()
+    model.lm_head.copy_(torch.eye(2560))
+    model.final_norm.weight.copy_(1.0 + 0.3 * torch.randn(2560, generator=torch.Generator().manual_seed(3)))
+    rng = random.Random(3)
+    sequences = [helpers.random_tokens(rng, config["vocab_size"], 4) for _ in range(4)]
+    got = _decode(model, sequences, 4, one_launch)
+    rows = weights["model.embed_tokens.weight"][torch.tensor(sequences)].double()
+    want = rows * (rows.pow(2).mean(-1, keepdim=True) + config["rms_norm_eps"]).rsqrt() * model.final_norm.weight.cpu().double()
+    assert int((got != want.bfloat16().float()).sum()) <= 16
 
 
 def test_some_rows_wanted():
