@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "smem_allowance.cuh"
 
 LSE_CHECK_DEFINE(lse_check_delta_memory_chunks)
 
@@ -353,6 +354,7 @@ delta_chunk_scan_kernel(const float* __restrict__ buffer, float* __restrict__ st
 // long as its slowest block.  So the scan asks for this where it has no more blocks than there are SMs.  One request of 501
 // rows, 16 heads of 128 (128 blocks): 82 to 54 us; 130 rows, the whole recurrence: 46 to 38, 2,048 rows: 400 to 288.
 constexpr size_t DC_LONE_SMEM = 116 * 1024;
+constexpr size_t DC_STATIC_SMEM = 4 * 1024;   // at least what the kernels hold beside their dynamic shared memory
 
 template <int NJ>
 int launch_delta_chunks(const float* q, const float* k, const float* v, const float* beta, const float* z, int z_partials,
@@ -364,20 +366,14 @@ int launch_delta_chunks(const float* q, const float* k, const float* v, const fl
   const int ep = (vdim + DCN - 1) / DCN * DCN;
   const size_t prepare_smem = sizeof(float) * 3 * DC * DP;
   const size_t scan_smem = sizeof(float) * (DP * DCS + 2 * (DP * 2 * DC + DP * DC + DP + 2 * DC * DC) + 8 * 512 + DC * DCN);
-  static bool configured = false;
-  static int sm_count = 0;
-  if (!configured) {
-    int device = 0;
-    cudaError_t got = cudaGetDevice(&device);
-    if (got == cudaSuccess) got = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
-    if (got != cudaSuccess) return (int)got;
-    cudaError_t err = cudaFuncSetAttribute(delta_chunk_prepare_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prepare_smem);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(delta_chunk_scan_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::max(scan_smem, DC_LONE_SMEM));
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  static SmemAllowance prepare_allowed, scan_allowed;
+  int device = 0, sm_count = 0;
+  cudaError_t err = cudaGetDevice(&device);
+  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+  // the largest heads' 48 KB would need no allowance but for the kernel's static shared memory beside them
+  if (err == cudaSuccess) err = allow_smem(delta_chunk_prepare_kernel<NJ>, prepare_smem + DC_STATIC_SMEM, prepare_allowed);
+  if (err == cudaSuccess) err = allow_smem(delta_chunk_scan_kernel<NJ>, std::max(scan_smem, DC_LONE_SMEM), scan_allowed);
+  if (err != cudaSuccess) return (int)err;
   lse_launch(delta_chunk_prepare_kernel<NJ>, dim3(max_chunks, heads), 128, prepare_smem, stream, q, k, v, beta, z, z_partials,
              z_stride, z_ld, dt_bias, a_log, segment_start, buffer, max_segments, heads, groups, dim, vdim, ep, min_rows);
   const bool lone = (long long)max_segments * heads * (ep / DCN) <= sm_count;

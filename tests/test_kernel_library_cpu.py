@@ -111,3 +111,55 @@ extern "C" int together() {
                                        (0, 90000, 7, 1), (0, 90000, 0, 1), (1, 90000, 0, 1), (1, 90000, 0, 0), (70, 90000, 0, 1)):
         assert trial.raise_(device, bytes_, err) == calls, (device, bytes_, err)
     assert trial.together() == 0
+
+
+def test_the_delta_memorys_scan_is_allowed_its_shared_memory_on_every_device(tmp_path):
+    """The launcher, compiled here and linked with a runtime that only keeps books: on a second device, and on one of fewer SMs,
+    every launch stays within what that device has been asked to allow (48 KB need no asking, static shared memory included, of which
+    these kernels have up to 4), and asks for an SM a block where that device has so many."""
+    (tmp_path / "books.cpp").write_text('''
+#include <cuda_runtime_api.h>
+#include <map>
+#include <utility>
+static int device, launches, refused, largest;
+static std::map<std::pair<int, const void*>, int> allowed;
+extern "C" {
+int use(int which) { device = which; launches = refused = largest = 0; return 0; }
+int refusals() { return launches == 2 ? refused : -1; }
+int most() { return largest; }
+void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void*) { return 0; }
+cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* out) { *out = device; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* out, cudaDeviceAttr, int which) { *out = which == 2 ? 20 : 148; return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute, int bytes) { allowed[{device, kernel}] = bytes; return cudaSuccess; }
+cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* kernel, void**) {
+  const int bytes = (int)config->dynamicSmemBytes;
+  const auto found = allowed.find({device, kernel});
+  ++launches;
+  if (bytes > largest) largest = bytes;
+  if (bytes > 44 * 1024 && (found == allowed.end() || bytes > found->second)) { ++refused; return cudaErrorInvalidValue; }
+  return cudaSuccess;
+}
+}
+''')
+    nvcc = [build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O1", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]
+    subprocess.run([*nvcc, "-c", str(build.CSRC / "delta_memory_chunks.cu"), "-o", str(tmp_path / "chunks.o")], check=True)
+    subprocess.run([*nvcc, "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic", str(tmp_path / "books.cpp"), str(tmp_path / "chunks.o"),
+                    "-o", str(tmp_path / "books.so")], check=True)     # its own runtime, also where another is in the process
+    books = ctypes.CDLL(str(tmp_path / "books.so"))
+    scan = books.lse_delta_chunk_scan
+    scan.argtypes = library._SIGNATURES["lse_delta_chunk_scan"]
+    for device, lone in ((0, True), (1, True), (0, True), (2, False), (70, True)):
+        for dim in (24, 64, 128, 200):
+            books.use(device)
+            # q .. beta, z, partials of z, bias and decay, state, segments, results, buffer; 10 chunks of one request, four heads
+            assert scan(*[None] * 5, 1, 0, 0, *[None] * 7, 10, 1, 4, 4, dim, 128, 1, 1, None) == 0
+            assert books.refusals() == 0, (device, dim)
+            assert lone == (books.most() >= 116 * 1024) or dim > 128
