@@ -529,12 +529,33 @@ def gemm_bf16_skinny(x: torch.Tensor, weight: torch.Tensor, splits: int | None =
 _PAIRS_ACT = {"silu": 0, "gelu_tanh": 1, "relu": 2, "clamped_swish": 3}
 
 
+def _pairs_operand_ok(operand: torch.Tensor) -> bool:
+    return (operand.is_cuda and operand.dtype == torch.bfloat16 and operand.dim() == 2 and 0 < operand.shape[0] < 2 ** 31
+            and operand.shape[1] % 8 == 0 and operand.stride(1) == 1 and operand.stride(0) % 8 == 0 and operand.data_ptr() % 16 == 0)
+
+
 def gemm_pairs_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether the product on pairs of SMs takes these operands (bfloat16, rows of whole 16-byte pieces)."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] > 0
-            and x.stride(1) == 1 and weight.stride(1) == 1 and x.stride(0) % 8 == 0 and weight.stride(0) % 8 == 0
-            and x.shape[1] % 8 == 0 and weight.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-            and max(x.shape[0], weight.shape[0]) < 2 ** 31)
+    return _pairs_operand_ok(x) and _pairs_operand_ok(weight)
+
+
+def _need_pairs(name: str, operands, outs, whole_scale: torch.Tensor | None = None, offsets: torch.Tensor | None = None,
+                sizes_fit: bool = True) -> None:
+    """Raises where the product on pairs of SMs would read or write something else than is meant.  ``outs``: (results, rows of
+    their operand, whether they may be float32)."""
+    if not all(_pairs_operand_ok(operand) for operand in operands):
+        raise KernelError(f"{name}: operands must be bfloat16, 16-byte aligned, rows of a multiple of 8 values")
+    for out, rows, float32_too in outs:
+        if (not out.is_cuda or out.dim() != 2 or out.shape[0] != rows or out.stride(1) != 1
+                or out.dtype != torch.bfloat16 and not (float32_too and out.dtype == torch.float32)):
+            raise KernelError(f"{name}: results must be rows of their operand, {'bfloat16 or float32' if float32_too else 'bfloat16'}, whole columns")
+    if whole_scale is not None and (whole_scale.dtype != torch.float32 or whole_scale.numel() != outs[-1][1] or not whole_scale.is_contiguous()):
+        raise KernelError(f"{name}: factors must be float32, one a row")
+    if offsets is not None and (offsets.dtype != torch.int32 or offsets.dim() != 1 or not offsets.is_contiguous()
+                                or not 0 < offsets.shape[0] <= PAIRS_MAX_GROUPS):
+        raise KernelError(f"{name}: ends of 1 to {PAIRS_MAX_GROUPS} groups must be int32")
+    if not sizes_fit:
+        raise KernelError(f"{name}: the weights are not of the operands' and results' sizes")
 
 
 def gated_product_wanted(x: torch.Tensor, weight: torch.Tensor) -> bool:
@@ -556,8 +577,7 @@ def gated_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, acti
     _need_cuda(x, weight, out)
     rows, k = x.shape
     inter = out.shape[1]
-    if not gemm_pairs_ok(x, weight) or weight.shape != (2 * inter, k) or out.shape[0] != rows or out.stride(1) != 1 or out.dtype != torch.bfloat16:
-        raise KernelError("gated_product: operands must be bfloat16, 16-byte aligned, rows of a multiple of 8 values")
+    _need_pairs("gated_product", (x, weight), ((out, rows, False),), sizes_fit=weight.shape == (2 * inter, k))
     check(library.load().lse_gemm_pairs(None, 0, 0, None, 0, 0, 0, None, 0, 0, 0.0, x.data_ptr(), rows, x.stride(0), inter, k,
                                         out.data_ptr(), out.stride(0), 0, None, float(limit), weight.data_ptr(), 2 * inter, k,
                                         weight.stride(0), _PAIRS_ACT[activation], sm_count(), _stream()), "gated_product")
@@ -572,11 +592,12 @@ def gated_product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tens
                          activation: str) -> None:
     """:func:`gated_product` of groups of rows of ``x`` (their ends: ``offsets``, int32), each with the next 2 * out.shape[1] rows of
     ``weight``, and of all rows of ``whole`` with the rows behind those, times ``whole_scale`` by row."""
-    _need_cuda(x, offsets, out, whole, weight)
+    _need_cuda(x, offsets, out, whole, whole_out, whole_scale, weight)
     k, routed, columns = x.shape[1], offsets.shape[0], out.shape[1]
-    assert offsets.dtype == torch.int32 and out.shape[0] == x.shape[0] and out.dtype == torch.bfloat16
-    if whole is not None:
-        assert whole.shape[1] == k and whole_out.shape[0] == whole.shape[0] and whole_out.dtype == torch.bfloat16
+    both = whole is not None
+    _need_pairs("gated_product_groups", (x, weight, whole) if both else (x, weight),
+                ((out, x.shape[0], False),) + (((whole_out, whole.shape[0], False),) if both else ()), whole_scale if both else None, offsets,
+                weight.shape == (2 * (routed * columns + (whole_out.shape[1] if both else 0)), k) and (not both or whole.shape[1] == k))
     check(library.load().lse_gemm_pairs(
         x.data_ptr(), x.shape[0], x.stride(0), offsets.data_ptr(), routed, columns, k, out.data_ptr(), out.stride(0), 0, float(limit),
         _ptr(whole), 0 if whole is None else whole.shape[0], 0 if whole is None else whole.stride(0),
@@ -589,9 +610,13 @@ def product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, wh
                    whole_out: torch.Tensor | None, weight: torch.Tensor) -> None:
     """out[t] = x[t] W_g^T for groups of rows of ``x`` (their ends: ``offsets``), W_g the g-th x.shape[1] columns of ``weight``
     (a multiple of 64), and whole_out = whole W^T with the columns behind those; bfloat16 or float32 results."""
-    _need_cuda(x, offsets, out, whole, weight)
+    _need_cuda(x, offsets, out, whole, whole_out, weight)
     k, routed, columns = x.shape[1], offsets.shape[0], weight.shape[0]
-    assert offsets.dtype == torch.int32 and out.shape == (x.shape[0], columns)
+    both = whole is not None
+    _need_pairs("product_groups", (x, weight, whole) if both else (x, weight),
+                ((out, x.shape[0], True),) + (((whole_out, whole.shape[0], True),) if both else ()), None, offsets,
+                k % 64 == 0 and weight.shape[1] == routed * k + (whole.shape[1] if both else 0) and out.shape[1] == columns
+                and (not both or whole_out.shape[1] == columns))
     check(library.load().lse_gemm_pairs(
         x.data_ptr(), x.shape[0], x.stride(0), offsets.data_ptr(), routed, columns, k, out.data_ptr(), out.stride(0),
         int(out.dtype == torch.float32), 0.0, _ptr(whole), 0 if whole is None else whole.shape[0], 0 if whole is None else whole.stride(0),

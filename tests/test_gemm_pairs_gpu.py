@@ -114,3 +114,41 @@ def test_what_the_product_does_not_take():
     assert not o.gemm_pairs_ok(_random(41, 64).flatten()[4:4 + 40 * 64].view(40, 64), w)
     with pytest.raises(o.KernelError):
         o.gated_product(x.float(), w, torch.empty(40, 64, device=DEV, dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("wrong", ["strided x", "strided whole", "float32 x", "float16 weight", "misaligned whole", "misaligned weight",
+                                   "rows of the result", "columns apart", "float32 result", "few weights", "int64 ends", "ends apart",
+                                   "factors", "float16 result"])
+def test_what_the_products_over_groups_do_not_take(wrong):
+    """Every operand is looked at before a launch, in both products: nothing is read as something that it is not."""
+    o = ops()
+
+    def refused(gated):
+        groups, columns, k, rows, whole = 2, 64, 128, 40, 24
+        x, everyone = _random(rows, k), _random(whole, k)
+        offsets, scale = torch.tensor([10, 40], device=DEV, dtype=torch.int32), torch.rand(whole, device=DEV)
+        weight = _random(2 * (groups + 1) * columns, k) if gated else _random(columns, (groups + 1) * k)
+        out, total = (torch.empty(count, columns, device=DEV, dtype=torch.bfloat16) for count in (rows, whole))
+        if wrong == "strided x": x = _random(k, rows).t()
+        if wrong == "strided whole": everyone = _random(whole, 2 * k)[:, ::2]
+        if wrong == "float32 x": x = x.float()
+        if wrong == "float16 weight": weight = weight.half()
+        if wrong == "misaligned whole": everyone = _random(whole + 1, k).flatten()[4:4 + whole * k].view(whole, k)
+        if wrong == "misaligned weight": weight = _random(weight.shape[0] + 1, weight.shape[1]).flatten()[1:1 + weight.numel()].view(weight.shape)
+        if wrong == "rows of the result": out = out[1:]
+        if wrong == "columns apart": total = torch.empty(columns, whole, device=DEV, dtype=torch.bfloat16).t()
+        if wrong == "float32 result": out = out.float()
+        if wrong == "float16 result": out = out.half()
+        if wrong == "few weights": weight = weight[:, :-64] if not gated else weight[:-64]
+        if wrong == "int64 ends": offsets = offsets.long()
+        if wrong == "ends apart": offsets = torch.zeros(4, device=DEV, dtype=torch.int32)[::2]
+        if wrong == "factors": scale = scale.half()
+        if not gated and wrong in ("float32 result", "factors"):      # this product's results may be float32, and it has no factors
+            return
+        with pytest.raises(o.KernelError):
+            if gated:
+                o.gated_product_groups(x, offsets, out, 0.0, everyone, total, scale, 0.0, weight, "silu")
+            else:
+                o.product_groups(x, offsets, out, everyone, total, weight)
+    refused(True)
+    refused(False)
