@@ -21,7 +21,10 @@
 // activations.
 //
 // The grid is persistent: pair p takes tiles p, p + pairs, ...; a group's row tiles follow one another under the same rows of w.
-// Every wait is bounded; a wait that gives up sets lse_gemm_pairs_error, and what the launch wrote is not to be used.
+// Every wait is bounded; a wait that gives up sets lse_gemm_pairs_error, and what the launch wrote is not to be used.  Both blocks of
+// the pair then stay until what is in flight has landed, whichever of their threads gave up.
+#include <atomic>
+
 #include "gate_act.cuh"
 #include "smem_allowance.cuh"
 #include "tcgen05.cuh"
@@ -35,6 +38,7 @@ constexpr int FINISHERS = 8;                                                 // 
 constexpr uint32_t ACC_COLS = 256;
 
 __device__ int lse_gemm_pairs_error;
+std::atomic<int> withhold{0};  // test hook
 
 struct Source {                // rows of x, and where their results go
   CUtensorMap rows[4];         // boxes of 32, 64, 96 and 128 rows
@@ -102,6 +106,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
                  "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr));
+}
+
+__device__ __forceinline__ void set_abort_there(uint32_t flag, int rank) {   // the other block's
+  asm volatile("{\n\t.reg .b32 there;\n\tmapa.shared::cluster.u32 there, %0, %1;\n\tst.shared::cluster.u32 [there], %2;\n\t}\n"
+               ::"r"(flag), "r"(rank), "r"(1) : "memory");
 }
 
 // Whether it went well for all threads of the warps that finish tiles (they meet at barriers: all go on or none).
@@ -241,7 +250,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128 + 32 * FINISHERS
           if (++stage == STAGES) { stage = 0; parity ^= 1u; }
         }
       }
-      if (!ok) for (int i = 0; i < 2000; ++i) __nanosleep(100);     // copies in flight land before the block leaves
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -272,6 +280,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128 + 32 * FINISHERS
         buffer ^= 1;
         if (buffer == 0) buffer_parity ^= 1u;
       }
+      if (!ok) set_abort_there(smem_u32(&s.abort), 1);   // the odd block's waits need not run out themselves
     }
     __syncwarp();
   } else if (warp >= 4) {          // finish the tiles: a warp reads 32 lanes and half of the columns
@@ -381,7 +390,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128 + 32 * FINISHERS
   }
   fence_before_sync();
   __syncthreads();
+  if (threadIdx.x == 0 && s.abort) set_abort_there(smem_u32(&s.abort), rank ^ 1);
   cluster_sync();                  // the other block may still count on this one's barriers, and the products on its operands
+  if (s.abort) {                   // loads and products in flight end (200 us: they take some) before either block leaves
+    if (threadIdx.x == 0) for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    __syncthreads();
+    cluster_sync();
+  }
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
 }
 
@@ -421,6 +436,12 @@ extern "C" int lse_gemm_pairs_status_reset(void) {
   const int zero = 0;
   return (int)cudaMemcpyToSymbol(lse_gemm_pairs_error, &zero, sizeof(int));
 }
+// Test hook.  withheld != 0: launches bring half of every box of x's rows, so that the wait for the rest gives up (after some
+// tenths of a second: the waits' limits are constants.  As an argument of the launch they made 2,048 x 1,536 x 8,960 take 96.3 us, not 93.2).
+extern "C" int lse_gemm_pairs_test_hook(int withheld) {
+  withhold = withheld;
+  return 0;
+}
 
 // Results of groups of rows, each with its own weights, and (whole_rows > 0) of all rows of another tensor with the weights behind
 // those.  x [x_rows, k] and whole_x [whole_rows, whole_k] bfloat16, rows ld elements apart; offsets int32 [routed] ends of
@@ -442,9 +463,10 @@ extern "C" int lse_gemm_pairs(const void* x, long long x_rows, long long ld_x, c
   // the boxes that the tiles of all rows take: every tile but the last has rows_a_tile rows
   const int a_tile = whole_rows ? rows_of_tiles(whole_rows) : 32;
   const int first_box = box_of(rows_of_tile(whole_rows, a_tile)), last_box = whole_rows ? box_of(rows_of_tile((whole_rows - 1) % a_tile + 1, a_tile)) : 0;
+  const int box_rows = withhold ? 16 : 32;
   for (int box = 1; box <= 4; ++box) {
-    if (routed && !make_rows_map(&args.source[0].rows[box - 1], x, x_rows, k, ld_x, 32 * box)) return LSE_ERR_BAD_ARGUMENT;
-    if (whole_rows && (box == first_box || box == last_box) && !make_rows_map(&args.source[1].rows[box - 1], whole_x, whole_rows, whole_k, ld_whole, 32 * box)) return LSE_ERR_BAD_ARGUMENT;
+    if (routed && !make_rows_map(&args.source[0].rows[box - 1], x, x_rows, k, ld_x, box_rows * box)) return LSE_ERR_BAD_ARGUMENT;
+    if (whole_rows && (box == first_box || box == last_box) && !make_rows_map(&args.source[1].rows[box - 1], whole_x, whole_rows, whole_k, ld_whole, box_rows * box)) return LSE_ERR_BAD_ARGUMENT;
   }
   if (!gated && routed && k % BLOCK_K) return LSE_ERR_BAD_ARGUMENT;      // a group's last k would meet the next one's weights
   args.source[0].out = out; args.source[0].ld_out = ld_out; args.source[0].out_f32 = out_f32; args.source[0].limit = limit;

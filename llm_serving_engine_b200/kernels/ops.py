@@ -625,6 +625,12 @@ def product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, wh
         weight.stride(0), -1, sm_count(), _stream()), "product_groups")
 
 
+def gemm_pairs_test_hook(withhold: bool = False) -> None:
+    """For tests of the bounded waits: launches bring half of x's rows, and the wait for the others gives up."""
+    torch.cuda.synchronize()
+    check(library.load().lse_gemm_pairs_test_hook(int(bool(withhold))), "gemm_pairs test hook")
+
+
 def gemm_bf16_skinny_test_hooks(spin_limit: int = 0, withhold: bool = False) -> None:
     """For tests of the bounded waits: ``spin_limit`` iterations before a wait gives up (0: the default),
     ``withhold``: every block leaves out its last weight tile, so that a wait runs out."""

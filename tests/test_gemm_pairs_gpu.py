@@ -152,3 +152,45 @@ def test_what_the_products_over_groups_do_not_take(wrong):
                 o.product_groups(x, offsets, out, everyone, total, weight)
     refused(True)
     refused(False)
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("rows", [40, 4000])
+def test_a_wait_that_runs_out_is_reported_and_the_kernel_returns(gated, rows):
+    """Half of x's rows do not come, and the wait for them gives up (after some tenths of a second); the other waits of both blocks of the pair
+    see it, for pairs of one tile and of several.  The launch ends, the status word reaches
+    the host as the sampler reads it, and after a reset the product is right.  Nothing faults: a load is simply not started."""
+    from llm_serving_engine_b200.kernels import library
+    from llm_serving_engine_b200.sampling.sampler import GenerationConfig, Sampler
+
+    o = ops()
+    torch.manual_seed(rows)
+    k, columns = 448, 2560
+    x, offsets = _random(rows, k), torch.tensor([rows], device=DEV, dtype=torch.int32)
+    weight = _random(2 * columns if gated else columns, k, k ** -0.5)
+    out = torch.empty(rows, columns, device=DEV, dtype=torch.bfloat16)
+
+    def product():
+        if gated:
+            o.gated_product(x, weight, out)
+        else:
+            o.product_groups(x, offsets, out, None, None, weight)
+        torch.cuda.synchronize()
+
+    sampler = Sampler(16, 1, torch.device(DEV))
+    product()
+    assert library.load().lse_gemm_pairs_status() == 0
+    o.gemm_pairs_test_hook(withhold=True)
+    try:
+        product()
+        assert library.load().lse_gemm_pairs_status() == 1
+        ticket = sampler.launch(torch.zeros(1, 16, device=DEV), [GenerationConfig()], [0])
+        with pytest.raises(o.KernelError, match="the product on pairs of SMs"):
+            sampler.collect(ticket)
+    finally:
+        o.gemm_pairs_test_hook()
+        o.kernel_status_reset()
+    product()
+    sums = x.double() @ weight.double().t()
+    _check(out, _act("silu", sums[:, :columns], sums[:, columns:], 0.0) if gated else sums, x, weight)
+    assert library.load().lse_gemm_pairs_status() == 0
