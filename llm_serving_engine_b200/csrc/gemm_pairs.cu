@@ -412,17 +412,31 @@ bool make_rows_map(CUtensorMap* map, const void* ptr, long long rows, long long 
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024;
+
+template <bool GATED, int ACT>
+cudaError_t allow() {
+  static SmemAllowance allowance;
+  return allow_smem(gemm_pairs_kernel<GATED, ACT>, SMEM, allowance);
+}
+
 template <bool GATED, int ACT>
 int launch(const Args& args, int blocks, cudaStream_t stream) {
-  static SmemAllowance allowance;
-  const size_t smem = (size_t)STAGES * STAGE + 1024;
-  cudaError_t err = allow_smem(gemm_pairs_kernel<GATED, ACT>, smem, allowance);
+  cudaError_t err = allow<GATED, ACT>();
   if (err != cudaSuccess) return (int)err;
-  err = lse_launch(gemm_pairs_kernel<GATED, ACT>, blocks, 128 + 32 * FINISHERS, smem, stream, args);
+  err = lse_launch(gemm_pairs_kernel<GATED, ACT>, blocks, 128 + 32 * FINISHERS, SMEM, stream, args);
   if (err != cudaSuccess) return (int)err;
   return (int)cudaGetLastError();
 }
 }  // namespace
+
+// The kernels loaded on the current device and allowed their shared memory, ahead of the first launch.
+extern "C" int lse_gemm_pairs_prepare(void) {
+  const cudaError_t errors[] = {allow<false, 0>(), allow<true, 0>(), allow<true, 1>(), allow<true, 2>(), allow<true, 3>()};
+  for (cudaError_t err : errors)
+    if (err != cudaSuccess) return (int)err;
+  return 0;
+}
 
 extern "C" int lse_gemm_pairs_status(void) {
   int value = 0;

@@ -218,6 +218,7 @@ _SIGNATURES = {
     "lse_gemm_pairs": [c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_float,
                        c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_float, c_void_p,
                        c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p],
+    "lse_gemm_pairs_prepare": [],
     "lse_gemm_pairs_status": [],
     "lse_gemm_pairs_status_async": [c_void_p, c_void_p],
     "lse_gemm_pairs_status_reset": [],

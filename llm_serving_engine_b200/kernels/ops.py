@@ -587,6 +587,16 @@ def gated_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, acti
 PAIRS_MAX_GROUPS = 256
 
 
+def gemm_pairs_prepare(device: torch.device) -> None:
+    """Have the product on pairs of SMs loaded on that device, with the shared memory that it needs: what its first use would do
+    otherwise, which is not to fall into a capture (a captured step's rows are rounded up, and may take it where no step launched
+    kernel by kernel has)."""
+    with torch.cuda.device(device):
+        code = library.load().lse_gemm_pairs_prepare()
+    if code:
+        raise KernelError(f"gemm_pairs_prepare: CUDA error {code}")
+
+
 def gated_product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, limit: float, whole: torch.Tensor | None,
                          whole_out: torch.Tensor | None, whole_scale: torch.Tensor | None, whole_limit: float, weight: torch.Tensor,
                          activation: str) -> None:

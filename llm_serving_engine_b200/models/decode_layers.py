@@ -11,8 +11,10 @@ import os
 
 import torch
 
+from ..config.model_config import ModelSpec
 from ..kernels import ops
 from ..parts.attention import GroupedQueryAttention
+from ..parts.base import BLOCKS, FEED_FORWARDS, MIXERS, NORMS, POSITION_ENCODINGS
 from ..parts.block import PreNormResidualBlock
 from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
@@ -46,12 +48,27 @@ class DecodeLayers:
                                  block.mixer_norm.weight, block.feed_forward_norm.weight])
             self.eps += [block.mixer_norm.eps, block.feed_forward_norm.eps]
 
+    @staticmethod
+    def described(spec: ModelSpec, dtype: torch.dtype) -> bool:
+        """Whether models of this description may be of that kind: then they have the kernel loaded when they are built."""
+        if (not ENABLED or dtype != torch.bfloat16 or spec.residual_streams != 1 or spec.position_table_name or spec.embedding_again
+                or NORMS.get(spec.final_norm.kind) is not RMSNorm):
+            return False
+        for layer in spec.layers:
+            mixer, ff = layer.mixer, layer.feed_forward
+            if (ff is None or layer.feed_forward_norm is None or BLOCKS.get(layer.block.kind) is not PreNormResidualBlock
+                    or MIXERS.get(mixer.kind) is not GroupedQueryAttention or FEED_FORWARDS.get(ff.kind) is not SwiGLU
+                    or NORMS.get(layer.mixer_norm.kind) is not RMSNorm or NORMS.get(layer.feed_forward_norm.kind) is not RMSNorm
+                    or POSITION_ENCODINGS.get(mixer.params["position"]["kind"]) is not RotaryEncoding
+                    or int(mixer.params["head_dim"]) != 128):
+                return False
+        return True
+
     @classmethod
     def of(cls, model) -> "DecodeLayers | None":
         """For a model whose layers are of that kind, else None."""
         spec = model.spec
-        if (not ENABLED or model.device.type != "cuda" or model.dtype != torch.bfloat16 or spec.residual_streams != 1
-                or model.position_table is not None or spec.embedding_again or type(model.final_norm) is not RMSNorm):
+        if model.device.type != "cuda" or not cls.described(spec, model.dtype):
             return None
         if model.embedding.dtype != torch.bfloat16 or model.lm_head.dtype != torch.bfloat16:
             return None

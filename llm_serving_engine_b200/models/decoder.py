@@ -111,6 +111,10 @@ def kernel_sources(spec: ModelSpec, dtype: torch.dtype) -> set[str]:
         for cls in classes:
             out.update(getattr(cls, "kernel_sources", ()))
     out.update(getattr(NORMS.get(spec.final_norm.kind), "kernel_sources", ()))
+    if DecodeLayers.described(spec, dtype):
+        out.add("decode_layers")
+    if dtype == torch.float32:
+        out.discard("gemm_pairs")       # products of bfloat16
     return out
 
 

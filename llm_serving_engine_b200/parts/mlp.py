@@ -24,7 +24,7 @@ class SwiGLU(FeedForward):
     on the way."""
 
     graph_safe = True
-    kernel_sources = ("elementwise",)
+    kernel_sources = ("elementwise", "gemm_pairs")
 
     def __init__(self, params, weights, ctx) -> None:
         super().__init__(params, weights, ctx)
@@ -39,6 +39,8 @@ class SwiGLU(FeedForward):
         names = {**_DEFAULT_NAMES, **params.get("tensor_names", {})}
         self.gate_up_weight = torch.cat([weights[names["gate"]], weights[names["up"]]], dim=0).contiguous()
         self.down_weight = weights[names["down"]].contiguous()
+        if self.gate_up_weight.is_cuda and self.gate_up_weight.dtype == torch.bfloat16:
+            ops.gemm_pairs_prepare(self.gate_up_weight.device)     # its first use may be one while a step is captured
 
     @classmethod
     def expected_tensors(cls, params, hidden_size):

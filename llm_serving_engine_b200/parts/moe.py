@@ -115,6 +115,8 @@ class ClampedMoE(FeedForward):
         # the engine's own products over groups of rows: gated experts whose columns are whole pieces of 64
         self._in_pairs = (self._grouped_gate_up is not None and self.activation in ("clamped_swish", "silu") and self.ff % 64 == 0
                           and self.shared_ff % 8 == 0 and self.experts <= ops.PAIRS_MAX_GROUPS)
+        if self._in_pairs and self.gate_up_weight.is_cuda:
+            ops.gemm_pairs_prepare(self.gate_up_weight.device)     # its first use may be one while a step is captured
 
     @classmethod
     def expected_tensors(cls, params, hidden_size):

@@ -76,6 +76,20 @@ def test_a_model_names_the_sources_of_its_parts_only():
     assert "elementwise" in needed["givelix"] and "residual_streams" in needed["givelix"] and "moe" not in needed["givelix"]
 
 
+def test_a_model_names_what_its_steps_choose_by_their_rows():
+    """The products and the decode step that only some numbers of rows take are loaded with the model, not by the step that first
+    takes them: that may be one that is being captured."""
+    from llm_serving_engine_b200.config import load_config
+    from llm_serving_engine_b200.models.decoder import kernel_sources
+
+    config = {"architectures": ["Qwen2ForCausalLM"], "model_type": "qwen2", "vocab_size": 528, "hidden_size": 192, "head_dim": 128,
+              "intermediate_size": 320, "num_hidden_layers": 2, "num_attention_heads": 2, "num_key_value_heads": 1,
+              "max_position_embeddings": 1024, "rope_theta": 10000.0, "rms_norm_eps": 1e-6, "tie_word_embeddings": False}
+    for head_dim, dtype, want in ((128, torch.bfloat16, {"decode_layers", "gemm_pairs"}), (64, torch.bfloat16, {"gemm_pairs"}), (128, torch.float32, set())):
+        _, _, spec = load_config({**config, "head_dim": head_dim})
+        assert kernel_sources(spec, dtype) & {"decode_layers", "gemm_pairs"} == want
+
+
 def test_libraries_share_the_switch_of_dependent_launches():
     """Two libraries in one process have one switch: built here (nvcc needs no GPU), loaded, compared by address."""
     paths = build.library_paths(["elementwise", "tanh_norm"], verbose=False)

@@ -134,3 +134,58 @@ def test_decode_steps_split_their_keys_by_the_contexts_and_not_by_the_tables(mon
         assert splits == [eager] and graphs.graph_replays == replays + 1 and len(graphs._graphs) == 2
         assert graphs._decode_key(64, graphs._pages_after([StepEntry(e.request_id, [], []) for e in entries]))[2] == kind, turn
         assert float((got - want).abs().max()) <= 2.0 ** -5 * float(want.abs().max())      # bfloat16, another order of sums
+
+
+_ROUNDED_UP = """
+import random, torch
+from llm_serving_engine_b200.cache import CacheManager
+from llm_serving_engine_b200.config import CacheConfig, load_config
+from llm_serving_engine_b200.engine import StepEntry, StepRunner
+from llm_serving_engine_b200.kernels import library, ops
+from llm_serving_engine_b200.models import DecoderModel, cache_requirements, expected_tensors
+
+config = {"architectures": ["Qwen2ForCausalLM"], "model_type": "qwen2", "vocab_size": 512, "hidden_size": 1536, "intermediate_size": 8960,
+          "num_hidden_layers": 2, "num_attention_heads": 12, "num_key_value_heads": 2, "max_position_embeddings": 2048,
+          "rope_theta": 1e6, "rms_norm_eps": 1e-6, "tie_word_embeddings": True}
+_, _, spec = load_config(config)
+torch.manual_seed(1)
+weights = {}
+for name, tensor in expected_tensors(spec).items():
+    value = torch.randn(tensor.shape, device="cuda") * (tensor.shape[-1] ** -0.5 if tensor.kind == "matrix" else 0.05)
+    weights[name] = value.bfloat16() if tensor.kind == "matrix" else value + (tensor.kind == "norm")
+model = DecoderModel(spec, weights, torch.bfloat16, "cuda")
+assert library.load().source_loaded("gemm_pairs") and library.load().source_loaded("decode_layers")
+calls = []
+product = ops.gated_product
+ops.gated_product = lambda *given: calls.append(1) or product(*given)
+rng = random.Random(1)
+prompts = [[rng.randrange(512) for _ in range(900)] for _ in range(3)]
+logits, counts = {}, []
+for graphs in (True, False):
+    cache = CacheManager(cache_requirements(spec), CacheConfig(16, 64), model.dtype, "cuda", 2048, num_state_slots=2)
+    runner = StepRunner(model, cache, 1024, 2, use_graphs=graphs)
+    logits[graphs] = []
+    for prompt in prompts:
+        cache.create("r")
+        logits[graphs].append(runner.run([StepEntry("r", prompt, [899])]).clone())
+        cache.free("r")
+        counts.append(len(calls))
+    if graphs:
+        assert runner.portion_graph_replays == 2
+assert counts == [0, 2, 2, 2, 2, 2], counts        # met first while a step is captured, of 1,024 rows, and replayed
+for got, want in zip(logits[True], logits[False]):
+    error = float((got - want).abs().max() / want.abs().max())
+    assert error <= 2.0 ** -5, error
+print("as launch by launch")
+"""
+
+
+def test_a_product_that_only_the_rows_of_a_captured_step_take():
+    """A portion of 900 rows runs launch by launch at first, then captured with 1,024: only there are the rows enough for the product
+    with its gate.  In a process of its own, without a warm-up, so that this is the product's first use."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    run = subprocess.run([sys.executable, "-c", _ROUNDED_UP], capture_output=True, text=True, timeout=600, cwd=Path(__file__).parents[1])
+    assert run.returncode == 0 and "as launch by launch" in run.stdout, run.stderr
