@@ -20,6 +20,8 @@ from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
 from ..parts.rope import RotaryEncoding
 
+HEAD = 128     # head size of the kernel
+
 # LSE_DECODE_LAYERS=0: decode steps launch by launch, for comparisons and for the timeline of single kernels
 ENABLED = os.environ.get("LSE_DECODE_LAYERS", "1") != "0"
 
@@ -33,20 +35,31 @@ ENABLED = os.environ.get("LSE_DECODE_LAYERS", "1") != "0"
 MOST_VALUES = 10240
 
 
+# A part whose class or instance has another ``forward`` (wrapped to look at what passes, replaced in a trial) is called, not read.
+_CALLED = {PreNormResidualBlock: "forward", GroupedQueryAttention: "forward", SwiGLU: "forward", RMSNorm: "forward",
+           RotaryEncoding: "encode_and_store"}
+_AS_WRITTEN = {cls: getattr(cls, name) for cls, name in _CALLED.items()}
+
+
+def _plain(part, cls) -> bool:
+    name = _CALLED[cls]
+    return type(part) is cls and name not in vars(part) and getattr(cls, name) is _AS_WRITTEN[cls]
+
+
+def _matrix(tensor, rows: int, columns: int) -> bool:
+    return (tensor.dtype == torch.bfloat16 and tensor.shape == (rows, columns) and tensor.is_contiguous() and tensor.data_ptr() % 16 == 0)
+
+
+def _vector(tensor, size: int) -> bool:
+    return tensor.dtype == torch.float32 and tensor.shape == (size,) and tensor.is_contiguous() and tensor.data_ptr() % 16 == 0
+
+
 class DecodeLayers:
-    """The layers of a model whose decode steps the one-launch kernel can run."""
+    """Decode steps of a model whose layers the one-launch kernel can run.  Nothing is kept of the layers: every step that is
+    launched (a captured one: when it is captured) reads the parts as they are then."""
 
     def __init__(self, model) -> None:
         self.model = model
-        first = model.blocks[model.spec.order[0]]
-        self.mixer, self.inter = first.mixer, first.feed_forward.inter
-        self.weights, self.eps = [], []
-        for index in model.spec.order:
-            block = model.blocks[index]
-            mixer, ff = block.mixer, block.feed_forward
-            self.weights.append([mixer.qkv_weight, mixer.o_weight, ff.gate_up_weight, ff.down_weight, mixer.qkv_bias,
-                                 block.mixer_norm.weight, block.feed_forward_norm.weight])
-            self.eps += [block.mixer_norm.eps, block.feed_forward_norm.eps]
 
     @staticmethod
     def described(spec: ModelSpec, dtype: torch.dtype) -> bool:
@@ -60,43 +73,61 @@ class DecodeLayers:
                     or MIXERS.get(mixer.kind) is not GroupedQueryAttention or FEED_FORWARDS.get(ff.kind) is not SwiGLU
                     or NORMS.get(layer.mixer_norm.kind) is not RMSNorm or NORMS.get(layer.feed_forward_norm.kind) is not RMSNorm
                     or POSITION_ENCODINGS.get(mixer.params["position"]["kind"]) is not RotaryEncoding
-                    or int(mixer.params["head_dim"]) != 128):
+                    or int(mixer.params["head_dim"]) != HEAD):
                 return False
         return True
 
     @classmethod
     def of(cls, model) -> "DecodeLayers | None":
         """For a model whose layers are of that kind, else None."""
-        spec = model.spec
-        if model.device.type != "cuda" or not cls.described(spec, model.dtype):
+        if model.device.type != "cuda" or not cls.described(model.spec, model.dtype):
             return None
-        if model.embedding.dtype != torch.bfloat16 or model.lm_head.dtype != torch.bfloat16:
-            return None
-        first = model.blocks[spec.order[0]]
-        for block in model.blocks:
-            mixer, ff = block.mixer, block.feed_forward
-            if (type(block) is not PreNormResidualBlock or type(mixer) is not GroupedQueryAttention or type(ff) is not SwiGLU
-                    or type(block.mixer_norm) is not RMSNorm or type(block.feed_forward_norm) is not RMSNorm
-                    or type(mixer.position) is not RotaryEncoding):
-                return None
-            if (mixer.head_dim != 128 or mixer.window or ff.activation != "silu" or ff.float32_output
-                    or (mixer.n_q, mixer.n_kv, ff.inter) != (first.mixer.n_q, first.mixer.n_kv, first.feed_forward.inter)
-                    or mixer.position.pairing != first.mixer.position.pairing
-                    or mixer.position.params.get("theta") != first.mixer.position.params.get("theta")):
-                return None
-            matrices = (mixer.qkv_weight, mixer.o_weight, ff.gate_up_weight, ff.down_weight)
-            if any(matrix.dtype != torch.bfloat16 for matrix in matrices):
-                return None
         made = cls(model)
-        tensors = [tensor for layer in made.weights for tensor in layer if tensor is not None] + [model.lm_head]
-        if any(tensor.data_ptr() % 16 or not tensor.is_contiguous() for tensor in tensors) or not made.supported(1):
+        return made if made._layers() is not None and made.supported(1) else None
+
+    def _layers(self):
+        """(weights, both norms' eps) of every layer run, from the parts as they are now; None where one is not what the kernel runs."""
+        model = self.model
+        hidden, final, first = model.spec.hidden_size, model.final_norm, self._first.mixer
+        if not (_plain(final, RMSNorm) and _vector(final.weight, hidden) and _matrix(model.lm_head, len(model.lm_head), hidden)
+                and _matrix(model.embedding, len(model.embedding), hidden)):
             return None
-        return made
+        weights, eps = [], []
+        for index in model.spec.order:
+            block = model.blocks[index]
+            if not _plain(block, PreNormResidualBlock):
+                return None
+            mixer, ff, norm1, norm2 = block.mixer, block.feed_forward, block.mixer_norm, block.feed_forward_norm
+            if not (_plain(mixer, GroupedQueryAttention) and _plain(ff, SwiGLU) and _plain(norm1, RMSNorm) and _plain(norm2, RMSNorm)
+                    and _plain(mixer.position, RotaryEncoding)):
+                return None
+            n_q, n_kv, inter, position = mixer.n_q, mixer.n_kv, ff.inter, mixer.position
+            if (mixer.head_dim != HEAD or mixer.window or ff.activation != "silu" or ff.float32_output
+                    or (n_q, n_kv, mixer.scale) != (first.n_q, first.n_kv, first.scale) or inter != self.inter
+                    or position.pairing != first.position.pairing or position.params.get("theta") != first.position.params.get("theta")):
+                return None
+            rows = (n_q + 2 * n_kv) * HEAD
+            if not (_matrix(mixer.qkv_weight, rows, hidden) and _matrix(mixer.o_weight, hidden, n_q * HEAD)
+                    and _matrix(ff.gate_up_weight, 2 * inter, hidden) and _matrix(ff.down_weight, hidden, inter)
+                    and _vector(norm1.weight, hidden) and _vector(norm2.weight, hidden)
+                    and (mixer.qkv_bias is None or _vector(mixer.qkv_bias, rows))):
+                return None
+            weights.append((mixer.qkv_weight, mixer.o_weight, ff.gate_up_weight, ff.down_weight, mixer.qkv_bias, norm1.weight, norm2.weight))
+            eps += [norm1.eps, norm2.eps]
+        return weights, eps
+
+    @property
+    def _first(self):
+        return self.model.blocks[self.model.spec.order[0]]
+
+    @property
+    def inter(self) -> int:
+        return self._first.feed_forward.inter
 
     def supported(self, rows: int) -> bool:
         spec = self.model.spec
-        return ops.decode_layers_supported(len(spec.order), rows, spec.hidden_size, self.inter, self.mixer.n_q, self.mixer.n_kv,
-                                           self.model.lm_head.shape[0])
+        mixer = self._first.mixer
+        return ops.decode_layers_supported(len(spec.order), rows, spec.hidden_size, self.inter, mixer.n_q, mixer.n_kv, len(self.model.lm_head))
 
     def wanted(self, rows: int) -> bool:
         """Whether a step of so many single tokens goes through the one launch."""
@@ -106,13 +137,18 @@ class DecodeLayers:
         """float32 logits of every row of a step of single tokens; None where the step has to go launch by launch."""
         model = self.model
         first = caches[0]
-        if not self.wanted(step.num_tokens) or first.keys.shape[2] % 16 or first.keys.dtype != torch.bfloat16:
+        if step.num_tokens * model.spec.hidden_size > MOST_VALUES or first.keys.shape[2] % 16 or first.keys.dtype != torch.bfloat16:
             return None
         if any(cache.group != first.group or cache.keys.shape != first.keys.shape for cache in caches):
             return None
-        pointers = [[None if tensor is None else tensor.data_ptr() for tensor in weights] + [cache.keys.data_ptr(), cache.values.data_ptr()]
-                    for weights, cache in zip(self.weights, caches)]
-        return ops.decode_layers(pointers, self.eps, model.embedding, model.spec.embedding_scale, model.lm_head,
-                                 model.final_norm.weight, model.final_norm.eps, self.mixer.position.inv_freq,
-                                 self.mixer.position.pairing, step.token_ids, step.positions, step.segment_of_token,
-                                 first.slot_mapping, first.block_tables, first.keys, self.inter, self.mixer.n_q, self.mixer.scale)
+        layers = self._layers()
+        if layers is None or not self.supported(step.num_tokens):
+            return None
+        weights, eps = layers
+        pointers = [[None if tensor is None else tensor.data_ptr() for tensor in of_layer] + [cache.keys.data_ptr(), cache.values.data_ptr()]
+                    for of_layer, cache in zip(weights, caches)]
+        mixer = self._first.mixer
+        return ops.decode_layers(pointers, eps, model.embedding, model.spec.embedding_scale, model.lm_head,
+                                 model.final_norm.weight, model.final_norm.eps, mixer.position.inv_freq, mixer.position.pairing,
+                                 step.token_ids, step.positions, step.segment_of_token, first.slot_mapping, first.block_tables,
+                                 first.keys, self.inter, mixer.n_q, mixer.scale)

@@ -196,6 +196,38 @@ def test_the_head_reads_rows_that_were_rounded_once(one_launch):
     assert int((got != want.bfloat16().float()).sum()) <= 16
 
 
+def test_the_parts_are_read_as_they_are(monkeypatch):
+    """A matrix that takes another's place is used by the next step, and a part that was wrapped, on the instance or on its class, is
+    called: the one launch keeps nothing of the layers as they were built."""
+    from llm_serving_engine_b200.kernels import ops
+    from llm_serving_engine_b200.parts.mlp import SwiGLU
+
+    config, model, _ = _build("small")
+    launches, passed = [], []
+    launch = ops.decode_layers
+    monkeypatch.setattr(ops, "decode_layers", lambda *given: launches.append(1) or launch(*given))
+    sequences = [[3], [8]]
+    before = _decode(model, sequences, 1, True)
+    assert len(launches) == 1
+    ff = model.blocks[1].feed_forward
+    ff.down_weight = (torch.randn(ff.down_weight.shape, generator=torch.Generator().manual_seed(9)) * 0.1).bfloat16().cuda()
+    got, want = (_decode(model, sequences, 1, one_launch) for one_launch in (True, False))
+    assert len(launches) == 2
+    limit = helpers.tolerance("bfloat16", want)
+    assert float((got - want).abs().max()) <= limit < float((got - before).abs().max())
+
+    mixer = model.blocks[2].mixer
+    whole = mixer.forward
+    mixer.forward = lambda *given: passed.append("instance") or whole(*given)
+    assert torch.equal(_decode(model, sequences, 1, True), want) and passed == ["instance"] and len(launches) == 2
+    del mixer.forward
+    act = SwiGLU.forward
+    monkeypatch.setattr(SwiGLU, "forward", lambda self, x: passed.append("class") or act(self, x))
+    assert torch.equal(_decode(model, sequences, 1, True), want) and passed[1:] == ["class"] * 3 and len(launches) == 2
+    monkeypatch.setattr(SwiGLU, "forward", act)
+    assert torch.equal(_decode(model, sequences, 1, True), got) and len(launches) == 3
+
+
 def test_some_rows_wanted():
     """A step launch by launch (no graph) that asks for some requests' logits only gives those, in their order."""
     from llm_serving_engine_b200.cache import CacheManager
