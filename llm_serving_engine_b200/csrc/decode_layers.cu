@@ -980,6 +980,7 @@ decode_layers_start_kernel(const __nv_bfloat16* __restrict__ table, const int* _
   }
 }
 
+constexpr int LSE_DECODE_LAYERS_REFUSED = -3;   // the blocks cannot all be on the GPU at once
 constexpr size_t SMEM_LIMIT = 232448;   // 227 KB a block, static shared memory included
 
 struct Plan {
@@ -1028,9 +1029,13 @@ bool make_plan(int blocks, int layers, int rows, int hidden, int inter, int n_q,
   return false;
 }
 
-int launch(const Args& args, int blocks, size_t smem, cudaStream_t stream) {
+cudaError_t allow(size_t smem) {
   static SmemAllowance allowance;
-  cudaError_t err = allow_smem(decode_layers_kernel, smem, allowance);
+  return allow_smem(decode_layers_kernel, smem, allowance);
+}
+
+int launch(const Args& args, int blocks, size_t smem, cudaStream_t stream) {
+  cudaError_t err = allow(smem);
   if (err != cudaSuccess) return (int)err;
   cudaLaunchConfig_t config = {};
   config.gridDim = blocks;
@@ -1043,8 +1048,12 @@ int launch(const Args& args, int blocks, size_t smem, cudaStream_t stream) {
   config.attrs = attribute;
   config.numAttrs = 1;
   err = cudaLaunchKernelEx(&config, decode_layers_kernel, args);
-  if (err != cudaSuccess) return (int)err;
-  return (int)cudaGetLastError();
+  if (err == cudaSuccess) err = cudaGetLastError();
+  if (err == cudaErrorCooperativeLaunchTooLarge || err == cudaErrorNotSupported) {   // a process that may use a part of the SMs only
+    cudaGetLastError();              // the step goes launch by launch, and is not to meet this error there
+    return LSE_DECODE_LAYERS_REFUSED;
+  }
+  return (int)err;
 }
 
 }  // namespace
@@ -1053,6 +1062,19 @@ int launch(const Args& args, int blocks, size_t smem, cudaStream_t stream) {
 extern "C" int lse_decode_layers_supported(int blocks, int layers, int rows, int hidden, int inter, int n_q, int n_kv, int vocab) {
   Plan plan;
   return layers >= 1 && layers <= MAX_LAYERS && make_plan(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, &plan) ? 1 : 0;
+}
+
+// Whether the current device takes the launch of a step of these sizes: all blocks at once.  Asked once, when a model is built.
+extern "C" int lse_decode_layers_fits(int blocks, int layers, int rows, int hidden, int inter, int n_q, int n_kv, int vocab) {
+  Plan plan;
+  int device = 0, cooperative = 0, sms = 0, a_sm = 0;
+  if (layers < 1 || layers > MAX_LAYERS || !make_plan(blocks, layers, rows, hidden, inter, n_q, n_kv, vocab, &plan)) return 0;
+  const bool answered = cudaGetDevice(&device) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && allow(plan.smem) == cudaSuccess &&
+                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a_sm, decode_layers_kernel, THREADS + 64, plan.smem) == cudaSuccess;
+  if (!answered) cudaGetLastError();
+  return answered && cooperative && (long long)a_sm * sms >= blocks ? 1 : 0;
 }
 
 // Bytes of scratch memory of a launch: the packets that blocks exchange, the abort word, and the norms' places.
@@ -1095,7 +1117,7 @@ extern "C" int lse_decode_layers_test_hooks(unsigned int spin_limit, int withhol
   return (int)cudaMemcpyToSymbol(lse_decode_layers_withhold, &withhold, sizeof(withhold));
 }
 
-// One decode step.  layer_pointers [layers][9]: qkv, o, gate_up, down, qkv_bias (may be 0), norm1, norm2, keys, values;
+// One decode step (LSE_DECODE_LAYERS_REFUSED: not taken, nothing of the step has happened).  layer_pointers [layers][9]: qkv, o, gate_up, down, qkv_bias (may be 0), norm1, norm2, keys, values;
 // layer_eps [layers][2].  All bfloat16 matrices row-major and 16-byte aligned (gate_up: gate rows, then up rows), norms and
 // biases float32.  Every row of the step is a request's next token (segment -1: padding).  logits float32 [rows][vocab].
 extern "C" int lse_decode_layers(const long long* layer_pointers, const float* layer_eps, int layers, const void* embedding,

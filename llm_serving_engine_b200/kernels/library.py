@@ -224,6 +224,7 @@ _SIGNATURES = {
     "lse_gemm_pairs_status_reset": [],
     "lse_gemm_pairs_test_hook": [c_int],
     "lse_decode_layers_supported": [c_int] * 8,
+    "lse_decode_layers_fits": [c_int] * 8,
     "lse_decode_layers_scratch": [c_int] * 8 + [c_void_p],
     "lse_decode_layers": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p, c_void_p, c_float, c_void_p, c_int,
                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

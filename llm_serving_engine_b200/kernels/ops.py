@@ -690,6 +690,11 @@ def decode_layers_supported(layers: int, rows: int, hidden: int, inter: int, n_q
     return bool(library.load().lse_decode_layers_supported(sm_count(), layers, rows, hidden, inter, n_q, n_kv, vocab))
 
 
+def decode_layers_fits(layers: int, rows: int, hidden: int, inter: int, n_q: int, n_kv: int, vocab: int) -> bool:
+    """Whether the current device takes the launch of a step of these sizes (it answers for the launch's blocks, all at once)."""
+    return bool(library.load().lse_decode_layers_fits(sm_count(), layers, rows, hidden, inter, n_q, n_kv, vocab))
+
+
 def decode_layers_test_hooks(spin_limit: int = 0, withhold: bool = False) -> None:
     """For tests of the bounded waits: ``spin_limit`` attempts before a wait gives up (0: the default), ``withhold``: a value
     that the first product waits for never comes."""
@@ -697,11 +702,15 @@ def decode_layers_test_hooks(spin_limit: int = 0, withhold: bool = False) -> Non
     check(library.load().lse_decode_layers_test_hooks(int(spin_limit), int(bool(withhold))), "decode_layers test hooks")
 
 
+DECODE_LAYERS_REFUSED = -3
+
+
 def decode_layers(layer_pointers: list, eps: list, embedding: torch.Tensor, embedding_scale: float, head: torch.Tensor,
                   final_norm: torch.Tensor, final_eps: float, inv_freq: torch.Tensor, pairing: int, token_ids: torch.Tensor,
                   positions: torch.Tensor, segment_of_token: torch.Tensor, slot_mapping: torch.Tensor, block_tables: torch.Tensor,
-                  keys: torch.Tensor, inter: int, n_q: int, scale: float) -> torch.Tensor:
-    """A step of single tokens through all layers and the head: float32 logits [rows, vocab].
+                  keys: torch.Tensor, inter: int, n_q: int, scale: float) -> torch.Tensor | None:
+    """A step of single tokens through all layers and the head: float32 logits [rows, vocab].  None where the device does not take
+    a launch of all blocks at once (a process that may use a part of the SMs only): nothing of the step has happened then.
 
     ``layer_pointers``: per layer the addresses of qkv, o, gate_up and down weights, the qkv bias (or None), both norms'
     weights, the cached keys and values; ``eps``: both norms' of every layer; ``keys``: one layer's cache, for its shape."""
@@ -716,12 +725,15 @@ def decode_layers(layer_pointers: list, eps: list, embedding: torch.Tensor, embe
         raise KernelError("decode_layers: a step of these sizes does not fit")
     scratch = torch.empty(places[10], dtype=torch.uint8, device=embedding.device)
     logits = torch.empty((rows, vocab), dtype=torch.float32, device=embedding.device)
-    check(lib.lse_decode_layers(flat, (c_float * (2 * layers))(*eps), layers, embedding.data_ptr(), embedding.shape[0],
-                                float(embedding_scale), head.data_ptr(), final_norm.data_ptr(), float(final_eps), inv_freq.data_ptr(),
-                                int(pairing), token_ids.data_ptr(), positions.data_ptr(), segment_of_token.data_ptr(),
-                                slot_mapping.data_ptr(), block_tables.data_ptr(), block_tables.stride(0), block_tables.shape[0], rows,
-                                hidden, inter, n_q, n_kv, vocab, page_size, pages, float(scale), scratch.data_ptr(),
-                                logits.data_ptr(), blocks, _stream()), "decode_layers")
+    code = lib.lse_decode_layers(flat, (c_float * (2 * layers))(*eps), layers, embedding.data_ptr(), embedding.shape[0],
+                                 float(embedding_scale), head.data_ptr(), final_norm.data_ptr(), float(final_eps), inv_freq.data_ptr(),
+                                 int(pairing), token_ids.data_ptr(), positions.data_ptr(), segment_of_token.data_ptr(),
+                                 slot_mapping.data_ptr(), block_tables.data_ptr(), block_tables.stride(0), block_tables.shape[0], rows,
+                                 hidden, inter, n_q, n_kv, vocab, page_size, pages, float(scale), scratch.data_ptr(),
+                                 logits.data_ptr(), blocks, _stream())
+    if code == DECODE_LAYERS_REFUSED:
+        return None
+    check(code, "decode_layers")
     return logits
 
 

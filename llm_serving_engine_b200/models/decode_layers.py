@@ -60,6 +60,7 @@ class DecodeLayers:
 
     def __init__(self, model) -> None:
         self.model = model
+        self.refused = False     # the device did not take the launch: it will not take the next one either
 
     @staticmethod
     def described(spec: ModelSpec, dtype: torch.dtype) -> bool:
@@ -83,7 +84,7 @@ class DecodeLayers:
         if model.device.type != "cuda" or not cls.described(model.spec, model.dtype):
             return None
         made = cls(model)
-        return made if made._layers() is not None and made.supported(1) else None
+        return made if made._layers() is not None and made._asked(ops.decode_layers_fits, 1) else None
 
     def _layers(self):
         """(weights, both norms' eps) of every layer run, from the parts as they are now; None where one is not what the kernel runs."""
@@ -125,9 +126,11 @@ class DecodeLayers:
         return self._first.feed_forward.inter
 
     def supported(self, rows: int) -> bool:
-        spec = self.model.spec
-        mixer = self._first.mixer
-        return ops.decode_layers_supported(len(spec.order), rows, spec.hidden_size, self.inter, mixer.n_q, mixer.n_kv, len(self.model.lm_head))
+        return self._asked(ops.decode_layers_supported, rows)
+
+    def _asked(self, question, rows: int) -> bool:
+        spec, mixer = self.model.spec, self._first.mixer
+        return question(len(spec.order), rows, spec.hidden_size, self.inter, mixer.n_q, mixer.n_kv, len(self.model.lm_head))
 
     def wanted(self, rows: int) -> bool:
         """Whether a step of so many single tokens goes through the one launch."""
@@ -137,7 +140,7 @@ class DecodeLayers:
         """float32 logits of every row of a step of single tokens; None where the step has to go launch by launch."""
         model = self.model
         first = caches[0]
-        if step.num_tokens * model.spec.hidden_size > MOST_VALUES or first.keys.shape[2] % 16 or first.keys.dtype != torch.bfloat16:
+        if self.refused or step.num_tokens * model.spec.hidden_size > MOST_VALUES or first.keys.shape[2] % 16 or first.keys.dtype != torch.bfloat16:
             return None
         if any(cache.group != first.group or cache.keys.shape != first.keys.shape for cache in caches):
             return None
@@ -148,7 +151,9 @@ class DecodeLayers:
         pointers = [[None if tensor is None else tensor.data_ptr() for tensor in of_layer] + [cache.keys.data_ptr(), cache.values.data_ptr()]
                     for of_layer, cache in zip(weights, caches)]
         mixer = self._first.mixer
-        return ops.decode_layers(pointers, eps, model.embedding, model.spec.embedding_scale, model.lm_head,
-                                 model.final_norm.weight, model.final_norm.eps, mixer.position.inv_freq, mixer.position.pairing,
-                                 step.token_ids, step.positions, step.segment_of_token, first.slot_mapping, first.block_tables,
-                                 first.keys, self.inter, mixer.n_q, mixer.scale)
+        logits = ops.decode_layers(pointers, eps, model.embedding, model.spec.embedding_scale, model.lm_head,
+                                   model.final_norm.weight, model.final_norm.eps, mixer.position.inv_freq, mixer.position.pairing,
+                                   step.token_ids, step.positions, step.segment_of_token, first.slot_mapping, first.block_tables,
+                                   first.keys, self.inter, mixer.n_q, mixer.scale)
+        self.refused = logits is None
+        return logits

@@ -228,6 +228,19 @@ def test_the_parts_are_read_as_they_are(monkeypatch):
     assert torch.equal(_decode(model, sequences, 1, True), got) and len(launches) == 3
 
 
+def test_a_launch_that_is_refused_goes_launch_by_launch(monkeypatch):
+    """The step's result is that of the kernels one by one, and the launch is not tried again."""
+    from llm_serving_engine_b200.kernels import library, ops
+
+    _, model, _ = _build("small")
+    asked = []
+    want = _decode(model, [[3], [8]], 1, False)
+    monkeypatch.setattr(library.load(), "lse_decode_layers", lambda *given: asked.append(1) or ops.DECODE_LAYERS_REFUSED)
+    for use_graphs in (False, True):
+        assert torch.equal(_decode(model, [[3], [8]], 1, True, use_graphs), want)
+    assert len(asked) == 1
+
+
 def test_some_rows_wanted():
     """A step launch by launch (no graph) that asks for some requests' logits only gives those, in their order."""
     from llm_serving_engine_b200.cache import CacheManager

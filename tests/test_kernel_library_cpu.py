@@ -127,20 +127,29 @@ extern "C" int together() {
     assert trial.together() == 0
 
 
-def test_the_delta_memorys_scan_is_allowed_its_shared_memory_on_every_device(tmp_path):
-    """The launcher, compiled here and linked with a runtime that only keeps books: on a second device, and on one of fewer SMs,
-    every launch stays within what that device has been asked to allow (48 KB need no asking, static shared memory included, of which
-    these kernels have up to 4), and asks for an SM a block where that device has so many."""
-    (tmp_path / "books.cpp").write_text('''
+_BOOKS = '''
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 #include <map>
+#include <string>
 #include <utility>
-static int device, launches, refused, largest;
+// A runtime that keeps books and runs nothing.  Device 2 has 20 SMs, device 3 takes no cooperative launches.
+static int device, launches, refused, largest, refuse_cooperative, a_sm = 1;
+static cudaError_t last = cudaSuccess;
 static std::map<std::pair<int, const void*>, int> allowed;
+static CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                       const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
+  return CUDA_SUCCESS;
+}
 extern "C" {
-int use(int which) { device = which; launches = refused = largest = 0; return 0; }
-int refusals() { return launches == 2 ? refused : -1; }
+int use(int which, int blocks_a_sm, int refuse) {
+  device = which; launches = refused = largest = 0; a_sm = blocks_a_sm; refuse_cooperative = refuse; last = cudaSuccess;
+  return 0;
+}
+int launched() { return launches; }
+int refusals() { return refused; }
 int most() { return largest; }
+int pending() { return (int)last; }
 void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
@@ -149,31 +158,80 @@ void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int)
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void*) { return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* out) { *out = device; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* out, cudaDeviceAttr, int which) { *out = which == 2 ? 20 : 148; return cudaSuccess; }
+cudaError_t cudaGetLastError() { const cudaError_t was = last; last = cudaSuccess; return was; }
+cudaError_t cudaDeviceGetAttribute(int* out, cudaDeviceAttr what, int which) {
+  *out = what == cudaDevAttrCooperativeLaunch ? which != 3 : which == 2 ? 20 : 148;
+  return cudaSuccess;
+}
 cudaError_t cudaFuncSetAttribute(const void* kernel, cudaFuncAttribute, int bytes) { allowed[{device, kernel}] = bytes; return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* out, const void*, int, size_t, unsigned) { *out = a_sm; return cudaSuccess; }
+#undef cudaGetDriverEntryPoint
+cudaError_t cudaGetDriverEntryPoint(const char* name, void** out, unsigned long long, cudaDriverEntryPointQueryResult* found) {
+  *out = std::string(name) == "cuTensorMapEncodeTiled" ? (void*)encode : nullptr;
+  *found = *out ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyFromSymbol(void*, const void*, size_t, size_t, cudaMemcpyKind) { return cudaErrorUnknown; }
+cudaError_t cudaMemcpyFromSymbolAsync(void*, const void*, size_t, size_t, cudaMemcpyKind, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t cudaMemcpyToSymbol(const void*, const void*, size_t, size_t, cudaMemcpyKind) { return cudaErrorUnknown; }
+cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return last = cudaErrorUnknown; }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* kernel, void**) {
   const int bytes = (int)config->dynamicSmemBytes;
   const auto found = allowed.find({device, kernel});
   ++launches;
   if (bytes > largest) largest = bytes;
-  if (bytes > 44 * 1024 && (found == allowed.end() || bytes > found->second)) { ++refused; return cudaErrorInvalidValue; }
+  if (bytes > 44 * 1024 && (found == allowed.end() || bytes > found->second)) { ++refused; return last = cudaErrorInvalidValue; }
+  if (config->attrs[0].id == cudaLaunchAttributeCooperative && refuse_cooperative) return last = cudaErrorCooperativeLaunchTooLarge;
   return cudaSuccess;
 }
 }
-''')
+'''
+
+
+def _with_books(source, folder):
+    """A source's launchers, compiled here and linked with a runtime that only keeps books."""
+    (folder / "books.cpp").write_text(_BOOKS)
     nvcc = [build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O1", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]
-    subprocess.run([*nvcc, "-c", str(build.CSRC / "delta_memory_chunks.cu"), "-o", str(tmp_path / "chunks.o")], check=True)
-    subprocess.run([*nvcc, "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic", str(tmp_path / "books.cpp"), str(tmp_path / "chunks.o"),
-                    "-o", str(tmp_path / "books.so")], check=True)     # its own runtime, also where another is in the process
-    books = ctypes.CDLL(str(tmp_path / "books.so"))
-    scan = books.lse_delta_chunk_scan
-    scan.argtypes = library._SIGNATURES["lse_delta_chunk_scan"]
+    subprocess.run([*nvcc, "-c", str(build.CSRC / f"{source}.cu"), "-o", str(folder / "source.o")], check=True)
+    subprocess.run([*nvcc, "-shared", "-cudart", "none", "-Xlinker", "-Bsymbolic", str(folder / "books.cpp"), str(folder / "source.o"),
+                    "-o", str(folder / "books.so")], check=True)     # its own runtime, also where another is in the process
+    books = ctypes.CDLL(str(folder / "books.so"))
+    for name, types in library._SIGNATURES.items():
+        if name in build.exported_names(build.CSRC / f"{source}.cu"):
+            getattr(books, name).argtypes = types
+    return books
+
+
+def test_the_delta_memorys_scan_is_allowed_its_shared_memory_on_every_device(tmp_path):
+    """On a second device, and on one of fewer SMs, every launch stays within what that device has been asked to allow (48 KB need no
+    asking, static shared memory included, of which these kernels have up to 4), and asks for an SM a block where that device has
+    so many."""
+    books = _with_books("delta_memory_chunks", tmp_path)
     for device, lone in ((0, True), (1, True), (0, True), (2, False), (70, True)):
         for dim in (24, 64, 128, 200):
-            books.use(device)
+            books.use(device, 1, 0)
             # q .. beta, z, partials of z, bias and decay, state, segments, results, buffer; 10 chunks of one request, four heads
-            assert scan(*[None] * 5, 1, 0, 0, *[None] * 7, 10, 1, 4, 4, dim, 128, 1, 1, None) == 0
-            assert books.refusals() == 0, (device, dim)
+            assert books.lse_delta_chunk_scan(*[None] * 5, 1, 0, 0, *[None] * 7, 10, 1, 4, 4, dim, 128, 1, 1, None) == 0
+            assert books.launched() == 2 and books.refusals() == 0, (device, dim)
             assert lone == (books.most() >= 116 * 1024) or dim > 128
+
+
+def test_a_device_that_does_not_take_the_one_launch_step_is_asked_and_leaves_no_error(tmp_path):
+    """A device without cooperative launches, or one on which not all blocks fit at once, is known when a model is built; a launch
+    that is refused all the same (a process that may use a part of the SMs only) says so, and the next launch does not meet its error."""
+    books = _with_books("decode_layers", tmp_path)
+    sizes = (2, 1, 192, 320, 2, 1, 528)           # layers, rows, hidden, feed-forward, query and key/value heads, vocabulary
+    for device, blocks_a_sm, blocks, want in ((0, 1, 148, 1), (0, 0, 148, 0), (3, 1, 148, 0), (2, 1, 148, 0), (2, 1, 20, 1), (0, 1, 20, 1)):
+        books.use(device, blocks_a_sm, 0)
+        assert books.lse_decode_layers_fits(blocks, *sizes) == want, (device, blocks_a_sm, blocks)
+        assert books.pending() == 0
+    layers = (ctypes.c_longlong * 18)()
+    eps = (ctypes.c_float * 4)()
+
+    def step():
+        return books.lse_decode_layers(layers, eps, 2, None, 528, 1.0, None, None, 1e-6, None, 0, None, None, None, None, None, 4, 1, 1, 192,
+                                       320, 2, 1, 528, 16, 8, 1.0, None, None, 148, None)
+    books.use(0, 1, 0)
+    assert step() == 0 and books.launched() == 2 and books.refusals() == 0
+    books.use(0, 1, 1)
+    assert step() == -3 and books.launched() == 2 and books.pending() == 0
