@@ -134,28 +134,52 @@ __host__ __device__ __forceinline__ int rows_of_tile(int left, int rows_a_tile) 
 }
 __host__ __device__ __forceinline__ int box_of(int rows) { return (rows / 2 + 31) / 32; }   // half a tile's rows, in boxes of 32
 
-// The groups' rows, tiles and pieces of w; one thread, once a block.
+// The groups' rows, tiles and pieces of w, in their order; one warp, once a block, 32 groups at a time.  (On one thread the prologue
+// of 256 groups took 40 us.)
 template <bool GATED>
-__device__ __noinline__ void lay_out(const Args& a, Shared& s) {
+__device__ __noinline__ void lay_out(const Args& a, Shared& s, int lane) {
   constexpr int W_TILE = GATED ? HALF_TILE : 2 * HALF_TILE;    // results a tile
-  int tiles = 0, count = 0;
-  auto add = [&](int lo, int hi, int index, int columns, int k, int source) {
-    if (hi <= lo) return;
+  int tiles = 0, count = 0, before = 0;
+  auto put = [&](int at, int tile0, int lo, int hi, int index, int columns, int k, int source) {
     Group g;
     g.lo = lo; g.hi = hi; g.source = source; g.columns = columns;
     g.w_row = (int)(index * a.w_rows); g.w_column = (int)(index * a.w_columns);
     g.k_blocks = (k + BLOCK_K - 1) / BLOCK_K;
     g.row_tiles = (hi - lo + 255) / 256;
     g.rows_a_tile = rows_of_tiles(hi - lo);
-    g.tile0 = tiles;
+    g.tile0 = tile0;
     g.w_tiles = (columns + W_TILE - 1) / W_TILE;
-    tiles += g.row_tiles * g.w_tiles;
-    s.group[count++] = g;
+    s.group[at] = g;
+    return g.row_tiles * g.w_tiles;
   };
-  if (a.whole) add(0, a.whole, a.routed, a.whole_columns, a.whole_k, a.whole_source);   // the largest first
-  for (int g = 0; g < a.routed; ++g) add(g ? a.offsets[g - 1] : 0, a.offsets[g], g, a.columns, a.k, 0);
-  s.groups = count;
-  s.tiles = tiles;
+  if (a.whole) {   // the largest first
+    if (lane == 0) tiles = put(0, 0, 0, a.whole, a.routed, a.whole_columns, a.whole_k, a.whole_source);
+    tiles = __shfl_sync(0xffffffffu, tiles, 0);
+    count = 1;
+  }
+  const int w_tiles = (a.columns + W_TILE - 1) / W_TILE;
+  for (int first = 0; first < a.routed; first += 32) {
+    const int g = first + lane, hi = g < a.routed ? a.offsets[g] : 0;
+    int lo = __shfl_up_sync(0xffffffffu, hi, 1);
+    if (lane == 0) lo = before;
+    before = __shfl_sync(0xffffffffu, hi, 31);
+    const bool some = g < a.routed && hi > lo;
+    const int mine = some ? (hi - lo + 255) / 256 * w_tiles : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += up;
+    }
+    const unsigned present = __ballot_sync(0xffffffffu, some);
+    if (some) put(count + __popc(present & ((1u << lane) - 1u)), tiles + upto - mine, lo, hi, g, a.columns, a.k, 0);
+    tiles += __shfl_sync(0xffffffffu, upto, 31);
+    count += __popc(present);
+  }
+  if (lane == 0) {
+    s.groups = count;
+    s.tiles = tiles;
+  }
 }
 
 struct Tile {
@@ -192,8 +216,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128 + 32 * FINISHERS
     }
     s.abort = 0;
     mbar_init_fence();
+  }
+  if (warp == 1) {
     if (a.routed) pdl_wait();                      // the groups' ranges are an earlier kernel's
-    lay_out<GATED>(a, s);
+    __syncwarp();
+    lay_out<GATED>(a, s, lane);
   }
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&s.tmem)) : "memory");

@@ -49,8 +49,8 @@ class ClampedMoE(FeedForward):
     * many bfloat16 rows: every (token, chosen expert) pair gets a row in a buffer grouped by expert (two small
       kernels), two products run over the groups and the shared expert at once, the activation inside the first, and a
       kernel adds each token's rows times their weights in float32, with the identity experts' share, onto the shared
-      expert's output.  (Experts without a gate, or of a width that is no multiple of 64: the library's grouped product
-      over views of the same stacked matrices, and the activation kernel.)"""
+      expert's output.  (Experts without a gate, or of a width that is no multiple of 64, and large groups of wide rows: the
+      library's grouped product over views of the same stacked matrices, and the activation kernel.)"""
 
     graph_safe = True
     kernel_sources = ("moe", "gemm_pairs")
@@ -153,7 +153,7 @@ class ClampedMoE(FeedForward):
         tokens, width = x.shape
         chosen = torch.empty((tokens, self.top), dtype=torch.int32, device=x.device)
         expert_weights, identity_weight, shared_gate = self._route(x, chosen)
-        if self._in_pairs:
+        if self._in_pairs and self._pairs_wanted(tokens):
             return self._grouped_in_pairs(x, chosen, expert_weights, identity_weight, shared_gate)
         y = None
         if self.shared_ff:   # the shared expert: two plain products, its gate folded into the activation
@@ -175,6 +175,16 @@ class ClampedMoE(FeedForward):
         out = y if y is not None else torch.empty((tokens, width), dtype=torch.float32, device=x.device)
         return ops.moe_combine(down, row_of, chosen, expert_weights, identity_weight if self.identity else None, x, out,
                                accumulate=y is not None)
+
+    def _pairs_wanted(self, tokens: int) -> bool:
+        """Whether the engine's products over groups are at least as fast as the library's: they save a launch and the gate and up values'
+        way through memory, and read more from the L2 where groups are large and k long.  Microseconds of the whole mixture, the
+        engine's / the library's, by rows a group.  8 experts, 2,048 wide, 2,688 and a shared one of 2,816 columns: 75 rows 116 / 148,
+        512 232 / 261, 2,048 689 / 734; 64 experts, 2,048 x 1,408 and 2,816: 28 265 / 316, 768 1,146 / 1,256; 128 of 768: 19 267 / 319,
+        512 859 / 862; 256 of 512, 1,024 wide: 4 215 / 238, 128 335 / 371.  Wider: 64 of 4,096 x 1,024, 97 rows 362 / 426, 188 419 / 440,
+        512 957 / 944, 1,024 1,777 / 1,698; 8 of 4,096 x 14,336, 194 601 / 635, 512 1,396 / 1,408, 1,024 2,784 / 2,692; 64 of 7,168 x 2,048,
+        73 1,029 / 1,315, 192 1,281 / 1,305, 216 1,675 / 1,539, 768 4,853 / 4,487."""
+        return self.router.shape[1] <= 2048 or tokens * self.top <= 200 * self.outputs
 
     def _grouped_in_pairs(self, x, chosen, expert_weights, identity_weight, shared_gate):
         """The experts and the shared expert together in two products of the engine's own, the activation inside the first."""

@@ -51,7 +51,8 @@ def test_gated_product(rows, k, inter, kind):
 
 @pytest.mark.parametrize("counts,k,columns,whole,whole_columns,kind", [
     ([64], 64, 64, 0, 0, "silu"), ([0, 1, 33, 0, 300], 128, 192, 40, 72, "clamped_swish"), ([256, 522, 5], 192, 128, 257, 200, "silu"),
-    ([2, 0, 3] + [1] * 60, 72, 64, 1, 8, "silu"), ([0, 0], 64, 64, 70, 136, "clamped_swish")])
+    ([2, 0, 3] + [1] * 60, 72, 64, 1, 8, "silu"), ([0, 0], 64, 64, 70, 136, "clamped_swish"),
+    ([0, 5, 300, 0] * 8 + [0] * 32 + [7, 0, 258] + [0, 1, 40] * 60 + [3], 64, 64, 33, 64, "silu"), ([1] * 31 + [0] * 224 + [520], 64, 128, 0, 0, "silu")])
 def test_groups_of_rows_with_weights_of_their_own(counts, k, columns, whole, whole_columns, kind):
     """Both products of a mixture of experts: rows behind the last group stay as they are, a group may have none."""
     torch.manual_seed(sum(counts) + k)
@@ -194,3 +195,31 @@ def test_a_wait_that_runs_out_is_reported_and_the_kernel_returns(gated, rows):
     sums = x.double() @ weight.double().t()
     _check(out, _act("silu", sums[:, :columns], sums[:, columns:], 0.0) if gated else sums, x, weight)
     assert library.load().lse_gemm_pairs_status() == 0
+
+
+@pytest.mark.parametrize("width,rows,pairs", [(2048, 401, True), (2560, 400, True), (2560, 401, False), (2560, 1000, False)])
+def test_which_experts_take_the_products_over_groups(width, rows, pairs, monkeypatch):
+    """Two experts of which each row chooses one: up to 200 rows an expert on average, or up to 2,048 columns.  Either way a value is
+    rounded at most five times to bfloat16 (2^-9 each) on its way to the result: 2^-6 of the whole between the two, in the 2-norm."""
+    from llm_serving_engine_b200.parts import FEED_FORWARDS
+    from llm_serving_engine_b200.parts.base import BuildContext
+
+    o = ops()
+    torch.manual_seed(rows + width)
+    ff = 64
+    weights = {"router": _random(2, width, width ** -0.5)}
+    for index in range(2):
+        weights.update({f"e{index}.gate": _random(ff, width, width ** -0.5), f"e{index}.up": _random(ff, width, width ** -0.5),
+                        f"e{index}.down": _random(width, ff, ff ** -0.5)})
+    params = {"experts": 2, "top": 1, "ff": ff, "activation": "silu", "correction": False}
+    part = FEED_FORWARDS.get("clamped_moe")(params, weights, BuildContext(torch.bfloat16, torch.device(DEV), width, 0, 64))
+    calls = []
+    product = o.product_groups
+    monkeypatch.setattr(o, "product_groups", lambda *given: calls.append(1) or product(*given))
+    x = _random(rows, width)
+    got = part.forward(x)
+    assert len(calls) == pairs
+    monkeypatch.setattr(part, "_pairs_wanted", lambda tokens: not pairs)
+    other = part.forward(x)
+    assert len(calls) == 1
+    assert float((got - other).norm() / other.norm()) <= 2.0 ** -6
