@@ -44,14 +44,19 @@ def _build(name, pairing="interleaved", layers=3):
     return config, DecoderModel(spec, held, torch.bfloat16, "cuda"), {key: value.float() for key, value in weights.items()}
 
 
-def _decode(model, sequences, steps, one_launch, use_graphs=False):
-    """Logits of the last ``steps`` tokens of every sequence, decoded together; the tokens before them come as portions."""
+def _decode(model, sequences, steps, one_launch, use_graphs=False, launches=None):
+    """Logits of the last ``steps`` tokens of every sequence, decoded together; the tokens before them come as portions.  The steps
+    take the one launch where they are meant to and nowhere else: ``launches`` of it, by default one a step (with graphs: ahead of
+    the capture and in it) or none."""
     from llm_serving_engine_b200.cache import CacheManager
     from llm_serving_engine_b200.config import CacheConfig
     from llm_serving_engine_b200.engine import StepEntry, StepRunner
+    from llm_serving_engine_b200.kernels import ops
     from llm_serving_engine_b200.models import cache_requirements
 
     held, model._decode_layers = model._decode_layers, model._decode_layers if one_launch else None
+    launch, calls = ops.decode_layers, []
+    ops.decode_layers = lambda *given: calls.append(1) or launch(*given)
     try:
         cache = CacheManager(cache_requirements(model.spec), CacheConfig(16, 16 * 40), model.dtype, "cuda", 1024, num_state_slots=16)
         for group in cache.groups:         # whatever lies behind a request's keys must not matter
@@ -62,12 +67,16 @@ def _decode(model, sequences, steps, one_launch, use_graphs=False):
             if len(tokens) > steps:
                 runner.run([StepEntry(str(index), tokens[:-steps], [])])
         out = []
+        calls.clear()
         for step in range(steps):
             entries = [StepEntry(str(index), [tokens[len(tokens) - steps + step]], [0]) for index, tokens in enumerate(sequences)]
             out.append(runner.run(entries).clone())
+        if launches is None:
+            launches = (2 if use_graphs else steps) if one_launch else 0
+        assert len(calls) == launches
         return torch.stack(out, dim=1).cpu()      # [requests, steps, vocab]
     finally:
-        model._decode_layers = held
+        model._decode_layers, ops.decode_layers = held, launch
 
 
 @pytest.mark.parametrize("name,rows,first", [("small", 1, 0), ("small", 3, 1), ("small", 4, 4), ("small", 4, 8), ("odd", 1, 9), ("odd", 2, 2),
@@ -80,17 +89,15 @@ def test_against_the_plain_implementation(name, rows, first):
     rng = random.Random(rows)
     steps = 2
     sequences = [helpers.random_tokens(rng, config["vocab_size"], context + steps) for context in CONTEXTS[first:first + rows]]
-    before = library.launches()
     got = _decode(model, sequences, steps, True, use_graphs=rows == 3)
     assert library.load().lse_decode_layers_status() == 0
-    assert library.launches() > before
     repeated = _decode(model, sequences, steps, True)
     assert torch.equal(got, repeated)              # every sum has its order
     for index, tokens in enumerate(sequences):
         want = qwen2_plain.forward_full(config, weights, tokens)[-steps:]
         limit = helpers.tolerance("bfloat16", want)
         assert float((got[index] - want).abs().max()) <= limit, (name, rows, index)
-        assert helpers.rms_ratio(got[index], want) <= helpers.RMS_RATIO_LARGE_LAYERS
+        assert helpers.rms_ratio(got[index], want) <= helpers.RMS_RATIO["bfloat16"]      # largest measured: 7.2e-3
 
 
 @pytest.mark.parametrize("name,rows", [("small", 4), ("odd", 3)])
@@ -199,33 +206,28 @@ def test_the_head_reads_rows_that_were_rounded_once(one_launch):
 def test_the_parts_are_read_as_they_are(monkeypatch):
     """A matrix that takes another's place is used by the next step, and a part that was wrapped, on the instance or on its class, is
     called: the one launch keeps nothing of the layers as they were built."""
-    from llm_serving_engine_b200.kernels import ops
     from llm_serving_engine_b200.parts.mlp import SwiGLU
 
     config, model, _ = _build("small")
-    launches, passed = [], []
-    launch = ops.decode_layers
-    monkeypatch.setattr(ops, "decode_layers", lambda *given: launches.append(1) or launch(*given))
+    passed = []
     sequences = [[3], [8]]
     before = _decode(model, sequences, 1, True)
-    assert len(launches) == 1
     ff = model.blocks[1].feed_forward
     ff.down_weight = (torch.randn(ff.down_weight.shape, generator=torch.Generator().manual_seed(9)) * 0.1).bfloat16().cuda()
     got, want = (_decode(model, sequences, 1, one_launch) for one_launch in (True, False))
-    assert len(launches) == 2
     limit = helpers.tolerance("bfloat16", want)
     assert float((got - want).abs().max()) <= limit < float((got - before).abs().max())
 
     mixer = model.blocks[2].mixer
     whole = mixer.forward
     mixer.forward = lambda *given: passed.append("instance") or whole(*given)
-    assert torch.equal(_decode(model, sequences, 1, True), want) and passed == ["instance"] and len(launches) == 2
+    assert torch.equal(_decode(model, sequences, 1, True, launches=0), want) and passed == ["instance"]
     del mixer.forward
     act = SwiGLU.forward
     monkeypatch.setattr(SwiGLU, "forward", lambda self, x: passed.append("class") or act(self, x))
-    assert torch.equal(_decode(model, sequences, 1, True), want) and passed[1:] == ["class"] * 3 and len(launches) == 2
+    assert torch.equal(_decode(model, sequences, 1, True, launches=0), want) and passed[1:] == ["class"] * 3
     monkeypatch.setattr(SwiGLU, "forward", act)
-    assert torch.equal(_decode(model, sequences, 1, True), got) and len(launches) == 3
+    assert torch.equal(_decode(model, sequences, 1, True), got)
 
 
 def test_a_launch_that_is_refused_goes_launch_by_launch(monkeypatch):
@@ -237,7 +239,7 @@ def test_a_launch_that_is_refused_goes_launch_by_launch(monkeypatch):
     want = _decode(model, [[3], [8]], 1, False)
     monkeypatch.setattr(library.load(), "lse_decode_layers", lambda *given: asked.append(1) or ops.DECODE_LAYERS_REFUSED)
     for use_graphs in (False, True):
-        assert torch.equal(_decode(model, [[3], [8]], 1, True, use_graphs), want)
+        assert torch.equal(_decode(model, [[3], [8]], 1, True, use_graphs, launches=0 if use_graphs else 1), want)
     assert len(asked) == 1
 
 

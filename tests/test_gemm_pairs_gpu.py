@@ -223,3 +223,30 @@ def test_which_experts_take_the_products_over_groups(width, rows, pairs, monkeyp
     other = part.forward(x)
     assert len(calls) == 1
     assert float((got - other).norm() / other.norm()) <= 2.0 ** -6
+
+
+@pytest.mark.parametrize("rows,in_the_product", [(1023, False), (1024, True), (1100, False), (2048, True)])
+def test_which_rows_of_a_feed_forward_take_the_product_with_its_gate(rows, in_the_product, monkeypatch):
+    """The dense feed-forward around the rows from which the gate goes into the product, and where the last tiles would leave the GPU
+    idle, against float64.  A value of the gated product carries up to three roundings to bfloat16 (2^-9 of it each; one where the gate
+    is inside), the result one more: 2^-7 of the whole in the 2-norm."""
+    from llm_serving_engine_b200.parts import FEED_FORWARDS
+    from llm_serving_engine_b200.parts.base import BuildContext
+
+    o = ops()
+    if o.sm_count() != 148:
+        pytest.skip("the rows are those of 148 SMs")
+    torch.manual_seed(rows)
+    hidden, inter = 1536, 8960
+    weights = {name: _random(*shape, scale=shape[1] ** -0.5) for name, shape in (
+        ("gate_proj.weight", (inter, hidden)), ("up_proj.weight", (inter, hidden)), ("down_proj.weight", (hidden, inter)))}
+    part = FEED_FORWARDS.get("swiglu")({"intermediate_size": inter}, weights, BuildContext(torch.bfloat16, torch.device(DEV), hidden, 0, 64))
+    calls = []
+    product = o.gated_product
+    monkeypatch.setattr(o, "gated_product", lambda *given: calls.append(1) or product(*given))
+    x = _random(rows, hidden)
+    got = part.forward(x).double()
+    assert bool(calls) == in_the_product
+    gate, up, down = (weights[name + "_proj.weight"].double() for name in ("gate", "up", "down"))
+    want = _act("silu", x.double() @ gate.t(), x.double() @ up.t(), 0.0) @ down.t()
+    assert float((got - want).norm() / want.norm()) <= 2.0 ** -7
