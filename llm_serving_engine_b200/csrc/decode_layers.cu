@@ -737,23 +737,23 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
           float m = -INFINITY;
 #pragma unroll
           for (int w = 0; w <= WARPS; ++w) m = fmaxf(m, s.ml[w][h][0]);
+          // A maximum is that of the numbers among the scores; where there are none, NaN among them still comes through the sums.
+          const float base = m > -INFINITY ? m : 0.f;
           float l = 0.f, v0 = 0.f, v1 = 0.f;
-          if (m > -INFINITY) {
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) {
-              const float f = fast_exp2(s.ml[w][h][0] - m);
-              const float2 sum = *reinterpret_cast<const float2*>(sums + (w * MAX_HEADS + h) * HEAD + d);
-              l += s.ml[w][h][1] * f;
-              v0 += sum.x * f;
-              v1 += sum.y * f;
-            }
-            if (own) {
-              const float f = fast_exp2(s.ml[WARPS][h][0] - m);
-              const float2 value = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(s.new_v + d));
-              l += f;
-              v0 += value.x * f;
-              v1 += value.y * f;
-            }
+          for (int w = 0; w < WARPS; ++w) {
+            const float f = fast_exp2(s.ml[w][h][0] - base);
+            const float2 sum = *reinterpret_cast<const float2*>(sums + (w * MAX_HEADS + h) * HEAD + d);
+            l += s.ml[w][h][1] * f;
+            v0 += sum.x * f;
+            v1 += sum.y * f;
+          }
+          if (own) {
+            const float f = fast_exp2(s.ml[WARPS][h][0] - base);
+            const float2 value = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(s.new_v + d));
+            l += f;
+            v0 += value.x * f;
+            v1 += value.y * f;
           }
           if (it.splits == 1) {
             store_packet(out + e, pack_bf16(v0 / l, v1 / l), epoch);
@@ -786,14 +786,12 @@ __global__ void __launch_bounds__(THREADS + 64, 1) decode_layers_kernel(const __
               for (int k = 0; k < AT_ONCE; ++k)
                 if (p0 + k < it.splits) {
                   const float its = __uint_as_float(ml[k].x);
-                  if (its > -INFINITY) {
-                    const float m_new = fmaxf(m, its);
-                    const float keep = fast_exp2(m - m_new), f = fast_exp2(its - m_new);
-                    l = l * keep + __uint_as_float(ml[k].z) * f;
-                    v0 = v0 * keep + __uint_as_float(o2[k].x) * f;
-                    v1 = v1 * keep + __uint_as_float(o2[k].z) * f;
-                    m = m_new;
-                  }
+                  const float m_new = fmaxf(m, its), base = m_new > -INFINITY ? m_new : 0.f;
+                  const float keep = fast_exp2(m - base), f = fast_exp2(its - base);
+                  l = l * keep + __uint_as_float(ml[k].z) * f;
+                  v0 = v0 * keep + __uint_as_float(o2[k].x) * f;
+                  v1 = v1 * keep + __uint_as_float(o2[k].z) * f;
+                  m = m_new;
                 }
             }
             store_packet(out + e, pack_bf16(v0 / l, v1 / l), epoch);

@@ -184,6 +184,35 @@ def test_long_contexts(name, layers, contexts, monkeypatch):
             assert helpers.rms_ratio(answer[None], want[None]) <= helpers.RMS_RATIO_LARGE_LAYERS
 
 
+@pytest.mark.parametrize("keys", [slice(256, 384), slice(300, 301), slice(0, 1280), slice(1279, 1280), slice(1280, 1280)])
+@pytest.mark.parametrize("what", ["keys", "values"])
+def test_nan_in_the_cache_reaches_the_logits(keys, what):
+    """As launch by launch: a share of the keys all of whose scores are NaN, a single such key, all of them, none; the same in the
+    values."""
+    from llm_serving_engine_b200.cache import CacheManager
+    from llm_serving_engine_b200.config import CacheConfig
+    from llm_serving_engine_b200.engine import StepEntry, StepRunner
+    from llm_serving_engine_b200.models import cache_requirements
+
+    _, model, _ = _build("small", layers=1)
+    kept = torch.randn(1280, 128, generator=torch.Generator().manual_seed(2)).bfloat16().cuda()
+    found = []
+    for one_launch in (True, False):
+        if not one_launch:
+            model._decode_layers = None
+        cache = CacheManager(cache_requirements(model.spec), CacheConfig(16, 81), model.dtype, "cuda", 2048, num_state_slots=1)
+        cache.create("a")
+        cache.reserve("a", 1280)
+        slots = torch.from_numpy(cache.slot_mapping(0, "a", 0, 1280)).cuda().long()
+        view = cache.layer_view(0)
+        for tensor in (view.keys, view.values):
+            tensor[slots // 16, 0, slots % 16] = kept
+        poisoned = view.keys if what == "keys" else view.values
+        poisoned[slots[keys] // 16, 0, slots[keys] % 16] = float("nan")
+        found.append(StepRunner(model, cache, 1, 1, use_graphs=False).run([StepEntry("a", [5], [0])]).isnan().cpu())
+    assert torch.equal(found[0], found[1]) and bool(found[0].all()) == (keys.stop > keys.start)
+
+
 @pytest.mark.parametrize("one_launch", [True, False])
 def test_the_head_reads_rows_that_were_rounded_once(one_launch):
     """Branches that add nothing and a head that is the identity: the logits are the normed embeddings as the product reads them,
