@@ -558,18 +558,26 @@ def _need_pairs(name: str, operands, outs, whole_scale: torch.Tensor | None = No
         raise KernelError(f"{name}: the weights are not of the operands' and results' sizes")
 
 
+# The dense gated product: k range from which it is the faster one and up to which, and multiplications and additions from which it is.
+GATED_PRODUCT_K, GATED_PRODUCT_WORK = (1024, 2048), 1.7e10
+
+
 def gated_product_wanted(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether :func:`gated_product` is faster than the library product and the activation kernel behind it: it saves writing and
-    reading the gate and up values (a k range of up to 2,048 leaves that a fifth of the product), and loses where few rows, rows that
-    do not fill their tiles of 256 or a last wave of tiles leave it idle.  Microseconds a call, 1,536 x 8,960, against the library's:
-    512 rows 28.0 / 27.3, 777 44.1 / 39.9, 1,024 46.5 / 48.7, 1,500 67.0 / 70.7, 2,048 87.5 / 94.2; 2,048 x 5,632, 2,048 rows
-    70.9 / 79.6, 1,349 54.5 / 54.9; 5,120 x 13,824, 2,048 rows 381 / 378."""
-    if not gemm_pairs_ok(x, weight) or x.shape[0] < 1024 or x.shape[1] > 2048:
+    reading the gate and up values (a k range of up to 2,048 leaves that a fifth of the product; a short one leaves the pairs waiting for
+    their tiles' epilogues), and loses where rows that do not fill their tiles of 256 or a last wave of tiles leave it idle, and in
+    small products.  Microseconds a call against the library's, operands from memory: 1,536 x 8,960, 1,024 rows 53.2 / 52.2, 1,280
+    61.4 / 66.6, 2,048 89.0 / 93.2, 8,192 315 / 370; 2,048 x 5,632, 1,280 51.2 / 48.1, 2,048 74.8 / 82.9; 2,048 x 11,008, 1,200 (tiles
+    filled to 0.908) 86.0 / 85.0, 1,500 98.3 / 109.6; of what it takes the worst found is 2,048 x 5,632, 2,000 rows (0.929), 80.9 / 78.8; 1,024 x 4,096, 2,300 45.1 / 42.0, 4,096 67.6 / 72.7; 1,024 x 2,816, 2,560
+    37.8 / 31.7; 768 x 3,072, 8,192 94.2 / 87.0; 512 x 2,048, 8,192 63.5 / 52.2; 5,120 x 13,824, 2,048 381 / 378."""
+    if not gemm_pairs_ok(x, weight) or not GATED_PRODUCT_K[0] <= x.shape[1] <= GATED_PRODUCT_K[1]:
         return False
     rows, pairs = x.shape[0], sm_count() // 2
+    if rows < 1024 or 0.5 * rows * x.shape[1] * weight.shape[0] < GATED_PRODUCT_WORK:
+        return False
     row_tiles, w_tiles = -(-rows // 256), -(-weight.shape[0] // 256)
     tiles = row_tiles * w_tiles
-    return 10 * rows * tiles >= 9 * row_tiles * 256 * pairs * -(-tiles // pairs)
+    return 100 * rows * tiles >= 91 * row_tiles * 256 * pairs * -(-tiles // pairs)
 
 
 def gated_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, activation: str = "silu", limit: float = 0.0) -> torch.Tensor:

@@ -159,20 +159,20 @@ calls = []
 product = ops.gated_product
 ops.gated_product = lambda *given: calls.append(1) or product(*given)
 rng = random.Random(1)
-prompts = [[rng.randrange(512) for _ in range(900)] for _ in range(3)]
+prompts = [[rng.randrange(512) for _ in range(1200)] for _ in range(3)]
 logits, counts = {}, []
 for graphs in (True, False):
-    cache = CacheManager(cache_requirements(spec), CacheConfig(16, 64), model.dtype, "cuda", 2048, num_state_slots=2)
-    runner = StepRunner(model, cache, 1024, 2, use_graphs=graphs)
+    cache = CacheManager(cache_requirements(spec), CacheConfig(16, 80), model.dtype, "cuda", 2048, num_state_slots=2)
+    runner = StepRunner(model, cache, 1280, 2, use_graphs=graphs)
     logits[graphs] = []
     for prompt in prompts:
         cache.create("r")
-        logits[graphs].append(runner.run([StepEntry("r", prompt, [899])]).clone())
+        logits[graphs].append(runner.run([StepEntry("r", prompt, [1199])]).clone())
         cache.free("r")
         counts.append(len(calls))
     if graphs:
         assert runner.portion_graph_replays == 2
-assert counts == [0, 2, 2, 2, 2, 2], counts        # met first while a step is captured, of 1,024 rows, and replayed
+assert counts == [0, 2, 2, 2, 2, 2], counts        # met first while a step is captured, of 1,280 rows, and replayed
 for got, want in zip(logits[True], logits[False]):
     error = float((got - want).abs().max() / want.abs().max())
     assert error <= 2.0 ** -5, error
@@ -181,7 +181,7 @@ print("as launch by launch")
 
 
 def test_a_product_that_only_the_rows_of_a_captured_step_take():
-    """A portion of 900 rows runs launch by launch at first, then captured with 1,024: only there are the rows enough for the product
+    """A portion of 1,200 rows runs launch by launch at first, then captured with 1,280: only there are the rows enough for the product
     with its gate.  In a process of its own, without a warm-up, so that this is the product's first use."""
     import subprocess
     import sys
