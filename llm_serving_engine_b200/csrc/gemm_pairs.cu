@@ -498,6 +498,8 @@ extern "C" int lse_gemm_pairs(const void* x, long long x_rows, long long ld_x, c
   if (routed < 0 || routed > MAX_GROUPS || act < -1 || act > 3 || blocks < 2) return LSE_ERR_BAD_ARGUMENT;
   if ((routed && (x_rows <= 0 || x_rows > 0x7fffffff)) || whole_rows < 0) return LSE_ERR_BAD_ARGUMENT;
   if (!routed && !whole_rows) return 0;
+  // whole 16-byte pieces (the tensor maps ask for aligned rows themselves)
+  if (ld_w % 8 || (routed && (k % 8 || ld_x % 8)) || (whole_rows && (whole_k % 8 || ld_whole % 8))) return LSE_ERR_BAD_ARGUMENT;
   const bool gated = act >= 0;
   Args args = {};
   if (!make_rows_map(&args.weights, w, w_total_rows, w_total_columns, ld_w, gated ? 64 : 128)) return LSE_ERR_BAD_ARGUMENT;

@@ -539,23 +539,13 @@ def gemm_pairs_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     return _pairs_operand_ok(x) and _pairs_operand_ok(weight)
 
 
-def _need_pairs(name: str, operands, outs, whole_scale: torch.Tensor | None = None, offsets: torch.Tensor | None = None,
-                sizes_fit: bool = True) -> None:
-    """Raises where the product on pairs of SMs would read or write something else than is meant.  ``outs``: (results, rows of
-    their operand, whether they may be float32)."""
-    if not all(_pairs_operand_ok(operand) for operand in operands):
-        raise KernelError(f"{name}: operands must be bfloat16, 16-byte aligned, rows of a multiple of 8 values")
-    for out, rows, float32_too in outs:
-        if (not out.is_cuda or out.dim() != 2 or out.shape[0] != rows or out.stride(1) != 1
-                or out.dtype != torch.bfloat16 and not (float32_too and out.dtype == torch.float32)):
-            raise KernelError(f"{name}: results must be rows of their operand, {'bfloat16 or float32' if float32_too else 'bfloat16'}, whole columns")
-    if whole_scale is not None and (whole_scale.dtype != torch.float32 or whole_scale.numel() != outs[-1][1] or not whole_scale.is_contiguous()):
-        raise KernelError(f"{name}: factors must be float32, one a row")
-    if offsets is not None and (offsets.dtype != torch.int32 or offsets.dim() != 1 or not offsets.is_contiguous()
-                                or not 0 < offsets.shape[0] <= PAIRS_MAX_GROUPS):
-        raise KernelError(f"{name}: ends of 1 to {PAIRS_MAX_GROUPS} groups must be int32")
-    if not sizes_fit:
-        raise KernelError(f"{name}: the weights are not of the operands' and results' sizes")
+_BFLOAT16, _RESULTS = torch.bfloat16, (torch.bfloat16, torch.float32)
+
+
+def _need_pairs(name: str, fits: bool) -> None:
+    if not fits:
+        raise KernelError(f"{name}: operands must be bfloat16 and results rows of their operand, columns side by side, ends of 1 to "
+                          f"{PAIRS_MAX_GROUPS} groups int32, factors float32, and the weights of the operands' and results' sizes")
 
 
 # The dense gated product: k range from which it is the faster one and up to which, and multiplications and additions from which it is.
@@ -568,8 +558,9 @@ def gated_product_wanted(x: torch.Tensor, weight: torch.Tensor) -> bool:
     their tiles' epilogues), and loses where rows that do not fill their tiles of 256 or a last wave of tiles leave it idle, and in
     small products.  Microseconds a call against the library's, operands from memory: 1,536 x 8,960, 1,024 rows 53.2 / 52.2, 1,280
     61.4 / 66.6, 2,048 89.0 / 93.2, 8,192 315 / 370; 2,048 x 5,632, 1,280 51.2 / 48.1, 2,048 74.8 / 82.9; 2,048 x 11,008, 1,200 (tiles
-    filled to 0.908) 86.0 / 85.0, 1,500 98.3 / 109.6; of what it takes the worst found is 2,048 x 5,632, 2,000 rows (0.929), 80.9 / 78.8; 1,024 x 4,096, 2,300 45.1 / 42.0, 4,096 67.6 / 72.7; 1,024 x 2,816, 2,560
-    37.8 / 31.7; 768 x 3,072, 8,192 94.2 / 87.0; 512 x 2,048, 8,192 63.5 / 52.2; 5,120 x 13,824, 2,048 381 / 378."""
+    filled to 0.908) 86.0 / 85.0, 1,500 98.3 / 109.6; 1,024 x 4,096, 2,300 45.1 / 42.0, 4,096 67.6 / 72.7; 1,024 x 2,816, 2,560
+    37.8 / 31.7; 768 x 3,072, 8,192 94.2 / 87.0; 512 x 2,048, 8,192 63.5 / 52.2; 5,120 x 13,824, 2,048 381 / 378.  The worst found of
+    what it takes is 2,048 x 5,632, 2,000 rows (tiles filled to 0.929), 80.9 / 78.8."""
     if not gemm_pairs_ok(x, weight) or not GATED_PRODUCT_K[0] <= x.shape[1] <= GATED_PRODUCT_K[1]:
         return False
     rows, pairs = x.shape[0], sm_count() // 2
@@ -585,7 +576,8 @@ def gated_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, acti
     _need_cuda(x, weight, out)
     rows, k = x.shape
     inter = out.shape[1]
-    _need_pairs("gated_product", (x, weight), ((out, rows, False),), sizes_fit=weight.shape == (2 * inter, k))
+    _need_pairs("gated_product", _pairs_operand_ok(x) and _pairs_operand_ok(weight) and out.dtype == _BFLOAT16 and out.shape[0] == rows
+                and out.stride(1) == 1 and weight.shape == (2 * inter, k))
     check(library.load().lse_gemm_pairs(None, 0, 0, None, 0, 0, 0, None, 0, 0, 0.0, x.data_ptr(), rows, x.stride(0), inter, k,
                                         out.data_ptr(), out.stride(0), 0, None, float(limit), weight.data_ptr(), 2 * inter, k,
                                         weight.stride(0), _PAIRS_ACT[activation], sm_count(), _stream()), "gated_product")
@@ -593,6 +585,12 @@ def gated_product(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, acti
 
 
 PAIRS_MAX_GROUPS = 256
+
+
+def _row_step(rows: torch.Tensor) -> int:
+    """From one row to the next one; 0 where the values of a row do not lie side by side."""
+    step, side_by_side = rows.stride()
+    return step if side_by_side == 1 else 0
 
 
 def gemm_pairs_prepare(device: torch.device) -> None:
@@ -611,16 +609,23 @@ def gated_product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tens
     """:func:`gated_product` of groups of rows of ``x`` (their ends: ``offsets``, int32), each with the next 2 * out.shape[1] rows of
     ``weight``, and of all rows of ``whole`` with the rows behind those, times ``whole_scale`` by row."""
     _need_cuda(x, offsets, out, whole, whole_out, whole_scale, weight)
-    k, routed, columns = x.shape[1], offsets.shape[0], out.shape[1]
-    both = whole is not None
-    _need_pairs("gated_product_groups", (x, weight, whole) if both else (x, weight),
-                ((out, x.shape[0], False),) + (((whole_out, whole.shape[0], False),) if both else ()), whole_scale if both else None, offsets,
-                weight.shape == (2 * (routed * columns + (whole_out.shape[1] if both else 0)), k) and (not both or whole.shape[1] == k))
+    # what the launcher does not see of the tensors (it looks at sizes, alignment and the rows' distances itself)
+    (rows, k), (out_rows, columns), (routed,) = x.shape, out.shape, offsets.shape
+    ld, ld_out = _row_step(x), _row_step(out)
+    all_rows = all_columns = ld_all = ld_all_out = 0
+    fits = (ld and ld_out and out_rows == rows and x.dtype == out.dtype == weight.dtype == _BFLOAT16 and offsets.dtype == torch.int32
+            and offsets.stride(0) == 1)
+    if whole is not None:
+        (all_rows, all_k), (all_out_rows, all_columns) = whole.shape, whole_out.shape
+        ld_all, ld_all_out = _row_step(whole), _row_step(whole_out)
+        fits = (fits and ld_all and ld_all_out and all_out_rows == all_rows and all_k == k and whole.dtype == whole_out.dtype == _BFLOAT16
+                and (whole_scale is None or whole_scale.dtype == torch.float32 and whole_scale.numel() == all_rows and whole_scale.is_contiguous()))
+    ld_weight = _row_step(weight)
+    _need_pairs("gated_product_groups", fits and ld_weight and weight.shape == (2 * (routed * columns + all_columns), k))
     check(library.load().lse_gemm_pairs(
-        x.data_ptr(), x.shape[0], x.stride(0), offsets.data_ptr(), routed, columns, k, out.data_ptr(), out.stride(0), 0, float(limit),
-        _ptr(whole), 0 if whole is None else whole.shape[0], 0 if whole is None else whole.stride(0),
-        0 if whole is None else whole_out.shape[1], k, _ptr(whole_out), 0 if whole is None else whole_out.stride(0), 0, _ptr(whole_scale),
-        float(whole_limit), weight.data_ptr(), weight.shape[0], k, weight.stride(0), _PAIRS_ACT[activation], sm_count(), _stream()),
+        x.data_ptr(), rows, ld, offsets.data_ptr(), routed, columns, k, out.data_ptr(), ld_out, 0, float(limit),
+        _ptr(whole), all_rows, ld_all, all_columns, k, _ptr(whole_out), ld_all_out, 0, _ptr(whole_scale),
+        float(whole_limit), weight.data_ptr(), weight.shape[0], k, ld_weight, _PAIRS_ACT[activation], sm_count(), _stream()),
         "gated_product_groups")
 
 
@@ -629,18 +634,22 @@ def product_groups(x: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, wh
     """out[t] = x[t] W_g^T for groups of rows of ``x`` (their ends: ``offsets``), W_g the g-th x.shape[1] columns of ``weight``
     (a multiple of 64), and whole_out = whole W^T with the columns behind those; bfloat16 or float32 results."""
     _need_cuda(x, offsets, out, whole, whole_out, weight)
-    k, routed, columns = x.shape[1], offsets.shape[0], weight.shape[0]
-    both = whole is not None
-    _need_pairs("product_groups", (x, weight, whole) if both else (x, weight),
-                ((out, x.shape[0], True),) + (((whole_out, whole.shape[0], True),) if both else ()), None, offsets,
-                k % 64 == 0 and weight.shape[1] == routed * k + (whole.shape[1] if both else 0) and out.shape[1] == columns
-                and (not both or whole_out.shape[1] == columns))
+    (rows, k), (columns, weight_columns), (routed,) = x.shape, weight.shape, offsets.shape
+    ld, ld_out, ld_weight = _row_step(x), _row_step(out), _row_step(weight)
+    all_rows = all_k = ld_all = ld_all_out = all_f32 = 0
+    fits = (ld and ld_out and ld_weight and out.shape == (rows, columns) and x.dtype == weight.dtype == _BFLOAT16 and out.dtype in _RESULTS
+            and offsets.dtype == torch.int32 and offsets.stride(0) == 1)
+    if whole is not None:
+        all_rows, all_k = whole.shape
+        ld_all, ld_all_out = _row_step(whole), _row_step(whole_out)
+        all_f32 = int(whole_out.dtype == torch.float32)
+        fits = (fits and ld_all and ld_all_out and whole_out.shape == (all_rows, columns) and whole.dtype == _BFLOAT16
+                and whole_out.dtype in _RESULTS)
+    _need_pairs("product_groups", fits and weight_columns == routed * k + all_k)
     check(library.load().lse_gemm_pairs(
-        x.data_ptr(), x.shape[0], x.stride(0), offsets.data_ptr(), routed, columns, k, out.data_ptr(), out.stride(0),
-        int(out.dtype == torch.float32), 0.0, _ptr(whole), 0 if whole is None else whole.shape[0], 0 if whole is None else whole.stride(0),
-        columns, 0 if whole is None else whole.shape[1], _ptr(whole_out), 0 if whole is None else whole_out.stride(0),
-        0 if whole is None else int(whole_out.dtype == torch.float32), None, 0.0, weight.data_ptr(), columns, weight.shape[1],
-        weight.stride(0), -1, sm_count(), _stream()), "product_groups")
+        x.data_ptr(), rows, ld, offsets.data_ptr(), routed, columns, k, out.data_ptr(), ld_out, int(out.dtype == torch.float32), 0.0,
+        _ptr(whole), all_rows, ld_all, columns, all_k, _ptr(whole_out), ld_all_out, all_f32, None, 0.0, weight.data_ptr(), columns,
+        weight_columns, ld_weight, -1, sm_count(), _stream()), "product_groups")
 
 
 def gemm_pairs_test_hook(withhold: bool = False) -> None:

@@ -115,6 +115,7 @@ class ClampedMoE(FeedForward):
         # the engine's own products over groups of rows: gated experts whose columns are whole pieces of 64
         self._in_pairs = (self._grouped_gate_up is not None and self.activation in ("clamped_swish", "silu") and self.ff % 64 == 0
                           and self.shared_ff % 8 == 0 and self.experts <= ops.PAIRS_MAX_GROUPS)
+        self._narrow, self._rows_in_pairs = width <= 2048, 200 * self.outputs     # see _pairs_wanted
         if self._in_pairs and self.gate_up_weight.is_cuda:
             ops.gemm_pairs_prepare(self.gate_up_weight.device)     # its first use may be one while a step is captured
 
@@ -184,7 +185,7 @@ class ClampedMoE(FeedForward):
         512 859 / 862; 256 of 512, 1,024 wide: 4 215 / 238, 128 335 / 371.  Wider: 64 of 4,096 x 1,024, 97 rows 362 / 426, 188 419 / 440,
         512 957 / 944, 1,024 1,777 / 1,698; 8 of 4,096 x 14,336, 194 601 / 635, 512 1,396 / 1,408, 1,024 2,784 / 2,692; 64 of 7,168 x 2,048,
         73 1,029 / 1,315, 192 1,281 / 1,305, 216 1,675 / 1,539, 768 4,853 / 4,487."""
-        return self.router.shape[1] <= 2048 or tokens * self.top <= 200 * self.outputs
+        return self._narrow or tokens * self.top <= self._rows_in_pairs
 
     def _grouped_in_pairs(self, x, chosen, expert_weights, identity_weight, shared_gate):
         """The experts and the shared expert together in two products of the engine's own, the activation inside the first."""
