@@ -26,8 +26,8 @@
 //     their order.
 // Sums do not depend on timing: every order is fixed.
 //
-// Measured against nine launches a layer, one B200: 28 layers of the 1.5B sizes and the head, one request of 100 keys, 879 us a
-// step against 1,158 (a layer 26 us, of which 14 are the weights' time at the memory's rate: QKV 2.5 us, attention 4, O 3,
+// Measured against nine launches a layer, one B200: 28 layers of the 1.5B sizes and the head, one request of 100 keys, 870 to 880
+// us a step against 1,174 (a layer 26 us, of which 14 are the weights' time at the memory's rate: QKV 2.5 us, attention 4, O 3,
 // gate/up 8, down 6, each 1.2 to 2 of it waiting for the others); more sizes beside the rule in models/decode_layers.py.
 //
 // Every wait is bounded: a block whose wait gives up sets the kernel's error word and the launch's abort word, the others see

@@ -7,7 +7,7 @@
 // A pair of blocks owns 256 rows of w (the M side of the instruction: 128 lanes of tensor memory in each block) and up to 256
 // rows of x (the N side; a group's last tile in steps of 32).  Each block brings its own half of both operands with TMA
 // (128-byte swizzle, six stages of 64 k), one thread of the even block issues the instructions for both, the sums lie in two
-// buffers of tensor memory, and four warps finish one tile while the next one's products run.  Gated, a block's 128 rows of w
+// buffers of tensor memory, and eight warps finish one tile while the next one's products run.  Gated, a block's 128 rows of w
 // are 64 rows of the gate and the 64 rows of the up projection beside them: the warps that read the up half hand it to those
 // that read the gate half through shared memory, the products' sums never leave the SM, and no kernel has to read them
 // (2,048 rows x 17,920 columns: 73 MB written and read again, 18 us of 95), and

@@ -28,10 +28,13 @@ ENABLED = os.environ.get("LSE_DECODE_LAYERS", "1") != "0"
 
 # Steps of at most so many values of the residual (rows x hidden size), and of at most the kernel's four rows, go through the
 # one launch.  It saves a layer's nine hand-overs (1.3 to 1.9 us each), and costs the exchange of every phase's rows between all
-# blocks, which grows with them.  One launch against launch by launch, microseconds a step: 28 layers of the 1.5B sizes (hidden
-# 1,536), one request of 100 keys 879 / 1,158, two of 2,048 keys 1,056 / 1,238, four of 500 1,109 / 1,215, of 4,000 1,192 / 1,357
-# (eight of 2,048 keys 1,338 / 1,310); four layers of the 7B sizes (3,584) and the head, one 511 / 597, two 543 / 594 (three
-# 600 / 603); four of the 14B sizes (5,120), two 670 / 729 (four 823 / 754).
+# blocks, which grows with them.  One launch against launch by launch, microseconds a step with its upload: 28 layers of the 1.5B
+# sizes (hidden 1,536), one request of 100 keys 920 / 1,232, of 30,000 1,316 / 1,615, two of 2,048 1,064 / 1,313, four of 500
+# 1,138 / 1,257, of 4,000 1,216 / 1,371, of 30,000 1,673 / 1,888 (eight of 2,048 keys 1,338 / 1,310); four layers of the 7B sizes
+# (3,584) and the head, one 519 / 617, two 556 / 620 (three 600 / 603); four of the 14B sizes (5,120), two 693 / 756 (four 823 /
+# 754).  The contexts do not change the answer: four layers of the 1.5B sizes, one request of 8,000 keys 250 / 316, of 100,000
+# 397 / 422, two of 100,000 423 / 437, four of 8,000 302 / 335; of the 7B sizes, two of 100,000 811 / 886; of the 14B sizes, two of
+# 8,000 751 / 801, of 100,000 1,159 / 1,279.
 MOST_VALUES = 10240
 
 
